@@ -109,6 +109,19 @@ int spsim_b200_qset_copy_q(const spsim_b200_qset *qs, float *hkl_host);
 int spsim_b200_qset_destroy(spsim_b200_qset *qs);
 
 /* ---- structure factor ---------------------------------------------------
+ * q sets made from a detector are oversampled: no atom's phase turns more than
+ * |dq/dx| |r - c|max cycles per pixel.  The FP32 forwards (one pattern, a
+ * batch, a spectrum) therefore evaluate the sum on a tensor grid of nodes, a
+ * little more than two per cycle along each axis, and interpolate it to the
+ * pixels in FP64, to 1e-8 of an outermost atom's amplitude and far less for
+ * the others; form factors and per-atom B factors belong to the interpolated
+ * sum, the global B factor and the centre phase are applied per pixel.  This
+ * is done where it is faster (patterns of more than about 1e7 terms), for
+ * whole batches or not at all; q lists, FP64, forced variants
+ * (spsim_b200_set_variant), detectors further than 1.2 detector distances off
+ * the beam axis and per-atom B factors beyond twice their largest at creation
+ * + 100 A^2 (checked on the device when they are rewritten there) take the
+ * sum on every pixel.
  * One pattern: F (complex64, interleaved re/im, npix) and I = |F|^2 (float)
  * into DEVICE buffers on `stream` (a cudaStream_t, NULL = legacy default).
  * rot: optional 3x3 row-major FP64 rotation applied to every q (q' = R q,
@@ -363,6 +376,11 @@ int spsim_b200_timing_read(double *ms, int cap, int *n);
  * reference's "atoms.pixel/s" self-report (src/diffraction.c:849-851). */
 int spsim_b200_last_forward_stats(double *terms, double *kernel_ms);
 
+/* Atom-point terms the last forward's structure-factor kernel evaluated: the
+ * terms of spsim_b200_last_forward_stats where it ran on every pixel, fewer
+ * where it ran on coarse grids (below). */
+int spsim_b200_last_terms_evaluated(double *terms);
+
 /* The reference-shaped calls (include/spsim.h) and
  * spsim_b200_structure_factor_host keep device scratch between calls on the
  * calling thread (grow-only buffers, the last molecule while its atom arrays
@@ -400,6 +418,9 @@ void spsim_b200_set_formula_seed(unsigned long long seed);
  * Forms 2, 3 and 4 read the reduced phase from a fixed-point phase word (three
  * FP64 FMAs) while |q|max |r - centre|max < 2^17 cycles, and reduce by FP64
  * rounding (six FP64 operations, up to 2^48 cycles) beyond.
+ * On coarse grids form 4's kernel for nodes runs, whose points each take their
+ * own FP64 phase; it has one shape, and the variant reported (the default's or
+ * the tuned threads and pixels per thread) is that of its size class on pixels.
  * threads < 0 restores automatic choice; autotune times every compiled
  * variant on the given workload and keeps the fastest for workloads of that
  * size class. */

@@ -21,7 +21,7 @@ from ._native import PRECISIONS, ChainOutputs, ChainParams, check, lib
 __all__ = [
     "Molecule", "QSet", "forward", "forward_batch", "adjoint", "detector_chain", "chain_params",
     "hkl_for_detector", "synchronize", "forward_spectrum", "timing", "autotune", "set_variant", "last_forward_stats",
-    "last_variant", "last_phase_word", "last_pair_narrow", "kernel_name", "autotune_batch", "clear_tuning",
+    "last_terms_evaluated", "last_variant", "last_phase_word", "last_pair_narrow", "kernel_name", "autotune_batch", "clear_tuning",
     "forward_nufft", "forward_nufft_batch", "last_nufft_grid",
 ]
 
@@ -386,6 +386,14 @@ def last_forward_stats():
     ms = c_double(0)
     check(lib().spsim_b200_last_forward_stats(byref(t), byref(ms)))
     return t.value, ms.value
+
+
+def last_terms_evaluated():
+    """Atom-point terms the last forward's kernel evaluated: fewer than
+    last_forward_stats' where it ran on coarse grids of nodes."""
+    t = c_double(0)
+    check(lib().spsim_b200_last_terms_evaluated(byref(t)))
+    return t.value
 
 
 FORMS = {0: "compensated FP32, one pixel per lane", 1: "compensated FP32, pixel pairs (f32x2)",

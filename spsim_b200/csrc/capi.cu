@@ -11,6 +11,7 @@
 #include <mutex>
 #include <thread>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/spsim_b200.h"
@@ -19,7 +20,7 @@
 #include "adjoint_kernels.cuh"
 #include "sf_kernels.cuh"
 #include "nufft_kernels.cuh"
-
+#include "coarse_kernels.cuh"
 
 using namespace spsim;
 
@@ -220,6 +221,8 @@ struct spsim_b200_molecule {
   int er = 0, kr = 11;
   float dr = 1, inv_dr = 1;
   int per_atom_b = 0, delta_atoms = 0;
+  float b_limit = 0;        // largest |per-atom B| the coarse grids are sized for
+  bool b_updated = false;   // B factors rewritten on the device: b_limit is checked there (d_flags[1])
   // device views of the buffers below
   float4 *d_atoms = nullptr;
   float4 *d_atoms2 = nullptr;  // pixel-pair layout of the same records
@@ -228,7 +231,7 @@ struct spsim_b200_molecule {
   int *d_perm = nullptr;
   float *d_wbase = nullptr;
   float *d_coeffs = nullptr;
-  int *d_flags = nullptr;  // [0] range error
+  int *d_flags = nullptr;  // [0] range error, [1] a rewritten B factor beyond b_limit
   // owned device memory; a new molecule may take over a dropped one's buffers
   DevBuf b_atoms, b_atoms2, b_atomsd, b_tiles, b_perm, b_wbase, b_coeffs, b_flags, b_inputs;
   void take_buffers(spsim_b200_molecule &o) {
@@ -308,6 +311,15 @@ static int molecule_create_impl(int natoms, const int32_t *Z, const PosT *pos, c
   m->er = ceil_log2_bound(m->rbound);
   m->dr = (float)std::ldexp(1.0, m->er - m->kr);
   m->inv_dr = (float)std::ldexp(1.0, m->kr - m->er);
+
+  // B factors may double (and rise by 100 A^2) in a refinement before its
+  // patterns leave the coarse grids
+  if (bfac) {
+    float bmax = 0.0f;
+    for (int j = 0; j < natoms; ++j)
+      if (Z[j]) bmax = std::max(bmax, std::isfinite(bfac[j]) ? std::fabs(bfac[j]) : 1e30f);
+    m->b_limit = 2.0f * bmax + 100.0f;
+  }
 
   // element segments (ascending Z), padded to ATOM_GROUP
   std::vector<int> seg_begin;
@@ -439,10 +451,13 @@ extern "C" int spsim_b200_molecule_update_device(spsim_b200_molecule *m, const v
   if (!m || !pos_dev) return fail(SPSIM_ERR_INVALID_ARG, "molecule or positions NULL");
   if (bfac_dev && !m->per_atom_b)
     return fail(SPSIM_ERR_INVALID_ARG, "molecule was created without per-atom B factors");
-  CUDA_TRY(cudaMemsetAsync(m->d_flags, 0, sizeof(int), (cudaStream_t)stream));  // the range word of this update
+  // the range word of this update, and the B factors' where they are rewritten
+  CUDA_TRY(cudaMemsetAsync(m->d_flags, 0, (bfac_dev ? 2 : 1) * sizeof(int), (cudaStream_t)stream));
+  if (bfac_dev) m->b_updated = true;
   CUDA_TRY(launch_atoms_update(m->d_atoms, m->d_atoms2, m->d_atomsd, m->d_perm, m->n_padded, pos_is_f64 ? nullptr : (const float *)pos_dev,
                                pos_is_f64 ? (const double *)pos_dev : nullptr, occ_dev, bfac_dev, m->d_wbase,
-                               m->center, m->dr, m->inv_dr, m->rbound, m->d_flags, (cudaStream_t)stream));
+                               m->center, m->dr, m->inv_dr, m->rbound, m->b_limit, m->d_flags,
+                               (cudaStream_t)stream));
   return SPSIM_OK;
 }
 
@@ -471,6 +486,8 @@ struct spsim_b200_qset {
   double pair_step = 0;  // largest |q[2m+1] - q[2m]| (the pixel-pair form's admission test)
   double quad_step1 = 0, quad_step2 = 0;  // largest one- and two-pixel steps from a quad's anchor (the quad form's)
   int row = 0;           // pixels per detector row (q sets made from a detector), 0 for a list
+  bool has_geom = false;  // q sets made from a detector: its geometry
+  DetGeom geom;
   ~spsim_b200_qset() {
     cudaFree(d_hkl);
     cudaFree(d_q64);
@@ -571,6 +588,23 @@ extern "C" int spsim_b200_qset_from_detector(int nx, int ny, float width, float 
   q->device = dev;
   q->npix = (long long)nx * ny;
   q->row = nx;
+  {
+    DetGeom &g = q->geom;
+    g.nx = nx;
+    g.ny = ny;
+    g.spherical = spherical ? 1 : 0;
+    g.width = width;
+    g.height = height;
+    g.distance = distance;
+    g.cx = center_x;
+    g.cy = center_y;
+    g.ewald = 1.0 / (double)wavelength;
+    g.px_size = (double)(width / nx);
+    g.py_size = (double)(height / ny);
+    g.fpx = 2 * std::sin(std::atan(g.px_size / distance) / 2) / wavelength;
+    g.fpy = 2 * std::sin(std::atan(g.py_size / distance) / 2) / wavelength;
+    q->has_geom = true;
+  }
   CUDA_TRY(cudaMalloc(&q->d_q64, 3 * q->npix * sizeof(double)));
   CUDA_TRY(launch_ewald(nx, ny, width, height, distance, center_x, center_y, wavelength, spherical, nullptr,
                         q->d_q64, 0));
@@ -637,8 +671,9 @@ struct Plan {
   DevBuf pats, items, acc, ff, flags;
   int n_items = 0, grid = 0, npat = 0;
   long long max_npix = 0;
-  double terms = 0;
+  double terms = 0, evaluated = 0;  // atom.pixel terms of the patterns, and those evaluated (on nodes: fewer)
   int precision = 0, nt = 128, ppt = 4, packed = 1;
+  int mode = PREC_MODE_POLY;
   bool perb = false;
   bool fixw = false;  // FP64-phase forms: fixed-point phase word (every pattern within 2^17 cycles)
   bool narrow = false;  // neighbour pairs: every step within 0.07 cycle (the NARROW second-pixel polynomial)
@@ -647,6 +682,16 @@ struct Plan {
   int spectrum = 0;                  // > 0: combine this many patterns into spec_F / spec_I
   DevBuf spec_w;
   float *spec_F = nullptr, *spec_I = nullptr;
+  // coarse grids: the descriptors hold npat node patterns, then the npat pixel
+  // patterns that the interpolation writes
+  bool coarse = false;
+  DevBuf tables, cpats, pix_acc, strip;
+  long long strip_size = 0;
+  int max_nx = 0, max_ny = 0, max_nyn = 0;
+  // the same patterns on every pixel, run where a B factor rewritten on the
+  // device is beyond what the coarse grids are sized for
+  std::unique_ptr<Plan> direct;
+  DevBuf gate;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   ~Plan() {
@@ -670,7 +715,7 @@ struct Variant {
 static std::map<long long, Variant> g_tuned;  // size class -> kernel variant
 static bool g_timing = false;
 static std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_timing_events;
-static thread_local double g_last_terms = 0, g_last_ms = 0;
+static thread_local double g_last_terms = 0, g_last_evaluated = 0, g_last_ms = 0;
 static thread_local int g_last_variant[3] = {0, 0, -1};  // threads, pixels per thread, form (-1: FP64 kernel)
 static thread_local int g_last_phase_word = 0;            // forms 2/3: fixed-point phase word used
 static thread_local int g_last_pair_narrow = 0;           // form 3: NARROW second-pixel polynomial used
@@ -726,14 +771,107 @@ static bool is_orthonormal(const double *R) {
 
 static thread_local long long g_split_pixels_hint = 0;  // pixels of the whole shot while a shot part is planned
 
+static double frobenius(const double *R) {
+  double s = 0;
+  for (int k = 0; k < 9; ++k) s += R[k] * R[k];
+  return std::sqrt(s);
+}
+
+// Node grid of one pattern (coarse_kernels.cuh): scale is the largest factor
+// by which the phases' q exceed the detector's own, bscale the same of the
+// per-atom B factors' |q|.  False where a grid is not admitted: a q list, a
+// molecule without atoms, a detector of fewer than 16 pixels a side or further
+// than 1.2 detector distances off the beam axis (where q no longer moves
+// evenly with the angle), form factors that fall by more than e^-60 across it,
+// or more nodes than 80 % of the pixels.
+struct CoarseGrid {
+  CoarseAxis x, y;
+};
+
+static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale,
+                       CoarseGrid *grid) {
+  const DetGeom &g = q->geom;
+  if (!q->has_geom || m->n_kept == 0 || g.nx < 16 || g.ny < 16) return false;
+  double bmax = m->per_atom_b ? (double)m->b_limit * bscale * bscale : 0.0;
+  if (!m->delta_atoms) {
+    double c = 0;
+    for (int e = 0; e < m->n_elem; ++e)
+      for (int k = 4; k < 8; ++k) c = std::max(c, (double)std::fabs(m->coeffs[9 * e + k]));
+    bmax += c;
+  }
+  grid->x = coarse_axis(g.nx, g.width, g.cx, g.distance, g.spherical != 0);
+  grid->y = coarse_axis(g.ny, g.height, g.cy, g.distance, g.spherical != 0);
+  for (int d = 0; d < 2; ++d) {
+    CoarseAxis &ax = d ? grid->y : grid->x;
+    // q over half the axis: an arc of the Ewald sphere, or a line
+    double arc = ax.half * g.ewald, reach = std::tan(ax.half) * g.ewald;
+    const double t = ax.angular ? std::tan(std::fabs(ax.mid) + ax.half) : 0.0;
+    if (!ax.angular) {
+      arc = d ? g.fpy * (0.5 * (g.ny - 1) / g.ny * g.height) / g.py_size
+              : g.fpx * (0.5 * (g.nx - 1) / g.nx * g.width) / g.px_size;
+      reach = arc;
+    }
+    const double c = 2.0 * M_PI * m->rbound * scale * arc * (t > 1.0 ? 1.02 : 1.0);
+    const double a = bmax * 0.25e-20 * reach * reach;
+    if (!(c <= 1.5 * COARSE_MAX_NODES) || !(t <= 1.2) || !(a <= 60.0)) return false;
+    const int n = coarse_node_count(c, t, a);
+    if (n > COARSE_MAX_NODES) return false;
+    coarse_set_nodes(ax, n);
+  }
+  return (double)grid->x.n * grid->y.n < 0.8 * (double)g.nx * g.ny;
+}
+
+// Whether the plan's patterns run on coarse grids, with their node counts.
+// All of them or none: a batch is one launch of one kernel.  The times weighed
+// are the measured rates on B200 (direct sum on neighbour quads 1.75e12 terms/s;
+// on nodes, each with its own FP64 phase, 1.3e12; the interpolation 1e13 FP64
+// multiply-adds/s) and the interpolation's launches and tail, ~4 us: patterns of
+// less than about 1e7 terms stay on the direct sum.
+static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
+                        const double *rot, int precision, const Spectrum *spec, std::vector<CoarseGrid> &nodes) {
+  if (precision == SPSIM_PREC_FP64 || g_force_nt > 0) return false;
+  double qscale = 1.0;
+  if (spec)
+    for (int i = 0; i < npat; ++i) qscale = std::max(qscale, std::fabs(spec->qscale[i]));
+  nodes.resize(npat);
+  double direct = 0, grid = 4e-6;
+  for (int i = 0; i < npat; ++i) {
+    double stretch = 1.0;  // of |q| under this pattern's matrix
+    if (rot && !is_orthonormal(rot + 9 * (size_t)i)) stretch = std::max(1.0, frobenius(rot + 9 * (size_t)i));
+    if (i > 0 && stretch == 1.0 && mols[i] == mols[i - 1] && qsets[i] == qsets[i - 1] &&
+        !(rot && !is_orthonormal(rot + 9 * (size_t)(i - 1)))) {
+      nodes[i] = nodes[i - 1];
+    } else if (!coarse_fit(mols[i], qsets[i], qscale * stretch, stretch, &nodes[i])) {
+      return false;
+    }
+    const double npix = (double)qsets[i]->npix, kept = mols[i]->n_kept;
+    const double nxn = nodes[i].x.n, nyn = nodes[i].y.n;
+    direct += kept * npix / 1.75e12;
+    grid += kept * nxn * nyn / 1.3e12 + 2.0 * (npix + qsets[i]->geom.nx * nxn) * nyn / 1e13;
+  }
+  return grid < 0.8 * direct;
+}
+
 static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
-                      cudaStream_t stream, const Spectrum *spec) {
+                      cudaStream_t stream, const Spectrum *spec, bool allow_coarse = true) {
   pl.npat = npat;
   pl.precision = precision;
+  std::vector<CoarseGrid> nodes;
+  for (int i = 0; i < npat; ++i)
+    if (!mols[i] || !qsets[i]) return fail(SPSIM_ERR_INVALID_ARG, "pattern %d: NULL molecule or q set", i);
+  pl.coarse = allow_coarse && coarse_plan(npat, mols, qsets, rot, precision, spec, nodes);
+  pl.mode = precision == SPSIM_PREC_F32_FAST && !pl.coarse ? PREC_MODE_MUFU : PREC_MODE_POLY;
+  // points each pattern's sum is evaluated on: its nodes or its pixels
+  std::vector<long long> points(npat);
+  for (int i = 0; i < npat; ++i) points[i] = pl.coarse ? (long long)nodes[i].x.n * nodes[i].y.n : qsets[i]->npix;
   std::vector<SfPattern> pats(npat);
-  // unique (molecule, q set) pairs share one form-factor table
-  std::map<std::pair<const void *, const void *>, size_t> ff_off;
+  // unique (molecule, q set, node grid) combinations share one form-factor table
+  typedef std::tuple<const void *, const void *, int, int> FfKey;
+  auto ff_key = [&](int i) {
+    return FfKey(mols[i], qsets[i], pl.coarse ? nodes[i].x.n : 0, pl.coarse ? nodes[i].y.n : 0);
+  };
+  std::map<FfKey, size_t> ff_off;
   size_t ff_total = 0, acc_total = 0;
   std::vector<size_t> acc_off(npat), ffo(npat);
   double terms = 0;
@@ -742,33 +880,67 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   for (int i = 0; i < npat; ++i) {
     const spsim_b200_molecule *m = mols[i];
     const spsim_b200_qset *q = qsets[i];
-    if (!m || !q) return fail(SPSIM_ERR_INVALID_ARG, "pattern %d: NULL molecule or q set", i);
-    auto key = std::make_pair((const void *)m, (const void *)q);
+    const auto key = ff_key(i);
     auto f = ff_off.find(key);
     if (f == ff_off.end()) {
       ff_off[key] = ff_total;
       ffo[i] = ff_total;
-      ff_total += (size_t)m->n_elem * q->npix;
+      ff_total += (size_t)m->n_elem * points[i];
     } else {
       ffo[i] = f->second;
     }
     acc_off[i] = acc_total;
-    acc_total += q->npix;
+    acc_total += points[i];
     terms += (double)q->npix * m->n_kept;
     total_npix += q->npix;
     perb = perb || m->per_atom_b;
   }
   pl.terms = terms;
+  pl.evaluated = 0;
+  for (int i = 0; i < npat; ++i) pl.evaluated += (double)points[i] * mols[i]->n_kept;
   pl.perb = perb;
   CUDA_TRY(pl.acc.ensure(std::max<size_t>(acc_total, 1) * sizeof(double2)));
   CUDA_TRY(pl.ff.ensure(std::max<size_t>(ff_total, 1) * sizeof(double)));
   CUDA_TRY(pl.flags.ensure(64));
   CUDA_TRY(cudaMemsetAsync(pl.flags.p, 0, 64, stream));  // queue head and the sticky error word
-  CUDA_TRY(pl.pats.ensure(std::max(npat, 1) * sizeof(SfPattern)));
+  CUDA_TRY(pl.pats.ensure((pl.coarse ? 2 : 1) * std::max(npat, 1) * sizeof(SfPattern)));
+
+  // node grids: one set of node q vectors and interpolation matrices per (q set, node counts)
+  typedef std::tuple<const void *, int, int> TabKey;
+  std::map<TabKey, size_t> tab_off;
+  size_t tab_total = 0;
+  auto tab_sizes = [&](int i, size_t n[3]) {
+    const DetGeom &g = qsets[i]->geom;
+    n[0] = ((size_t)3 * points[i] + 1) / 2 * 2;
+    n[1] = (size_t)g.nx * coarse_ld(nodes[i].x.n);
+    n[2] = (size_t)g.ny * coarse_ld(nodes[i].y.n);
+  };
+  size_t pix_total = 0;
+  std::vector<size_t> pix_off(npat);
+  if (pl.coarse) {
+    for (int i = 0; i < npat; ++i) {
+      const TabKey key(qsets[i], nodes[i].x.n, nodes[i].y.n);
+      if (!tab_off.count(key)) {
+        size_t n[3];
+        tab_sizes(i, n);
+        tab_off[key] = tab_total;
+        tab_total += n[0] + n[1] + n[2];
+      }
+      pix_off[i] = pix_total;
+      pix_total += qsets[i]->npix;
+    }
+    CUDA_TRY(pl.tables.ensure(tab_total * sizeof(double)));
+    CUDA_TRY(pl.cpats.ensure(npat * sizeof(CoarsePattern)));
+    if (spec) CUDA_TRY(pl.pix_acc.ensure(std::max<size_t>(pix_total, 1) * sizeof(double2)));
+  }
 
   Variant var = {128, 4, 1};
   if (precision != SPSIM_PREC_FP64) var = choose_variant(terms, total_npix, precision);
-  if (var.packed == 4) {
+  if (pl.coarse) {
+    // the quad form's kernel for nodes, reported with the size class's threads and pixels per thread
+    if (var.packed != 4) var = {var.nt, var.p, 4};
+    pl.narrow = false;
+  } else if (var.packed == 4) {
     // neighbour-quad form: every pattern needs its one-pixel steps within 1/8
     // cycle and its two-pixel steps within 0.16 cycle of the molecule's bound
     bool ok = precision != SPSIM_PREC_FP64;
@@ -813,7 +985,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   pl.nt = var.nt;
   pl.ppt = var.p;
   pl.packed = var.packed;
-  const long long tile_pix = (long long)nt * ppt;
+  const long long tile_pix = pl.coarse ? SF_NODES_TILE : (long long)nt * ppt;
 
   pl.max_npix = 0;
   pl.npix_of.resize(npat);
@@ -830,9 +1002,9 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     pt.n_elem = m->n_elem;
     pt.per_atom_b = m->per_atom_b;
     pt.ff = (double *)pl.ff.p + ffo[i];
-    pt.npix = q->npix;
-    pt.hkl = q->d_hkl;
-    pt.q64 = q->d_q64;
+    pt.npix = points[i];
+    pt.hkl = pl.coarse ? nullptr : q->d_hkl;
+    pt.q64 = pl.coarse ? (double *)pl.tables.p + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)] : q->d_q64;
     double qmax = q->qmax;
     if (rot) {
       const double *R = rot + 9 * (size_t)i;
@@ -860,8 +1032,8 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     pt.acc = (double2 *)pl.acc.p + acc_off[i];
     pt.F = F_dev ? (float2 *)F_dev[i] : nullptr;
     pt.I = I_dev ? I_dev[i] : nullptr;
-    pl.max_npix = std::max(pl.max_npix, q->npix);
-    pl.npix_of[i] = q->npix;
+    pl.max_npix = std::max(pl.max_npix, points[i]);
+    pl.npix_of[i] = points[i];
     if (precision != SPSIM_PREC_FP64 && pl.packed >= 2 && m->n_kept > 0 && q->npix > 0) {
       // FP64 phase: the half-cycle rounding needs |2 q.r| < 2^51
       const double qr = qmax * m->rbound;
@@ -892,7 +1064,57 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     }
     if (mols[i]->n_kept > 0 && qsets[i]->npix > 0 && qmax * mols[i]->rbound >= std::ldexp(1.0, 17)) pl.fixw = false;
   }
-  CUDA_TRY(cudaMemcpyAsync(pl.pats.p, pats.data(), npat * sizeof(SfPattern), cudaMemcpyHostToDevice, stream));
+  if (pl.coarse) {
+    std::vector<CoarsePattern> cp(npat);
+    pl.max_nx = pl.max_ny = pl.max_nyn = 0;
+    for (int i = 0; i < npat; ++i) {
+      const spsim_b200_qset *q = qsets[i];
+      size_t n[3];
+      tab_sizes(i, n);
+      const double *tab = pats[i].q64;
+      CoarsePattern &c = cp[i];
+      c.nodes = pats[i].acc;
+      c.mx = tab + n[0];
+      c.my = tab + n[0] + n[1];
+      c.nx = q->geom.nx;
+      c.ny = q->geom.ny;
+      c.nxn = nodes[i].x.n;
+      c.nyn = nodes[i].y.n;
+      c.ldx = coarse_ld(c.nxn);
+      c.ldy = coarse_ld(c.nyn);
+      c.B = B;
+      c.out = spec ? (double2 *)pl.pix_acc.p + pix_off[i] : nullptr;
+      pl.max_nx = std::max(pl.max_nx, c.nx);
+      pl.max_ny = std::max(pl.max_ny, c.ny);
+      pl.max_nyn = std::max(pl.max_nyn, c.nyn);
+    }
+    // the interpolation's strips: a group of patterns at a time, 64 MB of them
+    // (they are read back from L2), or one
+    const long long strip = (long long)pl.max_nyn * pl.max_nx;
+    pl.strip_size = strip * std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / strip));
+    CUDA_TRY(pl.strip.ensure(pl.strip_size * sizeof(double2)));
+    for (const auto &t : tab_off) {
+      size_t n[3];
+      int i = 0;  // a pattern with this table
+      while (TabKey(qsets[i], nodes[i].x.n, nodes[i].y.n) != t.first) ++i;
+      tab_sizes(i, n);
+      double *tab = (double *)pl.tables.p + t.second;
+      CUDA_TRY(launch_coarse_tables(qsets[i]->geom, nodes[i].x, nodes[i].y, tab, tab + n[0], tab + n[0] + n[1],
+                                    stream));
+    }
+    CUDA_TRY(cudaMemcpyAsync(pl.cpats.p, cp.data(), npat * sizeof(CoarsePattern), cudaMemcpyHostToDevice, stream));
+    // the pixel patterns behind the node patterns
+    pats.resize(2 * (size_t)npat);
+    for (int i = 0; i < npat; ++i) {
+      SfPattern &pt = pats[npat + i];
+      pt = pats[i];
+      pt.npix = qsets[i]->npix;
+      pt.q64 = qsets[i]->d_q64;
+      pt.ff = nullptr;
+      pt.acc = cp[i].out;
+    }
+  }
+  CUDA_TRY(cudaMemcpyAsync(pl.pats.p, pats.data(), pats.size() * sizeof(SfPattern), cudaMemcpyHostToDevice, stream));
   pl.host_pats = pats;
   pl.spectrum = spec ? spec->samples : 0;
   pl.spec_F = spec ? spec->F : nullptr;
@@ -904,12 +1126,11 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 
   if (precision != SPSIM_PREC_FP64) {
     // work items: pixel tile x atom-tile range, cost-sorted (largest first)
-    const int occ =
-        std::max(1, sf_f32_occupancy(precision == SPSIM_PREC_F32_FAST ? 1 : 0, nt, ppt, pl.packed, perb, pl.fixw,
-                                     pl.narrow));
+    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(perb, pl.fixw)
+                                          : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
     const long long slots = (long long)num_sms() * occ;
     long long total_ptiles = 0;
-    for (int i = 0; i < npat; ++i) total_ptiles += (qsets[i]->npix + tile_pix - 1) / tile_pix;
+    for (int i = 0; i < npat; ++i) total_ptiles += (points[i] + tile_pix - 1) / tile_pix;
     // a row chunk of a pipelined shot splits its atoms as the whole shot
     // would: the next chunk, on the other stream, fills this one's tail
     if (g_split_pixels_hint > 0) total_ptiles = std::max(total_ptiles, (g_split_pixels_hint + tile_pix - 1) / tile_pix);
@@ -918,14 +1139,14 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     std::vector<WorkItem> items;
     std::vector<double> cost;
     for (int i = 0; i < npat; ++i) {
-      const long long nptile = (qsets[i]->npix + tile_pix - 1) / tile_pix;
+      const long long nptile = (points[i] + tile_pix - 1) / tile_pix;
       const int ntile = (int)mols[i]->tiles.size();
-      if (ntile == 0 || qsets[i]->npix == 0) continue;
+      if (ntile == 0 || points[i] == 0) continue;
       int split = 1;
       if (total_ptiles < want) split = (int)std::min<long long>((want + total_ptiles - 1) / total_ptiles, ntile);
-      split = std::max(1, std::min(split, std::max(1, ntile / 2)));
+      split = std::max(1, std::min(split, std::max(1, pl.coarse ? ntile : ntile / 2)));
       for (long long t = 0; t < nptile; ++t) {
-        const long long pix_here = std::min(tile_pix, qsets[i]->npix - t * tile_pix);
+        const long long pix_here = std::min(tile_pix, points[i] - t * tile_pix);
         for (int s = 0; s < split; ++s) {
           WorkItem w;
           w.pattern = i;
@@ -952,15 +1173,25 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       CUDA_TRY(cudaMemcpyAsync(pl.items.p, sorted.data(), sorted.size() * sizeof(WorkItem), cudaMemcpyHostToDevice,
                                stream));
   }
-  // form-factor tables (per unique molecule / q set pair; fixed for the plan's life)
-  std::map<std::pair<const void *, const void *>, bool> done;
+  // form-factor tables (per unique molecule / q set pair; fixed for the plan's
+  // life); the interpolation applies the global B factor itself
+  std::map<FfKey, bool> done;
   for (int i = 0; i < npat; ++i) {
-    auto key = std::make_pair((const void *)mols[i], (const void *)qsets[i]);
+    const auto key = ff_key(i);
     if (done[key]) continue;
     done[key] = true;
-    const spsim_b200_qset *q = qsets[i];
-    CUDA_TRY(launch_ff_table(q->d_hkl, q->d_q64, q->npix, mols[i]->n_elem, mols[i]->d_coeffs, (double)B,
-                             mols[i]->delta_atoms, (double *)pl.ff.p + ffo[i], stream));
+    CUDA_TRY(launch_ff_table(pats[i].hkl, pats[i].q64, points[i], mols[i]->n_elem, mols[i]->d_coeffs,
+                             pl.coarse ? 0.0 : (double)B, mols[i]->delta_atoms, (double *)pl.ff.p + ffo[i], stream));
+  }
+  // B factors rewritten on the device are known there only: the plan on every
+  // pixel stands by for values beyond the molecule's limit
+  pl.direct.reset();
+  bool updated = false;
+  for (int i = 0; i < npat && pl.coarse; ++i) updated = updated || (mols[i]->per_atom_b && mols[i]->b_updated);
+  if (updated) {
+    pl.direct.reset(new Plan());
+    CUDA_TRY(pl.gate.ensure(sizeof(int)));
+    return build_plan(*pl.direct, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec, false);
   }
   return SPSIM_OK;
 }
@@ -968,28 +1199,46 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 // ---------------------------------------------------------------------------
 // enqueue, plan cache, forward entry points
 
-static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1) {
+// gate: a stand-by plan, run only where the device sets *gate (nullptr: always).
+static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, int *gate = nullptr) {
   cudaError_t e;
   long long acc_total = 0;
   for (long long n : pl.npix_of) acc_total += n;
-  if ((e = cudaMemsetAsync(pl.acc.p, 0, std::max<long long>(acc_total, 1) * sizeof(double2), stream))) return e;
-  if ((e = cudaMemsetAsync(pl.flags.p, 0, sizeof(int), stream))) return e;  // work queue head
+  if (gate) {
+    if ((e = launch_gate((const SfPattern *)pl.pats.p, pl.npat, pl.n_items, gate, (int *)pl.flags.p,
+                         (double2 *)pl.acc.p, acc_total, stream)))
+      return e;
+  } else {
+    if ((e = cudaMemsetAsync(pl.acc.p, 0, std::max<long long>(acc_total, 1) * sizeof(double2), stream))) return e;
+    if ((e = cudaMemsetAsync(pl.flags.p, 0, sizeof(int), stream))) return e;  // work queue head
+  }
   if (ev0 && (e = cudaEventRecord(ev0, stream))) return e;
   if (pl.precision == SPSIM_PREC_FP64) {
     for (int i = 0; i < pl.npat; ++i)
       if ((e = launch_sf_f64((const SfPattern *)pl.pats.p, i, pl.npix_of[i], stream))) return e;
   } else if (pl.n_items > 0) {
-    const int mode = pl.precision == SPSIM_PREC_F32_FAST ? PREC_MODE_MUFU : PREC_MODE_POLY;
     int *flags = (int *)pl.flags.p;
-    if ((e = launch_sf_f32(mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
-                           pl.n_items, flags, flags + 4, pl.grid, stream, pl.fixw, pl.narrow)))
-      return e;
+    if (pl.coarse)
+      e = launch_sf_nodes(pl.perb, pl.fixw, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p, pl.n_items, flags,
+                          flags + 4, pl.grid, stream);
+    else
+      e = launch_sf_f32(pl.mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
+                        pl.n_items, flags, flags + 4, pl.grid, stream, pl.fixw, pl.narrow);
+    if (e) return e;
   }
   if (ev1 && (e = cudaEventRecord(ev1, stream))) return e;
+  const SfPattern *pats = (const SfPattern *)pl.pats.p;
+  const int pixels = pl.coarse ? pl.npat : 0;  // the first pixel pattern
+  if (pl.coarse && (e = launch_coarse_interp(pats + pixels, (const CoarsePattern *)pl.cpats.p, pl.npat, pl.max_nx,
+                                             pl.max_ny, pl.max_nyn, (double2 *)pl.strip.p, pl.strip_size, stream)))
+    return e;
   if (pl.spectrum > 0)
-    return launch_spectrum_combine((const SfPattern *)pl.pats.p, 0, pl.spectrum, (const double *)pl.spec_w.p, pl.spec_F,
-                                   pl.spec_I, pl.npix_of.empty() ? 0 : pl.npix_of[0], stream);
-  return launch_finalize((const SfPattern *)pl.pats.p, 0, pl.npat, pl.max_npix, stream);
+    e = launch_spectrum_combine(pats, pixels, pl.spectrum, (const double *)pl.spec_w.p, pl.spec_F, pl.spec_I,
+                                pl.npat ? pl.host_pats[pixels].npix : 0, stream, gate);
+  else if (!pl.coarse)
+    e = launch_finalize(pats, 0, pl.npat, pl.max_npix, stream, gate);
+  if (e != cudaSuccess || !pl.direct) return e;
+  return enqueue_plan(*pl.direct, stream, nullptr, nullptr, (int *)pl.gate.p);
 }
 
 static void plan_key(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
@@ -1013,6 +1262,7 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
   for (int i = 0; i < npat; ++i) {
     kv.push_back((double)(mols[i] ? mols[i]->id : 0));
     kv.push_back((double)(qsets[i] ? qsets[i]->id : 0));
+    kv.push_back(mols[i] && mols[i]->b_updated ? 1.0 : 0.0);
     kp.push_back(F_dev ? (const void *)F_dev[i] : nullptr);
     kp.push_back(I_dev ? (const void *)I_dev[i] : nullptr);
   }
@@ -1030,13 +1280,20 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
 static cudaError_t refresh_rotations(Plan &pl, const double *rot, cudaStream_t stream) {
   if (!rot) return cudaSuccess;
   bool changed = false;
-  for (int i = 0; i < pl.npat; ++i)
-    if (memcmp(pl.host_pats[i].rot, rot + 9 * (size_t)i, 9 * sizeof(double)) != 0) {
-      memcpy(pl.host_pats[i].rot, rot + 9 * (size_t)i, 9 * sizeof(double));
+  for (size_t i = 0; i < pl.host_pats.size(); ++i) {
+    const double *R = rot + 9 * (i % (size_t)pl.npat);
+    if (memcmp(pl.host_pats[i].rot, R, 9 * sizeof(double)) != 0) {
+      memcpy(pl.host_pats[i].rot, R, 9 * sizeof(double));
       changed = true;
     }
+  }
+  if (pl.direct) {
+    const cudaError_t e = refresh_rotations(*pl.direct, rot, stream);
+    if (e != cudaSuccess) return e;
+  }
   if (!changed) return cudaSuccess;
-  return cudaMemcpyAsync(pl.pats.p, pl.host_pats.data(), pl.npat * sizeof(SfPattern), cudaMemcpyHostToDevice, stream);
+  return cudaMemcpyAsync(pl.pats.p, pl.host_pats.data(), pl.host_pats.size() * sizeof(SfPattern),
+                         cudaMemcpyHostToDevice, stream);
 }
 
 static int check_flags(Plan &pl) {
@@ -1052,7 +1309,7 @@ static int check_flags(Plan &pl) {
     cudaMemcpy((int *)pl.flags.p + 5, &z, sizeof(int), cudaMemcpyHostToDevice);
     return fail(SPSIM_ERR_RANGE, "atoms moved outside the molecule's creation-time bounds");
   }
-  return SPSIM_OK;
+  return pl.direct ? check_flags(*pl.direct) : SPSIM_OK;
 }
 
 // cache == false: a one-shot plan (host convenience path), synchronised before return
@@ -1123,6 +1380,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     if (st) return st;
   }
   g_last_terms = pl->terms;
+  g_last_evaluated = pl->evaluated;
   g_last_variant[0] = pl->precision == SPSIM_PREC_FP64 ? 256 : pl->nt;
   g_last_variant[1] = pl->precision == SPSIM_PREC_FP64 ? 1 : pl->ppt;
   g_last_variant[2] = pl->precision == SPSIM_PREC_FP64 ? -1 : pl->packed;
@@ -2145,6 +2403,12 @@ extern "C" int spsim_b200_timing_read(double *ms, int cap, int *n) {
 extern "C" int spsim_b200_last_forward_stats(double *terms, double *kernel_ms) {
   if (terms) *terms = g_last_terms;
   if (kernel_ms) *kernel_ms = g_last_ms;
+  return SPSIM_OK;
+}
+
+extern "C" int spsim_b200_last_terms_evaluated(double *terms) {
+  if (!terms) return fail(SPSIM_ERR_INVALID_ARG, "NULL argument");
+  *terms = g_last_evaluated;
   return SPSIM_OK;
 }
 

@@ -1,0 +1,303 @@
+// Coarse detector grids: node tables and the interpolation to pixels
+// (coarse_kernels.cuh says what they are for).
+#include "coarse_kernels.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace spsim {
+
+int coarse_node_count(double c, double t, double a) {
+  const double cc = c > 1.0 ? c : 1.0;
+  double n = 0.66 * cc + 8.9 * std::pow(cc, 0.253);
+  if (t > 0.0) n += (3.5 + 11.5 * std::sqrt(cc / 320.0)) * std::pow(t, 1.2);
+  if (a > 0.0) n += 6.6 * std::sqrt(a) / (1.0 + 0.5 * std::pow(cc / (8.0 * a), 0.6));
+  return (int)std::ceil(n);
+}
+
+CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, bool spherical) {
+  CoarseAxis a;
+  a.n_pix = n_pix;
+  a.angular = spherical ? 0 : 1;
+  a.size = size;
+  a.centre = centre;
+  a.distance = distance;
+  a.mid = 0.0;
+  a.half = 1.0;
+  a.n = 0;
+  a.alpha = a.asin_alpha = 0.0;
+  if (a.angular) {
+    const double edge = 0.5 * (n_pix - 1) / n_pix * size;
+    const double t0 = std::atan((-edge - centre) / distance), t1 = std::atan((edge - centre) / distance);
+    a.mid = 0.5 * (t0 + t1);
+    a.half = 0.5 * (t1 - t0);
+  }
+  return a;
+}
+
+void coarse_set_nodes(CoarseAxis &a, int n) {
+  a.n = n;
+  a.alpha = 1.0 / std::cosh(9.3 * std::cbrt((double)n) / n);
+  a.asin_alpha = std::asin(a.alpha);
+}
+
+// ---------------------------------------------------------------------------
+// node q vectors and interpolation matrices
+
+struct CoarseTables {
+  DetGeom g;
+  CoarseAxis x, y;
+  int ldx, ldy;
+  double *q64, *mx, *my;
+};
+
+// position on the detector (m) of node k of an axis
+__device__ __forceinline__ double coarse_node_pos(const CoarseAxis &a, int k) {
+  const double X = asin(a.alpha * cospi((double)k / (a.n - 1))) / a.asin_alpha;
+  if (a.angular) return a.distance * tan(a.mid + a.half * X);
+  return (0.5 * (a.n_pix - 1) * X / a.n_pix) * a.size - a.centre;
+}
+
+// One row (pixel p) of an interpolation matrix by one warp:
+// M[k] = (w_k / (xi - xi_k)) / sum_j w_j / (xi - xi_j), the barycentric weights
+// of the Chebyshev extreme points w_k = (-1)^k, halved at both ends.
+__device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, double *__restrict__ m) {
+  const int lane = threadIdx.x & 31, n = a.n;
+  double X = 2.0 * p / (a.n_pix - 1) - 1.0;
+  if (a.angular) {
+    const double pos = ((p - (a.n_pix - 1.0) / 2.0) / a.n_pix) * a.size - a.centre;
+    X = (atan(pos / a.distance) - a.mid) / a.half;
+  }
+  const double xi = sin(a.asin_alpha * X) / a.alpha;
+  double sum = 0.0;
+  int hit = -1;
+  for (int k = lane; k < n; k += 32) {
+    const double d = xi - cospi((double)k / (n - 1));
+    if (fabs(d) < 1e-14) hit = k;
+    const double w = ((k & 1) ? -1.0 : 1.0) * ((k == 0 || k == n - 1) ? 0.5 : 1.0);
+    sum += hit == k ? 0.0 : w / d;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    hit = max(hit, __shfl_xor_sync(0xffffffffu, hit, o));
+  }
+  for (int k = lane; k < ld; k += 32) {
+    double v = 0.0;
+    if (k < n) {
+      const double d = xi - cospi((double)k / (n - 1));
+      const double w = ((k & 1) ? -1.0 : 1.0) * ((k == 0 || k == n - 1) ? 0.5 : 1.0);
+      v = hit >= 0 ? (k == hit ? 1.0 : 0.0) : w / d / sum;
+    }
+    m[(long long)p * ld + k] = v;
+  }
+}
+
+__global__ void __launch_bounds__(256) coarse_tables_kernel(CoarseTables t) {
+  const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int nx = t.x.n_pix, ny = t.y.n_pix;
+  if (warp < nx) {
+    coarse_row(warp, t.x, t.ldx, t.mx);
+  } else if (warp < nx + ny) {
+    coarse_row(warp - nx, t.y, t.ldy, t.my);
+  } else {
+    const int i = (warp - nx - ny) * 32 + lane;
+    if (i >= t.x.n * t.y.n) return;
+    const double px = coarse_node_pos(t.x, i % t.x.n), py = coarse_node_pos(t.y, i / t.x.n);
+    double q0, q1, q2 = 0.0;
+    if (t.g.spherical) {
+      q0 = t.g.fpx * px / t.g.px_size;
+      q1 = t.g.fpy * py / t.g.py_size;
+    } else {
+      const double r = sqrt(px * px + py * py + t.g.distance * t.g.distance);
+      q0 = px / r * t.g.ewald;
+      q1 = py / r * t.g.ewald;
+      q2 = (t.g.distance / r - 1.0) * t.g.ewald;
+    }
+    t.q64[3 * i] = q0;
+    t.q64[3 * i + 1] = q1;
+    t.q64[3 * i + 2] = q2;
+  }
+}
+
+cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
+                                 double *my, cudaStream_t st) {
+  CoarseTables t;
+  t.g = g;
+  t.x = x;
+  t.y = y;
+  t.ldx = coarse_ld(x.n);
+  t.ldy = coarse_ld(y.n);
+  t.q64 = q64;
+  t.mx = mx;
+  t.my = my;
+  const long long warps = (long long)x.n_pix + y.n_pix + ((long long)x.n * y.n + 31) / 32;
+  coarse_tables_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(t);
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// Interpolation as two FP64 matrix products on the tensor pipe (m8n8k4):
+//   columns  strip[k][x] = sum_i M_x[x][i] nodes[k][i]
+//   rows     pixel[y][x] = sum_k M_y[y][k] strip[k][x]
+// with the complex values' parts as neighbouring columns of the right-hand
+// matrix, so that each lane's pair of results is one amplitude.  The rows'
+// kernel then applies the global B factor and the centre phase and writes F
+// and |F|^2 as sf_finalize_kernel does.  Fragments come straight from L1 / L2:
+// a warp's RM x RN tiles of 8 x 8 reuse each of its 2 (RM + RN) loads per four
+// k steps.  FP64 MMA runs at the FMA units' own rate but issues a quarter of
+// the loads of the same product written with FMAs from shared memory (50,000
+// atoms x 1024^2, 182 nodes a side: that form took 335 us).
+constexpr int INTERP_WARPS_M = 2, INTERP_WARPS_N = 2;
+constexpr int INTERP_THREADS = 32 * INTERP_WARPS_M * INTERP_WARPS_N;
+
+__device__ __forceinline__ void dmma(double c[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// ROWS: the second product, else the first.
+template <int RM, int RN, bool ROWS>
+__global__ void __launch_bounds__(INTERP_THREADS)
+    coarse_interp_kernel(const SfPattern *__restrict__ pats, const CoarsePattern *__restrict__ coarse, int pattern0,
+                         double2 *__restrict__ strips, long long strip_stride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const CoarsePattern cp = coarse[pattern0 + blockIdx.z];
+  double2 *__restrict__ strip = strips + blockIdx.z * strip_stride;
+  const int m_all = ROWS ? cp.ny : cp.nx;             // rows of the left matrix
+  const int n_all = 2 * (ROWS ? cp.nx : cp.nyn);      // columns of the right one (re, im pairs)
+  const int k_all = ROWS ? cp.nyn : cp.nxn;
+  const int ld = ROWS ? cp.ldy : cp.ldx;
+  const double *__restrict__ M = ROWS ? cp.my : cp.mx;
+  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
+  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);
+  if (m0 >= m_all || n0 >= n_all) return;
+  const int fr = lane >> 2, fc = lane & 3;
+
+  // lane's entries of the fragments: k steps 4 s .. 4 s + 3 of a group of eight
+  // hold k = 2 fc + s, so that the left matrix is read in pairs
+  const double2 *arow[RM];
+#pragma unroll
+  for (int i = 0; i < RM; ++i) arow[i] = (const double2 *)(M + (long long)min(m0 + 8 * i + fr, m_all - 1) * ld) + fc;
+  const double *bcol[RN];
+  const long long bstep = ROWS ? 2LL * cp.nx : 2;  // doubles from k to k + 1
+#pragma unroll
+  for (int j = 0; j < RN; ++j) {
+    const int n = min(n0 + 8 * j + fr, n_all - 1);
+    bcol[j] = ROWS ? (const double *)strip + n : (const double *)(cp.nodes + (long long)(n >> 1) * cp.nxn) + (n & 1);
+  }
+  double acc[RM][RN][2];
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < RN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int k = 0; k < k_all; k += 8) {
+    // beyond k_all the left matrix holds zeros; the right one is read in range
+    const long long kb0 = min(k + 2 * fc, k_all - 1) * bstep, kb1 = min(k + 2 * fc + 1, k_all - 1) * bstep;
+    double2 a[RM];
+    double b0[RN], b1[RN];
+#pragma unroll
+    for (int i = 0; i < RM; ++i) a[i] = arow[i][k / 2];
+#pragma unroll
+    for (int j = 0; j < RN; ++j) {
+      b0[j] = bcol[j][kb0];
+      b1[j] = bcol[j][kb1];
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < RN; ++j) dmma(acc[i][j], a[i].x, b0[j]);
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < RN; ++j) dmma(acc[i][j], a[i].y, b1[j]);
+  }
+
+  if (!ROWS) {
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+      const int x = m0 + 8 * i + fr;
+      if (x >= cp.nx) continue;
+#pragma unroll
+      for (int j = 0; j < RN; ++j) {
+        const int k = n0 / 2 + 4 * j + fc;
+        if (k < cp.nyn) strip[(long long)k * cp.nx + x] = make_double2(acc[i][j][0], acc[i][j][1]);
+      }
+    }
+    return;
+  }
+  const SfPattern &pt = pats[pattern0 + blockIdx.z];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int y = m0 + 8 * i + fr;
+    if (y >= cp.ny) continue;
+#pragma unroll
+    for (int j = 0; j < RN; ++j) {
+      const int x = n0 / 2 + 4 * j + fc;
+      if (x >= cp.nx) continue;
+      const long long p = (long long)y * cp.nx + x;
+      double re = acc[i][j][0], im = acc[i][j][1];
+      if (pt.F || cp.B != 0.0 || cp.out) {
+        const double a = pt.q64[3 * p], b = pt.q64[3 * p + 1], c = pt.q64[3 * p + 2];
+        if (cp.B != 0.0) {
+          const double e = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
+          re *= e;
+          im *= e;
+        }
+        if (cp.out) {
+          cp.out[p] = make_double2(re, im);
+          continue;
+        }
+        if (pt.F) {
+          double ux = a, uy = b, uz = c;
+          if (pt.has_rot) {
+            ux = pt.rot[0] * a + pt.rot[1] * b + pt.rot[2] * c;
+            uy = pt.rot[3] * a + pt.rot[4] * b + pt.rot[5] * c;
+            uz = pt.rot[6] * a + pt.rot[7] * b + pt.rot[8] * c;
+          }
+          double t = (ux * pt.center[0] + uy * pt.center[1] + uz * pt.center[2]) * pt.qscale;
+          t -= rint(t);
+          double sn, cs;
+          sincospi(2.0 * t, &sn, &cs);
+          pt.F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
+        }
+      }
+      if (pt.I) pt.I[p] = (float)(re * re + im * im);
+    }
+  }
+}
+
+template <int RM, int RN, bool ROWS>
+static void interp_t(const SfPattern *pats, const CoarsePattern *coarse, int pattern0, int n, int m_max, int n_max,
+                     double2 *strip, long long stride, cudaStream_t st) {
+  const int bm = 8 * RM * INTERP_WARPS_M, bn = 8 * RN * INTERP_WARPS_N;
+  dim3 grid((unsigned)((n_max + bn - 1) / bn), (unsigned)((m_max + bm - 1) / bm), (unsigned)n);
+  coarse_interp_kernel<RM, RN, ROWS><<<grid, INTERP_THREADS, 0, st>>>(pats, coarse, pattern0, strip, stride);
+}
+
+template <bool ROWS>
+static void interp_part(const SfPattern *pats, const CoarsePattern *coarse, int pattern0, int n, int m_max, int n_max,
+                        double2 *strip, long long stride, cudaStream_t st) {
+  // 32 x 32 tiles per warp where they fill the GPU a few times, else 16 x 16
+  const long long blocks = (long long)n * ((m_max + 63) / 64) * ((n_max + 63) / 64);
+  if (blocks >= 2 * 148)
+    interp_t<4, 4, ROWS>(pats, coarse, pattern0, n, m_max, n_max, strip, stride, st);
+  else
+    interp_t<2, 2, ROWS>(pats, coarse, pattern0, n, m_max, n_max, strip, stride, st);
+}
+
+cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coarse, int npat, int max_nx, int max_ny,
+                                 int max_nyn, double2 *strip, long long strip_size, cudaStream_t st) {
+  if (npat <= 0 || max_nx <= 0 || max_ny <= 0) return cudaSuccess;
+  const long long stride = (long long)max_nyn * max_nx;
+  const int group = (int)std::min<long long>(std::max<long long>(strip_size / stride, 1), 65535);
+  for (int p0 = 0; p0 < npat; p0 += group) {
+    const int n = std::min(group, npat - p0);
+    interp_part<false>(pats, coarse, p0, n, max_nx, 2 * max_nyn, strip, stride, st);
+    interp_part<true>(pats, coarse, p0, n, max_ny, 2 * max_nx, strip, stride, st);
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace spsim

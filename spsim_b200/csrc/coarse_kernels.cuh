@@ -1,0 +1,72 @@
+// Coarse detector grids (internal C++ interface).
+//
+// A pattern's centred amplitude A(x, y) = sum_e f_e sum_j w_j e^{-2 pi i q(x, y).(r_j - c)}
+// over the pixel coordinates of a detector is smooth: no atom's phase turns
+// faster than |dq/dx| |r - c|max cycles per pixel.  Where that is well below
+// half a cycle, the sum is evaluated on a tensor grid of nodes instead of on
+// every pixel and every pixel interpolates it: A = M_y A_nodes M_x^T in FP64.
+// Along each axis of a flat detector the coordinate is the scattering angle
+// atan(x / D), in which q moves along the Ewald sphere at (almost) constant
+// speed; a spherical detector's q is linear in the pixel index.  The nodes are
+// Chebyshev extreme points stretched towards equal spacing by
+// x = asin(alpha xi) / asin(alpha) (Kosloff and Tal-Ezer, J. Comput. Phys. 104
+// (1993) 457), so that little more than two of them per cycle are needed, and
+// the interpolation is the barycentric formula in xi (Salzer; Berrut and
+// Trefethen, SIAM Rev. 46 (2004) 501).
+#pragma once
+
+#include "sf_device.cuh"
+
+namespace spsim {
+
+// Pixel geometry of a detector q set, in the units of ewald_kernel.
+struct DetGeom {
+  int nx, ny;
+  int spherical;
+  double width, height, distance, cx, cy, ewald, fpx, fpy, px_size, py_size;
+};
+
+// One axis of a detector in the interpolation's coordinate X in [-1, 1]:
+// (atan(x / D) - mid) / half of the pixel's position x on a flat detector,
+// the scaled pixel index on a spherical one.
+struct CoarseAxis {
+  int n_pix, angular;
+  double size, centre, distance, mid, half;
+  int n;  // nodes
+  double alpha, asin_alpha;
+};
+
+constexpr int COARSE_MAX_NODES = 1024;  // per axis
+
+CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, bool spherical);
+// Nodes along one axis for phases of at most c radians over half of it, pixels
+// up to t detector distances off the beam axis and form factors falling as
+// exp(-a X^2): a fit, from above, to the smallest node counts that interpolate
+// every such function to 1e-8 of its maximum (tests/test_coarse_grid.py
+// restates it and measures the errors).
+int coarse_node_count(double c, double t, double a);
+void coarse_set_nodes(CoarseAxis &a, int n);
+
+// What the interpolation of one pattern reads and writes beside its
+// SfPattern of pixels.
+struct CoarsePattern {
+  const double2 *nodes;  // [nyn][nxn] centred amplitudes
+  const double *mx;      // [nx][ldx]: weight of node column i for pixel column x at mx[x * ldx + i]
+  const double *my;      // [ny][ldy]
+  int nx, ny, nxn, nyn, ldx, ldy;
+  double B;              // global B factor, applied per pixel
+  double2 *out;          // centred pixel amplitudes (FP64) instead of F and I, or nullptr
+};
+
+__host__ __device__ inline int coarse_ld(int n) { return (n + 7) / 8 * 8; }
+
+// Node q vectors [y.n * x.n][3] and both interpolation matrices of one detector.
+cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
+                                 double *my, cudaStream_t st);
+// Interpolates npat patterns: F, I of pats[i] (or coarse[i].out) from
+// coarse[i].nodes, in groups of as many patterns as the strip buffer holds
+// (strip_doubles2 complex values, at least max_nyn * max_nx).
+cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coarse, int npat, int max_nx, int max_ny,
+                                 int max_nyn, double2 *strip, long long strip_size, cudaStream_t st);
+
+}  // namespace spsim

@@ -131,6 +131,7 @@ def main():
     emit("HALF", 0.25 + 1.0 / 16, 4, 5, out)
     emit("QUAD", 0.125 + 1.0 / 16, 4, 4, out)
     emit("DHALF", 0.25, 4, 4, out)
+    emit("NODE", 0.25, 4, 5, out)
     emit("WIDE", 0.375, 5, 5, out)
     emit("NARROW", 0.32, 4, 5, out)
     emit("WIDER", 0.41, 5, 5, out)

@@ -128,6 +128,38 @@ __device__ __forceinline__ void bulk_copy_g2s(void *smem_dst, const void *gmem_s
       : "memory");
 }
 
+// Limits of the bounded waits on the atom-tile ring.
+constexpr long long kWaitCyclesDefault = 4000000000LL;  // ~2 s at 2 GHz
+constexpr long long kStallWaitCycles = 20000000LL;      // ~10 ms
+
+// ---------------------------------------------------------------------------
+// pixel set-up shared by the kernels: q (FP64) of pixel p, rotated
+
+__device__ __forceinline__ void load_q(const SfPattern &pt, long long p, double q[3]) {
+  double a, b, c;
+  if (pt.hkl) {
+    a = pt.hkl[3 * p];
+    b = pt.hkl[3 * p + 1];
+    c = pt.hkl[3 * p + 2];
+  } else {
+    a = pt.q64[3 * p];
+    b = pt.q64[3 * p + 1];
+    c = pt.q64[3 * p + 2];
+  }
+  if (pt.has_rot) {
+    q[0] = pt.rot[0] * a + pt.rot[1] * b + pt.rot[2] * c;
+    q[1] = pt.rot[3] * a + pt.rot[4] * b + pt.rot[5] * c;
+    q[2] = pt.rot[6] * a + pt.rot[7] * b + pt.rot[8] * c;
+  } else {
+    q[0] = a;
+    q[1] = b;
+    q[2] = c;
+  }
+  q[0] *= pt.qscale;
+  q[1] *= pt.qscale;
+  q[2] *= pt.qscale;
+}
+
 // ---------------------------------------------------------------------------
 // per-term arithmetic
 
@@ -181,6 +213,23 @@ __device__ __forceinline__ void sincos_dhalf_poly2(float2 y, float2 &S, float2 &
   pc = fma2(z, pc, f2(SPSIM_DHALF_C2));
   pc = fma2(z, pc, f2(SPSIM_DHALF_C1));
   pc = fma2(z, pc, f2(SPSIM_DHALF_C0));
+  S = mul2(y, ps);
+  C = pc;
+}
+
+// the NODE pair (|y| <= 1/4 cycle): DHALF with one more cosine coefficient,
+// whose error DHALF's five leave at +-6e-8 over whole ranges of the phase
+__device__ __forceinline__ void sincos_node_poly2(float2 y, float2 &S, float2 &C) {
+  const float2 z = mul2(y, y);
+  float2 ps = fma2(z, f2(SPSIM_NODE_S4), f2(SPSIM_NODE_S3));
+  ps = fma2(z, ps, f2(SPSIM_NODE_S2));
+  ps = fma2(z, ps, f2(SPSIM_NODE_S1));
+  ps = fma2(z, ps, f2(SPSIM_NODE_S0));
+  float2 pc = fma2(z, f2(SPSIM_NODE_C5), f2(SPSIM_NODE_C4));
+  pc = fma2(z, pc, f2(SPSIM_NODE_C3));
+  pc = fma2(z, pc, f2(SPSIM_NODE_C2));
+  pc = fma2(z, pc, f2(SPSIM_NODE_C1));
+  pc = fma2(z, pc, f2(SPSIM_NODE_C0));
   S = mul2(y, ps);
   C = pc;
 }

@@ -32,12 +32,10 @@ __host__ __device__ constexpr int sf_min_blocks(int mode) { return mode == PREC_
 // after kStallWaitCycles, so the exit path runs in milliseconds and without a
 // fault; read once per CTA at launch.
 __device__ int g_copy_stall = 0;
-constexpr long long kWaitCyclesDefault = 4000000000LL;  // ~2 s at 2 GHz
-constexpr long long kStallWaitCycles = 20000000LL;      // ~10 ms
-
 cudaError_t set_copy_stall(int on) {
   const int v = on ? 1 : 0;
-  return cudaMemcpyToSymbol(g_copy_stall, &v, sizeof(int));
+  const cudaError_t e = cudaMemcpyToSymbol(g_copy_stall, &v, sizeof(int));
+  return e != cudaSuccess ? e : set_nodes_copy_stall(on);
 }
 
 // ---------------------------------------------------------------------------
@@ -70,34 +68,6 @@ __global__ void ff_table_kernel(const float *__restrict__ hkl, const double *__r
     f += (double)c[8] * exp(-B * s2);
   }
   ff[(long long)e * npix + p] = f;
-}
-
-// ---------------------------------------------------------------------------
-// pixel set-up shared by the kernels: q (FP64) of pixel p, rotated
-
-__device__ __forceinline__ void load_q(const SfPattern &pt, long long p, double q[3]) {
-  double a, b, c;
-  if (pt.hkl) {
-    a = pt.hkl[3 * p];
-    b = pt.hkl[3 * p + 1];
-    c = pt.hkl[3 * p + 2];
-  } else {
-    a = pt.q64[3 * p];
-    b = pt.q64[3 * p + 1];
-    c = pt.q64[3 * p + 2];
-  }
-  if (pt.has_rot) {
-    q[0] = pt.rot[0] * a + pt.rot[1] * b + pt.rot[2] * c;
-    q[1] = pt.rot[3] * a + pt.rot[4] * b + pt.rot[5] * c;
-    q[2] = pt.rot[6] * a + pt.rot[7] * b + pt.rot[8] * c;
-  } else {
-    q[0] = a;
-    q[1] = b;
-    q[2] = c;
-  }
-  q[0] *= pt.qscale;
-  q[1] *= pt.qscale;
-  q[2] *= pt.qscale;
 }
 
 // ---------------------------------------------------------------------------
@@ -1354,7 +1324,9 @@ __global__ void __launch_bounds__(256) sf_f64_kernel(const SfPattern *__restrict
 // ---------------------------------------------------------------------------
 // finalize: F = e^{-2 pi i q.c} acc, I = |acc|^2
 
-__global__ void sf_finalize_kernel(const SfPattern *__restrict__ pats, int pattern0) {
+// gate: run only where *gate is set (nullptr: always)
+__global__ void sf_finalize_kernel(const SfPattern *__restrict__ pats, int pattern0, const int *__restrict__ gate) {
+  if (gate && !*gate) return;
   const SfPattern &pt = pats[pattern0 + blockIdx.y];
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
@@ -1378,7 +1350,8 @@ __global__ void sf_finalize_kernel(const SfPattern *__restrict__ pats, int patte
 // sum, each with its own centre phase e^{-2 pi i s_j q.c}, and I = |F|^2.
 __global__ void sf_spectrum_combine_kernel(const SfPattern *__restrict__ pats, int pattern0, int S,
                                            const double *__restrict__ weight, float2 *__restrict__ F,
-                                           float *__restrict__ I, long long npix) {
+                                           float *__restrict__ I, long long npix, const int *__restrict__ gate) {
+  if (gate && !*gate) return;
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p == 0 && pats[pattern0].mol_err && *pats[pattern0].mol_err) atomicOr(pats[pattern0].plan_err, 1);
   if (p >= npix) return;
@@ -1492,7 +1465,7 @@ __global__ void atoms_update_kernel(float4 *__restrict__ atoms, float4 *__restri
                                     const float *__restrict__ pos32, const double *__restrict__ pos64,
                                     const float *__restrict__ occ, const float *__restrict__ bfac,
                                     const float *__restrict__ wbase, double cx, double cy, double cz, float dr,
-                                    float inv_dr, double rbound, int *__restrict__ range_err) {
+                                    float inv_dr, double rbound, float b_limit, int *__restrict__ range_err) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n_padded) return;
   const int src = perm[j];
@@ -1519,7 +1492,10 @@ __global__ void atoms_update_kernel(float4 *__restrict__ atoms, float4 *__restri
   a1.y = (float)(r[1] - hy);
   a1.z = (float)(r[2] - hz);
   if (occ) a0.w = occ[src] * wbase[j];
-  if (bfac) a1.w = bfac[src];
+  if (bfac) {
+    a1.w = bfac[src];
+    if (!(fabsf(a1.w) <= b_limit)) atomicOr(range_err + 1, 1);
+  }
   atoms[2 * j] = a0;
   atoms[2 * j + 1] = a1;
   atoms2[4 * j] = make_float4(a0.x, a0.x, a0.y, a0.y);
@@ -1724,23 +1700,55 @@ cudaError_t launch_sf_f64(const SfPattern *pats, int pattern, long long npix, cu
 }
 
 cudaError_t launch_spectrum_combine(const SfPattern *pats, int pattern0, int S, const double *weight, float *F,
-                                    float *I, long long npix, cudaStream_t st) {
+                                    float *I, long long npix, cudaStream_t st, const int *gate) {
   if (npix <= 0) return cudaSuccess;
   sf_spectrum_combine_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(pats, pattern0, S, weight, (float2 *)F, I,
-                                                                            npix);
+                                                                            npix, gate);
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const SfPattern *pats, int pattern0, int npat, long long max_npix, cudaStream_t st) {
+cudaError_t launch_finalize(const SfPattern *pats, int pattern0, int npat, long long max_npix, cudaStream_t st,
+                            const int *gate) {
   if (max_npix <= 0 || npat <= 0) return cudaSuccess;
   for (int p0 = 0; p0 < npat; p0 += 65535) {
     const int n = npat - p0 < 65535 ? npat - p0 : 65535;
     dim3 grid((unsigned)((max_npix + 255) / 256), (unsigned)n);
-    sf_finalize_kernel<<<grid, 256, 0, st>>>(pats, pattern0 + p0);
+    sf_finalize_kernel<<<grid, 256, 0, st>>>(pats, pattern0 + p0, gate);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// Decides on the device whether a batch must run on every pixel: any of its
+// molecules holds a B factor beyond its limit.  The result goes to gate and,
+// as the first work item (all of them, or none left), to the queue head.
+__global__ void __launch_bounds__(256) sf_gate_kernel(const SfPattern *__restrict__ pats, int npat, int n_items,
+                                                      int *__restrict__ gate, int *__restrict__ queue) {
+  int any = 0;
+  for (int i = threadIdx.x; i < npat; i += blockDim.x) any |= pats[i].mol_err[1];
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    *gate = any;
+    *queue = any ? 0 : n_items;
+  }
+}
+
+__global__ void __launch_bounds__(256) sf_gated_zero_kernel(double2 *__restrict__ p, long long n,
+                                                            const int *__restrict__ gate) {
+  if (!*gate) return;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    p[i] = make_double2(0.0, 0.0);
+}
+
+cudaError_t launch_gate(const SfPattern *pats, int npat, int n_items, int *gate, int *queue, double2 *acc,
+                        long long n_acc, cudaStream_t st) {
+  sf_gate_kernel<<<1, 256, 0, st>>>(pats, npat, n_items, gate, queue);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || n_acc <= 0) return e;
+  const long long blocks = (n_acc + 255) / 256;
+  sf_gated_zero_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(acc, n_acc, gate);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_ewald(int nx, int ny, double width, double height, double distance, double cx, double cy,
@@ -1907,11 +1915,11 @@ cudaError_t launch_volume(int nx, int ny, int nz, float width, float height, flo
 
 cudaError_t launch_atoms_update(float4 *atoms, float4 *atoms2, AtomD *atomsd, const int *perm, int n_padded, const float *pos32,
                                 const double *pos64, const float *occ, const float *bfac, const float *wbase,
-                                const double c[3], float dr, float inv_dr, double rbound, int *range_err,
+                                const double c[3], float dr, float inv_dr, double rbound, float b_limit, int *range_err,
                                 cudaStream_t st) {
   if (n_padded <= 0) return cudaSuccess;
   atoms_update_kernel<<<(n_padded + 255) / 256, 256, 0, st>>>(atoms, atoms2, atomsd, perm, n_padded, pos32, pos64, occ, bfac, wbase,
-                                                             c[0], c[1], c[2], dr, inv_dr, rbound, range_err);
+                                                             c[0], c[1], c[2], dr, inv_dr, rbound, b_limit, range_err);
   return cudaGetLastError();
 }
 

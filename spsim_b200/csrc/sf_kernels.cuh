@@ -17,11 +17,17 @@ cudaError_t launch_sf_f32(int mode, int nt, int p, int packed, bool perb, const 
                           bool fixw = false, bool narrow = false);
 // The bounded-wait test hook (see g_copy_stall in sf_kernels.cu), current device.
 cudaError_t set_copy_stall(int on);
+cudaError_t set_nodes_copy_stall(int on);  // its part in sf_nodes.cu
 int sf_f32_occupancy(int mode, int nt, int p, int packed, bool perb, bool fixw = false, bool narrow = false);
+// The quad form on a coarse grid's nodes (work items of SF_NODES_TILE nodes).
+cudaError_t launch_sf_nodes(bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items, int *queue,
+                            int *err, int grid, cudaStream_t st);
+int sf_nodes_occupancy(bool perb, bool fixw);
+constexpr int SF_NODES_TILE = 256;
 bool sf_f32_variant_exists(int mode, int nt, int p, int packed);
 cudaError_t launch_sf_f64(const SfPattern *pats, int pattern, long long npix, cudaStream_t st);
 cudaError_t launch_spectrum_combine(const SfPattern *pats, int pattern0, int S, const double *weight, float *F,
-                                    float *I, long long npix, cudaStream_t st);
+                                    float *I, long long npix, cudaStream_t st, const int *gate = nullptr);
 cudaError_t launch_volume(int nx, int ny, int nz, float width, float height, float depth, float distance, float cx,
                           float cy, float cz, float wavelength, float *out32, cudaStream_t st);
 cudaError_t launch_crystal(long long npix, const float *hkl, const double cell[9], int na, int nb, int nc, float *F,
@@ -37,7 +43,14 @@ cudaError_t qset_steps(const float *hkl, const double *q64, long long npix, doub
 // four device words; waits for `st`).
 cudaError_t qset_stats(const float *hkl, long long npix, unsigned long long *scratch4, double *qmax, double steps[3],
                        cudaStream_t st);
-cudaError_t launch_finalize(const SfPattern *pats, int pattern0, int npat, long long max_npix, cudaStream_t st);
+// gate: the kernel does nothing where *gate is 0 (nullptr: it always runs)
+cudaError_t launch_finalize(const SfPattern *pats, int pattern0, int npat, long long max_npix, cudaStream_t st,
+                            const int *gate = nullptr);
+// *gate = whether any pattern's molecule holds a B factor beyond its limit;
+// the work queue's head is set to its first or past its last item, and acc
+// zeroed where the gate is set.
+cudaError_t launch_gate(const SfPattern *pats, int npat, int n_items, int *gate, int *queue, double2 *acc,
+                        long long n_acc, cudaStream_t st);
 cudaError_t launch_ewald(int nx, int ny, double width, double height, double distance, double cx, double cy,
                          double wavelength, int spherical, float *out32, double *out64, cudaStream_t st);
 // Atom records of a new molecule from the caller's positions (float or double),
@@ -48,7 +61,7 @@ cudaError_t launch_atoms_build(float4 *atoms, float4 *atoms2, AtomD *atomsd, con
                                const double c[3], double dr, double inv_dr, cudaStream_t st);
 cudaError_t launch_atoms_update(float4 *atoms, float4 *atoms2, AtomD *atomsd, const int *perm, int n_padded, const float *pos32,
                                 const double *pos64, const float *occ, const float *bfac, const float *wbase,
-                                const double c[3], float dr, float inv_dr, double rbound, int *range_err,
+                                const double c[3], float dr, float inv_dr, double rbound, float b_limit, int *range_err,
                                 cudaStream_t st);
 
 }  // namespace spsim

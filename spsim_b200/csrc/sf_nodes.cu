@@ -1,0 +1,239 @@
+// Structure-factor kernel on the nodes of coarse grids (sm_100a).
+#include "sf_kernels.cuh"
+
+namespace spsim {
+
+// Test hook of the bounded waits, as g_copy_stall in sf_kernels.cu.
+__device__ int g_nodes_copy_stall = 0;
+
+cudaError_t set_nodes_copy_stall(int on) {
+  const int v = on ? 1 : 0;
+  return cudaMemcpyToSymbol(g_nodes_copy_stall, &v, sizeof(int));
+}
+
+// ---------------------------------------------------------------------------
+// The quad form on the nodes of a coarse grid (coarse_kernels.cuh).  Nodes are
+// too far apart for FP32 steps, so all eight points of a thread (two runs of
+// four neighbours, as its two quads) take their own FP64 phase, and the NODE
+// polynomials, with the fewer points' time to spare, one more coefficient than
+// DHALF.  There are few nodes, so the warps of a CTA share one tile of 256 and
+// take its atoms in turn, groups of eight, adding their FP64 sums at the end
+// of the item: against 1,024 nodes per CTA that makes a work item a quarter as
+// long (the launch's tail) and lets a grid of some hundred nodes use the GPU.
+constexpr int NODE_THREADS = 128;
+constexpr int NODE_TILE = SF_NODES_TILE;  // nodes per work item: 8 per lane
+static_assert(NODE_TILE == 256, "eight nodes per lane");
+
+template <bool PERB, bool FIXW>
+__global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
+    const SfPattern *__restrict__ pats, const WorkItem *__restrict__ items, int n_items, int *__restrict__ queue,
+    int *__restrict__ err) {
+  constexpr int P = 8, NP = P / 2, WARPS = NODE_THREADS / 32;
+  __shared__ __align__(128) float4 ring[RING_STAGES][2 * TILE_ATOMS];
+  __shared__ __align__(16) double2 sacc[P * NODE_THREADS];  // per-thread FP64 sums of the current work item
+  __shared__ __align__(8) uint64_t full_bar[RING_STAGES];
+  __shared__ int s_item;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < RING_STAGES; ++s) mbar_init(&full_bar[s], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  uint32_t g_issue = 0, g_cons = 0;
+  const bool stall = g_nodes_copy_stall != 0;
+  const long long kWaitCycles = stall ? kStallWaitCycles : kWaitCyclesDefault;
+  const double M52 = 6755399441055744.0;  // 1.5 * 2^52
+  constexpr double kQScale = FIXW ? 2.0 : 1.0;
+  constexpr bool LOGW = PERB && FIXW;  // the weight folded into the exponent, as in sf_dquad_kernel
+
+  for (;;) {
+    if (tid == 0) s_item = atomicAdd(queue, 1);
+    __syncthreads();
+    const int it = s_item;
+    if (it >= n_items) break;
+    const WorkItem wi = items[it];
+    const SfPattern &pt = pats[wi.pattern];
+    const long long npix = pt.npix;
+    const AtomD *__restrict__ atomsd = pt.atomsd;
+    const TileDesc *__restrict__ tiles = pt.tiles;
+
+    // node i of this lane: pix0 + 128 (i / 4) + i % 4
+    const long long pix0 = (long long)wi.pixel_tile * NODE_TILE + 4 * lane;
+    double qx[P], qy[P], qz[P];
+    float s2n[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const long long p = pix0 + 128 * (i / 4) + i % 4;
+      double q[3] = {0.0, 0.0, 0.0};
+      if (p < npix) load_q(pt, p, q);
+      qx[i] = kQScale * q[0];
+      qy[i] = kQScale * q[1];
+      qz[i] = kQScale * q[2];
+      s2n[i] = (float)(-0.25 * (q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) * 1e-20 * pt.s2scale * 1.4426950408889634);
+    }
+    float2 shc[NP], slc[NP], shs[NP], sls[NP];
+#pragma unroll
+    for (int j = 0; j < NP; ++j) shc[j] = slc[j] = shs[j] = sls[j] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < P; ++i) sacc[i * NODE_THREADS + tid] = make_double2(0.0, 0.0);
+
+    const int k0 = wi.k0, k1 = wi.k1;
+    if (tid == 0) {
+      for (int k = k0; k < k1 && k < k0 + RING_STAGES; ++k) {
+        const TileDesc td = tiles[k];
+        const uint32_t st = g_issue % RING_STAGES;
+        const uint32_t bytes = (uint32_t)td.count * (uint32_t)sizeof(AtomD);
+        mbar_arrive_expect_tx(&full_bar[st], bytes);
+        if (!(stall && g_issue == 0))  // the stall hook skips the CTA's first copy
+          bulk_copy_g2s(&ring[st][0], atomsd + td.atom_begin, bytes, &full_bar[st]);
+        ++g_issue;
+      }
+    }
+
+    for (int k = k0; k < k1; ++k) {
+      const uint32_t st = g_cons % RING_STAGES;
+      const uint32_t par = (g_cons / RING_STAGES) & 1u;
+      const bool ok = mbar_wait_bounded(&full_bar[st], par, kWaitCycles);
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) {
+          atomicOr(err, 1);
+          for (uint32_t g = g_cons; g < g_issue; ++g)
+            mbar_wait_bounded(&full_bar[g % RING_STAGES], (g / RING_STAGES) & 1u, kWaitCycles);
+        }
+        return;
+      }
+      const TileDesc td = tiles[k];
+      const float4 *__restrict__ ta = ring[st];
+      // this warp's groups of eight atoms, two of them per FP32 sum
+      for (int a = ATOM_GROUP * warp; a < td.count; a += 2 * ATOM_GROUP * WARPS) {
+        float2 bc[NP], bs[NP];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) bc[j] = bs[j] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int g = 0; g < 2 * ATOM_GROUP; ++g) {
+          if (g == ATOM_GROUP && a + ATOM_GROUP * WARPS >= td.count) break;
+          const int at = g < ATOM_GROUP ? a + g : a + ATOM_GROUP * (WARPS - 1) + g;
+          const float4 d0 = ta[2 * at], d1 = ta[2 * at + 1];
+          const double rx = __hiloint2double(__float_as_int(d0.y), __float_as_int(d0.x));
+          const double ry = __hiloint2double(__float_as_int(d0.w), __float_as_int(d0.z));
+          const double rz = __hiloint2double(__float_as_int(d1.y), __float_as_int(d1.x));
+          const float W = d1.z;
+          const float lw = LOGW ? lg2_approx(fabsf(W)) : 0.0f;
+          const double wbase = LOGW && W < 0.0f ? PHASE_WORD_BASE_HALF + 1.0 : PHASE_WORD_BASE_HALF;
+#pragma unroll
+          for (int j = 0; j < NP; ++j) {
+            float y[2], w[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int i = 2 * j + h;
+              uint32_t kb;
+              if (FIXW) {
+                const double t = phase_word(qx[i], qy[i], qz[i], rx, ry, rz, wbase);
+                reduce_phase_word<PREC_MODE_POLY>(t, y[h], kb);
+              } else {
+                double u = qx[i] * rx;
+                u = fma(qy[i], ry, u);
+                u = fma(qz[i], rz, u);
+                const double t = fma(u, 2.0, M52);
+                y[h] = __double2float_rn(fma(t - M52, -0.5, u));
+                kb = (uint32_t)__double2loint(t);
+              }
+              w[h] = LOGW ? ex2_approx(fmaf(d1.w, s2n[i], lw)) : PERB ? W * ex2_approx(d1.w * s2n[i]) : W;
+              w[h] = sign_by_parity_alu(w[h], kb);
+            }
+            const float2 yy = FIXW ? mul2(make_float2(y[0], y[1]), f2(word_to_phase<PREC_MODE_POLY>()))
+                                   : make_float2(y[0], y[1]);
+            float2 S, C;
+            sincos_node_poly2(yy, S, C);
+            const float2 ws = make_float2(w[0], w[1]);
+            bc[j] = fma2(ws, C, bc[j]);
+            bs[j] = fma2(ws, S, bs[j]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          ff_accumulate2(shc[j], slc[j], bc[j]);
+          ff_accumulate2(shs[j], sls[j], bs[j]);
+        }
+      }
+      if (td.last || k == k1 - 1) {
+        const double *__restrict__ ffe = pt.ff + (long long)td.elem * npix;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int i = 2 * j + h;
+            const long long p = pix0 + 128 * (i / 4) + i % 4;
+            if (p < npix) {
+              const double f = ffe[p];
+              const double re = h ? (double)shc[j].y + (double)slc[j].y : (double)shc[j].x + (double)slc[j].x;
+              const double sm = h ? (double)shs[j].y + (double)sls[j].y : (double)shs[j].x + (double)sls[j].x;
+              double2 v = sacc[i * NODE_THREADS + tid];
+              v.x = fma(f, re, v.x);
+              v.y = fma(-f, sm, v.y);
+              sacc[i * NODE_THREADS + tid] = v;
+            }
+          }
+          shc[j] = slc[j] = shs[j] = sls[j] = make_float2(0.f, 0.f);
+        }
+      }
+      __syncthreads();
+      if (tid == 0 && k + RING_STAGES < k1) {
+        const TileDesc tn = tiles[k + RING_STAGES];
+        const uint32_t bytes = (uint32_t)tn.count * (uint32_t)sizeof(AtomD);
+        mbar_arrive_expect_tx(&full_bar[st], bytes);
+        bulk_copy_g2s(&ring[st][0], atomsd + tn.atom_begin, bytes, &full_bar[st]);
+        ++g_issue;
+      }
+      ++g_cons;
+    }
+    // item done: the warps' sums of each node added, one write per node (a plain
+    // store when the item covers every atom tile of the molecule)
+    const bool whole = k0 == 0 && k1 == pt.n_tiles;
+#pragma unroll
+    for (int r = 0; r < P / WARPS; ++r) {
+      const int i = warp * (P / WARPS) + r;
+      const long long p = pix0 + 128 * (i / 4) + i % 4;
+      double2 v = sacc[i * NODE_THREADS + lane];
+#pragma unroll
+      for (int w = 1; w < WARPS; ++w) {
+        const double2 u = sacc[i * NODE_THREADS + 32 * w + lane];
+        v.x += u.x;
+        v.y += u.y;
+      }
+      if (p < npix) {
+        if (whole) {
+          pt.acc[p] = v;
+        } else {
+          atomicAdd(&pt.acc[p].x, v.x);
+          atomicAdd(&pt.acc[p].y, v.y);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+cudaError_t launch_sf_nodes(bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items, int *queue,
+                            int *err, int grid, cudaStream_t st) {
+  if (perb)
+    fixw ? sf_dquad_nodes_kernel<true, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err)
+         : sf_dquad_nodes_kernel<true, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err);
+  else
+    fixw ? sf_dquad_nodes_kernel<false, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err)
+         : sf_dquad_nodes_kernel<false, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err);
+  return cudaGetLastError();
+}
+
+int sf_nodes_occupancy(bool perb, bool fixw) {
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &n, perb ? (fixw ? sf_dquad_nodes_kernel<true, true> : sf_dquad_nodes_kernel<true, false>)
+               : (fixw ? sf_dquad_nodes_kernel<false, true> : sf_dquad_nodes_kernel<false, false>),
+      NODE_THREADS, 0);
+  return n;
+}
+
+}  // namespace spsim

@@ -1,0 +1,163 @@
+"""Forwards on coarse grids of nodes against the FP64 oracle, at the FP32
+tolerance of the sum on every pixel (floored maximum relative |F|^2 error 1e-5,
+L2 1e-6; tests/test_gpu_sf.py): tile edges of the interpolation's 8 x 8
+fragments, detectors off the beam axis, wide and spherical ones, every weight
+and B factor, and the calls that must not take the grids."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import intensity_errors
+from oracle import oracle as O
+from spsim_b200 import core, synth
+
+pytestmark = pytest.mark.gpu
+
+TOL = (1e-5, 1e-6)
+
+
+def _det(nx, ny, pixel=150e-6, distance=0.2, wavelength=0.2e-9, **kw):
+    return dict(nx=nx, ny=ny, width=nx * pixel, height=ny * pixel, distance=distance, wavelength=wavelength, **kw)
+
+
+def _q(d):
+    return O.hkl_detector(d["nx"], d["ny"], d["width"], d["height"], d["distance"], d["wavelength"],
+                          center_x=d.get("center_x", 0.0), center_y=d.get("center_y", 0.0),
+                          spherical=d.get("spherical", False))
+
+
+def _check(F, I, Z, pos, q, **kw):
+    F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q, **kw)
+    e_max, e_l2 = intensity_errors(I.cpu().numpy(), I64)
+    assert e_max < TOL[0] and e_l2 < TOL[1], (e_max, e_l2)
+    if F is not None:
+        assert np.abs(F.cpu().numpy() - F64).max() < 1e-5 * np.abs(F64).max()
+
+
+def _on_grid(yes=True):
+    terms = core.last_forward_stats()[0]
+    assert (core.last_terms_evaluated() < terms) == yes
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 250), (127, 130), (129, 95), (200, 61), (257, 256), (1000, 17)])
+@pytest.mark.parametrize("precision", ["f32", "f32_fast"])
+def test_ragged_detectors(cuda, nx, ny, precision):
+    Z, pos = synth.random_molecule(3000, 3.0e-9, 201)
+    pos += np.float32(5e-9)  # a centre phase
+    d = _det(nx, ny)
+    R = synth.haar_rotations(1, 202)[0]
+    F, I = core.forward(core.Molecule(Z, pos), core.QSet.from_detector(**d), rot=R, B=7.5, precision=precision)
+    _on_grid()
+    _check(F, I, Z, pos, _q(d) @ R.T, B=7.5)
+
+
+@pytest.mark.parametrize("kw", [dict(center_x=0.012), dict(spherical=True), dict(distance=0.012),
+                                dict(wavelength=0.06e-9), dict(pixel=2e-3, distance=0.5)],
+                         ids=["off_axis", "spherical", "wide_angle", "hard_x_rays", "large_pixels"])
+def test_geometries(cuda, kw):
+    # wide_angle: pixels to 0.9 detector distances off the axis, form factors
+    # falling over their whole range; hard_x_rays: phases up to ~0.1 cycle per pixel
+    Z, pos = synth.random_molecule(2500, 2.8e-9, 203)
+    d = _det(144, 140, **kw)
+    F, I = core.forward(core.Molecule(Z, pos), core.QSet.from_detector(**d))
+    _on_grid()
+    _check(F, I, Z, pos, _q(d))
+
+
+def test_panel_off_the_beam_axis(cuda):
+    # no bright pixels near the beam: the FP32 terms' own noise reaches 1.5e-5 of
+    # the dimmest intensities with the sum on every pixel, which bounds the grid's
+    Z, pos = synth.random_molecule(2500, 2.8e-9, 203)
+    d = _det(144, 140, center_x=-0.05, center_y=0.03)
+    q, qs, mol = _q(d), core.QSet.from_detector(**d), core.Molecule(Z, pos)
+    _, I64 = O.structure_factor(Z, pos.astype(np.float64), q)
+    _, I = core.forward(mol, qs)
+    _on_grid()
+    try:
+        core.set_variant(128, 8, 4)
+        _, Ip = core.forward(mol, qs)
+        _on_grid(False)
+    finally:
+        core.set_variant(-1)
+    got, bound = (intensity_errors(v.cpu().numpy(), I64) for v in (I, Ip))
+    assert got[0] <= max(TOL[0], bound[0]) and got[1] <= max(TOL[1], bound[1]), (got, bound)
+
+
+def test_weights_and_b_factors(cuda):
+    Z, pos = synth.random_molecule(2000, 2.5e-9, 204)
+    Z[::7] = 0
+    Z[::11] = 19  # potassium: the widest form factor of common elements
+    rng = np.random.Generator(np.random.PCG64(205))
+    occ = rng.uniform(-0.5, 1.0, len(Z)).astype(np.float32)
+    b = rng.uniform(0.0, 60.0, len(Z)).astype(np.float32)
+    d = _det(130, 140, distance=0.05)
+    q, qs = _q(d), core.QSet.from_detector(**d)
+    for occ_, b_, B in ((occ, None, 0.0), (occ, b, 0.0), (None, b, 12.0)):
+        F, I = core.forward(core.Molecule(Z, pos, occ=occ_, bfac=b_), qs, B=B)
+        _on_grid()
+        _check(F, I, Z, pos, q, occ=occ_, bfac=b_, B=B)
+
+
+def test_b_factors_rewritten_beyond_the_grids_limit(cuda):
+    # the limit is 2 * 20 + 100 = 140 A^2: on either side of it, and back, in a
+    # batch of orientations with a molecule that stays within it
+    Z, pos = synth.random_molecule(1500, 2.5e-9, 206)
+    rng = np.random.Generator(np.random.PCG64(207))
+    b0 = rng.uniform(0.0, 20.0, len(Z)).astype(np.float32)
+    b0[0] = 20.0
+    d = _det(128, 120, distance=0.03)
+    q, qs = _q(d), core.QSet.from_detector(**d)
+    mol, other = core.Molecule(Z, pos, bfac=b0), core.Molecule(Z, pos, bfac=b0)
+    R = synth.haar_rotations(2, 208)
+    p = torch.from_numpy(pos).cuda()
+    for top in (100.0, 3000.0, 139.0):
+        b = b0.copy()
+        b[5:400:9] = top
+        mol.update_device(p, bfac=torch.from_numpy(b).cuda())
+        F, I = core.forward_batch([other, mol], [qs, qs], rots=R)
+        _on_grid()
+        for k, bk in enumerate((b0, b)):
+            _check(F[k], I[k], Z, pos, q @ R[k].T, bfac=bk)
+
+
+def test_general_matrices_and_spectrum(cuda):
+    Z, pos = synth.random_molecule(2500, 2.6e-9, 209)
+    d = _det(132, 136)
+    q, qs, mol = _q(d), core.QSet.from_detector(**d), core.Molecule(Z, pos)
+    R = synth.haar_rotations(1, 210)[0] @ np.diag([1.0, 1.3, 0.8])  # not a rotation: it stretches q
+    F, I = core.forward(mol, qs, rot=R)
+    _on_grid()
+    # the oracle takes form factors at |R q|, the library's at |q|: point atoms compare the sum
+    point = core.Molecule(Z, pos, delta_atoms=True)
+    F, I = core.forward(point, qs, rot=R)
+    _on_grid()
+    u = q @ R.T
+    F64 = np.exp(-2j * np.pi * (u @ pos.astype(np.float64).T)).sum(1)
+    e_max, e_l2 = intensity_errors(I.cpu().numpy(), np.abs(F64) ** 2)
+    assert e_max < TOL[0] and e_l2 < TOL[1], (e_max, e_l2)
+    F, I = core.forward_spectrum(mol, qs, d["wavelength"], 0.1, 4)
+    _on_grid()
+    _, I64 = O.structure_factor_spectrum(Z, pos.astype(np.float64), q, d["wavelength"], 0.1, 4)
+    e_max, e_l2 = intensity_errors(I.cpu().numpy(), I64)
+    assert e_max < TOL[0] and e_l2 < TOL[1], (e_max, e_l2)
+
+
+def test_calls_that_stay_on_every_pixel(cuda):
+    Z, pos = synth.random_molecule(4000, 3.0e-9, 211)
+    mol = core.Molecule(Z, pos)
+    d = _det(128, 128)
+    qs = core.QSet.from_detector(**d)
+    cases = [(qs, "fp64"), (core.QSet.from_list(qs.q()), "f32"), (core.QSet.from_detector(**_det(15, 2000)), "f32"),
+             (core.QSet.from_detector(**_det(128, 128, pixel=1e-3, distance=0.05)), "f32"),  # 64 mm at 50 mm
+             (core.QSet.from_detector(**_det(128, 128, wavelength=0.01e-9)), "f32")]  # undersampled
+    for q, precision in cases:
+        F, I = core.forward(mol, q, precision=precision)
+        _on_grid(False)
+        _, I64 = O.structure_factor(Z, pos.astype(np.float64), q.q().astype(np.float64))
+        assert np.abs(I.cpu().numpy() - I64).max() < 1e-4 * I64.max()
+    # a batch with one such pattern runs on every pixel as a whole
+    core.forward_batch([mol, mol], [qs, cases[2][0]])
+    _on_grid(False)
+    # no atoms: zeros
+    _, I = core.forward(core.Molecule(np.zeros(5, np.int32), pos[:5]), qs)
+    assert not I.any()
