@@ -117,7 +117,9 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
  * the others; form factors and per-atom B factors belong to the interpolated
  * sum, the global B factor and the centre phase are applied per pixel.  This
  * is done where it is faster (patterns of more than about 1e7 terms), for
- * whole batches or not at all; q lists, FP64, forced variants
+ * whole batches or not at all, and in FP64 for molecules rewritten on the
+ * device (refinements: a node's rounding error would enter the pixels around it
+ * alike and add up in a gradient); q lists, FP64, forced variants
  * (spsim_b200_set_variant), detectors further than 1.2 detector distances off
  * the beam axis and per-atom B factors beyond twice their largest at creation
  * + 100 A^2 (checked on the device when they are rewritten there) take the
@@ -250,7 +252,9 @@ int spsim_b200_structure_factor_host_noalloc(int natoms, const int32_t *Z, const
  * atoms x pixels is stored.  The outputs are overwritten.  The form-factor
  * table, atom blocks and work items of a (molecule, q set, pattern count, B,
  * precision) are built on the first call and reused by the next ones, which
- * allocate nothing; calls that share such a plan run in call order, whatever
+ * allocate nothing.  Where the forward's coarse grids serve (see the structure
+ * factor above), dL/dI F is taken to the nodes by the transposed interpolation
+ * and the sum runs there in FP64; calls that share such a plan run in call order, whatever
  * their streams. */
 int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200_qset *qs, int npat,
                        const double *rot, float B, int precision, const float *F_dev, const float *G_dev,

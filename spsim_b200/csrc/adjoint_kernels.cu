@@ -43,6 +43,14 @@ __device__ __forceinline__ void adj_pixel(const AdjParams &prm, int elem, long l
     q[1] = b;
     q[2] = c;
   }
+  s2 = (q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) * 1e-20 * 0.25;
+  const double f = prm.ff[(long long)elem * prm.npix + p];
+  if (prm.H) {  // a coarse grid's node
+    const double2 h = prm.H[gp];
+    hr = f * h.x;
+    hi = f * h.y;
+    return;
+  }
   // centred amplitude A = e^{+2 pi i q.c} F
   double t = q[0] * prm.cx + q[1] * prm.cy + q[2] * prm.cz;
   t -= rint(t);
@@ -51,10 +59,9 @@ __device__ __forceinline__ void adj_pixel(const AdjParams &prm, int elem, long l
   const float2 F = prm.F[gp];
   const double ar = F.x * cs - F.y * sn;
   const double ai = F.x * sn + F.y * cs;
-  const double h = (double)prm.G[gp] * prm.ff[(long long)elem * prm.npix + p];
+  const double h = (double)prm.G[gp] * f;
   hr = h * ar;
   hi = h * ai;
-  s2 = (q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) * 1e-20 * 0.25;
 }
 
 template <int MODE>
@@ -91,6 +98,7 @@ __device__ __forceinline__ void adj_sincos(const float4 a0, const float4 a1, con
 
 template <int MODE, int NT, int A, bool PERB>
 __global__ void __launch_bounds__(NT) adj_kernel(AdjParams prm) {
+  if (prm.gate && (*prm.gate != 0) != (prm.gate_set != 0)) return;
   __shared__ __align__(16) float4 pix[ADJ_PIX_TILE * 4];
   const int tid = threadIdx.x;
   const AdjItem item = prm.items[blockIdx.x];
@@ -205,6 +213,7 @@ __global__ void __launch_bounds__(NT) adj_kernel(AdjParams prm) {
 template <int NT, int A, bool PERB, bool FIXW>
 __global__ void __launch_bounds__(NT) adj_dphase_kernel(AdjParams prm, uint32_t m31) {
   static_assert(A % 2 == 0, "atoms per thread must be even");
+  if (prm.gate && (*prm.gate != 0) != (prm.gate_set != 0)) return;
   constexpr int NP = A / 2;
   // pixel records of the block's (at most two) elements
   __shared__ __align__(16) double2 pq_all[2][ADJ_PIX_TILE * 2];
@@ -389,6 +398,111 @@ __global__ void __launch_bounds__(NT) adj_dphase_kernel(AdjParams prm, uint32_t 
   }
 }
 
+// The adjoint on a coarse grid's nodes, FP64 throughout: blocks and phases as adj_dphase_kernel's, H = |H| e^{i phi}
+// entering as phi / 2 pi in the phase sum, so that the polynomials' cos / sin are
+// the products with H.  The nodes are a few per cent of the pixels, each stands
+// for many, and a loss's gradient is what is left of terms that mostly cancel:
+// with FP32 sin / cos and sums it had up to 2.5 times the error of the sum on
+// every pixel.  26 FP64 operations per term bind it (5,000 atoms x 8 x 841
+// nodes).
+//   pq[2i] = {qx, qy}  pq[2i+1] = {qz, phi / 2 pi}
+//   pm[2i] = {|H| qx, |H| qy}  pm[2i+1] = {|H| qz, |H|}  ps[i] = {|H| s2, s2n}
+constexpr int ADJ_NODE_TILE = 128;
+
+template <int NT, int A, bool PERB>
+__global__ void __launch_bounds__(NT) adj_nodes_kernel(AdjParams prm) {
+  if (prm.gate && (*prm.gate != 0) != (prm.gate_set != 0)) return;
+  __shared__ __align__(16) double2 pq_all[2][ADJ_NODE_TILE * 2], pm_all[2][ADJ_NODE_TILE * 2], ps_all[2][ADJ_NODE_TILE];
+  const int tid = threadIdx.x;
+  const AdjItem item = prm.items[blockIdx.x];
+  const AdjBlock blk = prm.blocks[item.block];
+  const double M52 = 6755399441055744.0;  // 1.5 * 2^52
+  const int a_first = blk.atom_begin + A * tid;
+  const int slot = (blk.elem2 >= 0 && a_first >= blk.split) ? 1 : 0;
+  const int nslot = blk.elem2 >= 0 ? 2 : 1;
+  const double2 *__restrict__ pq = pq_all[slot];
+  const double2 *__restrict__ pm = pm_all[slot];
+  const double2 *__restrict__ ps = ps_all[slot];
+
+  double rx[A], ry[A], rz[A], gx[A], gy[A], gz[A], go[A], gb[A];
+  double bfac[A];
+#pragma unroll
+  for (int k = 0; k < A; ++k) {
+    rx[k] = ry[k] = rz[k] = gx[k] = gy[k] = gz[k] = go[k] = gb[k] = 0.0;
+    bfac[k] = 0.0;
+    if (a_first + k < blk.atom_end) {
+      const AtomD a = prm.atomsd[a_first + k];
+      rx[k] = a.x;
+      ry[k] = a.y;
+      rz[k] = a.z;
+      bfac[k] = a.b;
+    }
+  }
+  for (long long base = item.pix_begin; base < item.pix_end; base += ADJ_NODE_TILE) {
+    const int n = (int)min((long long)ADJ_NODE_TILE, item.pix_end - base);
+    __syncthreads();
+    for (int c = tid; c < ADJ_NODE_TILE * nslot; c += NT) {
+      const int i = c % ADJ_NODE_TILE, sl = c / ADJ_NODE_TILE;
+      if (i >= n) continue;
+      double q[3], hr, hi, s2;
+      adj_pixel(prm, sl ? blk.elem2 : blk.elem, base + i, q, hr, hi, s2);
+      const double mag = hypot(hr, hi);
+      const double phi = mag > 0.0 ? atan2(hi, hr) : 0.0;
+      pq_all[sl][2 * i] = make_double2(q[0], q[1]);
+      pq_all[sl][2 * i + 1] = make_double2(q[2], phi * 0.15915494309189535);
+      pm_all[sl][2 * i] = make_double2(mag * q[0], mag * q[1]);
+      pm_all[sl][2 * i + 1] = make_double2(mag * q[2], mag);
+      ps_all[sl][i] = make_double2(mag * s2, -s2 * 1.4426950408889634);
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int i = 0; i < n; ++i) {
+      const double2 qa = pq[2 * i], qb = pq[2 * i + 1], ma = pm[2 * i], mb = pm[2 * i + 1], sv = ps[i];
+#pragma unroll
+      for (int k = 0; k < A; ++k) {
+        double u = fma(qa.x, rx[k], qb.y);
+        u = fma(qa.y, ry[k], u);
+        u = fma(qb.x, rz[k], u);
+        const double t = fma(u, 2.0, M52);  // rint(2u) in the low bits
+        const double y = fma(t - M52, -0.5, u);
+        double w = PERB ? exp2_poly(bfac[k] * sv.y) : 1.0;
+        w = __hiloint2double(__double2hiint(w) ^ (__double2loint(t) << 31), __double2loint(w));
+        const double z = y * y;
+        double sp = fma(z, SPSIM_NODE64_S5, SPSIM_NODE64_S4);
+        double cp = fma(z, SPSIM_NODE64_C6, SPSIM_NODE64_C5);
+        sp = fma(z, sp, SPSIM_NODE64_S3);
+        cp = fma(z, cp, SPSIM_NODE64_C4);
+        sp = fma(z, sp, SPSIM_NODE64_S2);
+        cp = fma(z, cp, SPSIM_NODE64_C3);
+        sp = fma(z, sp, SPSIM_NODE64_S1);
+        cp = fma(z, cp, SPSIM_NODE64_C2);
+        sp = fma(z, sp, SPSIM_NODE64_S0);
+        cp = fma(z, cp, SPSIM_NODE64_C1);
+        cp = fma(z, cp, SPSIM_NODE64_C0);
+        const double zr = w * cp, zn = w * y * sp;  // zn = -Im
+        gx[k] = fma(-zn, ma.x, gx[k]);
+        gy[k] = fma(-zn, ma.y, gy[k]);
+        gz[k] = fma(-zn, mb.x, gz[k]);
+        go[k] = fma(zr, mb.y, go[k]);
+        gb[k] = fma(zr, sv.x, gb[k]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < A; ++k) {
+    if (a_first + k >= blk.atom_end) continue;
+    const int src = prm.perm[a_first + k];
+    if (src < 0) continue;
+    const double w = prm.atomsd[a_first + k].w, wb = prm.wbase[a_first + k];
+    const double kp = 4.0 * 3.14159265358979323846 * w;
+    atomicAdd(&prm.dpos[3 * src], kp * gx[k]);
+    atomicAdd(&prm.dpos[3 * src + 1], kp * gy[k]);
+    atomicAdd(&prm.dpos[3 * src + 2], kp * gz[k]);
+    if (prm.docc) atomicAdd(&prm.docc[src], 2.0 * wb * go[k]);
+    if (prm.dB) atomicAdd(&prm.dB[src], -2.0 * w * gb[k]);
+  }
+}
+
 // plain FP64 adjoint: same decomposition, FP64 phase and sincos
 template <int NT>
 __global__ void __launch_bounds__(NT) adj_f64_kernel(AdjParams prm) {
@@ -460,7 +574,12 @@ __global__ void __launch_bounds__(NT) adj_f64_kernel(AdjParams prm) {
 
 int adjoint_occupancy(int precision_mode, bool perb) {
   int n = 0;
-  if (precision_mode == 2)
+  if (precision_mode == ADJ_MODE_NODES)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &n, perb ? adj_nodes_kernel<ADJ_THREADS, ADJ_NODES_ATOMS_PER_THREAD, true>
+                 : adj_nodes_kernel<ADJ_THREADS, ADJ_NODES_ATOMS_PER_THREAD, false>,
+        ADJ_THREADS, 0);
+  else if (precision_mode == 2)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adj_f64_kernel<ADJ_THREADS>, ADJ_THREADS, 0);
   else if (precision_mode == 3 || precision_mode == 4) {
     const bool fw = precision_mode == 4;
@@ -488,7 +607,12 @@ int adjoint_occupancy(int precision_mode, bool perb) {
 
 cudaError_t launch_adjoint(int precision_mode, const AdjParams &prm, int n_items, cudaStream_t st) {
   if (n_items <= 0) return cudaSuccess;
-  if (precision_mode == 2) {
+  if (precision_mode == ADJ_MODE_NODES) {
+    if (prm.per_atom_b)
+      adj_nodes_kernel<ADJ_THREADS, ADJ_NODES_ATOMS_PER_THREAD, true><<<n_items, ADJ_THREADS, 0, st>>>(prm);
+    else
+      adj_nodes_kernel<ADJ_THREADS, ADJ_NODES_ATOMS_PER_THREAD, false><<<n_items, ADJ_THREADS, 0, st>>>(prm);
+  } else if (precision_mode == 2) {
     adj_f64_kernel<ADJ_THREADS><<<n_items, ADJ_THREADS, 0, st>>>(prm);
   } else if (precision_mode == 3) {
     if (prm.per_atom_b)

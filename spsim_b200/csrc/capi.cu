@@ -222,6 +222,7 @@ struct spsim_b200_molecule {
   float dr = 1, inv_dr = 1;
   int per_atom_b = 0, delta_atoms = 0;
   float b_limit = 0;        // largest |per-atom B| the coarse grids are sized for
+  bool updated = false;     // atoms rewritten on the device
   bool b_updated = false;   // B factors rewritten on the device: b_limit is checked there (d_flags[1])
   // device views of the buffers below
   float4 *d_atoms = nullptr;
@@ -453,6 +454,7 @@ extern "C" int spsim_b200_molecule_update_device(spsim_b200_molecule *m, const v
     return fail(SPSIM_ERR_INVALID_ARG, "molecule was created without per-atom B factors");
   // the range word of this update, and the B factors' where they are rewritten
   CUDA_TRY(cudaMemsetAsync(m->d_flags, 0, (bfac_dev ? 2 : 1) * sizeof(int), (cudaStream_t)stream));
+  m->updated = true;
   if (bfac_dev) m->b_updated = true;
   CUDA_TRY(launch_atoms_update(m->d_atoms, m->d_atoms2, m->d_atomsd, m->d_perm, m->n_padded, pos_is_f64 ? nullptr : (const float *)pos_dev,
                                pos_is_f64 ? (const double *)pos_dev : nullptr, occ_dev, bfac_dev, m->d_wbase,
@@ -674,6 +676,7 @@ struct Plan {
   double terms = 0, evaluated = 0;  // atom.pixel terms of the patterns, and those evaluated (on nodes: fewer)
   int precision = 0, nt = 128, ppt = 4, packed = 1;
   int mode = PREC_MODE_POLY;
+  int node_tile = 0;  // coarse grids: nodes per work item, which selects the kernel (launch_sf_nodes)
   bool perb = false;
   bool fixw = false;  // FP64-phase forms: fixed-point phase word (every pattern within 2^17 cycles)
   bool narrow = false;  // neighbour pairs: every step within 0.07 cycle (the NARROW second-pixel polynomial)
@@ -985,7 +988,14 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   pl.nt = var.nt;
   pl.ppt = var.p;
   pl.packed = var.packed;
-  const long long tile_pix = pl.coarse ? SF_NODES_TILE : (long long)nt * ppt;
+  if (pl.coarse) {
+    // the FP64 kernel (sf_nodes.cu) for molecules rewritten on the device and for
+    // grids that latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
+    bool updated = false;
+    for (int i = 0; i < npat; ++i) updated = updated || mols[i]->updated;
+    pl.node_tile = pl.evaluated <= 4e6 ? SF_NODES64_SMALL_TILE : updated ? SF_NODES64_TILE : SF_NODES_TILE;
+  }
+  const long long tile_pix = pl.coarse ? pl.node_tile : (long long)nt * ppt;
 
   pl.max_npix = 0;
   pl.npix_of.resize(npat);
@@ -1126,7 +1136,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 
   if (precision != SPSIM_PREC_FP64) {
     // work items: pixel tile x atom-tile range, cost-sorted (largest first)
-    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(perb, pl.fixw)
+    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw)
                                           : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
     const long long slots = (long long)num_sms() * occ;
     long long total_ptiles = 0;
@@ -1219,8 +1229,8 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   } else if (pl.n_items > 0) {
     int *flags = (int *)pl.flags.p;
     if (pl.coarse)
-      e = launch_sf_nodes(pl.perb, pl.fixw, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p, pl.n_items, flags,
-                          flags + 4, pl.grid, stream);
+      e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
+                          pl.n_items, flags, flags + 4, pl.grid, stream);
     else
       e = launch_sf_f32(pl.mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
                         pl.n_items, flags, flags + 4, pl.grid, stream, pl.fixw, pl.narrow);
@@ -1262,7 +1272,7 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
   for (int i = 0; i < npat; ++i) {
     kv.push_back((double)(mols[i] ? mols[i]->id : 0));
     kv.push_back((double)(qsets[i] ? qsets[i]->id : 0));
-    kv.push_back(mols[i] && mols[i]->b_updated ? 1.0 : 0.0);
+    kv.push_back(mols[i] ? (mols[i]->updated ? 1.0 : 0.0) + (mols[i]->b_updated ? 2.0 : 0.0) : 0.0);
     kp.push_back(F_dev ? (const void *)F_dev[i] : nullptr);
     kp.push_back(I_dev ? (const void *)I_dev[i] : nullptr);
   }
@@ -2753,8 +2763,16 @@ struct AdjPlan {
   unsigned long long mol_id = 0, qs_id = 0;
   int npat = 0, mode = 0, device = 0;
   float B = 0;
+  double stretch = 1.0;  // of |q| under matrices that are not rotations
   int n_items = 0;
+  long long points = 0;  // per pattern: nodes of a coarse grid, or pixels
   DevBuf ff, blocks, items, rot;
+  // coarse grids: the sum runs on the nodes, from the pixels' dL/d|F|^2 and
+  // amplitudes taken to them by the transposed interpolation
+  bool coarse = false;
+  CoarseGrid grid;
+  int group = 1;  // patterns at a time
+  DevBuf tables, H, strip, nodes;
   std::vector<double> host_rot;  // the rotations as last uploaded
   // recorded after each call's launch: the next call, on whatever stream,
   // waits for it before it rewrites the rotations the last launch reads
@@ -2770,6 +2788,209 @@ static void adjoint_release(int dev) {
   std::lock_guard<std::mutex> lk(g_mu);
   for (size_t i = g_adj_plans.size(); i-- > 0;)
     if (g_adj_plans[i]->device == dev) g_adj_plans.erase(g_adj_plans.begin() + i);
+}
+
+// Offsets (doubles) of an adjoint plan's tables: node q, the interpolation
+// matrices and their transposes.
+struct AdjTables {
+  size_t mx, my, tx, ty, total;
+  AdjTables(const DetGeom &g, const CoarseGrid &c) {
+    const size_t nx = c.x.n, ny = c.y.n;
+    mx = (3 * nx * ny + 1) / 2 * 2;
+    my = mx + (size_t)g.nx * coarse_ld(c.x.n);
+    tx = my + (size_t)g.ny * coarse_ld(c.y.n);
+    ty = tx + nx * coarse_ld(g.nx);
+    total = ty + ny * coarse_ld(g.ny);
+  }
+};
+
+// The plan of one adjoint in kernel mode `mode` (launch_adjoint), on the nodes
+// of a coarse grid or on every pixel; *out stays owned by the cache.
+static int adjoint_plan(const spsim_b200_molecule *m, const spsim_b200_qset *qs, int npat, float B, int mode, int dev,
+                        double stretch, const CoarseGrid *grid, cudaStream_t st, AdjPlan **out) {
+  for (size_t i = 0; i < g_adj_plans.size(); ++i) {
+    AdjPlan &c = *g_adj_plans[i];
+    if (c.mol_id == m->id && c.qs_id == qs->id && c.npat == npat && c.B == B && c.mode == mode && c.device == dev &&
+        c.coarse == (grid != nullptr) && c.stretch == stretch) {
+      std::unique_ptr<AdjPlan> keep = std::move(g_adj_plans[i]);
+      g_adj_plans.erase(g_adj_plans.begin() + i);
+      g_adj_plans.push_back(std::move(keep));
+      *out = g_adj_plans.back().get();
+      return SPSIM_OK;
+    }
+  }
+  std::unique_ptr<AdjPlan> np(new AdjPlan());
+  np->mol_id = m->id;
+  np->qs_id = qs->id;
+  np->npat = npat;
+  np->B = B;
+  np->mode = mode;
+  np->device = dev;
+  np->stretch = stretch;
+  np->coarse = grid != nullptr;
+  np->points = qs->npix;
+  if (grid) {
+    np->grid = *grid;
+    np->points = (long long)grid->x.n * grid->y.n;
+  }
+  const bool dphase = mode >= 3;
+  // atom blocks x pixel chunks.  The FP64-phase adjoint's blocks are
+  // consecutive runs of the element-sorted atoms that may span two element
+  // segments (each thread's atoms stay in one), so short segments do not leave
+  // blocks mostly empty; the other adjoints take one element per block.
+  const int block_atoms = mode == ADJ_MODE_NODES ? ADJ_NODES_BLOCK_ATOMS
+                          : mode == 2            ? ADJ_THREADS
+                                                 : (dphase ? ADJ_DPHASE_BLOCK_ATOMS : ADJ_BLOCK_ATOMS);
+  std::vector<AdjBlock> blocks;
+  {
+    struct Seg {
+      int elem, begin, end;
+    };
+    std::vector<Seg> segs;
+    int e = -1, seg0 = 0;
+    for (size_t k = 0; k <= m->tiles.size(); ++k) {
+      const bool end = k == m->tiles.size();
+      if (end || m->tiles[k].elem != e) {
+        if (e >= 0) segs.push_back({e, seg0, m->tiles[k - 1].atom_begin + m->tiles[k - 1].count});
+        if (!end) {
+          e = m->tiles[k].elem;
+          seg0 = m->tiles[k].atom_begin;
+        }
+      }
+    }
+    if (dphase) {
+      size_t s0 = 0;
+      int a = segs.empty() ? 0 : segs[0].begin;
+      while (s0 < segs.size()) {
+        AdjBlock b = {a, std::min(a + block_atoms, segs[s0].end), segs[s0].elem, -1, 0, 0};
+        b.split = b.atom_end;
+        if (b.atom_end == segs[s0].end && b.atom_end - a < block_atoms && s0 + 1 < segs.size()) {
+          // fill the rest of the block from the next segment (segments are contiguous)
+          b.elem2 = segs[s0 + 1].elem;
+          b.split = segs[s0 + 1].begin;
+          b.atom_end = std::min(a + block_atoms, segs[s0 + 1].end);
+        }
+        blocks.push_back(b);
+        a = b.atom_end;
+        while (s0 < segs.size() && a >= segs[s0].end) ++s0;
+      }
+    } else {
+      for (const Seg &sg : segs)
+        for (int a = sg.begin; a < sg.end; a += block_atoms)
+          blocks.push_back({a, std::min(a + block_atoms, sg.end), sg.elem, -1, std::min(a + block_atoms, sg.end), 0});
+    }
+  }
+  // pixel chunks per block so that the equal-cost CTAs fill at most four whole
+  // waves of the resident slots (a last wave of a few CTAs would leave the GPU
+  // idle for one item's length: 1,190 CTAs on 592 slots ran as three waves)
+  const long long total = np->points * npat;
+  const long long slots = (long long)num_sms() * std::max(1, adjoint_occupancy(mode, m->per_atom_b != 0));
+  long long nchunk = std::max<long long>(1, 4 * slots / (long long)blocks.size());
+  long long chunk = (total + nchunk - 1) / nchunk;
+  const long long unit = mode == ADJ_MODE_NODES ? 128 : 256;  // points per shared-memory tile
+  chunk = (chunk + unit - 1) / unit * unit;
+  std::vector<AdjItem> items;
+  for (size_t b = 0; b < blocks.size(); ++b)
+    for (long long p0 = 0; p0 < total; p0 += chunk) items.push_back({(int)b, 0, p0, std::min(total, p0 + chunk)});
+  np->n_items = (int)items.size();
+  CUDA_TRY(np->ff.ensure(std::max<size_t>((size_t)m->n_elem * np->points, 1) * sizeof(double)));
+  CUDA_TRY(np->blocks.ensure(blocks.size() * sizeof(AdjBlock)));
+  CUDA_TRY(np->items.ensure(items.size() * sizeof(AdjItem)));
+  CUDA_TRY(np->rot.ensure(9 * (size_t)npat * sizeof(double)));
+  CUDA_TRY(cudaMemcpyAsync(np->blocks.p, blocks.data(), blocks.size() * sizeof(AdjBlock), cudaMemcpyHostToDevice, st));
+  CUDA_TRY(cudaMemcpyAsync(np->items.p, items.data(), items.size() * sizeof(AdjItem), cudaMemcpyHostToDevice, st));
+  if (grid) {
+    const int nx = qs->geom.nx, ny = qs->geom.ny, nxn = grid->x.n, nyn = grid->y.n;
+    AdjTables t(qs->geom, *grid);
+    CUDA_TRY(np->tables.ensure(t.total * sizeof(double)));
+    double *tab = (double *)np->tables.p;
+    CUDA_TRY(launch_coarse_tables(qs->geom, grid->x, grid->y, tab, tab + t.mx, tab + t.my, st, tab + t.tx, tab + t.ty));
+    // 64 MB of pixels at a time: they are read back from L2
+    np->group = (int)std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / qs->npix));
+    np->group = std::min(np->group, 65535);
+    CUDA_TRY(np->H.ensure((size_t)np->group * nx * ny * sizeof(double2)));
+    CUDA_TRY(np->strip.ensure((size_t)np->group * nxn * ny * sizeof(double2)));
+    CUDA_TRY(np->nodes.ensure((size_t)total * sizeof(double2)));
+    CUDA_TRY(launch_ff_table(nullptr, tab, np->points, m->n_elem, m->d_coeffs, 0.0, m->delta_atoms, (double *)np->ff.p,
+                             st));
+  } else {
+    CUDA_TRY(launch_ff_table(qs->d_hkl, qs->d_q64, qs->npix, m->n_elem, m->d_coeffs, (double)B, m->delta_atoms,
+                             (double *)np->ff.p, st));
+  }
+  CUDA_TRY(cudaEventCreateWithFlags(&np->done, cudaEventDisableTiming));
+  CUDA_TRY(cudaEventRecord(np->done, st));
+  if (g_adj_plans.size() >= kMaxAdjPlans) {
+    cudaDeviceSynchronize();  // the evicted plan's buffers may still be in use
+    g_adj_plans.erase(g_adj_plans.begin());
+  }
+  g_adj_plans.push_back(std::move(np));
+  *out = g_adj_plans.back().get();
+  return SPSIM_OK;
+}
+
+// One adjoint launch on its plan; gate as AdjParams::gate.
+static int adjoint_run(AdjPlan *pl, const spsim_b200_molecule *m, const spsim_b200_qset *qs, const double *rot,
+                       float dq, float inv_dq, const float *F_dev, const float *G_dev, double *dpos_dev,
+                       double *docc_dev, double *dB_dev, const int *gate, int gate_set, cudaStream_t st) {
+  const int npat = pl->npat;
+  CUDA_TRY(cudaStreamWaitEvent(st, pl->done, 0));
+  // this call's rotations, uploaded when they differ from the last call's
+  if (rot && (pl->host_rot.size() != 9 * (size_t)npat ||
+              memcmp(pl->host_rot.data(), rot, 9 * (size_t)npat * sizeof(double)) != 0)) {
+    pl->host_rot.assign(rot, rot + 9 * (size_t)npat);
+    CUDA_TRY(cudaMemcpyAsync(pl->rot.p, pl->host_rot.data(), 9 * (size_t)npat * sizeof(double),
+                             cudaMemcpyHostToDevice, st));
+  }
+  AdjParams prm;
+  memset(&prm, 0, sizeof(prm));
+  prm.atoms = m->d_atoms;
+  prm.atomsd = m->d_atomsd;
+  prm.perm = m->d_perm;
+  prm.wbase = m->d_wbase;
+  prm.blocks = (const AdjBlock *)pl->blocks.p;
+  prm.items = (const AdjItem *)pl->items.p;
+  prm.hkl = pl->coarse ? nullptr : qs->d_hkl;
+  prm.q64 = pl->coarse ? (const double *)pl->tables.p : qs->d_q64;
+  prm.rot = rot ? (const double *)pl->rot.p : nullptr;
+  prm.ff = (const double *)pl->ff.p;
+  prm.F = (const float2 *)F_dev;
+  prm.G = G_dev;
+  prm.npix = pl->points;
+  prm.cx = m->center[0];
+  prm.cy = m->center[1];
+  prm.cz = m->center[2];
+  prm.dq = dq;
+  prm.inv_dq = inv_dq;
+  prm.per_atom_b = m->per_atom_b;
+  prm.dpos = dpos_dev;
+  prm.docc = docc_dev;
+  prm.dB = dB_dev;
+  prm.gate = gate;
+  prm.gate_set = gate_set;
+  if (pl->coarse) {
+    const AdjTables t(qs->geom, pl->grid);
+    const double *tab = (const double *)pl->tables.p;
+    CoarseAdjoint a;
+    a.F = prm.F;
+    a.G = prm.G;
+    a.q64 = qs->d_q64;
+    a.rot = prm.rot;
+    memcpy(a.center, m->center, sizeof(a.center));
+    a.B = pl->B;
+    a.npix = qs->npix;
+    a.nx = qs->geom.nx;
+    a.ny = qs->geom.ny;
+    a.nxn = pl->grid.x.n;
+    a.nyn = pl->grid.y.n;
+    a.tx = tab + t.tx;
+    a.ty = tab + t.ty;
+    CUDA_TRY(launch_coarse_adjoint(a, npat, (double2 *)pl->H.p, pl->group, (double2 *)pl->strip.p,
+                                   (double2 *)pl->nodes.p, st));
+    prm.H = (const double2 *)pl->nodes.p;
+  }
+  CUDA_TRY(launch_adjoint(pl->mode, prm, pl->n_items, st));
+  CUDA_TRY(cudaEventRecord(pl->done, st));
+  return SPSIM_OK;
 }
 
 extern "C" int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200_qset *qs, int npat,
@@ -2813,146 +3034,44 @@ extern "C" int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200
   if (m->n_kept == 0 || total == 0) return SPSIM_OK;
 
   // mode 4: the FP64-phase adjoint with the fixed-point phase word (phases within 2^17 cycles)
-  const bool fixw = dphase && qmax * m->rbound < std::ldexp(1.0, 17);
+  const bool fixw = qmax * m->rbound < std::ldexp(1.0, 17);
   const int mode =
       precision == SPSIM_PREC_FP64 ? 2 : (precision == SPSIM_PREC_F32_FAST ? 1 : (dphase ? (fixw ? 4 : 3) : 0));
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_mu);
-  AdjPlan *pl = nullptr;
-  for (size_t i = 0; i < g_adj_plans.size(); ++i) {
-    AdjPlan &c = *g_adj_plans[i];
-    if (c.mol_id == m->id && c.qs_id == qs->id && c.npat == npat && c.B == B && c.mode == mode &&
-        c.device == dev) {
-      std::unique_ptr<AdjPlan> keep = std::move(g_adj_plans[i]);
-      g_adj_plans.erase(g_adj_plans.begin() + i);
-      g_adj_plans.push_back(std::move(keep));
-      pl = g_adj_plans.back().get();
-      break;
-    }
+  // the sum on a coarse grid's nodes where that is faster than on every pixel
+  // (measured: the adjoint's terms 1.15e12/s on pixels, 5e11/s in FP64 on nodes;
+  // the transposed interpolation 8e12 FP64 multiply-adds/s, its pixels 40 B at
+  // 4 TB/s, its launches ~15 us); both FP32 precisions take the FP64 kernel there
+  const double stretch = qs->qmax > 0 ? qmax / qs->qmax : 1.0;
+  CoarseGrid grid;
+  bool coarse = precision != SPSIM_PREC_FP64 && g_force_nt <= 0 && coarse_fit(m, qs, stretch, stretch, &grid);
+  if (coarse) {
+    const double nxn = grid.x.n, nyn = grid.y.n, pix = (double)npix;
+    const double on_nodes = npat * (m->n_kept * nxn * nyn / 5e11 + 2 * (pix * nxn + nxn * nyn * qs->geom.ny) / 8e12 +
+                                    pix * 40 / 4e12) + 15e-6;
+    coarse = on_nodes < 0.8 * npat * m->n_kept * pix / 1.15e12;
   }
-  if (!pl) {
-    std::unique_ptr<AdjPlan> np(new AdjPlan());
-    np->mol_id = m->id;
-    np->qs_id = qs->id;
-    np->npat = npat;
-    np->B = B;
-    np->mode = mode;
-    np->device = dev;
-    // atom blocks x pixel chunks.  The FP64-phase adjoint's blocks are
-    // consecutive runs of the element-sorted atoms that may span two element
-    // segments (each thread's atoms stay in one), so short segments do not leave
-    // blocks mostly empty; the other adjoints take one element per block.
-    const int block_atoms =
-        precision == SPSIM_PREC_FP64 ? ADJ_THREADS : (dphase ? ADJ_DPHASE_BLOCK_ATOMS : ADJ_BLOCK_ATOMS);
-    std::vector<AdjBlock> blocks;
-    {
-      struct Seg {
-        int elem, begin, end;
-      };
-      std::vector<Seg> segs;
-      int e = -1, seg0 = 0;
-      for (size_t k = 0; k <= m->tiles.size(); ++k) {
-        const bool end = k == m->tiles.size();
-        if (end || m->tiles[k].elem != e) {
-          if (e >= 0) segs.push_back({e, seg0, m->tiles[k - 1].atom_begin + m->tiles[k - 1].count});
-          if (!end) {
-            e = m->tiles[k].elem;
-            seg0 = m->tiles[k].atom_begin;
-          }
-        }
-      }
-      if (dphase) {
-        size_t s0 = 0;
-        int a = segs.empty() ? 0 : segs[0].begin;
-        while (s0 < segs.size()) {
-          AdjBlock b = {a, std::min(a + block_atoms, segs[s0].end), segs[s0].elem, -1, 0, 0};
-          b.split = b.atom_end;
-          if (b.atom_end == segs[s0].end && b.atom_end - a < block_atoms && s0 + 1 < segs.size()) {
-            // fill the rest of the block from the next segment (segments are contiguous)
-            b.elem2 = segs[s0 + 1].elem;
-            b.split = segs[s0 + 1].begin;
-            b.atom_end = std::min(a + block_atoms, segs[s0 + 1].end);
-          }
-          blocks.push_back(b);
-          a = b.atom_end;
-          while (s0 < segs.size() && a >= segs[s0].end) ++s0;
-        }
-      } else {
-        for (const Seg &sg : segs)
-          for (int a = sg.begin; a < sg.end; a += block_atoms)
-            blocks.push_back({a, std::min(a + block_atoms, sg.end), sg.elem, -1, std::min(a + block_atoms, sg.end), 0});
-      }
-    }
-    // pixel chunks per block so that the equal-cost CTAs fill at most four whole
-    // waves of the resident slots (a last wave of a few CTAs would leave the GPU
-    // idle for one item's length: 1,190 CTAs on 592 slots ran as three waves)
-    const long long slots = (long long)num_sms() * std::max(1, adjoint_occupancy(mode, m->per_atom_b != 0));
-    long long nchunk = std::max<long long>(1, 4 * slots / (long long)blocks.size());
-    long long chunk = (total + nchunk - 1) / nchunk;
-    chunk = (chunk + 255) / 256 * 256;
-    std::vector<AdjItem> items;
-    for (size_t b = 0; b < blocks.size(); ++b)
-      for (long long p0 = 0; p0 < total; p0 += chunk) items.push_back({(int)b, 0, p0, std::min(total, p0 + chunk)});
-    np->n_items = (int)items.size();
-    CUDA_TRY(np->ff.ensure(std::max<size_t>((size_t)m->n_elem * npix, 1) * sizeof(double)));
-    CUDA_TRY(np->blocks.ensure(blocks.size() * sizeof(AdjBlock)));
-    CUDA_TRY(np->items.ensure(items.size() * sizeof(AdjItem)));
-    CUDA_TRY(np->rot.ensure(9 * (size_t)npat * sizeof(double)));
-    CUDA_TRY(cudaMemcpyAsync(np->blocks.p, blocks.data(), blocks.size() * sizeof(AdjBlock), cudaMemcpyHostToDevice,
-                             st));
-    CUDA_TRY(cudaMemcpyAsync(np->items.p, items.data(), items.size() * sizeof(AdjItem), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(launch_ff_table(qs->d_hkl, qs->d_q64, npix, m->n_elem, m->d_coeffs, (double)B, m->delta_atoms,
-                             (double *)np->ff.p, st));
-    CUDA_TRY(cudaEventCreateWithFlags(&np->done, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventRecord(np->done, st));
-    if (g_adj_plans.size() >= kMaxAdjPlans) {
-      cudaDeviceSynchronize();  // the evicted plan's buffers may still be in use
-      g_adj_plans.erase(g_adj_plans.begin());
-    }
-    g_adj_plans.push_back(std::move(np));
-    pl = g_adj_plans.back().get();
-  }
-  CUDA_TRY(cudaStreamWaitEvent(st, pl->done, 0));
-  // this call's rotations, uploaded when they differ from the last call's
-  if (rot && (pl->host_rot.size() != 9 * (size_t)npat ||
-              memcmp(pl->host_rot.data(), rot, 9 * (size_t)npat * sizeof(double)) != 0)) {
-    pl->host_rot.assign(rot, rot + 9 * (size_t)npat);
-    CUDA_TRY(cudaMemcpyAsync(pl->rot.p, pl->host_rot.data(), 9 * (size_t)npat * sizeof(double),
-                             cudaMemcpyHostToDevice, st));
-  }
-  AdjParams prm;
-  memset(&prm, 0, sizeof(prm));
-  prm.atoms = m->d_atoms;
-  prm.atomsd = m->d_atomsd;
-  prm.perm = m->d_perm;
-  prm.wbase = m->d_wbase;
-  prm.blocks = (const AdjBlock *)pl->blocks.p;
-  prm.items = (const AdjItem *)pl->items.p;
-  prm.hkl = qs->d_hkl;
-  prm.q64 = qs->d_q64;
-  prm.rot = rot ? (const double *)pl->rot.p : nullptr;
-  prm.ff = (const double *)pl->ff.p;
-  prm.F = (const float2 *)F_dev;
-  prm.G = G_dev;
-  prm.npix = npix;
-  prm.cx = m->center[0];
-  prm.cy = m->center[1];
-  prm.cz = m->center[2];
-  prm.dq = dq;
-  prm.inv_dq = (float)std::ldexp(1.0, kq - eq);
-  prm.per_atom_b = m->per_atom_b;
-  prm.dpos = dpos_dev;
-  prm.docc = docc_dev;
-  prm.dB = dB_dev;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (g_timing) {
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     CUDA_TRY(cudaEventRecord(e0, st));
   }
-  CUDA_TRY(launch_adjoint(mode, prm, pl->n_items, st));
-  CUDA_TRY(cudaEventRecord(pl->done, st));
+  const float inv_dq = (float)std::ldexp(1.0, kq - eq);
+  // B factors rewritten on the device may be beyond the grid's limit: there,
+  // by the device's word, the sum runs on every pixel instead
+  const bool gated = coarse && m->per_atom_b && m->b_updated;
+  for (int on_grid = coarse ? 1 : 0; on_grid >= (coarse && !gated ? 1 : 0); --on_grid) {
+    AdjPlan *pl = nullptr;
+    int status = adjoint_plan(m, qs, npat, B, on_grid ? ADJ_MODE_NODES : mode, dev, stretch, on_grid ? &grid : nullptr, st,
+                              &pl);
+    if (status) return status;
+    status = adjoint_run(pl, m, qs, rot, dq, inv_dq, F_dev, G_dev, dpos_dev, docc_dev, dB_dev,
+                         gated ? m->d_flags + 1 : nullptr, on_grid ? 0 : 1, st);
+    if (status) return status;
+  }
   if (g_timing) {
     CUDA_TRY(cudaEventRecord(e1, st));
     g_timing_events.push_back({e0, e1});

@@ -47,8 +47,8 @@ void coarse_set_nodes(CoarseAxis &a, int n) {
 struct CoarseTables {
   DetGeom g;
   CoarseAxis x, y;
-  int ldx, ldy;
-  double *q64, *mx, *my;
+  int ldx, ldy, ltx, lty;
+  double *q64, *mx, *my, *tx, *ty;
 };
 
 // position on the detector (m) of node k of an axis
@@ -61,7 +61,9 @@ __device__ __forceinline__ double coarse_node_pos(const CoarseAxis &a, int k) {
 // One row (pixel p) of an interpolation matrix by one warp:
 // M[k] = (w_k / (xi - xi_k)) / sum_j w_j / (xi - xi_j), the barycentric weights
 // of the Chebyshev extreme points w_k = (-1)^k, halved at both ends.
-__device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, double *__restrict__ m) {
+// mt: the transpose, [node][lt], or nullptr.
+__device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, double *__restrict__ m, int lt,
+                                           double *__restrict__ mt) {
   const int lane = threadIdx.x & 31, n = a.n;
   double X = 2.0 * p / (a.n_pix - 1) - 1.0;
   if (a.angular) {
@@ -89,6 +91,11 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
       v = hit >= 0 ? (k == hit ? 1.0 : 0.0) : w / d / sum;
     }
     m[(long long)p * ld + k] = v;
+    if (mt && k < n) {
+      mt[(long long)k * lt + p] = v;
+      if (p == a.n_pix - 1)
+        for (int z = p + 1; z < lt; ++z) mt[(long long)k * lt + z] = 0.0;
+    }
   }
 }
 
@@ -96,9 +103,9 @@ __global__ void __launch_bounds__(256) coarse_tables_kernel(CoarseTables t) {
   const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   const int nx = t.x.n_pix, ny = t.y.n_pix;
   if (warp < nx) {
-    coarse_row(warp, t.x, t.ldx, t.mx);
+    coarse_row(warp, t.x, t.ldx, t.mx, t.ltx, t.tx);
   } else if (warp < nx + ny) {
-    coarse_row(warp - nx, t.y, t.ldy, t.my);
+    coarse_row(warp - nx, t.y, t.ldy, t.my, t.lty, t.ty);
   } else {
     const int i = (warp - nx - ny) * 32 + lane;
     if (i >= t.x.n * t.y.n) return;
@@ -120,7 +127,7 @@ __global__ void __launch_bounds__(256) coarse_tables_kernel(CoarseTables t) {
 }
 
 cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
-                                 double *my, cudaStream_t st) {
+                                 double *my, cudaStream_t st, double *tx, double *ty) {
   CoarseTables t;
   t.g = g;
   t.x = x;
@@ -130,6 +137,10 @@ cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const Co
   t.q64 = q64;
   t.mx = mx;
   t.my = my;
+  t.ltx = coarse_ld(x.n_pix);
+  t.lty = coarse_ld(y.n_pix);
+  t.tx = tx;
+  t.ty = ty;
   const long long warps = (long long)x.n_pix + y.n_pix + ((long long)x.n * y.n + 31) / 32;
   coarse_tables_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(t);
   return cudaGetLastError();
@@ -156,43 +167,24 @@ __device__ __forceinline__ void dmma(double c[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
-// ROWS: the second product, else the first.
-template <int RM, int RN, bool ROWS>
-__global__ void __launch_bounds__(INTERP_THREADS)
-    coarse_interp_kernel(const SfPattern *__restrict__ pats, const CoarsePattern *__restrict__ coarse, int pattern0,
-                         double2 *__restrict__ strips, long long strip_stride) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const CoarsePattern cp = coarse[pattern0 + blockIdx.z];
-  double2 *__restrict__ strip = strips + blockIdx.z * strip_stride;
-  const int m_all = ROWS ? cp.ny : cp.nx;             // rows of the left matrix
-  const int n_all = 2 * (ROWS ? cp.nx : cp.nyn);      // columns of the right one (re, im pairs)
-  const int k_all = ROWS ? cp.nyn : cp.nxn;
-  const int ld = ROWS ? cp.ldy : cp.ldx;
-  const double *__restrict__ M = ROWS ? cp.my : cp.mx;
-  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
-  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);
-  if (m0 >= m_all || n0 >= n_all) return;
-  const int fr = lane >> 2, fc = lane & 3;
-
-  // lane's entries of the fragments: k steps 4 s .. 4 s + 3 of a group of eight
-  // hold k = 2 fc + s, so that the left matrix is read in pairs
+// RM x RN tiles of 8 x 8 of M B by one warp, M's rows from m0 (in range, clamped)
+// and B's columns at bcol[j], bstep doubles from one k to the next.  Of each
+// group of eight k the lane's entries are k = 2 fc + s in step s, so that M is
+// read in pairs; M holds zeros from k_all to its padded end, where B is read at
+// its last row.
+template <int RM, int RN>
+__device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, int m0, int m_all,
+                                          const double *const bcol[RN], long long bstep, int k_all,
+                                          double acc[RM][RN][2]) {
+  const int lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
   const double2 *arow[RM];
 #pragma unroll
   for (int i = 0; i < RM; ++i) arow[i] = (const double2 *)(M + (long long)min(m0 + 8 * i + fr, m_all - 1) * ld) + fc;
-  const double *bcol[RN];
-  const long long bstep = ROWS ? 2LL * cp.nx : 2;  // doubles from k to k + 1
-#pragma unroll
-  for (int j = 0; j < RN; ++j) {
-    const int n = min(n0 + 8 * j + fr, n_all - 1);
-    bcol[j] = ROWS ? (const double *)strip + n : (const double *)(cp.nodes + (long long)(n >> 1) * cp.nxn) + (n & 1);
-  }
-  double acc[RM][RN][2];
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < RN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   for (int k = 0; k < k_all; k += 8) {
-    // beyond k_all the left matrix holds zeros; the right one is read in range
     const long long kb0 = min(k + 2 * fc, k_all - 1) * bstep, kb1 = min(k + 2 * fc + 1, k_all - 1) * bstep;
     double2 a[RM];
     double b0[RN], b1[RN];
@@ -212,6 +204,34 @@ __global__ void __launch_bounds__(INTERP_THREADS)
 #pragma unroll
       for (int j = 0; j < RN; ++j) dmma(acc[i][j], a[i].y, b1[j]);
   }
+}
+
+// ROWS: the second product, else the first.
+template <int RM, int RN, bool ROWS>
+__global__ void __launch_bounds__(INTERP_THREADS)
+    coarse_interp_kernel(const SfPattern *__restrict__ pats, const CoarsePattern *__restrict__ coarse, int pattern0,
+                         double2 *__restrict__ strips, long long strip_stride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const CoarsePattern cp = coarse[pattern0 + blockIdx.z];
+  double2 *__restrict__ strip = strips + blockIdx.z * strip_stride;
+  const int m_all = ROWS ? cp.ny : cp.nx;             // rows of the left matrix
+  const int n_all = 2 * (ROWS ? cp.nx : cp.nyn);      // columns of the right one (re, im pairs)
+  const int k_all = ROWS ? cp.nyn : cp.nxn;
+  const int ld = ROWS ? cp.ldy : cp.ldx;
+  const double *__restrict__ M = ROWS ? cp.my : cp.mx;
+  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
+  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);
+  if (m0 >= m_all || n0 >= n_all) return;
+  const int fr = lane >> 2, fc = lane & 3;
+
+  const double *bcol[RN];
+#pragma unroll
+  for (int j = 0; j < RN; ++j) {
+    const int n = min(n0 + 8 * j + fr, n_all - 1);
+    bcol[j] = ROWS ? (const double *)strip + n : (const double *)(cp.nodes + (long long)(n >> 1) * cp.nxn) + (n & 1);
+  }
+  double acc[RM][RN][2];
+  dmma_tile<RM, RN>(M, ld, m0, m_all, bcol, ROWS ? 2LL * cp.nx : 2LL, k_all, acc);
 
   if (!ROWS) {
 #pragma unroll
@@ -296,6 +316,90 @@ cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coa
     const int n = std::min(group, npat - p0);
     interp_part<false>(pats, coarse, p0, n, max_nx, 2 * max_nyn, strip, stride, st);
     interp_part<true>(pats, coarse, p0, n, max_ny, 2 * max_nx, strip, stride, st);
+  }
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// the adjoint of the interpolation: H_nodes = M_y^T H M_x with
+// H = dL/d|F|^2 A e^{-B s^2} per pixel, A the centred amplitude
+
+__global__ void __launch_bounds__(256)
+    coarse_adjoint_pixels_kernel(CoarseAdjoint a, int pattern0, double2 *__restrict__ H) {
+  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= a.npix) return;
+  const int pat = pattern0 + blockIdx.y;
+  const double q0 = a.q64[3 * p], q1 = a.q64[3 * p + 1], q2 = a.q64[3 * p + 2];
+  double ux = q0, uy = q1, uz = q2;
+  if (a.rot) {
+    const double *R = a.rot + 9LL * pat;
+    ux = R[0] * q0 + R[1] * q1 + R[2] * q2;
+    uy = R[3] * q0 + R[4] * q1 + R[5] * q2;
+    uz = R[6] * q0 + R[7] * q1 + R[8] * q2;
+  }
+  double t = ux * a.center[0] + uy * a.center[1] + uz * a.center[2];
+  t -= rint(t);
+  double sn, cs;
+  sincospi(2.0 * t, &sn, &cs);
+  const float2 F = a.F[pat * a.npix + p];
+  double h = a.G[pat * a.npix + p];
+  if (a.B != 0.0) h *= exp(-a.B * 0.25e-20 * (q0 * q0 + q1 * q1 + q2 * q2));
+  H[blockIdx.y * a.npix + p] = make_double2(h * (F.x * cs - F.y * sn), h * (F.x * sn + F.y * cs));
+}
+
+// out[m][n] = sum_k L[m][k] R[n][k] for complex R of n_all rows, k_all long, and
+// real L of m_all rows, ld long; blockIdx.z: pattern.
+template <int RM, int RN>
+__global__ void __launch_bounds__(INTERP_THREADS)
+    coarse_product_kernel(const double *__restrict__ L, int ld, int m_all, const double2 *__restrict__ R, int n_all,
+                          int k_all, double2 *__restrict__ out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
+  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
+  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);  // of 2 n_all real columns
+  if (m0 >= m_all || n0 >= 2 * n_all) return;
+  R += (long long)blockIdx.z * n_all * k_all;
+  out += (long long)blockIdx.z * m_all * n_all;
+  const double *bcol[RN];
+#pragma unroll
+  for (int j = 0; j < RN; ++j) {
+    const int n = min(n0 + 8 * j + fr, 2 * n_all - 1);
+    bcol[j] = (const double *)(R + (long long)(n >> 1) * k_all) + (n & 1);
+  }
+  double acc[RM][RN][2];
+  dmma_tile<RM, RN>(L, ld, m0, m_all, bcol, 2LL, k_all, acc);
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int m = m0 + 8 * i + fr;
+    if (m >= m_all) continue;
+#pragma unroll
+    for (int j = 0; j < RN; ++j) {
+      const int n = n0 / 2 + 4 * j + fc;
+      if (n < n_all) out[(long long)m * n_all + n] = make_double2(acc[i][j][0], acc[i][j][1]);
+    }
+  }
+}
+
+static void product(const double *L, int ld, int m, const double2 *R, int n, int k, double2 *out, int npat,
+                    cudaStream_t st) {
+  const long long blocks = (long long)npat * ((m + 63) / 64) * ((2 * n + 63) / 64);
+  if (blocks >= 4 * 148) {
+    dim3 grid((unsigned)((2 * n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)npat);
+    coarse_product_kernel<4, 4><<<grid, INTERP_THREADS, 0, st>>>(L, ld, m, R, n, k, out);
+  } else {
+    dim3 grid((unsigned)((2 * n + 31) / 32), (unsigned)((m + 31) / 32), (unsigned)npat);
+    coarse_product_kernel<2, 2><<<grid, INTERP_THREADS, 0, st>>>(L, ld, m, R, n, k, out);
+  }
+}
+
+cudaError_t launch_coarse_adjoint(const CoarseAdjoint &a, int npat, double2 *H, int group, double2 *strip,
+                                  double2 *nodes, cudaStream_t st) {
+  for (int p0 = 0; p0 < npat; p0 += group) {
+    const int n = std::min(group, npat - p0);
+    dim3 grid((unsigned)((a.npix + 255) / 256), (unsigned)n);
+    coarse_adjoint_pixels_kernel<<<grid, 256, 0, st>>>(a, p0, H);
+    // strip[i][y] = sum_x M_x[x][i] H[y][x], then nodes[k][i] = sum_y M_y[y][k] strip[i][y]
+    product(a.tx, coarse_ld(a.nx), a.nxn, H, a.ny, a.nx, strip, n, st);
+    product(a.ty, coarse_ld(a.ny), a.nyn, strip, a.nxn, a.ny, nodes + (long long)p0 * a.nyn * a.nxn, n, st);
   }
   return cudaGetLastError();
 }

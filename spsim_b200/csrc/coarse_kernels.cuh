@@ -60,13 +60,30 @@ struct CoarsePattern {
 
 __host__ __device__ inline int coarse_ld(int n) { return (n + 7) / 8 * 8; }
 
-// Node q vectors [y.n * x.n][3] and both interpolation matrices of one detector.
+// Node q vectors [y.n * x.n][3] and both interpolation matrices of one
+// detector; tx, ty: also their transposes, [nodes][coarse_ld(pixels)].
 cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
-                                 double *my, cudaStream_t st);
+                                 double *my, cudaStream_t st, double *tx = nullptr, double *ty = nullptr);
 // Interpolates npat patterns: F, I of pats[i] (or coarse[i].out) from
 // coarse[i].nodes, in groups of as many patterns as the strip buffer holds
-// (strip_doubles2 complex values, at least max_nyn * max_nx).
+// (strip_size complex values, at least max_nyn * max_nx).
 cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coarse, int npat, int max_nx, int max_ny,
                                  int max_nyn, double2 *strip, long long strip_size, cudaStream_t st);
+
+// The adjoint of the interpolation: per pattern, from the forward's F and
+// G = dL/d|F|^2 on the pixels to the amplitudes H on the nodes.
+struct CoarseAdjoint {
+  const float2 *F;      // [npat][npix]
+  const float *G;       // [npat][npix]
+  const double *q64, *rot;
+  double center[3], B;
+  long long npix;
+  int nx, ny, nxn, nyn;
+  const double *tx, *ty;  // transposed interpolation matrices
+};
+// Groups of `group` patterns at a time through H (group * npix complex values)
+// and strip (group * nxn * ny).
+cudaError_t launch_coarse_adjoint(const CoarseAdjoint &a, int npat, double2 *H, int group, double2 *strip,
+                                  double2 *nodes, cudaStream_t st);
 
 }  // namespace spsim

@@ -121,6 +121,26 @@ def emit(name, Y, sdeg, cdeg, out):
         out.append("#define SPSIM_%s_C%d %.9ef" % (name, k, c))
 
 
+def emit64(name, Y, sdeg, cdeg, out):
+    """FP64 pair: the same fit with unrounded constants, S_0 = 2 pi."""
+    z_hi = Y * Y
+    z_lo = z_hi * 1e-4  # below, the quotients cancel and their weight vanishes
+    s0 = 2 * np.pi
+    gs = lambda z: (np.sin(2 * np.pi * np.sqrt(z)) / np.sqrt(z) - s0) / z
+    gc = lambda z: (np.cos(2 * np.pi * np.sqrt(z)) - 1.0) / z
+    ps = np.concatenate([[s0], remez(gs, lambda z: z ** 1.5, z_lo, z_hi, sdeg - 1)])
+    pc = np.concatenate([[1.0], remez(gc, lambda z: z, z_lo, z_hi, cdeg - 1)])
+    y = np.linspace(-Y, Y, 200001)
+    z = y * y
+    es = np.max(np.abs(y * np.polyval(ps[::-1], z) - np.sin(2 * np.pi * y)))
+    ec = np.max(np.abs(np.polyval(pc[::-1], z) - np.cos(2 * np.pi * y)))
+    out.append("/* %s: |y| <= %.6f cycles, FP64: sin max %.1e, cos max %.1e */" % (name, Y, es, ec))
+    for k, c in enumerate(ps):
+        out.append("#define SPSIM_%s_S%d %.17e" % (name, k, c))
+    for k, c in enumerate(pc):
+        out.append("#define SPSIM_%s_C%d %.17e" % (name, k, c))
+
+
 def main():
     out = [
         "/* Generated by gen_sincos_poly.py (Remez minimax, float32 coefficients).",
@@ -135,6 +155,7 @@ def main():
     emit("WIDE", 0.375, 5, 5, out)
     emit("NARROW", 0.32, 4, 5, out)
     emit("WIDER", 0.41, 5, 5, out)
+    emit64("NODE64", 0.25, 5, 6, out)
     out += ["#endif", ""]
     print("\n".join(out))
 

@@ -346,6 +346,29 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// 2^x in FP64, |x| < 1000, to 1e-11: rint(x) into the exponent, the Taylor
+// polynomial of 2^f on |f| <= 1/2.  For the weights on coarse grids' nodes,
+// where ex2_approx's 1e-7, a smooth function of its argument, would not average
+// out over the pixels as it does in the sums on every pixel.
+__device__ __forceinline__ double exp2_poly(double x) {
+  const double M52 = 6755399441055744.0;  // 1.5 * 2^52
+  constexpr double L = 0.69314718055994530942;
+  constexpr double c2 = L * L / 2, c3 = c2 * L / 3, c4 = c3 * L / 4, c5 = c4 * L / 5, c6 = c5 * L / 6, c7 = c6 * L / 7,
+                   c8 = c7 * L / 8, c9 = c8 * L / 9;
+  const double t = x + M52;
+  const double f = x - (t - M52);
+  double p = fma(f, c9, c8);
+  p = fma(f, p, c7);
+  p = fma(f, p, c6);
+  p = fma(f, p, c5);
+  p = fma(f, p, c4);
+  p = fma(f, p, c3);
+  p = fma(f, p, c2);
+  p = fma(f, p, L);
+  p = fma(f, p, 1.0);
+  return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
+}
+
 // log2(x) by the XU pipe's approximation (PTX lg2.approx.ftz.f32; -inf at 0)
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;

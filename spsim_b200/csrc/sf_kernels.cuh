@@ -19,11 +19,12 @@ cudaError_t launch_sf_f32(int mode, int nt, int p, int packed, bool perb, const 
 cudaError_t set_copy_stall(int on);
 cudaError_t set_nodes_copy_stall(int on);  // its part in sf_nodes.cu
 int sf_f32_occupancy(int mode, int nt, int p, int packed, bool perb, bool fixw = false, bool narrow = false);
-// The quad form on a coarse grid's nodes (work items of SF_NODES_TILE nodes).
-cudaError_t launch_sf_nodes(bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items, int *queue,
-                            int *err, int grid, cudaStream_t st);
-int sf_nodes_occupancy(bool perb, bool fixw);
-constexpr int SF_NODES_TILE = 256;
+// The sum on a coarse grid's nodes, in work items of `tile` nodes: SF_NODES_TILE
+// selects the FP32 quad form, the other two the FP64 kernel.
+constexpr int SF_NODES_TILE = 256, SF_NODES64_TILE = 128, SF_NODES64_SMALL_TILE = 64;
+cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items,
+                            int *queue, int *err, int grid, cudaStream_t st);
+int sf_nodes_occupancy(int tile, bool perb, bool fixw);
 bool sf_f32_variant_exists(int mode, int nt, int p, int packed);
 cudaError_t launch_sf_f64(const SfPattern *pats, int pattern, long long npix, cudaStream_t st);
 cudaError_t launch_spectrum_combine(const SfPattern *pats, int pattern0, int S, const double *weight, float *F,

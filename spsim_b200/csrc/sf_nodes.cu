@@ -20,6 +20,12 @@ cudaError_t set_nodes_copy_stall(int on) {
 // take its atoms in turn, groups of eight, adding their FP64 sums at the end
 // of the item: against 1,024 nodes per CTA that makes a work item a quarter as
 // long (the launch's tail) and lets a grid of some hundred nodes use the GPU.
+// Bound by the FMA and FP64 pipes, which add up: 14.6 FP32 and 3 FP64 lane
+// operations per term allow 1.75e12 terms/s.  Measured on 50,000 atoms x 26,244
+// nodes: 1.29e12 (1.27e12 with the sign on the ALU pipe, 1.24e12 with a full /
+// empty barrier pair per stage instead of the CTA barrier, 1.28e12 with three
+// CTAs per SM; FP32 sums of 16 atoms take the same time and have half as much
+// error again).
 constexpr int NODE_THREADS = 128;
 constexpr int NODE_TILE = SF_NODES_TILE;  // nodes per work item: 8 per lane
 static_assert(NODE_TILE == 256, "eight nodes per lane");
@@ -27,7 +33,7 @@ static_assert(NODE_TILE == 256, "eight nodes per lane");
 template <bool PERB, bool FIXW>
 __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
     const SfPattern *__restrict__ pats, const WorkItem *__restrict__ items, int n_items, int *__restrict__ queue,
-    int *__restrict__ err) {
+    int *__restrict__ err, uint32_t m31) {
   constexpr int P = 8, NP = P / 2, WARPS = NODE_THREADS / 32;
   __shared__ __align__(128) float4 ring[RING_STAGES][2 * TILE_ATOMS];
   __shared__ __align__(16) double2 sacc[P * NODE_THREADS];  // per-thread FP64 sums of the current work item
@@ -106,15 +112,17 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
       }
       const TileDesc td = tiles[k];
       const float4 *__restrict__ ta = ring[st];
-      // this warp's groups of eight atoms, two of them per FP32 sum
-      for (int a = ATOM_GROUP * warp; a < td.count; a += 2 * ATOM_GROUP * WARPS) {
+      // this warp's groups of eight atoms, in FP32 sums of four: of bright nodes'
+      // sums, all of one sign, the rounding errors grow with the sum
+      for (int a = ATOM_GROUP * warp; a < td.count; a += ATOM_GROUP * WARPS)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
         float2 bc[NP], bs[NP];
 #pragma unroll
         for (int j = 0; j < NP; ++j) bc[j] = bs[j] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int g = 0; g < 2 * ATOM_GROUP; ++g) {
-          if (g == ATOM_GROUP && a + ATOM_GROUP * WARPS >= td.count) break;
-          const int at = g < ATOM_GROUP ? a + g : a + ATOM_GROUP * (WARPS - 1) + g;
+        for (int g = 0; g < ATOM_GROUP / 2; ++g) {
+          const int at = a + ATOM_GROUP / 2 * half + g;
           const float4 d0 = ta[2 * at], d1 = ta[2 * at + 1];
           const double rx = __hiloint2double(__float_as_int(d0.y), __float_as_int(d0.x));
           const double ry = __hiloint2double(__float_as_int(d0.w), __float_as_int(d0.z));
@@ -141,7 +149,7 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
                 kb = (uint32_t)__double2loint(t);
               }
               w[h] = LOGW ? ex2_approx(fmaf(d1.w, s2n[i], lw)) : PERB ? W * ex2_approx(d1.w * s2n[i]) : W;
-              w[h] = sign_by_parity_alu(w[h], kb);
+              w[h] = sign_by_parity(w[h], kb, m31);
             }
             const float2 yy = FIXW ? mul2(make_float2(y[0], y[1]), f2(word_to_phase<PREC_MODE_POLY>()))
                                    : make_float2(y[0], y[1]);
@@ -216,19 +224,203 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
   }
 }
 
-cudaError_t launch_sf_nodes(bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items, int *queue,
-                            int *err, int grid, cudaStream_t st) {
-  if (perb)
-    fixw ? sf_dquad_nodes_kernel<true, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err)
-         : sf_dquad_nodes_kernel<true, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err);
+// The same sum in FP64 throughout, phases by rounding.  B200's FP64 pipe runs at half the FP32 rate, and without the split
+// phase and the compensated sums a term is 21 operations, so this takes 1.8
+// times as long as the FP32 kernel (7.2e11 terms/s on 50,000 atoms x 26,244
+// nodes, P = 4; 80 % of the pipe).  It runs
+//   - for molecules rewritten on the device, that is in refinements: a node's
+//     rounding error goes into all the pixels around it alike, and the gradient
+//     of a loss adds it up where the pixels' own errors would average out (up
+//     to 6 times the gradient's error on a heavily oversampled detector);
+//   - for small grids, which latency bounds: with P = 2 a work item is 64 nodes
+//     (1,000 atoms x 340 nodes: 12 us against 17 us in FP32; 5,000 x 840 even).
+template <int P, bool PERB>
+__global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPattern *__restrict__ pats,
+                                                                  const WorkItem *__restrict__ items, int n_items,
+                                                                  int *__restrict__ queue, int *__restrict__ err) {
+  constexpr int WARPS = NODE_THREADS / 32;
+  __shared__ __align__(128) float4 ring[RING_STAGES][2 * TILE_ATOMS];
+  __shared__ __align__(16) double2 sacc[P * NODE_THREADS];
+  __shared__ __align__(8) uint64_t full_bar[RING_STAGES];
+  __shared__ int s_item;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < RING_STAGES; ++s) mbar_init(&full_bar[s], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  uint32_t g_issue = 0, g_cons = 0;
+  const bool stall = g_nodes_copy_stall != 0;
+  const long long kWaitCycles = stall ? kStallWaitCycles : kWaitCyclesDefault;
+  const double M52 = 6755399441055744.0;  // 1.5 * 2^52
+
+  for (;;) {
+    if (tid == 0) s_item = atomicAdd(queue, 1);
+    __syncthreads();
+    const int it = s_item;
+    if (it >= n_items) break;
+    const WorkItem wi = items[it];
+    const SfPattern &pt = pats[wi.pattern];
+    const long long npix = pt.npix;
+    const AtomD *__restrict__ atomsd = pt.atomsd;
+    const TileDesc *__restrict__ tiles = pt.tiles;
+
+    const long long pix0 = (long long)wi.pixel_tile * (32 * P) + lane;  // node i of this lane: pix0 + 32 i
+    double qx[P], qy[P], qz[P];
+    double s2n[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      double q[3] = {0.0, 0.0, 0.0};
+      if (pix0 + 32 * i < npix) load_q(pt, pix0 + 32 * i, q);
+      qx[i] = q[0];
+      qy[i] = q[1];
+      qz[i] = q[2];
+      s2n[i] = -0.25 * (q[0] * q[0] + q[1] * q[1] + q[2] * q[2]) * 1e-20 * pt.s2scale * 1.4426950408889634;
+    }
+    double fre[P], fim[P], ec[P], es[P];  // the item's sums, and the current element's
+#pragma unroll
+    for (int i = 0; i < P; ++i) fre[i] = fim[i] = ec[i] = es[i] = 0.0;
+
+    const int k0 = wi.k0, k1 = wi.k1;
+    if (tid == 0) {
+      for (int k = k0; k < k1 && k < k0 + RING_STAGES; ++k) {
+        const TileDesc td = tiles[k];
+        const uint32_t st = g_issue % RING_STAGES;
+        const uint32_t bytes = (uint32_t)td.count * (uint32_t)sizeof(AtomD);
+        mbar_arrive_expect_tx(&full_bar[st], bytes);
+        if (!(stall && g_issue == 0))  // the stall hook skips the CTA's first copy
+          bulk_copy_g2s(&ring[st][0], atomsd + td.atom_begin, bytes, &full_bar[st]);
+        ++g_issue;
+      }
+    }
+
+    for (int k = k0; k < k1; ++k) {
+      const uint32_t st = g_cons % RING_STAGES;
+      const uint32_t par = (g_cons / RING_STAGES) & 1u;
+      const bool ok = mbar_wait_bounded(&full_bar[st], par, kWaitCycles);
+      if (__syncthreads_or(!ok)) {
+        if (tid == 0) {
+          atomicOr(err, 1);
+          for (uint32_t g = g_cons; g < g_issue; ++g)
+            mbar_wait_bounded(&full_bar[g % RING_STAGES], (g / RING_STAGES) & 1u, kWaitCycles);
+        }
+        return;
+      }
+      const TileDesc td = tiles[k];
+      const float4 *__restrict__ ta = ring[st];
+#pragma unroll 2
+      for (int a = warp; a < td.count; a += WARPS) {
+        const float4 d0 = ta[2 * a], d1 = ta[2 * a + 1];
+        const double rx = __hiloint2double(__float_as_int(d0.y), __float_as_int(d0.x));
+        const double ry = __hiloint2double(__float_as_int(d0.w), __float_as_int(d0.z));
+        const double rz = __hiloint2double(__float_as_int(d1.y), __float_as_int(d1.x));
+        const double W = d1.z, Bj = d1.w;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          double u = qx[i] * rx;
+          u = fma(qy[i], ry, u);
+          u = fma(qz[i], rz, u);
+          const double t = fma(u, 2.0, M52);  // rint(2u) in the low bits
+          const double y = fma(t - M52, -0.5, u);
+          double w = PERB ? W * exp2_poly(Bj * s2n[i]) : W;
+          w = __hiloint2double(__double2hiint(w) ^ (__double2loint(t) << 31), __double2loint(w));
+          const double z = y * y;
+          double ps = fma(z, SPSIM_NODE64_S5, SPSIM_NODE64_S4);
+          double pc = fma(z, SPSIM_NODE64_C6, SPSIM_NODE64_C5);
+          ps = fma(z, ps, SPSIM_NODE64_S3);
+          pc = fma(z, pc, SPSIM_NODE64_C4);
+          ps = fma(z, ps, SPSIM_NODE64_S2);
+          pc = fma(z, pc, SPSIM_NODE64_C3);
+          ps = fma(z, ps, SPSIM_NODE64_S1);
+          pc = fma(z, pc, SPSIM_NODE64_C2);
+          ps = fma(z, ps, SPSIM_NODE64_S0);
+          pc = fma(z, pc, SPSIM_NODE64_C1);
+          pc = fma(z, pc, SPSIM_NODE64_C0);
+          ec[i] = fma(w, pc, ec[i]);
+          es[i] = fma(w * y, ps, es[i]);
+        }
+      }
+      if (td.last || k == k1 - 1) {
+        const double *__restrict__ ffe = pt.ff + (long long)td.elem * npix;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          const double f = pix0 + 32 * i < npix ? ffe[pix0 + 32 * i] : 0.0;
+          fre[i] = fma(f, ec[i], fre[i]);
+          fim[i] = fma(-f, es[i], fim[i]);
+          ec[i] = es[i] = 0.0;
+        }
+      }
+      __syncthreads();
+      if (tid == 0 && k + RING_STAGES < k1) {
+        const TileDesc tn = tiles[k + RING_STAGES];
+        const uint32_t bytes = (uint32_t)tn.count * (uint32_t)sizeof(AtomD);
+        mbar_arrive_expect_tx(&full_bar[st], bytes);
+        bulk_copy_g2s(&ring[st][0], atomsd + tn.atom_begin, bytes, &full_bar[st]);
+        ++g_issue;
+      }
+      ++g_cons;
+    }
+#pragma unroll
+    for (int i = 0; i < P; ++i) sacc[i * NODE_THREADS + tid] = make_double2(fre[i], fim[i]);
+    __syncthreads();
+    const bool whole = k0 == 0 && k1 == pt.n_tiles;
+    for (int i = warp; i < P; i += WARPS) {
+      double2 v = sacc[i * NODE_THREADS + lane];
+#pragma unroll
+      for (int w = 1; w < WARPS; ++w) {
+        const double2 u = sacc[i * NODE_THREADS + 32 * w + lane];
+        v.x += u.x;
+        v.y += u.y;
+      }
+      const long long p = pix0 + 32 * i;
+      if (p < npix) {
+        if (whole) {
+          pt.acc[p] = v;
+        } else {
+          atomicAdd(&pt.acc[p].x, v.x);
+          atomicAdd(&pt.acc[p].y, v.y);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// f(the kernel of node form `tile`), called with its arguments or queried for its occupancy
+template <typename F>
+static void with_nodes64(int tile, bool perb, F f) {
+  if (tile == SF_NODES64_TILE)
+    perb ? f(sf_nodes64_kernel<4, true>) : f(sf_nodes64_kernel<4, false>);
   else
-    fixw ? sf_dquad_nodes_kernel<false, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err)
-         : sf_dquad_nodes_kernel<false, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err);
+    perb ? f(sf_nodes64_kernel<2, true>) : f(sf_nodes64_kernel<2, false>);
+}
+
+cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items,
+                            int *queue, int *err, int grid, cudaStream_t st) {
+  if (tile != SF_NODES_TILE)
+    with_nodes64(tile, perb,
+                 [&](auto kernel) { kernel<<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err); });
+  else if (perb)
+    fixw ? sf_dquad_nodes_kernel<true, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err, 0x80000000u)
+         : sf_dquad_nodes_kernel<true, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err,
+                                                                            0x80000000u);
+  else
+    fixw ? sf_dquad_nodes_kernel<false, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err,
+                                                                            0x80000000u)
+         : sf_dquad_nodes_kernel<false, false><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err,
+                                                                             0x80000000u);
   return cudaGetLastError();
 }
 
-int sf_nodes_occupancy(bool perb, bool fixw) {
+int sf_nodes_occupancy(int tile, bool perb, bool fixw) {
   int n = 0;
+  if (tile != SF_NODES_TILE) {
+    with_nodes64(tile, perb,
+                 [&](auto kernel) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NODE_THREADS, 0); });
+    return n;
+  }
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &n, perb ? (fixw ? sf_dquad_nodes_kernel<true, true> : sf_dquad_nodes_kernel<true, false>)
                : (fixw ? sf_dquad_nodes_kernel<false, true> : sf_dquad_nodes_kernel<false, false>),

@@ -161,3 +161,56 @@ def test_calls_that_stay_on_every_pixel(cuda):
     # no atoms: zeros
     _, I = core.forward(core.Molecule(np.zeros(5, np.int32), pos[:5]), qs)
     assert not I.any()
+
+
+def _rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("nx,ny", [(96, 70), (129, 65), (61, 200)])
+@pytest.mark.parametrize("precision", ["f32", "f32_fast"])
+@pytest.mark.parametrize("with_b", [False, True])
+def test_adjoint(cuda, nx, ny, precision, with_b):
+    # the gradient through the nodes against the oracle's vector-Jacobian
+    # product, at the adjoint's tolerance (1e-4 relative L2): an odd number of
+    # patterns, elements whose segments share a block, a centre phase, global B
+    Z, pos = synth.random_molecule(1403, 2.4e-9, 221)
+    pos += np.float32(4e-9)
+    rng = np.random.Generator(np.random.PCG64(222))
+    occ = rng.uniform(0.5, 1.0, len(Z)).astype(np.float32)
+    b = rng.uniform(0.0, 30.0, len(Z)).astype(np.float32) if with_b else None
+    B = 0.0 if with_b else 9.0
+    d = _det(nx, ny)
+    R = synth.haar_rotations(3, 223)
+    q = np.concatenate([_q(d) @ r.T for r in R])
+    g = rng.normal(size=q.shape[0]).astype(np.float32)
+    mol, qs = core.Molecule(Z, pos, occ=occ, bfac=b), core.QSet.from_detector(**d)
+    F, _ = core.forward_batch([mol] * 3, [qs] * 3, rots=R, B=B, precision=precision)
+    dpos, docc, dB = core.adjoint(mol, qs, torch.cat(F), torch.from_numpy(g).cuda(), rots=R, B=B, precision=precision)
+    # the oracle's gradient has no global B: the same factor on every atom
+    ball = np.full(len(Z), B, np.float32) if b is None else b
+    dp, do, db = O.structure_factor_vjp(Z, pos.astype(np.float64), q, g.astype(np.float64), occ=occ, bfac=ball)
+    assert _rel(dpos.cpu().numpy(), dp) < 1e-4
+    assert _rel(docc.cpu().numpy(), do) < 1e-4
+    if with_b:
+        assert _rel(dB.cpu().numpy(), db) < 1e-4
+
+
+def test_adjoint_of_b_factors_beyond_the_grids_limit(cuda):
+    Z, pos = synth.random_molecule(1500, 2.5e-9, 224)
+    rng = np.random.Generator(np.random.PCG64(225))
+    b0 = rng.uniform(0.0, 20.0, len(Z)).astype(np.float32)
+    d = _det(128, 120, distance=0.03)
+    q, qs = _q(d), core.QSet.from_detector(**d)
+    mol = core.Molecule(Z, pos, bfac=b0)
+    g = rng.normal(size=q.shape[0]).astype(np.float32)
+    for top in (90.0, 2500.0, 60.0):
+        b = b0.copy()
+        b[3:300:7] = top
+        mol.update_device(torch.from_numpy(pos).cuda(), bfac=torch.from_numpy(b).cuda())
+        F, _ = core.forward(mol, qs)
+        dpos, docc, dB = core.adjoint(mol, qs, F, torch.from_numpy(g).cuda())
+        dp, do, db = O.structure_factor_vjp(Z, pos.astype(np.float64), q, g.astype(np.float64), bfac=b)
+        assert _rel(dpos.cpu().numpy(), dp) < 1e-4
+        assert _rel(docc.cpu().numpy(), do) < 1e-4
+        assert _rel(dB.cpu().numpy(), db) < 1e-4
