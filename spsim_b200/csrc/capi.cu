@@ -1239,9 +1239,15 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   if (ev1 && (e = cudaEventRecord(ev1, stream))) return e;
   const SfPattern *pats = (const SfPattern *)pl.pats.p;
   const int pixels = pl.coarse ? pl.npat : 0;  // the first pixel pattern
-  if (pl.coarse && (e = launch_coarse_interp(pats + pixels, (const CoarsePattern *)pl.cpats.p, pl.npat, pl.max_nx,
-                                             pl.max_ny, pl.max_nyn, (double2 *)pl.strip.p, pl.strip_size, stream)))
-    return e;
+  if (pl.coarse) {
+    CoarseBatch b;
+    memset(&b, 0, sizeof(b));
+    b.pats = pats + pixels;
+    b.coarse = (const CoarsePattern *)pl.cpats.p;
+    if ((e = launch_coarse_interp(b, pl.npat, pl.max_nx, pl.max_ny, pl.max_nyn, (double2 *)pl.strip.p, pl.strip_size,
+                                  stream)))
+      return e;
+  }
   if (pl.spectrum > 0)
     e = launch_spectrum_combine(pats, pixels, pl.spectrum, (const double *)pl.spec_w.p, pl.spec_F, pl.spec_I,
                                 pl.npat ? pl.host_pats[pixels].npix : 0, stream, gate);
@@ -1887,6 +1893,8 @@ extern "C" int spsim_b200_structure_factor_host_spectrum(int natoms, const int32
 
 struct NufftCtx {
   DevBuf small, fa, fb, packed, dec, tw, seg, keys, flags, rots;
+  DevBuf ntab, nodes, strip;      // the interpolation through a detector's coarse grid
+  std::vector<double> ntab_key;   // detector and node counts the tables in ntab are for
   FftAxis ax[3];  // the pruned FFT passes (twiddle tables in tw)
   std::vector<double> geom_key;   // inputs the q box was read for
   std::vector<double> size_key;   // q box, bound, elements, eps the grids were sized for
@@ -1949,6 +1957,61 @@ static int nufft_width(double eps) {
   return std::min(std::max(w, NUFFT_MIN_W), NUFFT_MAX_W - 1);
 }
 
+// Step 4 through the detector's coarse grid: the stencils at its nodes only
+// (each its own, the tile path shares nothing between nodes pixels apart), then
+// the interpolation to the pixels.  From 2^16 pixels on, where the stencils at
+// every pixel (1 ns each) take longer than the grid's three launches; 50,000
+// atoms x 1024^2 at 26,244 nodes: 1.07 ms -> 0.11 ms.
+static cudaError_t nufft_interp_coarse(NufftCtx &c, const NufftInterp &pixels, const spsim_b200_qset *qs,
+                                       const CoarseGrid &grid, cudaStream_t st) {
+  const DetGeom &g = qs->geom;
+  const int nxn = grid.x.n, nyn = grid.y.n, ldx = coarse_ld(nxn), ldy = coarse_ld(nyn);
+  const size_t points = (size_t)nxn * nyn, at_x = (3 * points + 1) / 2 * 2, at_y = at_x + (size_t)g.nx * ldx;
+  const std::vector<double> key = {(double)g.nx, (double)g.ny, (double)g.spherical, g.width, g.height,    g.distance,
+                                   g.cx,         g.cy,         g.ewald,             (double)nxn, (double)nyn};
+  const long long strip = (long long)nyn * g.nx;
+  const long long strips = strip * std::min<long long>(pixels.npat, std::max<long long>(1, (4LL << 20) / strip));
+  cudaError_t e;
+  if ((e = c.nodes.ensure(points * pixels.npat * sizeof(double2))) || (e = c.strip.ensure(strips * sizeof(double2))))
+    return e;
+  if (key != c.ntab_key) {
+    c.ntab_key.clear();
+    if ((e = c.ntab.ensure((at_y + (size_t)g.ny * ldy) * sizeof(double)))) return e;
+    double *tab = (double *)c.ntab.p;
+    if ((e = launch_coarse_tables(g, grid.x, grid.y, tab, tab + at_x, tab + at_y, st))) return e;
+    c.ntab_key = key;
+  }
+  const double *tab = (const double *)c.ntab.p;
+  NufftInterp a = pixels;
+  a.hkl = nullptr;
+  a.q64 = tab;
+  a.npix = (long long)points;
+  a.tile_nx = 0;
+  if ((e = nufft_nodes(a, (double2 *)c.nodes.p, st))) return e;
+  if (!pixels.rots && pixels.has_rot) {  // one rotation: beside the tables' users on the stream
+    if ((e = c.rots.ensure(9 * sizeof(double)))) return e;
+    if ((e = cudaMemcpyAsync(c.rots.p, pixels.rot, 9 * sizeof(double), cudaMemcpyHostToDevice, st))) return e;
+  }
+  CoarseBatch b;
+  memset(&b, 0, sizeof(b));
+  b.one.nodes = (const double2 *)c.nodes.p;
+  b.one.mx = tab + at_x;
+  b.one.my = tab + at_y;
+  b.one.nx = g.nx;
+  b.one.ny = g.ny;
+  b.one.nxn = nxn;
+  b.one.nyn = nyn;
+  b.one.ldx = ldx;
+  b.one.ldy = ldy;
+  b.one.B = pixels.B;
+  b.q64 = qs->d_q64;
+  b.rots = pixels.rots || pixels.has_rot ? (const double *)c.rots.p : nullptr;
+  memcpy(b.center, pixels.g.center, sizeof(b.center));
+  b.F = pixels.F;
+  b.I = pixels.I;
+  return launch_coarse_interp(b, pixels.npat, g.nx, g.ny, nyn, (double2 *)c.strip.p, strips, st);
+}
+
 // npat patterns of one molecule and q set, pattern i rotated by rot[9 i] (or
 // none), outputs [npat][npix].  ball: size the grid for the ball |R q| <=
 // |q|max instead of the box of the rotated list, so that it holds for every
@@ -1959,7 +2022,7 @@ static int nufft_width(double eps) {
 // outputs are zeros).
 static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs, int npat, const double *rot,
                          bool ball, float B, double eps, float *F_dev, float *I_dev, cudaStream_t st,
-                         NufftInterp *deferred = nullptr, bool *deferred_empty = nullptr) {
+                         NufftInterp *deferred = nullptr, bool *deferred_empty = nullptr, bool allow_nodes = true) {
   if (!m || !qs) return fail(SPSIM_ERR_INVALID_ARG, "NULL handle");
   if (npat < 1 || npat > 65535) return fail(SPSIM_ERR_INVALID_ARG, "npatterns %d outside [1, 65535]", npat);
   if (!(eps >= 1e-14 && eps <= 1e-2)) return fail(SPSIM_ERR_INVALID_ARG, "eps %g outside [1e-14, 1e-2]", eps);
@@ -1995,11 +2058,19 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
   if (!c.has_done) CUDA_TRY(cudaMemsetAsync(c.flags.p, 0, sizeof(int), st));
 
   const int n_elem = m->n_elem;
+  CoarseGrid coarse;
+  const double stretch = qs->qmax > 0 ? qball / qs->qmax : 1.0;
+  const bool on_nodes = allow_nodes && !deferred && nufft_interp_mode() == 0 && npix * npat >= (1 << 16) &&
+                        coarse_fit(m, qs, stretch, stretch, &coarse);
+  // a grid point more per axis than stencils at every pixel take: an error at a
+  // bright node enters the dim pixels around it (without it the maximum error
+  // was up to twice theirs, with it a tenth)
+  const int w = std::min(nufft_width(eps) + (on_nodes ? 1 : 0), NUFFT_MAX_W - 1);
   std::vector<double> key;
   if (ball) {
-    key = {-1.0, qball, m->rbound, (double)n_elem, eps};
+    key = {-1.0, qball, m->rbound, (double)n_elem, (double)w, eps, on_nodes ? 1.0 : 0.0};
   } else {
-    key = {(double)qs->id, (double)npix, m->rbound, (double)n_elem, eps, rot ? 1.0 : 0.0};
+    key = {(double)qs->id, (double)npix, m->rbound, (double)n_elem, (double)w, eps, on_nodes ? 1.0 : 0.0, rot ? 1.0 : 0.0};
     if (rot) key.insert(key.end(), rot, rot + 9);
   }
   if (key != c.geom_key) {
@@ -2028,7 +2099,8 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
     // the grids follow from the q box, the molecule's bound, the elements and
     // eps: an unchanged box (a new list of the same detector, say) keeps them
     // (the molecule's bound enters only through the spreading grid's size n1)
-    std::vector<double> size_key = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], (double)n_elem, eps};
+    std::vector<double> size_key = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], (double)n_elem, (double)w,
+                                    on_nodes ? 1.0 : 0.0};
     {
       const int w1 = std::min(nufft_width(eps) + 3, NUFFT_MAX_W);
       for (int d = 0; d < 3; ++d) {
@@ -2039,11 +2111,10 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
     }
     if (size_key != c.size_key) {
       c.size_key.clear();
-      const int w = nufft_width(eps);
       const double sigma1 = 1.5, sigma2 = 2.0;  // spreading-grid and FFT-grid upsampling
       NufftGeom g;
       std::memset(&g, 0, sizeof(g));
-      g.w1 = std::min(w + 3, NUFFT_MAX_W);
+      g.w1 = std::min(nufft_width(eps) + 3, NUFFT_MAX_W);
       g.w2 = w;
       g.beta1 = 0.97 * M_PI * g.w1 * (1.0 - 0.5 / sigma1);
       g.beta2 = 0.97 * M_PI * g.w2 * (1.0 - 0.5 / sigma2);
@@ -2066,6 +2137,7 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
         const double tlo = (lo[d] - g.cq[d]) * g.L[d], thi = (hi[d] - g.cq[d]) * g.L[d];
         g.pmin[d] = (int)std::floor(tlo - 0.5 * w) - 2;
         g.m[d] = (int)std::ceil(thi - 0.5 * w) + w - 1 + 2 - g.pmin[d] + 1;
+        if (on_nodes && d == 0) g.m[d] += g.m[d] & 1;  // whole pairs of cells (nufft_nodes_kernel)
         cells1 *= (size_t)g.n1[d];
         cells2 *= (size_t)g.m[d];
       }
@@ -2079,10 +2151,15 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
       const size_t bytes1 = one1 * c.copies;
       const size_t bytes_a = (size_t)n_elem * g.n1[2] * g.n1[1] * g.m[0] * sizeof(double2);
       const size_t bytes_b = (size_t)n_elem * g.n1[2] * g.m[1] * g.m[0] * sizeof(double2);
-      const size_t bytes3 = cells2 * nufft_pack_groups(n_elem) * nufft_pack_halves(n_elem) * sizeof(float4);
+      const size_t bytes3 = cells2 * nufft_pack_groups(n_elem) * nufft_pack_halves(n_elem) * sizeof(float4) *
+                            (on_nodes ? 2 : 1);  // FP64 for the nodes, else FP32
       size_t free_b = 0, total_b = 0;
       CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
       const size_t have = free_b + c.small.cap + c.fa.cap + c.fb.cap + c.packed.cap;
+      if (bytes1 + bytes_a + bytes_b + bytes3 > have / 10 * 9 && on_nodes) {
+        lk.unlock();  // the FP32 grid of the stencils at every pixel is half as large
+        return nufft_forward(m, qs, npat, rot, ball, B, eps, F_dev, I_dev, st, deferred, deferred_empty, false);
+      }
       if (bytes1 + bytes_a + bytes_b + bytes3 > have / 10 * 9)
         return fail(SPSIM_ERR_INVALID_ARG, "NUFFT: grids of %.3g GB do not fit; use the direct sum",
                     (double)(bytes1 + bytes_a + bytes_b + bytes3) * 1e-9);
@@ -2133,7 +2210,7 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
   CUDA_TRY(nufft_spread(m->d_atomsd, (const int *)c.seg.p, n_elem, m->n_padded, g, (double *)c.small.p, c.copies,
                         (int *)c.flags.p, st));
   CUDA_TRY(nufft_fft3((const double *)c.small.p, c.copies, (const double *)c.dec.p, g, n_elem, c.ax,
-                      (double2 *)c.fa.p, (double2 *)c.fb.p, (float4 *)c.packed.p, st));
+                      (double2 *)c.fa.p, (double2 *)c.fb.p, c.packed.p, on_nodes, st));
   const long long cells2 = (long long)g.m[0] * g.m[1] * g.m[2];
   NufftInterp a;
   std::memset(&a, 0, sizeof(a));
@@ -2167,6 +2244,8 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
     *deferred = a;
     c.shot_open = true;
     c.shot_owner = std::this_thread::get_id();
+  } else if (on_nodes) {
+    CUDA_TRY(nufft_interp_coarse(c, a, qs, coarse, st));
   } else {
     CUDA_TRY(nufft_interp(a, st));
   }

@@ -209,10 +209,12 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, 
 // ROWS: the second product, else the first.
 template <int RM, int RN, bool ROWS>
 __global__ void __launch_bounds__(INTERP_THREADS)
-    coarse_interp_kernel(const SfPattern *__restrict__ pats, const CoarsePattern *__restrict__ coarse, int pattern0,
-                         double2 *__restrict__ strips, long long strip_stride) {
+    coarse_interp_kernel(const __grid_constant__ CoarseBatch batch, int pattern0, double2 *__restrict__ strips,
+                         long long strip_stride) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const CoarsePattern cp = coarse[pattern0 + blockIdx.z];
+  const int pattern = pattern0 + blockIdx.z;
+  CoarsePattern cp = batch.pats ? batch.coarse[pattern] : batch.one;
+  if (!batch.pats) cp.nodes += (long long)pattern * cp.nyn * cp.nxn;
   double2 *__restrict__ strip = strips + blockIdx.z * strip_stride;
   const int m_all = ROWS ? cp.ny : cp.nx;             // rows of the left matrix
   const int n_all = 2 * (ROWS ? cp.nx : cp.nyn);      // columns of the right one (re, im pairs)
@@ -246,8 +248,21 @@ __global__ void __launch_bounds__(INTERP_THREADS)
     }
     return;
   }
-  const SfPattern &pt = pats[pattern0 + blockIdx.z];
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
+  const long long npix = (long long)cp.nx * cp.ny;
+  const double *q64 = batch.q64, *rot = batch.rots ? batch.rots + 9LL * pattern : nullptr, *center = batch.center;
+  double qscale = 1.0;
+  float2 *F = batch.F ? batch.F + pattern * npix : nullptr;
+  float *I = batch.I ? batch.I + pattern * npix : nullptr;
+  if (batch.pats) {
+    const SfPattern &pt = batch.pats[pattern];
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
+    q64 = pt.q64;
+    rot = pt.has_rot ? pt.rot : nullptr;
+    center = pt.center;
+    qscale = pt.qscale;
+    F = pt.F;
+    I = pt.I;
+  }
 #pragma unroll
   for (int i = 0; i < RM; ++i) {
     const int y = m0 + 8 * i + fr;
@@ -258,8 +273,8 @@ __global__ void __launch_bounds__(INTERP_THREADS)
       if (x >= cp.nx) continue;
       const long long p = (long long)y * cp.nx + x;
       double re = acc[i][j][0], im = acc[i][j][1];
-      if (pt.F || cp.B != 0.0 || cp.out) {
-        const double a = pt.q64[3 * p], b = pt.q64[3 * p + 1], c = pt.q64[3 * p + 2];
+      if (F || cp.B != 0.0 || cp.out) {
+        const double a = q64[3 * p], b = q64[3 * p + 1], c = q64[3 * p + 2];
         if (cp.B != 0.0) {
           const double e = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
           re *= e;
@@ -269,53 +284,53 @@ __global__ void __launch_bounds__(INTERP_THREADS)
           cp.out[p] = make_double2(re, im);
           continue;
         }
-        if (pt.F) {
+        if (F) {
           double ux = a, uy = b, uz = c;
-          if (pt.has_rot) {
-            ux = pt.rot[0] * a + pt.rot[1] * b + pt.rot[2] * c;
-            uy = pt.rot[3] * a + pt.rot[4] * b + pt.rot[5] * c;
-            uz = pt.rot[6] * a + pt.rot[7] * b + pt.rot[8] * c;
+          if (rot) {
+            ux = rot[0] * a + rot[1] * b + rot[2] * c;
+            uy = rot[3] * a + rot[4] * b + rot[5] * c;
+            uz = rot[6] * a + rot[7] * b + rot[8] * c;
           }
-          double t = (ux * pt.center[0] + uy * pt.center[1] + uz * pt.center[2]) * pt.qscale;
+          double t = (ux * center[0] + uy * center[1] + uz * center[2]) * qscale;
           t -= rint(t);
           double sn, cs;
           sincospi(2.0 * t, &sn, &cs);
-          pt.F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
+          F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
         }
       }
-      if (pt.I) pt.I[p] = (float)(re * re + im * im);
+      if (I) I[p] = (float)(re * re + im * im);
     }
   }
 }
 
 template <int RM, int RN, bool ROWS>
-static void interp_t(const SfPattern *pats, const CoarsePattern *coarse, int pattern0, int n, int m_max, int n_max,
-                     double2 *strip, long long stride, cudaStream_t st) {
+static void interp_t(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip, long long stride,
+                     cudaStream_t st) {
   const int bm = 8 * RM * INTERP_WARPS_M, bn = 8 * RN * INTERP_WARPS_N;
   dim3 grid((unsigned)((n_max + bn - 1) / bn), (unsigned)((m_max + bm - 1) / bm), (unsigned)n);
-  coarse_interp_kernel<RM, RN, ROWS><<<grid, INTERP_THREADS, 0, st>>>(pats, coarse, pattern0, strip, stride);
+  coarse_interp_kernel<RM, RN, ROWS><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
 }
 
 template <bool ROWS>
-static void interp_part(const SfPattern *pats, const CoarsePattern *coarse, int pattern0, int n, int m_max, int n_max,
-                        double2 *strip, long long stride, cudaStream_t st) {
+static void interp_part(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip,
+                        long long stride, cudaStream_t st) {
   // 32 x 32 tiles per warp where they fill the GPU a few times, else 16 x 16
   const long long blocks = (long long)n * ((m_max + 63) / 64) * ((n_max + 63) / 64);
   if (blocks >= 2 * 148)
-    interp_t<4, 4, ROWS>(pats, coarse, pattern0, n, m_max, n_max, strip, stride, st);
+    interp_t<4, 4, ROWS>(b, pattern0, n, m_max, n_max, strip, stride, st);
   else
-    interp_t<2, 2, ROWS>(pats, coarse, pattern0, n, m_max, n_max, strip, stride, st);
+    interp_t<2, 2, ROWS>(b, pattern0, n, m_max, n_max, strip, stride, st);
 }
 
-cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coarse, int npat, int max_nx, int max_ny,
-                                 int max_nyn, double2 *strip, long long strip_size, cudaStream_t st) {
+cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
+                                 long long strip_size, cudaStream_t st) {
   if (npat <= 0 || max_nx <= 0 || max_ny <= 0) return cudaSuccess;
   const long long stride = (long long)max_nyn * max_nx;
   const int group = (int)std::min<long long>(std::max<long long>(strip_size / stride, 1), 65535);
   for (int p0 = 0; p0 < npat; p0 += group) {
     const int n = std::min(group, npat - p0);
-    interp_part<false>(pats, coarse, p0, n, max_nx, 2 * max_nyn, strip, stride, st);
-    interp_part<true>(pats, coarse, p0, n, max_ny, 2 * max_nx, strip, stride, st);
+    interp_part<false>(b, p0, n, max_nx, 2 * max_nyn, strip, stride, st);
+    interp_part<true>(b, p0, n, max_ny, 2 * max_nx, strip, stride, st);
   }
   return cudaGetLastError();
 }

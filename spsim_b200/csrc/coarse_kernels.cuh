@@ -64,11 +64,22 @@ __host__ __device__ inline int coarse_ld(int n) { return (n + 7) / 8 * 8; }
 // detector; tx, ty: also their transposes, [nodes][coarse_ld(pixels)].
 cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
                                  double *my, cudaStream_t st, double *tx = nullptr, double *ty = nullptr);
-// Interpolates npat patterns: F, I of pats[i] (or coarse[i].out) from
-// coarse[i].nodes, in groups of as many patterns as the strip buffer holds
+// The patterns of one interpolation: either described one by one (pats, coarse)
+// or, pats == nullptr, alike: pattern i reads one.nodes + i * nyn * nxn, takes
+// the rotation rots + 9 i (or none) and writes F + i * npix and I + i * npix.
+struct CoarseBatch {
+  const SfPattern *pats;
+  const CoarsePattern *coarse;
+  CoarsePattern one;
+  const double *q64, *rots;
+  double center[3];
+  float2 *F;
+  float *I;
+};
+// Interpolates npat patterns in groups of as many as the strip buffer holds
 // (strip_size complex values, at least max_nyn * max_nx).
-cudaError_t launch_coarse_interp(const SfPattern *pats, const CoarsePattern *coarse, int npat, int max_nx, int max_ny,
-                                 int max_nyn, double2 *strip, long long strip_size, cudaStream_t st);
+cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
+                                 long long strip_size, cudaStream_t st);
 
 // The adjoint of the interpolation: per pattern, from the forward's F and
 // G = dL/d|F|^2 on the pixels to the amplitudes H on the nodes.

@@ -322,10 +322,10 @@ __global__ void __launch_bounds__(FFT_THREADS, 3) nufft_fft_y_kernel(const __gri
 }
 
 // z pass: columns of [E][n1z][my][mx] for elements [e0, e0 + per_elem) and
-// per_cta neighbouring x of one y; out: the interpolation's FP32 grid,
-// float2 slots [group][nout][my][mx][slots], element e in group e / slots,
-// slot e mod slots; slots past the last element are written as zeros
-template <bool PAD>
+// per_cta neighbouring x of one y; out: the interpolation's grid, complex
+// slots [group][nout][my][mx][slots] (FP32, or FP64 for F64), element e in
+// group e / slots, slot e mod slots; slots past the last element are zeros
+template <bool PAD, bool F64>
 __global__ void __launch_bounds__(FFT_THREADS, 3) nufft_fft_z_kernel(const __grid_constant__ FftPassZ a) {
   extern __shared__ double2 sm[];
   const FftAxis &ax = a.ax;
@@ -365,15 +365,15 @@ __global__ void __launch_bounds__(FFT_THREADS, 3) nufft_fft_z_kernel(const __gri
   const int el = threadIdx.x % nw, c = (threadIdx.x / nw) % nc, o0 = threadIdx.x / lw, step = FFT_THREADS / lw;
   if (o0 >= step) return;
   const int e = e0 + el, grp = e / a.slots;
-  float2 *out = a.packed + (((long long)grp * ax.nout * a.my + py) * a.mx + x0 + c) * a.slots + (e - grp * a.slots);
+  const long long out0 = (((long long)grp * ax.nout * a.my + py) * a.mx + x0 + c) * a.slots + (e - grp * a.slots);
   const long long ostride = plane * a.slots;
   for (int o = o0; o < ax.nout; o += step) {
-    float2 v = make_float2(0.0f, 0.0f);
-    if (el < ne) {
-      const double2 d = r[(el * nc + c) * ax.ld + out_pos<PAD>(o, ax)];
-      v = make_float2((float)d.x, (float)d.y);
-    }
-    out[o * ostride] = v;
+    double2 d = make_double2(0.0, 0.0);
+    if (el < ne) d = r[(el * nc + c) * ax.ld + out_pos<PAD>(o, ax)];
+    if (F64)
+      ((double2 *)a.packed)[out0 + o * ostride] = d;
+    else
+      ((float2 *)a.packed)[out0 + o * ostride] = make_float2((float)d.x, (float)d.y);
   }
 }
 
@@ -429,8 +429,10 @@ static cudaError_t smem_opt_in() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev == done_dev) return e;
   for (const void *f : {(const void *)nufft_fft_x_kernel<false>, (const void *)nufft_fft_y_kernel<false>,
-                        (const void *)nufft_fft_z_kernel<false>, (const void *)nufft_fft_x_kernel<true>,
-                        (const void *)nufft_fft_y_kernel<true>, (const void *)nufft_fft_z_kernel<true>}) {
+                        (const void *)nufft_fft_z_kernel<false, false>, (const void *)nufft_fft_z_kernel<false, true>,
+                         (const void *)nufft_fft_x_kernel<true>,
+                        (const void *)nufft_fft_y_kernel<true>, (const void *)nufft_fft_z_kernel<true, false>,
+                         (const void *)nufft_fft_z_kernel<true, true>}) {
     e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
     if (e != cudaSuccess) return e;
   }
@@ -445,7 +447,7 @@ static int lines_for(const FftAxis &ax, int cap) {
 }
 
 cudaError_t nufft_fft3(const double *small, int copies, const double *dec, const NufftGeom &g, int n_elem,
-                       const FftAxis ax[3], double2 *fa, double2 *fb, float4 *packed, cudaStream_t st) {
+                       const FftAxis ax[3], double2 *fa, double2 *fb, void *packed, bool f64, cudaStream_t st) {
   cudaError_t e = smem_opt_in();
   if (e != cudaSuccess) return e;
   const int mx = ax[0].nout, my = ax[1].nout;
@@ -489,7 +491,7 @@ cudaError_t nufft_fft3(const double *small, int copies, const double *dec, const
     FftPassZ p;
     p.ax = ax[2];
     p.in = fb;
-    p.packed = (float2 *)packed;
+    p.packed = packed;
     p.mx = mx;
     p.my = my;
     p.n_elem = n_elem;
@@ -506,10 +508,12 @@ cudaError_t nufft_fft3(const double *small, int copies, const double *dec, const
     const size_t smem = 2 * (size_t)p.per_elem * p.per_cta * ax[2].ld * sizeof(double2);
     const dim3 grid((unsigned)((mx + p.per_cta - 1) / p.per_cta), (unsigned)my,
                     (unsigned)((n_elem + p.per_elem - 1) / p.per_elem));
-    if (p.ax.pad)
-      nufft_fft_z_kernel<true><<<grid, FFT_THREADS, smem, st>>>(p);
+    if (f64)
+      p.ax.pad ? nufft_fft_z_kernel<true, true><<<grid, FFT_THREADS, smem, st>>>(p)
+               : nufft_fft_z_kernel<false, true><<<grid, FFT_THREADS, smem, st>>>(p);
     else
-      nufft_fft_z_kernel<false><<<grid, FFT_THREADS, smem, st>>>(p);
+      p.ax.pad ? nufft_fft_z_kernel<true, false><<<grid, FFT_THREADS, smem, st>>>(p)
+               : nufft_fft_z_kernel<false, false><<<grid, FFT_THREADS, smem, st>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;

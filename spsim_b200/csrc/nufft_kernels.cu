@@ -6,6 +6,8 @@
 // form factor of |q| with the B factor (src/diffraction.c:390-400).
 #include "nufft_kernels.cuh"
 
+#include <type_traits>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -520,6 +522,18 @@ __global__ void __launch_bounds__(INTERP_THREADS, 3) nufft_interp_tile_kernel(co
   if (active) write_pixel(a, (long long)blockIdx.y * a.npix + p, s, fr, fi);
 }
 
+// f(std::integral_constant of the stencil width w)
+template <typename F>
+static cudaError_t with_width(int w, F f) {
+  switch (w) {
+#define W(n) \
+  case n: return f(std::integral_constant<int, n>{});
+    W(4) W(5) W(6) W(7) W(8) W(9) W(10) W(11) W(12) W(13) W(14) W(15)
+#undef W
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 template <int W>
 static cudaError_t interp_t(const NufftInterp &a, cudaStream_t st) {
   long long blocks = (a.npix + INTERP_THREADS - 1) / INTERP_THREADS;
@@ -551,27 +565,128 @@ static cudaError_t interp_t(const NufftInterp &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Interpolation at a coarse grid's nodes, FP64 throughout: what a node is off
+// by goes into the pixels around it, a bright one's error into dim pixels (the
+// FP32 grid's 4e-9 of the brightest gave up to twice the maximum error of
+// stencils at every pixel).  A warp takes one node, its lanes (element slot,
+// neighbouring x, four rows of the stencil): neighbouring nodes' warps, eight to
+// a block, find most of each other's rows in L1.  Bound by the L1 data path
+// (W^3 x 64 B per node).
+constexpr int NODE_WARPS = 8;
+
+template <int W, int SLOTS>
+__global__ void __launch_bounds__(32 * NODE_WARPS) nufft_nodes_kernel(const __grid_constant__ NufftInterp a,
+                                                                      double2 *__restrict__ out) {
+  __shared__ double wgt[NODE_WARPS][3][W];
+  constexpr int XS = 2, ROWS = 32 / (SLOTS * XS), NX = (W + XS) / XS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long p = (long long)blockIdx.x * NODE_WARPS + warp;
+  if (p >= a.npix) return;
+  const NufftGeom &g = a.g;
+  const double h0 = a.q64[3 * p], h1 = a.q64[3 * p + 1], h2 = a.q64[3 * p + 2];
+  double q[3] = {h0, h1, h2};
+  const double *R = a.rots ? a.rots + 9 * blockIdx.y : (a.has_rot ? a.rot : nullptr);
+  if (R) {
+    q[0] = R[0] * h0 + R[1] * h1 + R[2] * h2;
+    q[1] = R[3] * h0 + R[4] * h1 + R[5] * h2;
+    q[2] = R[6] * h0 + R[7] * h1 + R[8] * h2;
+  }
+  int b[3];
+  double D = 1.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double qp = q[d] - g.cq[d];
+    const double t = qp * g.L[d];
+    const double p0 = ceil(t - 0.5 * W);
+    b[d] = min(max((int)p0 - g.pmin[d], 0), g.m[d] - W);
+    if (lane < W) wgt[warp][d][lane] = es_kernel(t - p0 - lane, 2.0 / W, g.beta2);
+    // psi1hat(xi) = sum_k a_k cos(2 pi xi k / 4), a term or two per lane
+    double s = 0.0;
+    for (int k = lane; k < a.n_coef; k += 32) s = fma(a.psi_a[k], cospi(0.5 * k * g.h[d] * qp), s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    D *= s;
+  }
+  __syncwarp();
+  const double s2 = (h0 * h0 + h1 * h1 + h2 * h2) * 0.25e-20;
+  const int el = lane % SLOTS, xs = lane / SLOTS % XS, r0 = lane / (SLOTS * XS);
+  const double *wy = wgt[warp][1], *wz = wgt[warp][2];
+  // this lane's x, in aligned pairs of cells (the box is of even width): a warp's
+  // load is then four whole 128-byte lines
+  const int off = b[0] & 1;
+  double wx[NX];
+#pragma unroll
+  for (int k = 0; k < NX; ++k) {
+    const int i = XS * k + xs - off;
+    wx[k] = i >= 0 && i < W ? wgt[warp][0][i] : 0.0;
+  }
+  const long long row_stride = (long long)g.m[0] * SLOTS, plane_stride = row_stride * g.m[1];
+  double fr = 0.0, fi = 0.0;
+  for (int grp = 0; grp < a.n_groups; ++grp) {
+    const double2 *gr = (const double2 *)a.packed + grp * a.cell2 * SLOTS + (long long)b[2] * plane_stride +
+                        b[1] * row_stride + (long long)(b[0] - off) * SLOTS + el;
+    double re = 0.0, im = 0.0;
+#pragma unroll 3
+    for (int r = r0; r < W * W; r += ROWS) {
+      const int jz = r / W, jy = r - jz * W;
+      const double2 *row = gr + jz * plane_stride + jy * row_stride + xs * SLOTS;
+      double2 v[NX];
+#pragma unroll
+      for (int k = 0; k < NX; ++k)
+        v[k] = wx[k] != 0.0 ? __ldg(row + XS * k * SLOTS) : make_double2(0.0, 0.0);
+      double sr = 0.0, si = 0.0;
+#pragma unroll
+      for (int k = 0; k < NX; ++k) {
+        sr = fma(wx[k], v[k].x, sr);
+        si = fma(wx[k], v[k].y, si);
+      }
+      const double w = wz[jz] * wy[jy];
+      re = fma(w, sr, re);
+      im = fma(w, si, im);
+    }
+    for (int o = SLOTS; o < 32; o *= 2) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    const int e = grp * SLOTS + el;
+    double f = e < a.n_elem ? 1.0 : 0.0;
+    if (!a.delta_atoms && e < a.n_elem) {
+      const float *c = a.coeffs + 9 * e;
+      f = c[8];
+      for (int i = 0; i < 4; ++i) f += (double)c[i] * exp(-(double)c[i + 4] * s2);
+    }
+    fr = fma(f, re, fr);
+    fi = fma(f, im, fi);
+  }
+  for (int o = 1; o < SLOTS; o *= 2) {
+    fr += __shfl_xor_sync(0xffffffffu, fr, o);
+    fi += __shfl_xor_sync(0xffffffffu, fi, o);
+  }
+  if (lane == 0) out[blockIdx.y * a.npix + p] = make_double2(fr / D, fi / D);
+}
+
+template <int W>
+static cudaError_t nodes_t(const NufftInterp &a, double2 *out, cudaStream_t st) {
+  const dim3 grid((unsigned)((a.npix + NODE_WARPS - 1) / NODE_WARPS), (unsigned)std::max(a.npat, 1));
+  if (a.halves == 1)
+    nufft_nodes_kernel<W, 2><<<grid, 32 * NODE_WARPS, 0, st>>>(a, out);
+  else
+    nufft_nodes_kernel<W, 4><<<grid, 32 * NODE_WARPS, 0, st>>>(a, out);
+  return cudaGetLastError();
+}
+
+cudaError_t nufft_nodes(const NufftInterp &a, double2 *out, cudaStream_t st) {
+  if (a.npix <= 0) return cudaSuccess;
+  if (a.halves != 1 && a.halves != 2) return cudaErrorInvalidValue;
+  return with_width(a.g.w2, [&](auto w) { return nodes_t<w()>(a, out, st); });
+}
+
 void nufft_set_interp_mode(int mode) { g_interp_mode = mode; }
 int nufft_interp_mode() { return g_interp_mode; }
 
 cudaError_t nufft_interp(const NufftInterp &a, cudaStream_t st) {
   if (a.npix <= 0) return cudaSuccess;
   if (a.halves != 1 && a.halves != 2) return cudaErrorInvalidValue;
-  switch (a.g.w2) {
-    case 4: return interp_t<4>(a, st);
-    case 5: return interp_t<5>(a, st);
-    case 6: return interp_t<6>(a, st);
-    case 7: return interp_t<7>(a, st);
-    case 8: return interp_t<8>(a, st);
-    case 9: return interp_t<9>(a, st);
-    case 10: return interp_t<10>(a, st);
-    case 11: return interp_t<11>(a, st);
-    case 12: return interp_t<12>(a, st);
-    case 13: return interp_t<13>(a, st);
-    case 14: return interp_t<14>(a, st);
-    case 15: return interp_t<15>(a, st);
-    default: return cudaErrorInvalidValue;
-  }
+  return with_width(a.g.w2, [&](auto w) { return interp_t<w()>(a, st); });
 }
 
 }  // namespace spsim

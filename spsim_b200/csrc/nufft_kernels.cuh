@@ -75,7 +75,7 @@ struct FftPassY {
 struct FftPassZ {
   FftAxis ax;
   const double2 *in;     // [E][n1z][my][mx]
-  float2 *packed;        // [groups][mz][my][mx][slots]
+  void *packed;          // [groups][mz][my][mx][slots], float2 or double2
   int mx, my, n_elem, slots, n_groups;
   int per_cta, per_elem;
 };
@@ -126,16 +126,20 @@ cudaError_t nufft_pad(const double2 *small, double2 *fine, const NufftGeom &g, i
 // Steps 2-3 by the hand-written passes: x (with the sum of the spreading-grid
 // copies and the deconvolution), y, z (with the FP32 element-interleaved
 // output of nufft_pack_groups(n_elem) x box cells x nufft_pack_halves(n_elem)
-// float4).  fa: E n1z n1y m_x, fb: E n1z m_y m_x double2.
+// float4; f64: the same cells in FP64, for nufft_nodes).  fa: E n1z n1y m_x, fb:
+// E n1z m_y m_x double2.
 int nufft_pack_halves(int n_elem);
 int nufft_pack_groups(int n_elem);
 int nufft_fft_axis(int n, int nin, int pmin, int nout, const double2 *tw, FftAxis *ax);  // 0, or -1: n unsupported
 void nufft_fft_twiddles(int n, double2 *tw);  // host table exp(-2 pi i k / n)
 cudaError_t nufft_fft3(const double *small, int copies, const double *dec, const NufftGeom &g, int n_elem,
-                       const FftAxis ax[3], double2 *fa, double2 *fb, float4 *packed, cudaStream_t st);
+                       const FftAxis ax[3], double2 *fa, double2 *fb, void *packed, bool f64, cudaStream_t st);
 // Step 4.  Detector q sets (tile_nx > 0) take the tile path unless the mode is
 // 1 (the per-pixel path everywhere; both give the same bits).
 cudaError_t nufft_interp(const NufftInterp &a, cudaStream_t st);
+// Step 4 at the nodes of a coarse grid (a.q64, row-major): centred amplitudes
+// out[npat][npix] in FP64, without F, I and B, from the FP64 grid (a.packed).
+cudaError_t nufft_nodes(const NufftInterp &a, double2 *out, cudaStream_t st);
 void nufft_set_interp_mode(int mode);
 int nufft_interp_mode();
 

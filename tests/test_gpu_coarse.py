@@ -214,3 +214,28 @@ def test_adjoint_of_b_factors_beyond_the_grids_limit(cuda):
         assert _rel(dpos.cpu().numpy(), dp) < 1e-4
         assert _rel(docc.cpu().numpy(), do) < 1e-4
         assert _rel(dB.cpu().numpy(), db) < 1e-4
+
+
+@pytest.mark.parametrize("eps", [1e-3, 1e-6, 1e-8, 1e-12])
+@pytest.mark.parametrize("elements", [(6, 8), (6, 7, 8, 16), (1, 6, 7, 8, 16, 26)], ids=["2", "4", "6"])
+def test_nufft_at_the_nodes(cuda, eps, elements):
+    # 2^16 pixels: the NUFFT's stencils at the nodes of the detector's grid, two
+    # and four element slots a cell and two groups, narrow and wide stencils, one
+    # rotated pattern and a batch, with a global B and a centre phase; tolerances
+    # of the NUFFT against the sum (relative L2 max(3 eps, 2e-7), maximum
+    # max(30 eps, 2e-6) of the largest amplitude)
+    _, pos = synth.random_molecule(2000, 2.6e-9, 231)
+    pos += np.float32(6e-9)
+    Z = np.random.Generator(np.random.PCG64(232)).choice(elements, len(pos)).astype(np.int32)
+    d = _det(250, 263)
+    R = synth.haar_rotations(2, 233)
+    mol, qs = core.Molecule(Z, pos), core.QSet.from_detector(**d)
+    F1, I1 = core.forward_nufft(mol, qs, rot=R[0], B=5.0, eps=eps)
+    F2, I2 = core.forward_nufft_batch(mol, qs, R, B=5.0, eps=eps)
+    core.synchronize()
+    for F, I, r in ((F1, I1, R[0]), (F2[0], I2[0], R[0]), (F2[1], I2[1], R[1])):
+        F64, I64 = O.structure_factor(Z, pos.astype(np.float64), _q(d) @ r.T, B=5.0)
+        dF = np.abs(F.cpu().numpy() - F64)
+        assert np.linalg.norm(dF) < max(3 * eps, 2e-7) * np.linalg.norm(F64)
+        assert dF.max() < max(30 * eps, 2e-6) * np.abs(F64).max()
+        assert np.abs(I.cpu().numpy() - I64).max() < max(60 * eps, 4e-6) * I64.max()
