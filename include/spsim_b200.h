@@ -33,7 +33,7 @@ extern "C" {
 #define SPSIM_ERR_UNSUPPORTED 7
 
 /* ---- precision of the structure-factor sum ----------------------------- */
-#define SPSIM_PREC_FP64 0        /* plain FP64 per-pixel kernel (FP64 phase, sincos, sum)      */
+#define SPSIM_PREC_FP64 0        /* FP64 phase, sincos and sum                                  */
 #define SPSIM_PREC_F32 1         /* FP64 (or compensated FP32) phase, FMA-pipe minimax sin/cos,*/
                                  /* float-float segment sums, FP64 cross-tile/element sum;     */
                                  /* <= 1e-5 relative |F|^2 error against FP64                  */
@@ -110,16 +110,16 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
 
 /* ---- structure factor ---------------------------------------------------
  * q sets made from a detector are oversampled: no atom's phase turns more than
- * |dq/dx| |r - c|max cycles per pixel.  The FP32 forwards (one pattern, a
- * batch, a spectrum) therefore evaluate the sum on a tensor grid of nodes, a
+ * |dq/dx| |r - c|max cycles per pixel.  The forwards (one pattern, a batch, a
+ * spectrum) therefore evaluate the sum on a tensor grid of nodes, a
  * little more than two per cycle along each axis, and interpolate it to the
- * pixels in FP64, to 1e-8 of an outermost atom's amplitude and far less for
- * the others; form factors and per-atom B factors belong to the interpolated
+ * pixels in FP64, to 1e-8 of an outermost atom's amplitude (1e-12 with
+ * SPSIM_PREC_FP64) and far less for the others; form factors and per-atom B factors belong to the interpolated
  * sum, the global B factor and the centre phase are applied per pixel.  This
  * is done where it is faster (patterns of more than about 1e7 terms), for
  * whole batches or not at all, and in FP64 for molecules rewritten on the
  * device (refinements: a node's rounding error would enter the pixels around it
- * alike and add up in a gradient); q lists, FP64, forced variants
+ * alike and add up in a gradient); q lists, forced variants
  * (spsim_b200_set_variant), detectors further than 1.2 detector distances off
  * the beam axis and per-atom B factors beyond twice their largest at creation
  * + 100 A^2 (checked on the device when they are rewritten there) take the

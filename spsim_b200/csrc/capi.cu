@@ -791,10 +791,12 @@ struct CoarseGrid {
   CoarseAxis x, y;
 };
 
+// fp64: nodes for FP64 sums (1e-12 instead of 1e-8).
 static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale,
-                       CoarseGrid *grid) {
+                       CoarseGrid *grid, bool fp64 = false) {
   const DetGeom &g = q->geom;
   if (!q->has_geom || m->n_kept == 0 || g.nx < 16 || g.ny < 16) return false;
+  if (!(q->qmax * scale * m->rbound < std::ldexp(1.0, 40))) return false;  // the FP64 sums' rounding reduction
   double bmax = m->per_atom_b ? (double)m->b_limit * bscale * bscale : 0.0;
   if (!m->delta_atoms) {
     double c = 0;
@@ -817,7 +819,7 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
     const double c = 2.0 * M_PI * m->rbound * scale * arc * (t > 1.0 ? 1.02 : 1.0);
     const double a = bmax * 0.25e-20 * reach * reach;
     if (!(c <= 1.5 * COARSE_MAX_NODES) || !(t <= 1.2) || !(a <= 60.0)) return false;
-    const int n = coarse_node_count(c, t, a);
+    const int n = coarse_node_count(c, t, a, fp64);
     if (n > COARSE_MAX_NODES) return false;
     coarse_set_nodes(ax, n);
   }
@@ -827,12 +829,13 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
 // Whether the plan's patterns run on coarse grids, with their node counts.
 // All of them or none: a batch is one launch of one kernel.  The times weighed
 // are the measured rates on B200 (direct sum on neighbour quads 1.75e12 terms/s;
-// on nodes, each with its own FP64 phase, 1.3e12; the interpolation 1e13 FP64
-// multiply-adds/s) and the interpolation's launches and tail, ~4 us: patterns of
+// on nodes, each with its own FP64 phase, 1.3e12; in FP64 on pixels 2e11, on
+// nodes 7e11; the interpolation 1e13 FP64 multiply-adds/s) and the interpolation's launches and tail, ~4 us: patterns of
 // less than about 1e7 terms stay on the direct sum.
 static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                         const double *rot, int precision, const Spectrum *spec, std::vector<CoarseGrid> &nodes) {
-  if (precision == SPSIM_PREC_FP64 || g_force_nt > 0) return false;
+  const bool fp64 = precision == SPSIM_PREC_FP64;
+  if (!fp64 && g_force_nt > 0) return false;
   double qscale = 1.0;
   if (spec)
     for (int i = 0; i < npat; ++i) qscale = std::max(qscale, std::fabs(spec->qscale[i]));
@@ -841,16 +844,17 @@ static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const 
   for (int i = 0; i < npat; ++i) {
     double stretch = 1.0;  // of |q| under this pattern's matrix
     if (rot && !is_orthonormal(rot + 9 * (size_t)i)) stretch = std::max(1.0, frobenius(rot + 9 * (size_t)i));
+    if (fp64 && mols[i]->per_atom_b && mols[i]->b_updated) return false;  // no plan on every pixel stands by
     if (i > 0 && stretch == 1.0 && mols[i] == mols[i - 1] && qsets[i] == qsets[i - 1] &&
         !(rot && !is_orthonormal(rot + 9 * (size_t)(i - 1)))) {
       nodes[i] = nodes[i - 1];
-    } else if (!coarse_fit(mols[i], qsets[i], qscale * stretch, stretch, &nodes[i])) {
+    } else if (!coarse_fit(mols[i], qsets[i], qscale * stretch, stretch, &nodes[i], fp64)) {
       return false;
     }
     const double npix = (double)qsets[i]->npix, kept = mols[i]->n_kept;
     const double nxn = nodes[i].x.n, nyn = nodes[i].y.n;
-    direct += kept * npix / 1.75e12;
-    grid += kept * nxn * nyn / 1.3e12 + 2.0 * (npix + qsets[i]->geom.nx * nxn) * nyn / 1e13;
+    direct += kept * npix / (fp64 ? 2e11 : 1.75e12);
+    grid += kept * nxn * nyn / (fp64 ? 7e11 : 1.3e12) + 2.0 * (npix + qsets[i]->geom.nx * nxn) * nyn / 1e13;
   }
   return grid < 0.8 * direct;
 }
@@ -989,11 +993,13 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   pl.ppt = var.p;
   pl.packed = var.packed;
   if (pl.coarse) {
-    // the FP64 kernel (sf_nodes.cu) for molecules rewritten on the device and for
-    // grids that latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
+    // the FP64 kernel (sf_nodes.cu) for FP64, for molecules rewritten on the device
+    // and for grids that latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
     bool updated = false;
     for (int i = 0; i < npat; ++i) updated = updated || mols[i]->updated;
-    pl.node_tile = pl.evaluated <= 4e6 ? SF_NODES64_SMALL_TILE : updated ? SF_NODES64_TILE : SF_NODES_TILE;
+    pl.node_tile = pl.evaluated <= 4e6                            ? SF_NODES64_SMALL_TILE
+                   : updated || precision == SPSIM_PREC_FP64 ? SF_NODES64_TILE
+                                                             : SF_NODES_TILE;
   }
   const long long tile_pix = pl.coarse ? pl.node_tile : (long long)nt * ppt;
 
@@ -1134,7 +1140,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     CUDA_TRY(cudaMemcpyAsync(pl.spec_w.p, spec->weight, npat * sizeof(double), cudaMemcpyHostToDevice, stream));
   }
 
-  if (precision != SPSIM_PREC_FP64) {
+  if (precision != SPSIM_PREC_FP64 || pl.coarse) {
     // work items: pixel tile x atom-tile range, cost-sorted (largest first)
     const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw)
                                           : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
@@ -1223,7 +1229,7 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
     if ((e = cudaMemsetAsync(pl.flags.p, 0, sizeof(int), stream))) return e;  // work queue head
   }
   if (ev0 && (e = cudaEventRecord(ev0, stream))) return e;
-  if (pl.precision == SPSIM_PREC_FP64) {
+  if (pl.precision == SPSIM_PREC_FP64 && !pl.coarse) {
     for (int i = 0; i < pl.npat; ++i)
       if ((e = launch_sf_f64((const SfPattern *)pl.pats.p, i, pl.npix_of[i], stream))) return e;
   } else if (pl.n_items > 0) {

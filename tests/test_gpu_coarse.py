@@ -40,7 +40,7 @@ def _on_grid(yes=True):
 
 
 @pytest.mark.parametrize("nx,ny", [(64, 250), (127, 130), (129, 95), (200, 61), (257, 256), (1000, 17)])
-@pytest.mark.parametrize("precision", ["f32", "f32_fast"])
+@pytest.mark.parametrize("precision", ["f32", "f32_fast", "fp64"])
 def test_ragged_detectors(cuda, nx, ny, precision):
     Z, pos = synth.random_molecule(3000, 3.0e-9, 201)
     pos += np.float32(5e-9)  # a centre phase
@@ -120,6 +120,23 @@ def test_b_factors_rewritten_beyond_the_grids_limit(cuda):
             _check(F[k], I[k], Z, pos, q @ R[k].T, bfac=bk)
 
 
+def test_fp64_at_its_own_tolerance(cuda):
+    # 2e-7 floored maximum, 1e-7 L2: the float32 outputs' rounding; weights, B factors, a wide detector
+    Z, pos = synth.random_molecule(1500, 2.5e-9, 212)
+    rng = np.random.Generator(np.random.PCG64(213))
+    occ = rng.uniform(-0.5, 1.0, len(Z)).astype(np.float32)
+    b = rng.uniform(0.0, 60.0, len(Z)).astype(np.float32)
+    for d in (_det(130, 141), _det(128, 97, distance=0.02), _det(100, 120, spherical=True)):
+        q, qs = _q(d), core.QSet.from_detector(**d)
+        for b_, B in ((None, 0.0), (b, 6.0)):
+            F, I = core.forward(core.Molecule(Z, pos, occ=occ, bfac=b_), qs, B=B, precision="fp64")
+            _on_grid()
+            F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q, occ=occ, bfac=b_, B=B)
+            e_max, e_l2 = intensity_errors(I.cpu().numpy(), I64)
+            assert e_max < 2e-7 and e_l2 < 1e-7, (e_max, e_l2)
+            assert np.linalg.norm(F.cpu().numpy() - F64) < 1e-7 * np.linalg.norm(F64)
+
+
 def test_general_matrices_and_spectrum(cuda):
     Z, pos = synth.random_molecule(2500, 2.6e-9, 209)
     d = _det(132, 136)
@@ -147,7 +164,7 @@ def test_calls_that_stay_on_every_pixel(cuda):
     mol = core.Molecule(Z, pos)
     d = _det(128, 128)
     qs = core.QSet.from_detector(**d)
-    cases = [(qs, "fp64"), (core.QSet.from_list(qs.q()), "f32"), (core.QSet.from_detector(**_det(15, 2000)), "f32"),
+    cases = [(core.QSet.from_list(qs.q()), "fp64"), (core.QSet.from_list(qs.q()), "f32"), (core.QSet.from_detector(**_det(15, 2000)), "f32"),
              (core.QSet.from_detector(**_det(128, 128, pixel=1e-3, distance=0.05)), "f32"),  # 64 mm at 50 mm
              (core.QSet.from_detector(**_det(128, 128, wavelength=0.01e-9)), "f32")]  # undersampled
     for q, precision in cases:
