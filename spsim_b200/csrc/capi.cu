@@ -670,7 +670,11 @@ struct Plan {
   std::vector<const void *> key_ptrs;
   std::vector<double> key_vals;
   // device state
-  DevBuf pats, items, acc, ff, flags;
+  int device = 0;
+  cudaStream_t stream = nullptr;
+  // acc: a head of 64 bytes (ints 4 and 5 the sticky error words, int 8 the work
+  // queue's), then the sums; a launch clears from the queue's head on at once
+  DevBuf pats, items, acc, ff;
   int n_items = 0, grid = 0, npat = 0;
   long long max_npix = 0;
   double terms = 0, evaluated = 0;  // atom.pixel terms of the patterns, and those evaluated (on nodes: fewer)
@@ -688,7 +692,10 @@ struct Plan {
   // coarse grids: the descriptors hold npat node patterns, then the npat pixel
   // patterns that the interpolation writes
   bool coarse = false;
-  DevBuf tables, cpats, pix_acc, strip;
+  DevBuf grids;  // the four below
+  double *tables = nullptr;
+  CoarsePattern *cpats = nullptr;
+  double2 *pix_acc = nullptr, *strip = nullptr;
   long long strip_size = 0;
   int max_nx = 0, max_ny = 0, max_nyn = 0;
   // the same patterns on every pixel, run where a B factor rewritten on the
@@ -697,9 +704,21 @@ struct Plan {
   DevBuf gate;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  ~Plan() {
+  cudaEvent_t done = nullptr;  // recorded after each launch of a cached plan
+  int *head() { return (int *)acc.p; }
+  double2 *sums() { return (double2 *)((char *)acc.p + 64); }
+  size_t bytes() const {
+    return pats.cap + items.cap + acc.cap + ff.cap + grids.cap + spec_w.cap + gate.cap + (direct ? direct->bytes() : 0);
+  }
+  void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
+    exec = nullptr;
+    graph = nullptr;
+  }
+  ~Plan() {
+    drop_graph();
+    if (done) cudaEventDestroy(done);
   }
 };
 
@@ -710,12 +729,14 @@ struct OneShot {  // per-thread scratch plan of uncached calls; lives until the 
 };
 static thread_local OneShot g_oneshot;
 static const size_t kMaxPlans = 8;
+static const size_t kMaxKeptBytes = 256u << 20;  // of a plan whose buffers its successor may take over
 static int g_force_nt = -1, g_force_p = -1, g_force_pk = 3;
 struct Variant {
   int nt, p, packed;
   int p_fallback = 0;  // pixels per thread where form 4 or 3 is not admitted (0: p's nearest)
 };
 static std::map<long long, Variant> g_tuned;  // size class -> kernel variant
+static long long g_tunings = 0;               // changes of g_tuned: plans made before one are not matched after it
 static bool g_timing = false;
 static std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_timing_events;
 static thread_local double g_last_terms = 0, g_last_evaluated = 0, g_last_ms = 0;
@@ -906,10 +927,9 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   pl.evaluated = 0;
   for (int i = 0; i < npat; ++i) pl.evaluated += (double)points[i] * mols[i]->n_kept;
   pl.perb = perb;
-  CUDA_TRY(pl.acc.ensure(std::max<size_t>(acc_total, 1) * sizeof(double2)));
+  CUDA_TRY(pl.acc.ensure(64 + std::max<size_t>(acc_total, 1) * sizeof(double2)));
   CUDA_TRY(pl.ff.ensure(std::max<size_t>(ff_total, 1) * sizeof(double)));
-  CUDA_TRY(pl.flags.ensure(64));
-  CUDA_TRY(cudaMemsetAsync(pl.flags.p, 0, 64, stream));  // queue head and the sticky error word
+  CUDA_TRY(cudaMemsetAsync(pl.acc.p, 0, 64, stream));  // queue head and the sticky error words
   CUDA_TRY(pl.pats.ensure((pl.coarse ? 2 : 1) * std::max(npat, 1) * sizeof(SfPattern)));
 
   // node grids: one set of node q vectors and interpolation matrices per (q set, node counts)
@@ -936,9 +956,26 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       pix_off[i] = pix_total;
       pix_total += qsets[i]->npix;
     }
-    CUDA_TRY(pl.tables.ensure(tab_total * sizeof(double)));
-    CUDA_TRY(pl.cpats.ensure(npat * sizeof(CoarsePattern)));
-    if (spec) CUDA_TRY(pl.pix_acc.ensure(std::max<size_t>(pix_total, 1) * sizeof(double2)));
+    pl.max_nx = pl.max_ny = pl.max_nyn = 0;
+    for (int i = 0; i < npat; ++i) {
+      pl.max_nx = std::max(pl.max_nx, qsets[i]->geom.nx);
+      pl.max_ny = std::max(pl.max_ny, qsets[i]->geom.ny);
+      pl.max_nyn = std::max(pl.max_nyn, nodes[i].y.n);
+    }
+    // the interpolation's strips: a group of patterns at a time, 64 MB of them
+    // (they are read back from L2), or one
+    const long long strip = (long long)pl.max_nyn * pl.max_nx;
+    pl.strip_size = strip * std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / strip));
+    auto round = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t at_cpats = round(tab_total * sizeof(double));
+    const size_t at_strip = at_cpats + round(npat * sizeof(CoarsePattern));
+    const size_t at_acc = at_strip + round(pl.strip_size * sizeof(double2));
+    CUDA_TRY(pl.grids.ensure(at_acc + (spec ? pix_total * sizeof(double2) : 0)));
+    char *base = (char *)pl.grids.p;
+    pl.tables = (double *)base;
+    pl.cpats = (CoarsePattern *)(base + at_cpats);
+    pl.strip = (double2 *)(base + at_strip);
+    pl.pix_acc = (double2 *)(base + at_acc);
   }
 
   Variant var = {128, 4, 1};
@@ -1020,7 +1057,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     pt.ff = (double *)pl.ff.p + ffo[i];
     pt.npix = points[i];
     pt.hkl = pl.coarse ? nullptr : q->d_hkl;
-    pt.q64 = pl.coarse ? (double *)pl.tables.p + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)] : q->d_q64;
+    pt.q64 = pl.coarse ? pl.tables + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)] : q->d_q64;
     double qmax = q->qmax;
     if (rot) {
       const double *R = rot + 9 * (size_t)i;
@@ -1040,12 +1077,12 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     qmax *= std::fabs(pt.qscale);
     memcpy(pt.center, m->center, sizeof(pt.center));
     pt.mol_err = m->d_flags;
-    pt.plan_err = (int *)pl.flags.p + 5;
+    pt.plan_err = pl.head() + 5;
     const int eq = ceil_log2_bound(std::max(qmax, 1e-300));
     const int kq = 22 - m->kr;
     pt.dq = (float)std::ldexp(1.0, eq - kq);
     pt.inv_dq = (float)std::ldexp(1.0, kq - eq);
-    pt.acc = (double2 *)pl.acc.p + acc_off[i];
+    pt.acc = pl.sums() + acc_off[i];
     pt.F = F_dev ? (float2 *)F_dev[i] : nullptr;
     pt.I = I_dev ? I_dev[i] : nullptr;
     pl.max_npix = std::max(pl.max_npix, points[i]);
@@ -1082,7 +1119,6 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   }
   if (pl.coarse) {
     std::vector<CoarsePattern> cp(npat);
-    pl.max_nx = pl.max_ny = pl.max_nyn = 0;
     for (int i = 0; i < npat; ++i) {
       const spsim_b200_qset *q = qsets[i];
       size_t n[3];
@@ -1099,26 +1135,18 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       c.ldx = coarse_ld(c.nxn);
       c.ldy = coarse_ld(c.nyn);
       c.B = B;
-      c.out = spec ? (double2 *)pl.pix_acc.p + pix_off[i] : nullptr;
-      pl.max_nx = std::max(pl.max_nx, c.nx);
-      pl.max_ny = std::max(pl.max_ny, c.ny);
-      pl.max_nyn = std::max(pl.max_nyn, c.nyn);
+      c.out = spec ? pl.pix_acc + pix_off[i] : nullptr;
     }
-    // the interpolation's strips: a group of patterns at a time, 64 MB of them
-    // (they are read back from L2), or one
-    const long long strip = (long long)pl.max_nyn * pl.max_nx;
-    pl.strip_size = strip * std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / strip));
-    CUDA_TRY(pl.strip.ensure(pl.strip_size * sizeof(double2)));
     for (const auto &t : tab_off) {
       size_t n[3];
       int i = 0;  // a pattern with this table
       while (TabKey(qsets[i], nodes[i].x.n, nodes[i].y.n) != t.first) ++i;
       tab_sizes(i, n);
-      double *tab = (double *)pl.tables.p + t.second;
+      double *tab = pl.tables + t.second;
       CUDA_TRY(launch_coarse_tables(qsets[i]->geom, nodes[i].x, nodes[i].y, tab, tab + n[0], tab + n[0] + n[1],
                                     stream));
     }
-    CUDA_TRY(cudaMemcpyAsync(pl.cpats.p, cp.data(), npat * sizeof(CoarsePattern), cudaMemcpyHostToDevice, stream));
+    CUDA_TRY(cudaMemcpyAsync(pl.cpats, cp.data(), npat * sizeof(CoarsePattern), cudaMemcpyHostToDevice, stream));
     // the pixel patterns behind the node patterns
     pats.resize(2 * (size_t)npat);
     for (int i = 0; i < npat; ++i) {
@@ -1201,11 +1229,11 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   }
   // B factors rewritten on the device are known there only: the plan on every
   // pixel stands by for values beyond the molecule's limit
-  pl.direct.reset();
   bool updated = false;
   for (int i = 0; i < npat && pl.coarse; ++i) updated = updated || (mols[i]->per_atom_b && mols[i]->b_updated);
+  if (!updated) pl.direct.reset();
   if (updated) {
-    pl.direct.reset(new Plan());
+    if (!pl.direct) pl.direct.reset(new Plan());
     CUDA_TRY(pl.gate.ensure(sizeof(int)));
     return build_plan(*pl.direct, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec, false);
   }
@@ -1221,25 +1249,24 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   long long acc_total = 0;
   for (long long n : pl.npix_of) acc_total += n;
   if (gate) {
-    if ((e = launch_gate((const SfPattern *)pl.pats.p, pl.npat, pl.n_items, gate, (int *)pl.flags.p,
-                         (double2 *)pl.acc.p, acc_total, stream)))
+    if ((e = launch_gate((const SfPattern *)pl.pats.p, pl.npat, pl.n_items, gate, pl.head() + 8, pl.sums(), acc_total,
+                         stream)))
       return e;
-  } else {
-    if ((e = cudaMemsetAsync(pl.acc.p, 0, std::max<long long>(acc_total, 1) * sizeof(double2), stream))) return e;
-    if ((e = cudaMemsetAsync(pl.flags.p, 0, sizeof(int), stream))) return e;  // work queue head
+  } else if ((e = cudaMemsetAsync(pl.head() + 8, 0, 32 + acc_total * sizeof(double2), stream))) {  // queue and sums
+    return e;
   }
   if (ev0 && (e = cudaEventRecord(ev0, stream))) return e;
   if (pl.precision == SPSIM_PREC_FP64 && !pl.coarse) {
     for (int i = 0; i < pl.npat; ++i)
       if ((e = launch_sf_f64((const SfPattern *)pl.pats.p, i, pl.npix_of[i], stream))) return e;
   } else if (pl.n_items > 0) {
-    int *flags = (int *)pl.flags.p;
+    int *queue = pl.head() + 8, *err = pl.head() + 4;
     if (pl.coarse)
       e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
-                          pl.n_items, flags, flags + 4, pl.grid, stream);
+                          pl.n_items, queue, err, pl.grid, stream);
     else
       e = launch_sf_f32(pl.mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
-                        pl.n_items, flags, flags + 4, pl.grid, stream, pl.fixw, pl.narrow);
+                        pl.n_items, queue, err, pl.grid, stream, pl.fixw, pl.narrow);
     if (e) return e;
   }
   if (ev1 && (e = cudaEventRecord(ev1, stream))) return e;
@@ -1249,9 +1276,8 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
     CoarseBatch b;
     memset(&b, 0, sizeof(b));
     b.pats = pats + pixels;
-    b.coarse = (const CoarsePattern *)pl.cpats.p;
-    if ((e = launch_coarse_interp(b, pl.npat, pl.max_nx, pl.max_ny, pl.max_nyn, (double2 *)pl.strip.p, pl.strip_size,
-                                  stream)))
+    b.coarse = pl.cpats;
+    if ((e = launch_coarse_interp(b, pl.npat, pl.max_nx, pl.max_ny, pl.max_nyn, pl.strip, pl.strip_size, stream)))
       return e;
   }
   if (pl.spectrum > 0)
@@ -1264,8 +1290,11 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
 }
 
 static void plan_key(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
-                     const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
-                     const Spectrum *spec, std::vector<const void *> &kp, std::vector<double> &kv) {
+                     const double *rot, float B, int precision, cudaStream_t stream, const Spectrum *spec,
+                     std::vector<const void *> &kp, std::vector<double> &kv) {
+  // a plan belongs to one stream, whose order keeps its launches apart (forwards
+  // on several streams run side by side, each with its own sums)
+  kp.push_back(stream);
   kv.push_back(npat);
   kv.push_back(spec ? spec->samples : 0);
   if (spec) {
@@ -1281,12 +1310,11 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
   kv.push_back(g_force_nt);
   kv.push_back(g_force_p);
   kv.push_back(g_force_pk);
+  kv.push_back((double)g_tunings);
   for (int i = 0; i < npat; ++i) {
     kv.push_back((double)(mols[i] ? mols[i]->id : 0));
     kv.push_back((double)(qsets[i] ? qsets[i]->id : 0));
     kv.push_back(mols[i] ? (mols[i]->updated ? 1.0 : 0.0) + (mols[i]->b_updated ? 2.0 : 0.0) : 0.0);
-    kp.push_back(F_dev ? (const void *)F_dev[i] : nullptr);
-    kp.push_back(I_dev ? (const void *)I_dev[i] : nullptr);
   }
   // Orthonormal rotations only change the descriptors, which are re-uploaded
   // per call; any other matrix changes the phase grid, so it keys the plan.
@@ -1298,37 +1326,53 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
     for (long long k = 0; k < 9LL * npat; ++k) kv.push_back(rot[k]);
 }
 
-// Write this call's rotations into the plan's descriptors (device copy ordered on `stream`).
-static cudaError_t refresh_rotations(Plan &pl, const double *rot, cudaStream_t stream) {
-  if (!rot) return cudaSuccess;
-  bool changed = false;
+// Write this call's rotations and outputs into the plan's descriptors (device
+// copy ordered on `stream`).  New outputs cannot be written while the stream is
+// being captured: the copy's source would be read again at every replay.
+static cudaError_t refresh_descriptors(Plan &pl, const double *rot, float *const *F_dev, float *const *I_dev,
+                                       cudaStream_t stream) {
+  bool changed = false, moved = false;
+  const size_t outputs = pl.coarse ? pl.npat : 0;  // the first pattern with pixels to write
   for (size_t i = 0; i < pl.host_pats.size(); ++i) {
-    const double *R = rot + 9 * (i % (size_t)pl.npat);
-    if (memcmp(pl.host_pats[i].rot, R, 9 * sizeof(double)) != 0) {
-      memcpy(pl.host_pats[i].rot, R, 9 * sizeof(double));
+    SfPattern &pt = pl.host_pats[i];
+    const size_t k = i % (size_t)pl.npat;
+    if (rot && memcmp(pt.rot, rot + 9 * k, 9 * sizeof(double)) != 0) {
+      memcpy(pt.rot, rot + 9 * k, 9 * sizeof(double));
       changed = true;
     }
+    if (i < outputs || pl.spectrum) continue;  // (a spectrum's are the launch's arguments)
+    float2 *F = F_dev ? (float2 *)F_dev[k] : nullptr;
+    float *I = I_dev ? I_dev[k] : nullptr;
+    moved = moved || pt.F != F || pt.I != I;
+    pt.F = F;
+    pt.I = I;
   }
   if (pl.direct) {
-    const cudaError_t e = refresh_rotations(*pl.direct, rot, stream);
+    const cudaError_t e = refresh_descriptors(*pl.direct, rot, F_dev, I_dev, stream);
     if (e != cudaSuccess) return e;
   }
-  if (!changed) return cudaSuccess;
+  if (!changed && !moved) return cudaSuccess;
+  if (moved && stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    if (e != cudaSuccess) return e;
+    if (capture != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
+  }
   return cudaMemcpyAsync(pl.pats.p, pl.host_pats.data(), pl.host_pats.size() * sizeof(SfPattern),
                          cudaMemcpyHostToDevice, stream);
 }
 
 static int check_flags(Plan &pl) {
   int h[8] = {0};
-  CUDA_TRY(cudaMemcpy(h, pl.flags.p, sizeof(h), cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemcpy(h, pl.head(), sizeof(h), cudaMemcpyDeviceToHost));
   if (h[4]) {
     int z = 0;
-    cudaMemcpy((int *)pl.flags.p + 4, &z, sizeof(int), cudaMemcpyHostToDevice);
+    cudaMemcpy(pl.head() + 4, &z, sizeof(int), cudaMemcpyHostToDevice);
     return fail(SPSIM_ERR_TIMEOUT, "structure-factor kernel: an atom-tile copy did not complete in time");
   }
   if (h[5]) {
     int z = 0;
-    cudaMemcpy((int *)pl.flags.p + 5, &z, sizeof(int), cudaMemcpyHostToDevice);
+    cudaMemcpy(pl.head() + 5, &z, sizeof(int), cudaMemcpyHostToDevice);
     return fail(SPSIM_ERR_RANGE, "atoms moved outside the molecule's creation-time bounds");
   }
   return pl.direct ? check_flags(*pl.direct) : SPSIM_OK;
@@ -1357,7 +1401,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
   std::lock_guard<std::mutex> lk(g_mu);
   std::vector<const void *> kp;
   std::vector<double> kv;
-  plan_key(npat, mols, qsets, rot, B, precision, F_dev, I_dev, spec, kp, kv);
+  plan_key(npat, mols, qsets, rot, B, precision, stream, spec, kp, kv);
   Plan *pl = nullptr;
   if (cache) {
     for (size_t i = 0; i < g_plans.size(); ++i) {
@@ -1371,15 +1415,24 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     }
   }
   if (!pl && cache) {
-    std::unique_ptr<Plan> np(new Plan());
+    // the least recently used plan's place, once its last launch is done, and its
+    // buffers with it (allocating and freeing them anew takes longer than most
+    // launches, and a free waits for the whole device) unless they are large
+    std::unique_ptr<Plan> np;
+    if (g_plans.size() >= kMaxPlans) {
+      np = std::move(g_plans.front());
+      g_plans.erase(g_plans.begin());
+      if (np->done) CUDA_TRY(cudaEventSynchronize(np->done));
+      np->drop_graph();
+      if (np->device != dev || np->bytes() > kMaxKeptBytes) np.reset();
+    }
+    if (!np) np.reset(new Plan());
     np->key_ptrs = kp;
     np->key_vals = kv;
+    np->device = dev;
+    if (!np->done) CUDA_TRY(cudaEventCreateWithFlags(&np->done, cudaEventDisableTiming));
     st = build_plan(*np, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec);
     if (st) return st;
-    if (g_plans.size() >= kMaxPlans) {
-      cudaDeviceSynchronize();  // the evicted plan's buffers may still be in use
-      g_plans.erase(g_plans.begin());
-    }
     g_plans.push_back(std::move(np));
     pl = g_plans.back().get();
   } else if (!pl) {
@@ -1412,7 +1465,9 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
               pl->fixw && pl->narrow
           ? 1
           : 0;
-  CUDA_TRY(refresh_rotations(*pl, rot, stream));
+  // a destroyed stream's handle may come back as another stream's: its last launch first
+  if (cache && stream) CUDA_TRY(cudaStreamWaitEvent(stream, pl->done, 0));
+  CUDA_TRY(refresh_descriptors(*pl, rot, F_dev, I_dev, stream));
   if (g_timing || !cache || stream == nullptr) {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (g_timing) {
@@ -1434,6 +1489,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     }
     CUDA_TRY(cudaGraphLaunch(pl->exec, stream));
   }
+  if (cache) CUDA_TRY(cudaEventRecord(pl->done, stream));
   if (!cache && sync) {
     CUDA_TRY(cudaStreamSynchronize(stream));
     return check_flags(*pl);
@@ -1944,14 +2000,31 @@ static double es_host(double u, double w, double beta) {
   return a >= 0.0 ? std::exp(beta * (std::sqrt(a) - 1.0)) : 0.0;
 }
 
-// Fourier transform of the ES kernel, int es(u) e^{-2 pi i xi u} du, by the
-// trapezoid rule at spacing d (spectrally accurate: the kernel is smooth and
-// vanishes to e^{-beta} at its ends)
-static double es_hat_host(double xi, double w, double beta, double d) {
-  const int n = (int)std::floor(0.5 * w / d);
-  double s = 0.5 * es_host(0.0, w, beta);
-  for (int i = 1; i <= n; ++i) s += es_host(i * d, w, beta) * std::cos(2.0 * M_PI * xi * i * d);
-  return 2.0 * d * s;
+// Fourier transform of the ES kernel, int es(u) e^{-2 pi i xi u} du, at xi =
+// k / n for k = 0 .. count - 1 by the trapezoid rule at spacing 0.01 (spectrally
+// accurate: the kernel is smooth and vanishes to e^{-beta} at its ends).  The
+// kernel's values are taken once and the cosines by rotation from an exact one
+// every 64 (2 ms of host time per new grid when every term took its own).
+static void es_hat_host(int n, int count, double w, double beta, std::vector<double> &out) {
+  const double d = 0.01;
+  const int terms = (int)std::floor(0.5 * w / d);
+  std::vector<double> es(terms + 1);
+  for (int i = 0; i <= terms; ++i) es[i] = es_host(i * d, w, beta);
+  out.resize(count);
+  for (int k = 0; k < count; ++k) {
+    const double step = 2.0 * M_PI * ((double)k / n) * d, cs = std::cos(step), sn = std::sin(step);
+    double s = 0.5 * es[0];
+    for (int i0 = 1; i0 <= terms; i0 += 64) {
+      double c = std::cos(step * i0), v = std::sin(step * i0);
+      for (int i = i0; i < std::min(i0 + 64, terms + 1); ++i) {
+        s += es[i] * c;
+        const double t = c * cs - v * sn;
+        v = v * cs + c * sn;
+        c = t;
+      }
+    }
+    out[k] = 2.0 * d * s;
+  }
 }
 
 // Interpolation kernel width (grid points) for a requested relative error of
@@ -2171,9 +2244,11 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
                     (double)(bytes1 + bytes_a + bytes_b + bytes3) * 1e-9);
       // 1 / phi2hat per spreading-grid index, and psi1hat's trapezoid coefficients
       std::vector<double> dec;
-      for (int d = 0; d < 3; ++d)
-        for (int l = 0; l < g.n1[d]; ++l)
-          dec.push_back(1.0 / es_hat_host((double)(l - g.n1[d] / 2) / g.n2[d], g.w2, g.beta2, 0.01));
+      for (int d = 0; d < 3; ++d) {
+        std::vector<double> hat;  // even in l - n1 / 2
+        es_hat_host(g.n2[d], g.n1[d] / 2 + 1, g.w2, g.beta2, hat);
+        for (int l = 0; l < g.n1[d]; ++l) dec.push_back(1.0 / hat[std::abs(l - g.n1[d] / 2)]);
+      }
       c.n_coef = (int)std::floor(0.5 * g.w1 / 0.25) + 1;
       for (int k = 0; k < c.n_coef; ++k) c.psi_a[k] = 0.25 * (k == 0 ? 1.0 : 2.0) * es_host(0.25 * k, g.w1, g.beta1);
       // twiddle tables of the three transforms, after dec in one upload
@@ -2616,6 +2691,7 @@ static int autotune_impl(int npat, const spsim_b200_molecule *const *mols, const
   {
     std::lock_guard<std::mutex> lk(g_mu);
     g_tuned[size_class(terms) * 4 + precision] = {bt, bp, bk};
+    ++g_tunings;
   }
   if (best_threads) *best_threads = bt;
   if (best_pixels_per_thread) *best_pixels_per_thread = bp;
@@ -2633,6 +2709,7 @@ extern "C" int spsim_b200_autotune(const spsim_b200_molecule *m, const spsim_b20
 extern "C" int spsim_b200_clear_tuning(void) {
   std::lock_guard<std::mutex> lk(g_mu);
   g_tuned.clear();
+  ++g_tunings;
   return SPSIM_OK;
 }
 
@@ -2859,6 +2936,9 @@ struct AdjPlan {
   int group = 1;  // patterns at a time
   DevBuf tables, H, strip, nodes;
   std::vector<double> host_rot;  // the rotations as last uploaded
+  size_t bytes() const {
+    return ff.cap + blocks.cap + items.cap + rot.cap + tables.cap + H.cap + strip.cap + nodes.cap;
+  }
   // recorded after each call's launch: the next call, on whatever stream,
   // waits for it before it rewrites the rotations the last launch reads
   cudaEvent_t done = nullptr;
@@ -2867,7 +2947,7 @@ struct AdjPlan {
   }
 };
 static std::vector<std::unique_ptr<AdjPlan>> g_adj_plans;  // most recent last
-static const size_t kMaxAdjPlans = 4;
+static const size_t kMaxAdjPlans = 8;  // a refinement takes two, on the nodes and on every pixel
 
 static void adjoint_release(int dev) {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -2904,7 +2984,17 @@ static int adjoint_plan(const spsim_b200_molecule *m, const spsim_b200_qset *qs,
       return SPSIM_OK;
     }
   }
-  std::unique_ptr<AdjPlan> np(new AdjPlan());
+  // the least recently used plan's place and, unless they are large, its buffers,
+  // as in run_forward
+  std::unique_ptr<AdjPlan> np;
+  if (g_adj_plans.size() >= kMaxAdjPlans) {
+    np = std::move(g_adj_plans.front());
+    g_adj_plans.erase(g_adj_plans.begin());
+    if (np->done) CUDA_TRY(cudaEventSynchronize(np->done));
+    if (np->device != dev || np->bytes() > kMaxKeptBytes) np.reset();
+  }
+  if (!np) np.reset(new AdjPlan());
+  np->host_rot.clear();
   np->mol_id = m->id;
   np->qs_id = qs->id;
   np->npat = npat;
@@ -3002,12 +3092,8 @@ static int adjoint_plan(const spsim_b200_molecule *m, const spsim_b200_qset *qs,
     CUDA_TRY(launch_ff_table(qs->d_hkl, qs->d_q64, qs->npix, m->n_elem, m->d_coeffs, (double)B, m->delta_atoms,
                              (double *)np->ff.p, st));
   }
-  CUDA_TRY(cudaEventCreateWithFlags(&np->done, cudaEventDisableTiming));
+  if (!np->done) CUDA_TRY(cudaEventCreateWithFlags(&np->done, cudaEventDisableTiming));
   CUDA_TRY(cudaEventRecord(np->done, st));
-  if (g_adj_plans.size() >= kMaxAdjPlans) {
-    cudaDeviceSynchronize();  // the evicted plan's buffers may still be in use
-    g_adj_plans.erase(g_adj_plans.begin());
-  }
   g_adj_plans.push_back(std::move(np));
   *out = g_adj_plans.back().get();
   return SPSIM_OK;
