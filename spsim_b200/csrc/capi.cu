@@ -2772,13 +2772,13 @@ static int chain_dev(const spsim_b200_chain_params *p, ChainDev *c) {
   c->polarization = p->polarization;
   c->unbinned = (c->bx == 1 && c->by == 1 && c->bz == 1);
   c->clamp = p->clamp_to_maximum;
-  c->width = p->width;
-  c->height = p->height;
   c->distance = p->distance;
+  c->step_x = (double)p->width / p->nx;
+  c->step_y = (double)p->height / p->ny;
+  c->inv_dd = 1.0 / (c->distance * c->distance);
+  c->omega0 = (double)p->pixel_width * p->pixel_height / (c->distance * c->distance);
   c->cx = p->center_x;
   c->cy = p->center_y;
-  c->pw = p->pixel_width;
-  c->ph = p->pixel_height;
   c->beam_intensity = p->beam_intensity;
   c->qe = p->quantum_efficiency;
   // src/amplification.c:56-61 and :121-123

@@ -35,7 +35,6 @@ struct PhiloxStream {
   uint32_t ctr[4];
   uint32_t k0, k1;
   uint32_t buf[4];
-  int left;
   __device__ PhiloxStream(uint32_t item, uint32_t pattern, uint32_t sid, uint64_t seed) {
     ctr[0] = item;
     ctr[1] = pattern;
@@ -43,43 +42,61 @@ struct PhiloxStream {
     ctr[3] = 0;
     k0 = (uint32_t)seed;
     k1 = (uint32_t)(seed >> 32);
-    left = 0;
   }
-  __device__ float uniform() {  // (0, 1)
-    if (left == 0) {
-      buf[0] = ctr[0];
-      buf[1] = ctr[1];
-      buf[2] = ctr[2];
-      buf[3] = ctr[3];
-      philox4x32_10(buf, k0, k1);
-      ++ctr[3];
-      left = 4;
-    }
-    const uint32_t x = buf[4 - left--];
-    return ((float)(x >> 8) + 0.5f) * 5.9604644775390625e-8f;
+  __device__ void refill() {
+    buf[0] = ctr[0];
+    buf[1] = ctr[1];
+    buf[2] = ctr[2];
+    buf[3] = ctr[3];
+    philox4x32_10(buf, k0, k1);
+    ++ctr[3];
   }
-  __device__ float normal() {  // Box-Muller, first of the pair
-    const float a = uniform(), b = uniform();
+  // Box-Muller, first of the pair, of a fresh block
+  __device__ float normal() {
+    refill();
+    return normal_of(buf[0], buf[1]);
+  }
+  __device__ static float unit(uint32_t x) { return ((float)(x >> 8) + 0.5f) * 5.9604644775390625e-8f; }  // (0, 1]
+  __device__ static float normal_of(uint32_t x, uint32_t y) {
+    const float a = unit(x), b = unit(y);
     return sqrtf(-2.0f * logf(a)) * cosf(6.2831853071795864f * b);
   }
 };
 
+// 1 / k, rounded to nearest, for the Poisson inversion
+struct InverseTable {
+  float v[201];
+};
+constexpr InverseTable make_inverse_table() {
+  InverseTable t{};
+  for (int k = 1; k <= 200; ++k) t.v[k] = 1.0f / (float)k;
+  return t;
+}
+__constant__ InverseTable c_inverse = make_inverse_table();
+
 // Poisson(lam): inversion below 10, Hormann's PTRS transformed rejection
 // (Insurance: Math. & Econ. 12 (1993) 39-45) up to 1000, and the reference's
 // Gaussian approximation (int)(lam + N(0, sqrt(lam))) above (src/noise.c:42-46).
+// The stream's first block is drawn before the branches: a warp that holds
+// several of the ranges draws it once.  Each trial of the rejection takes two
+// words, so a block serves an even trial and the odd one after it.
 __device__ float poisson_sample(PhiloxStream &s, float lam) {
   if (!(lam > 0.0f)) return 0.0f;
+  s.refill();
   if (lam >= 1000.0f) {
-    const float v = lam + sqrtf(lam) * s.normal();
+    const float v = lam + sqrtf(lam) * PhiloxStream::normal_of(s.buf[0], s.buf[1]);
     return (float)(int)v;
   }
   if (lam < 10.0f) {
-    const float u = s.uniform();
+    const float u = PhiloxStream::unit(s.buf[0]);
     float p = expf(-lam), F = p;
     int k = 0;
     while (u > F && k < 200) {
       ++k;
-      p *= lam / (float)k;
+      // lam / k as the division rounds it (Markstein: the quotient by the
+      // rounded reciprocal, corrected by its exact remainder)
+      const float inv = c_inverse.v[k], q = lam * inv;
+      p *= fmaf(fmaf(-q, (float)k, lam), inv, q);
       F += p;
     }
     return (float)k;
@@ -90,8 +107,9 @@ __device__ float poisson_sample(PhiloxStream &s, float lam) {
   const float inv_alpha = 1.1239f + 1.1328f / (b - 3.4f);
   const float vr = 0.9277f - 3.6224f / (b - 2.0f);
   for (int it = 0; it < 64; ++it) {
-    const float U = s.uniform() - 0.5f;
-    const float V = s.uniform();
+    if (it > 0 && !(it & 1)) s.refill();
+    const float U = PhiloxStream::unit(it & 1 ? s.buf[2] : s.buf[0]) - 0.5f;
+    const float V = PhiloxStream::unit(it & 1 ? s.buf[3] : s.buf[1]);
     const float us = 0.5f - fabsf(U);
     const float k = floorf((2.0f * a / us + b) * U + lam + 0.43f);
     if (us >= 0.07f && V <= vr) return k;
@@ -103,49 +121,67 @@ __device__ float poisson_sample(PhiloxStream &s, float lam) {
 
 // ---- per-pixel geometry factors --------------------------------------------
 
-__device__ __forceinline__ float thomson_factor(const ChainDev &c, int x, int y) {
+// Pixel i's row and column; small: i < 2^31 (64-bit divisions take a hundred
+// instructions each).
+__device__ __forceinline__ void pixel_xy(const ChainDev &c, long long i, bool small, int &x, int &y) {
+  if (small) {
+    const unsigned r = (unsigned)i / (unsigned)c.nx;
+    x = (int)((unsigned)i - r * (unsigned)c.nx);
+    y = c.nz > 1 ? (int)(r % (unsigned)c.ny) : (int)r;
+  } else {
+    x = (int)(i % c.nx);
+    y = (int)((i / c.nx) % c.ny);
+  }
+}
+
+// The squared positions x^2 and y^2 of a pixel on the detector, and the cosine
+// of its angle off the beam, D / sqrt(x^2 + y^2 + D^2).
+struct PixelPos {
+  double xx, yy, cosine;
+};
+__device__ __forceinline__ PixelPos pixel_pos(const ChainDev &c, int x, int y) {
+  const double px = (x - (c.nx - 1.0) / 2.0) * c.step_x - c.cx;
+  const double py = (y - (c.ny - 1.0) / 2.0) * c.step_y - c.cy;
+  const double xx = px * px, yy = py * py;
+  return {xx, yy, rsqrt(1.0 + (xx + yy) * c.inv_dd)};
+}
+
+// The reference's cos^2 chi with sin chi = y / r, x / r or sqrt(x^2 + y^2) / r
+// (r^2 = x^2 + y^2 + D^2) is a quotient of squares.
+__device__ __forceinline__ float thomson_factor(const ChainDev &c, const PixelPos &p) {
   const double r0 = 2.81794e-15;
   double pf = 1.0;
-  if (c.polarization != 0) {
-    const double px = ((x - (c.nx - 1.0) / 2.0) / c.nx) * c.width - c.cx;
-    const double py = ((y - (c.ny - 1.0) / 2.0) / c.ny) * c.height - c.cy;
-    const double r = sqrt(px * px + py * py + c.distance * c.distance);
-    if (c.polarization == 1) {
-      const double chi = asin(py / r);
-      pf = cos(chi) * cos(chi);
-    } else if (c.polarization == 2) {
-      const double chi = asin(px / r);
-      pf = cos(chi) * cos(chi);
-    } else if (c.polarization == 3) {
-      const double chi = asin(sqrt(px * px + py * py) / r);
-      pf = (1.0 + cos(chi) * cos(chi)) / 2.0;
-    }
+  if (c.polarization == 3) {
+    pf = (1.0 + p.cosine * p.cosine) / 2.0;
+  } else if (c.polarization == 1 || c.polarization == 2) {
+    const double dd = c.distance * c.distance;
+    pf = ((c.polarization == 1 ? p.xx : p.yy) + dd) / (p.xx + p.yy + dd);
   }
   return (float)((r0 * r0) * pf);
 }
 
-__device__ __forceinline__ float solid_angle_factor(const ChainDev &c, int x, int y) {
-  if (c.nz > 1 || c.spherical) {
-    const double r = c.distance;
-    return (float)(c.pw * c.ph / (r * r));
-  }
-  const double px = ((x - (c.nx - 1.0) / 2.0) / c.nx) * c.width - c.cx;
-  const double py = ((y - (c.ny - 1.0) / 2.0) / c.ny) * c.height - c.cy;
-  double inc = atan(sqrt(px * px + py * py) / c.distance);
-  inc = cos(inc);
-  inc = inc * inc * inc;
-  return (float)(c.pw * c.ph / (c.distance * c.distance) * inc);
+// cos^3(atan(sqrt(x^2 + y^2) / D)) is the cube of that cosine
+__device__ __forceinline__ float solid_angle_factor(const ChainDev &c, const PixelPos &p) {
+  if (c.nz > 1 || c.spherical) return (float)c.omega0;
+  return (float)(c.omega0 * (p.cosine * p.cosine * p.cosine));
 }
 
 // ---- fused chain -------------------------------------------------------------
 
-__global__ void chain_pixel_kernel(ChainDev c, const float *__restrict__ I, ChainOut o) {
+// Bound by the instructions it issues (two Philox blocks, logarithms, the
+// samplers' loops; 51 MB at 1536 x 1030 pixels with every output would take
+// 8 us).  There 57 us with the angles by asin, atan and cos in FP64, 64-bit
+// pixel indices and a division per Poisson term; 41 us without those; 35 us
+// with a block drawn before the samplers' branches and one rsqrt for both
+// angles; 33 us at 40 registers (six blocks per SM instead of four).
+__global__ void __launch_bounds__(256, 6) chain_pixel_kernel(ChainDev c, const float *__restrict__ I, ChainOut o, bool small) {
   const long long i = c.i0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.i1) return;
-  const int x = (int)(i % c.nx);
-  const int y = (int)((i / c.nx) % c.ny);
-  const float T = thomson_factor(c, x, y);
-  const float Om = solid_angle_factor(c, x, y);
+  int x, y;
+  pixel_xy(c, i, small, x, y);
+  const PixelPos pos = pixel_pos(c, x, y);
+  const float T = thomson_factor(c, pos);
+  const float Om = solid_angle_factor(c, pos);
   if (o.thomson) o.thomson[i] = T;
   if (o.solid_angle) o.solid_angle[i] = Om;
   if (!I) return;
@@ -263,7 +299,7 @@ cudaError_t launch_chain(const ChainDev &c, const float *I, const ChainOut &o, f
     po.noiseless = nullptr;
     po.real_out = nullptr;
   }
-  chain_pixel_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(c, I, po);
+  chain_pixel_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(c, I, po, c.i1 < (1LL << 31));
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || c.unbinned || (!o.noiseless && !o.real_out) || !I) return e;
   const long long nb = c.b1 - c.b0;

@@ -13,7 +13,9 @@ struct ChainDev {
   int spherical, polarization;
   int unbinned;          // bx == by == bz == 1
   int clamp;
-  double width, height, distance, cx, cy, pw, ph;
+  double distance, cx, cy;
+  double step_x, step_y;  // width / nx, height / ny: the reference's pixel pitch
+  double inv_dd, omega0;  // 1 / distance^2; pixel area / distance^2
   float beam_intensity;
   float qe;
   float epp;             // electrons per photon for counts (1 when e_hole == 0), src/amplification.c:57-61
