@@ -168,15 +168,18 @@ __device__ __forceinline__ void dmma(double c[2], double a, double b) {
       : "d"(a), "d"(b));
 }
 
-// RM x RN tiles of 8 x 8 of M B by one warp, M's rows from m0 (in range, clamped)
-// and B's columns at bcol[j], bstep doubles from one k to the next.  Of each
-// group of eight k the lane's entries are k = 2 fc + s in step s, so that M is
-// read in pairs; M holds zeros from k_all to its padded end, where B is read at
-// its last row.
-template <int RM, int RN>
+// M B by one warp for RM x RN tiles of 8 x 8 complex values: M's rows from m0
+// (in range, clamped), B's column n0 + 8 j + fr from bcol[j], bstep values from
+// one k to the next.  A tile's real and imaginary parts are two MMA tiles, so
+// that a lane reads a complex value at a time.  Of each group of eight k the
+// lane's entries are k = 2 fc + s in step s, so that M is read in pairs; M
+// holds zeros from k_all to its padded end, where B is read at its last row.
+// AHEAD: the groups whose fragments are read ahead of the one multiplied (L2's
+// latency bounds the small tiles, registers the large ones).
+template <int RM, int RN, int AHEAD>
 __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, int m0, int m_all,
-                                          const double *const bcol[RN], long long bstep, int k_all,
-                                          double acc[RM][RN][2]) {
+                                          const double2 *const bcol[RN], long long bstep, int k_all, int k_first,
+                                          int k_end, double re[RM][RN][2], double im[RM][RN][2]) {
   const int lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
   const double2 *arow[RM];
 #pragma unroll
@@ -184,32 +187,48 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, 
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < RN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  for (int k = 0; k < k_all; k += 8) {
+    for (int j = 0; j < RN; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+  double2 a[AHEAD + 1][RM], b0[AHEAD + 1][RN], b1[AHEAD + 1][RN];
+  auto load = [&](int k, int slot) {
     const long long kb0 = min(k + 2 * fc, k_all - 1) * bstep, kb1 = min(k + 2 * fc + 1, k_all - 1) * bstep;
-    double2 a[RM];
-    double b0[RN], b1[RN];
 #pragma unroll
-    for (int i = 0; i < RM; ++i) a[i] = arow[i][k / 2];
+    for (int i = 0; i < RM; ++i) a[slot][i] = arow[i][k / 2];
 #pragma unroll
     for (int j = 0; j < RN; ++j) {
-      b0[j] = bcol[j][kb0];
-      b1[j] = bcol[j][kb1];
+      b0[slot][j] = bcol[j][kb0];
+      b1[slot][j] = bcol[j][kb1];
     }
+  };
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+  for (int s = 0; s < AHEAD; ++s)
+    if (k_first + 8 * s < k_end) load(k_first + 8 * s, s);
+  for (int k0 = k_first; k0 < k_end; k0 += 8 * (AHEAD + 1)) {
 #pragma unroll
-      for (int j = 0; j < RN; ++j) dmma(acc[i][j], a[i].x, b0[j]);
+    for (int s = 0; s <= AHEAD; ++s) {
+      const int k = k0 + 8 * s;
+      if (k >= k_end) break;
+      if (k + 8 * AHEAD < k_end) load(k + 8 * AHEAD, (s + AHEAD) % (AHEAD + 1));
 #pragma unroll
-    for (int i = 0; i < RM; ++i)
+      for (int i = 0; i < RM; ++i)
 #pragma unroll
-      for (int j = 0; j < RN; ++j) dmma(acc[i][j], a[i].y, b1[j]);
+        for (int j = 0; j < RN; ++j) {
+          dmma(re[i][j], a[s][i].x, b0[s][j].x);
+          dmma(im[i][j], a[s][i].x, b0[s][j].y);
+        }
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) {
+          dmma(re[i][j], a[s][i].y, b1[s][j].x);
+          dmma(im[i][j], a[s][i].y, b1[s][j].y);
+        }
+    }
   }
 }
 
 // ROWS: the second product, else the first.
-template <int RM, int RN, bool ROWS>
-__global__ void __launch_bounds__(INTERP_THREADS)
+template <int RM, int RN, int AHEAD, bool ROWS>
+__global__ void __launch_bounds__(INTERP_THREADS, 7)
     coarse_interp_kernel(const __grid_constant__ CoarseBatch batch, int pattern0, double2 *__restrict__ strips,
                          long long strip_stride) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -218,7 +237,7 @@ __global__ void __launch_bounds__(INTERP_THREADS)
   if (!batch.pats) cp.nodes += (long long)pattern * cp.nyn * cp.nxn;
   double2 *__restrict__ strip = strips + blockIdx.z * strip_stride;
   const int m_all = ROWS ? cp.ny : cp.nx;             // rows of the left matrix
-  const int n_all = 2 * (ROWS ? cp.nx : cp.nyn);      // columns of the right one (re, im pairs)
+  const int n_all = ROWS ? cp.nx : cp.nyn;            // columns of the right one
   const int k_all = ROWS ? cp.nyn : cp.nxn;
   const int ld = ROWS ? cp.ldy : cp.ldx;
   const double *__restrict__ M = ROWS ? cp.my : cp.mx;
@@ -227,14 +246,14 @@ __global__ void __launch_bounds__(INTERP_THREADS)
   if (m0 >= m_all || n0 >= n_all) return;
   const int fr = lane >> 2, fc = lane & 3;
 
-  const double *bcol[RN];
+  const double2 *bcol[RN];
 #pragma unroll
   for (int j = 0; j < RN; ++j) {
     const int n = min(n0 + 8 * j + fr, n_all - 1);
-    bcol[j] = ROWS ? (const double *)strip + n : (const double *)(cp.nodes + (long long)(n >> 1) * cp.nxn) + (n & 1);
+    bcol[j] = ROWS ? strip + n : cp.nodes + (long long)n * cp.nxn;
   }
-  double acc[RM][RN][2];
-  dmma_tile<RM, RN>(M, ld, m0, m_all, bcol, ROWS ? 2LL * cp.nx : 2LL, k_all, acc);
+  double re_[RM][RN][2], im_[RM][RN][2];
+  dmma_tile<RM, RN, AHEAD>(M, ld, m0, m_all, bcol, ROWS ? cp.nx : 1, k_all, 0, k_all, re_, im_);
 
   if (!ROWS) {
 #pragma unroll
@@ -242,9 +261,9 @@ __global__ void __launch_bounds__(INTERP_THREADS)
       const int x = m0 + 8 * i + fr;
       if (x >= cp.nx) continue;
 #pragma unroll
-      for (int j = 0; j < RN; ++j) {
-        const int k = n0 / 2 + 4 * j + fc;
-        if (k < cp.nyn) strip[(long long)k * cp.nx + x] = make_double2(acc[i][j][0], acc[i][j][1]);
+      for (int j = 0; j < 2 * RN; ++j) {
+        const int k = n0 + 8 * (j >> 1) + 2 * fc + (j & 1);
+        if (k < cp.nyn) strip[(long long)k * cp.nx + x] = make_double2(re_[i][j >> 1][j & 1], im_[i][j >> 1][j & 1]);
       }
     }
     return;
@@ -264,63 +283,61 @@ __global__ void __launch_bounds__(INTERP_THREADS)
     F = pt.F;
     I = pt.I;
   }
+  // the tile by rows of neighbouring pixels, one per lane: coalesced, and the
+  // phase's code once instead of once per accumulator
+  constexpr int TN = 8 * RN, TLD = TN + 1;
+  __shared__ double2 tiles[INTERP_WARPS_M * INTERP_WARPS_N][8 * RM * TLD];
+  double2 *tile = tiles[warp];
 #pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    const int y = m0 + 8 * i + fr;
-    if (y >= cp.ny) continue;
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < RN; ++j) {
-      const int x = n0 / 2 + 4 * j + fc;
-      if (x >= cp.nx) continue;
-      const long long p = (long long)y * cp.nx + x;
-      double re = acc[i][j][0], im = acc[i][j][1];
-      if (F || cp.B != 0.0 || cp.out) {
-        const double a = q64[3 * p], b = q64[3 * p + 1], c = q64[3 * p + 2];
-        if (cp.B != 0.0) {
-          const double e = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
-          re *= e;
-          im *= e;
-        }
-        if (cp.out) {
-          cp.out[p] = make_double2(re, im);
-          continue;
-        }
-        if (F) {
-          double ux = a, uy = b, uz = c;
-          if (rot) {
-            ux = rot[0] * a + rot[1] * b + rot[2] * c;
-            uy = rot[3] * a + rot[4] * b + rot[5] * c;
-            uz = rot[6] * a + rot[7] * b + rot[8] * c;
-          }
-          double t = (ux * center[0] + uy * center[1] + uz * center[2]) * qscale;
-          t -= rint(t);
-          double sn, cs;
-          sincospi(2.0 * t, &sn, &cs);
-          F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
-        }
+    for (int j = 0; j < 2 * RN; ++j)
+      tile[(8 * i + fr) * TLD + 8 * (j >> 1) + 2 * fc + (j & 1)] =
+          make_double2(re_[i][j >> 1][j & 1], im_[i][j >> 1][j & 1]);
+  __syncwarp();
+  const bool need_q = F || cp.B != 0.0 || cp.out;
+#pragma unroll 1
+  for (int e = lane; e < 8 * RM * TN; e += 32) {
+    const int y = m0 + e / TN, x = n0 + e % TN;
+    if (y >= cp.ny || x >= cp.nx) continue;
+    const long long p = (long long)y * cp.nx + x;
+    const double2 v = tile[e / TN * TLD + e % TN];
+    double re = v.x, im = v.y;
+    if (need_q) {
+      const double a = q64[3 * p], b = q64[3 * p + 1], c = q64[3 * p + 2];
+      if (cp.B != 0.0) {
+        const double w = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
+        re *= w;
+        im *= w;
       }
-      if (I) I[p] = (float)(re * re + im * im);
+      if (cp.out) {
+        cp.out[p] = make_double2(re, im);
+        continue;
+      }
+      if (F) {
+        double ux = a, uy = b, uz = c;
+        if (rot) {
+          ux = rot[0] * a + rot[1] * b + rot[2] * c;
+          uy = rot[3] * a + rot[4] * b + rot[5] * c;
+          uz = rot[6] * a + rot[7] * b + rot[8] * c;
+        }
+        double t = (ux * center[0] + uy * center[1] + uz * center[2]) * qscale;
+        t -= rint(t);
+        double sn, cs;
+        sincospi(2.0 * t, &sn, &cs);
+        F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
+      }
     }
+    if (I) I[p] = (float)(re * re + im * im);
   }
 }
 
-template <int RM, int RN, bool ROWS>
+template <int RM, int RN, int AHEAD, bool ROWS>
 static void interp_t(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip, long long stride,
                      cudaStream_t st) {
   const int bm = 8 * RM * INTERP_WARPS_M, bn = 8 * RN * INTERP_WARPS_N;
   dim3 grid((unsigned)((n_max + bn - 1) / bn), (unsigned)((m_max + bm - 1) / bm), (unsigned)n);
-  coarse_interp_kernel<RM, RN, ROWS><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
-}
-
-template <bool ROWS>
-static void interp_part(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip,
-                        long long stride, cudaStream_t st) {
-  // 32 x 32 tiles per warp where they fill the GPU a few times, else 16 x 16
-  const long long blocks = (long long)n * ((m_max + 63) / 64) * ((n_max + 63) / 64);
-  if (blocks >= 2 * 148)
-    interp_t<4, 4, ROWS>(b, pattern0, n, m_max, n_max, strip, stride, st);
-  else
-    interp_t<2, 2, ROWS>(b, pattern0, n, m_max, n_max, strip, stride, st);
+  coarse_interp_kernel<RM, RN, AHEAD, ROWS><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
 }
 
 cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
@@ -330,8 +347,15 @@ cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int
   const int group = (int)std::min<long long>(std::max<long long>(strip_size / stride, 1), 65535);
   for (int p0 = 0; p0 < npat; p0 += group) {
     const int n = std::min(group, npat - p0);
-    interp_part<false>(b, p0, n, max_nx, 2 * max_nyn, strip, stride, st);
-    interp_part<true>(b, p0, n, max_ny, 2 * max_nx, strip, stride, st);
+    // Columns: 8 x 8 values per warp (50,000 atoms x 1024^2, 161 nodes a side:
+    // 10.3 us, with 16 x 8 11.8, 16 x 16 14).  Rows: 16 x 8 (46 us; 8 x 8 64,
+    // 32 x 16 46.5), but 8 x 8 where those leave most SMs without two blocks
+    // (one 512^2 pattern: 6.4 us instead of 8.8; eight: 43 instead of 34).
+    interp_t<1, 1, 2, false>(b, p0, n, max_nx, max_nyn, strip, stride, st);
+    if ((long long)n * ((max_ny + 31) / 32) * ((max_nx + 15) / 16) < 2 * 148)
+      interp_t<1, 1, 2, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
+    else
+      interp_t<2, 1, 1, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
   }
   return cudaGetLastError();
 }
@@ -364,47 +388,42 @@ __global__ void __launch_bounds__(256)
 }
 
 // out[m][n] = sum_k L[m][k] R[n][k] for complex R of n_all rows, k_all long, and
-// real L of m_all rows, ld long; blockIdx.z: pattern.
-template <int RM, int RN>
-__global__ void __launch_bounds__(INTERP_THREADS)
+// real L of m_all rows, ld long; blockIdx.z: pattern.  Few results of long sums
+// (30 nodes a side, k a side of the detector): one 8 x 8 tile per block, its
+// warps taking a quarter of k each, their parts added in a fixed order.  Eight
+// 512^2 patterns (k = 512 both times): 16.5 and 6.5 us; 45 and 44 us with 16 x 16
+// tiles of all of k per warp, 18 and 14 with 8 x 8 tiles of all of k.
+constexpr int PRODUCT_SPLIT = 4;
+__global__ void __launch_bounds__(32 * PRODUCT_SPLIT)
     coarse_product_kernel(const double *__restrict__ L, int ld, int m_all, const double2 *__restrict__ R, int n_all,
                           int k_all, double2 *__restrict__ out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
-  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
-  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);  // of 2 n_all real columns
-  if (m0 >= m_all || n0 >= 2 * n_all) return;
+  const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 8;
   R += (long long)blockIdx.z * n_all * k_all;
   out += (long long)blockIdx.z * m_all * n_all;
-  const double *bcol[RN];
+  const double2 *bcol[1] = {R + (long long)min(n0 + fr, n_all - 1) * k_all};
+  const int part = (k_all + 8 * PRODUCT_SPLIT - 1) / (8 * PRODUCT_SPLIT) * 8;
+  double re[1][1][2], im[1][1][2];
+  dmma_tile<1, 1, 3>(L, ld, m0, m_all, bcol, 1, k_all, warp * part, min((warp + 1) * part, k_all), re, im);
+  __shared__ double2 parts[PRODUCT_SPLIT][64];
 #pragma unroll
-  for (int j = 0; j < RN; ++j) {
-    const int n = min(n0 + 8 * j + fr, 2 * n_all - 1);
-    bcol[j] = (const double *)(R + (long long)(n >> 1) * k_all) + (n & 1);
+  for (int h = 0; h < 2; ++h) parts[warp][8 * fr + 2 * fc + h] = make_double2(re[0][0][h], im[0][0][h]);
+  __syncthreads();
+  const int m = m0 + threadIdx.x / 8, n = n0 + threadIdx.x % 8;
+  if (threadIdx.x >= 64 || m >= m_all || n >= n_all) return;
+  double2 v = parts[0][threadIdx.x];
+#pragma unroll
+  for (int w = 1; w < PRODUCT_SPLIT; ++w) {
+    v.x += parts[w][threadIdx.x].x;
+    v.y += parts[w][threadIdx.x].y;
   }
-  double acc[RM][RN][2];
-  dmma_tile<RM, RN>(L, ld, m0, m_all, bcol, 2LL, k_all, acc);
-#pragma unroll
-  for (int i = 0; i < RM; ++i) {
-    const int m = m0 + 8 * i + fr;
-    if (m >= m_all) continue;
-#pragma unroll
-    for (int j = 0; j < RN; ++j) {
-      const int n = n0 / 2 + 4 * j + fc;
-      if (n < n_all) out[(long long)m * n_all + n] = make_double2(acc[i][j][0], acc[i][j][1]);
-    }
-  }
+  out[(long long)m * n_all + n] = v;
 }
 
 static void product(const double *L, int ld, int m, const double2 *R, int n, int k, double2 *out, int npat,
                     cudaStream_t st) {
-  const long long blocks = (long long)npat * ((m + 63) / 64) * ((2 * n + 63) / 64);
-  if (blocks >= 4 * 148) {
-    dim3 grid((unsigned)((2 * n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)npat);
-    coarse_product_kernel<4, 4><<<grid, INTERP_THREADS, 0, st>>>(L, ld, m, R, n, k, out);
-  } else {
-    dim3 grid((unsigned)((2 * n + 31) / 32), (unsigned)((m + 31) / 32), (unsigned)npat);
-    coarse_product_kernel<2, 2><<<grid, INTERP_THREADS, 0, st>>>(L, ld, m, R, n, k, out);
-  }
+  dim3 grid((unsigned)((n + 7) / 8), (unsigned)((m + 7) / 8), (unsigned)npat);
+  coarse_product_kernel<<<grid, 32 * PRODUCT_SPLIT, 0, st>>>(L, ld, m, R, n, k, out);
 }
 
 cudaError_t launch_coarse_adjoint(const CoarseAdjoint &a, int npat, double2 *H, int group, double2 *strip,
