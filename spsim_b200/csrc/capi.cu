@@ -205,6 +205,19 @@ struct PinnedBuf {
 };
 static PinnedBuf g_upload_stage;  // molecule uploads, under g_mu
 
+// A molecule's atoms by the cells of a lattice (coarse_kernels.cuh), for plans
+// whose node sums run cell by cell.
+struct MoleculeCells {
+  CellLattice lattice;
+  int n = 0;                    // cells with atoms
+  std::vector<double> shift;    // [n][3]: centres, from the molecule's
+  std::vector<int> tile_begin;  // [n + 1]: each cell's tiles
+  std::vector<TileDesc> tiles;
+  DevBuf buf;
+  AtomD *d_atoms = nullptr;
+  TileDesc *d_tiles = nullptr;
+};
+
 struct spsim_b200_molecule {
   unsigned long long id = 0;
   int device = 0;
@@ -235,6 +248,8 @@ struct spsim_b200_molecule {
   int *d_flags = nullptr;  // [0] range error, [1] a rewritten B factor beyond b_limit
   // owned device memory; a new molecule may take over a dropped one's buffers
   DevBuf b_atoms, b_atoms2, b_atomsd, b_tiles, b_perm, b_wbase, b_coeffs, b_flags, b_inputs;
+  // by index of kCellSizes, made when a plan first wants them, under g_mu
+  mutable std::map<int, std::unique_ptr<MoleculeCells>> cells;
   void take_buffers(spsim_b200_molecule &o) {
     b_atoms.swap(o.b_atoms);
     b_atoms2.swap(o.b_atoms2);
@@ -698,6 +713,10 @@ struct Plan {
   double2 *pix_acc = nullptr, *strip = nullptr;
   long long strip_size = 0;
   int max_nx = 0, max_ny = 0, max_nyn = 0;
+  // cells: the last npat descriptors hold the patterns on their own nodes, which
+  // the interpolation of the cells' sums writes
+  int n_cells = 0, cell_nx = 0, cell_ny = 0, cell_nyn = 0;
+  long long acc_total = 0;  // FP64 sums
   // the same patterns on every pixel, run where a B factor rewritten on the
   // device is beyond what the coarse grids are sized for
   std::unique_ptr<Plan> direct;
@@ -813,8 +832,10 @@ struct CoarseGrid {
 };
 
 // fp64: nodes for FP64 sums (1e-12 instead of 1e-8).
+// rbound: of the atoms about the centre of their phases (0: the molecule's).
 static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale,
-                       CoarseGrid *grid, bool fp64 = false) {
+                       CoarseGrid *grid, bool fp64 = false, double rbound = 0.0) {
+  if (!(rbound > 0.0)) rbound = m->rbound;
   const DetGeom &g = q->geom;
   if (!q->has_geom || m->n_kept == 0 || g.nx < 16 || g.ny < 16) return false;
   if (!(q->qmax * scale * m->rbound < std::ldexp(1.0, 40))) return false;  // the FP64 sums' rounding reduction
@@ -837,7 +858,7 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
               : g.fpx * (0.5 * (g.nx - 1) / g.nx * g.width) / g.px_size;
       reach = arc;
     }
-    const double c = 2.0 * M_PI * m->rbound * scale * arc * (t > 1.0 ? 1.02 : 1.0);
+    const double c = 2.0 * M_PI * rbound * scale * arc * (t > 1.0 ? 1.02 : 1.0);
     const double a = bmax * 0.25e-20 * reach * reach;
     if (!(c <= 1.5 * COARSE_MAX_NODES) || !(t <= 1.2) || !(a <= 60.0)) return false;
     const int n = coarse_node_count(c, t, a, fp64);
@@ -880,6 +901,168 @@ static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const 
   return grid < 0.8 * direct;
 }
 
+// Cells.  A pattern of many nodes is itself summed in two levels: the atoms of
+// each cell of a lattice (coarse_kernels.cuh) have phases about the cell's
+// centre that turn as much slower as the cell is smaller than the molecule, so
+// each cell's sum runs on a coarser grid of its own, which is interpolated to
+// the pattern's nodes and multiplied there by the phase of the cell's centre.
+// 50,000 atoms on 167^2 nodes, 1,065 us of node kernel: 65 cells of 71^2 nodes
+// take 256 us, and 75 us to interpolate; 128 orientations of 20,000 atoms on
+// 38^2 nodes 2,890 us: 65 cells of 22^2, 1,361 and 232 us.  The cells' size is
+// the cheapest of these by the measured rates.
+struct CellSize {
+  double a;   // lattice constant per bound of the molecule
+  int cells;  // that hold atoms of a ball: sizes just above those where a shell of cells comes in
+};
+static const CellSize kCellSizes[] = {{1.07, 15}, {0.85, 27},  {0.74, 51},  {0.65, 59},  {0.57, 65},
+                                      {0.495, 113}, {0.46, 137}, {0.41, 169}, {0.39, 181}, {0.36, 259},
+                                      {0.32, 331}, {0.275, 531}, {0.25, 609}, {0.225, 868}, {0.2, 1133}};
+
+// Node kernel's rate (terms/s) and, per (cell, element), the atoms that the
+// padding, the flush and the idle warps of a short run cost.
+static double node_rate(bool fp64) { return fp64 ? 7e11 : 1.3e12; }
+constexpr double kRunAtoms = 50.0;
+
+// The cheapest cells of one pattern: index into kCellSizes or -1, their grid,
+// and the time saved against the sum of all atoms on `outer`.
+static int choose_cells(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale, bool fp64,
+                        const CoarseGrid &outer, CoarseGrid *inner, double *saved) {
+  const double no = (double)outer.x.n * outer.y.n, whole = m->n_kept * no / node_rate(fp64);
+  int best = -1;
+  double best_time = 0.85 * whole;
+  *saved = 0.0;
+  if (whole < 2e-6) return best;
+  for (int k = 0; k < (int)(sizeof(kCellSizes) / sizeof(kCellSizes[0])); ++k) {
+    const double cells = kCellSizes[k].cells;
+    CoarseGrid g;
+    if (!coarse_fit(m, q, scale, bscale, &g, fp64, 0.5591 * kCellSizes[k].a * m->rbound)) continue;
+    const double ni = (double)g.x.n * g.y.n;
+    const double tile = fp64 ? SF_NODES64_TILE : SF_NODES_TILE;
+    const double time = (m->n_kept + cells * m->n_elem * kRunAtoms) * std::ceil(ni / tile) * tile / node_rate(fp64) +
+                        cells * (2.0 * outer.x.n * g.y.n * (g.x.n + outer.y.n) / 6e12 + no / 1.2e11);
+    if (time < best_time) {
+      best = k;
+      best_time = time;
+      *inner = g;
+    }
+  }
+  *saved = best >= 0 ? whole - best_time : 0.0;
+  return best;
+}
+
+// The molecule's cells of size k; nullptr while the stream is being captured
+// and they are not there yet.  Complete before return.
+static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stream, const MoleculeCells **out) {
+  *out = nullptr;
+  auto &slot = m->cells[k];
+  if (slot) {
+    *out = slot.get();
+    return SPSIM_OK;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return SPSIM_OK;
+  }
+  std::unique_ptr<MoleculeCells> c(new MoleculeCells());
+  c->lattice.a = kCellSizes[k].a * m->rbound;
+  c->lattice.reach = (int)std::ceil(1.0 / kCellSizes[k].a) + 1;
+  c->lattice.dim = 2 * c->lattice.reach + 1;
+  const int dim = c->lattice.dim, n_elem = m->n_elem, keys = 2 * dim * dim * dim * n_elem;
+  // one allocation: records, tiles (at most one, of a run's last atoms, besides
+  // the full ones), and the kernels' scratch
+  const size_t runs = std::min(keys, m->n_kept), most = (size_t)m->n_kept + (ATOM_GROUP - 1) * runs;
+  const size_t rec = most * sizeof(AtomD), desc = (most / TILE_ATOMS + runs) * sizeof(TileDesc);
+  CUDA_TRY(c->buf.ensure(rec + desc + (most + m->n_padded + 3 * (size_t)keys) * sizeof(int)));
+  c->d_atoms = (AtomD *)c->buf.p;
+  c->d_tiles = (TileDesc *)((char *)c->buf.p + rec);
+  int *order = (int *)((char *)c->buf.p + rec + desc);
+  int *key = order + most, *count = key + m->n_padded, *run = count + keys, *cursor = run + keys;
+  CUDA_TRY(cudaMemsetAsync(count, 0, keys * sizeof(int), stream));
+  CUDA_TRY(launch_cells_count(c->lattice, m->d_atomsd, m->d_perm, m->d_tiles, (int)m->tiles.size(), n_elem, key, count,
+                              stream));
+  std::vector<int> counts(keys), begin(keys, 0);
+  CUDA_TRY(cudaMemcpyAsync(counts.data(), count, keys * sizeof(int), cudaMemcpyDeviceToHost, stream));
+  CUDA_TRY(cudaStreamSynchronize(stream));
+  int slots = 0;
+  for (int cell = 0; cell < keys / n_elem; ++cell) {
+    const size_t first = c->tiles.size();
+    for (int e = 0; e < n_elem; ++e) {
+      const int n = counts[(size_t)cell * n_elem + e], padded = (n + ATOM_GROUP - 1) / ATOM_GROUP * ATOM_GROUP;
+      begin[(size_t)cell * n_elem + e] = slots;
+      for (int a = 0; a < padded; a += TILE_ATOMS) {
+        TileDesc t;
+        t.atom_begin = slots + a;
+        t.count = std::min(TILE_ATOMS, padded - a);
+        t.elem = e;
+        t.last = a + TILE_ATOMS >= padded ? 1 : 0;
+        c->tiles.push_back(t);
+      }
+      slots += padded;
+    }
+    if (c->tiles.size() == first) continue;
+    c->tile_begin.push_back((int)first);
+    const int at[3] = {cell % dim, cell / dim % dim, cell / (dim * dim) % dim}, sub = cell / (dim * dim * dim);
+    for (int d = 0; d < 3; ++d) c->shift.push_back(c->lattice.a * (at[d] - c->lattice.reach + 0.5 * sub));
+    ++c->n;
+  }
+  c->tile_begin.push_back((int)c->tiles.size());
+  CUDA_TRY(cudaMemcpyAsync(run, begin.data(), keys * sizeof(int), cudaMemcpyHostToDevice, stream));
+  CUDA_TRY(cudaMemsetAsync(cursor, 0, keys * sizeof(int), stream));
+  CUDA_TRY(cudaMemcpyAsync(c->d_tiles, c->tiles.data(), c->tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice, stream));
+  CUDA_TRY(launch_cells_build(c->lattice, m->d_atomsd, m->d_perm, m->n_padded, n_elem, key, count, run, cursor, order,
+                              c->d_atoms, slots, stream));
+  CUDA_TRY(cudaStreamSynchronize(stream));
+  slot = std::move(c);
+  *out = slot.get();
+  return SPSIM_OK;
+}
+
+// Cells for the patterns of a plan on coarse grids: where they save more than
+// their two launches, in all less than kMaxCellSums of sums.
+struct PatternCells {
+  const MoleculeCells *list = nullptr;
+  CoarseGrid grid;  // of each cell
+};
+constexpr double kMaxCellSums = 4e9, kCellsMinSaved = 15e-6;
+static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
+                      const double *rot, int precision, const Spectrum *spec, const std::vector<CoarseGrid> &nodes,
+                      cudaStream_t stream, std::vector<PatternCells> &cells) {
+  cells.assign(npat, PatternCells());
+  const bool fp64 = precision == SPSIM_PREC_FP64;
+  std::vector<int> size(npat, -1);
+  std::vector<CoarseGrid> grid(npat);
+  double saved = 0.0, bytes = 0.0;
+  double qscale = 1.0;
+  if (spec)
+    for (int i = 0; i < npat; ++i) qscale = std::max(qscale, std::fabs(spec->qscale[i]));
+  double last = 0.0;
+  for (int i = 0; i < npat; ++i) {
+    // positions rewritten on the device have left their cells
+    if (mols[i]->updated) continue;
+    double stretch = 1.0;
+    if (rot && !is_orthonormal(rot + 9 * (size_t)i)) stretch = std::max(1.0, frobenius(rot + 9 * (size_t)i));
+    if (i > 0 && stretch == 1.0 && mols[i] == mols[i - 1] && qsets[i] == qsets[i - 1] &&
+        nodes[i].x.n == nodes[i - 1].x.n && nodes[i].y.n == nodes[i - 1].y.n) {
+      size[i] = size[i - 1];
+      grid[i] = grid[i - 1];
+    } else {
+      size[i] = choose_cells(mols[i], qsets[i], qscale * stretch, stretch, fp64, nodes[i], &grid[i], &last);
+    }
+    saved += last;
+  }
+  if (saved < kCellsMinSaved) return SPSIM_OK;
+  for (int i = 0; i < npat; ++i) {
+    if (size[i] < 0) continue;
+    const int st = molecule_cells(mols[i], size[i], stream, &cells[i].list);
+    if (st) return st;
+    cells[i].grid = grid[i];
+    if (cells[i].list) bytes += (double)cells[i].list->n * grid[i].x.n * grid[i].y.n * sizeof(double2);
+  }
+  if (bytes > kMaxCellSums) cells.assign(npat, PatternCells());
+  return SPSIM_OK;
+}
+
 static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
                       cudaStream_t stream, const Spectrum *spec, bool allow_coarse = true) {
@@ -890,18 +1073,32 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     if (!mols[i] || !qsets[i]) return fail(SPSIM_ERR_INVALID_ARG, "pattern %d: NULL molecule or q set", i);
   pl.coarse = allow_coarse && coarse_plan(npat, mols, qsets, rot, precision, spec, nodes);
   pl.mode = precision == SPSIM_PREC_F32_FAST && !pl.coarse ? PREC_MODE_MUFU : PREC_MODE_POLY;
-  // points each pattern's sum is evaluated on: its nodes or its pixels
+  // cells, and the grid of each pattern's sums: its cells' or its own
+  std::vector<PatternCells> cells(npat);
+  if (pl.coarse) {
+    const int st = plan_cells(npat, mols, qsets, rot, precision, spec, nodes, stream, cells);
+    if (st) return st;
+  }
+  std::vector<CoarseGrid> sum_grid(nodes);
+  pl.n_cells = 0;
+  for (int i = 0; i < npat; ++i)
+    if (cells[i].list) {
+      sum_grid[i] = cells[i].grid;
+      pl.n_cells += cells[i].list->n;
+    }
+  // points each pattern's sum is evaluated on: nodes or its pixels
   std::vector<long long> points(npat);
-  for (int i = 0; i < npat; ++i) points[i] = pl.coarse ? (long long)nodes[i].x.n * nodes[i].y.n : qsets[i]->npix;
+  for (int i = 0; i < npat; ++i)
+    points[i] = pl.coarse ? (long long)sum_grid[i].x.n * sum_grid[i].y.n : qsets[i]->npix;
   std::vector<SfPattern> pats(npat);
   // unique (molecule, q set, node grid) combinations share one form-factor table
   typedef std::tuple<const void *, const void *, int, int> FfKey;
   auto ff_key = [&](int i) {
-    return FfKey(mols[i], qsets[i], pl.coarse ? nodes[i].x.n : 0, pl.coarse ? nodes[i].y.n : 0);
+    return FfKey(mols[i], qsets[i], pl.coarse ? sum_grid[i].x.n : 0, pl.coarse ? sum_grid[i].y.n : 0);
   };
   std::map<FfKey, size_t> ff_off;
   size_t ff_total = 0, acc_total = 0;
-  std::vector<size_t> acc_off(npat), ffo(npat);
+  std::vector<size_t> acc_off(npat), node_off(npat), ffo(npat);  // node_off: the pattern's own nodes
   double terms = 0;
   long long total_npix = 0;
   bool perb = false;
@@ -917,8 +1114,12 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     } else {
       ffo[i] = f->second;
     }
-    acc_off[i] = acc_total;
+    acc_off[i] = node_off[i] = acc_total;
     acc_total += points[i];
+    if (cells[i].list) {
+      node_off[i] = acc_off[i] + (size_t)cells[i].list->n * points[i];
+      acc_total = node_off[i] + (size_t)nodes[i].x.n * nodes[i].y.n;
+    }
     terms += (double)q->npix * m->n_kept;
     total_npix += q->npix;
     perb = perb || m->per_atom_b;
@@ -930,7 +1131,8 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   CUDA_TRY(pl.acc.ensure(64 + std::max<size_t>(acc_total, 1) * sizeof(double2)));
   CUDA_TRY(pl.ff.ensure(std::max<size_t>(ff_total, 1) * sizeof(double)));
   CUDA_TRY(cudaMemsetAsync(pl.acc.p, 0, 64, stream));  // queue head and the sticky error words
-  CUDA_TRY(pl.pats.ensure((pl.coarse ? 2 : 1) * std::max(npat, 1) * sizeof(SfPattern)));
+  pl.acc_total = (long long)acc_total;
+  CUDA_TRY(pl.pats.ensure((pl.n_cells ? 3 : pl.coarse ? 2 : 1) * std::max(npat, 1) * sizeof(SfPattern)));
 
   // node grids: one set of node q vectors and interpolation matrices per (q set, node counts)
   typedef std::tuple<const void *, int, int> TabKey;
@@ -938,9 +1140,20 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   size_t tab_total = 0;
   auto tab_sizes = [&](int i, size_t n[3]) {
     const DetGeom &g = qsets[i]->geom;
-    n[0] = ((size_t)3 * points[i] + 1) / 2 * 2;
+    n[0] = ((size_t)3 * nodes[i].x.n * nodes[i].y.n + 1) / 2 * 2;
     n[1] = (size_t)g.nx * coarse_ld(nodes[i].x.n);
     n[2] = (size_t)g.ny * coarse_ld(nodes[i].y.n);
+  };
+  // and of the cells' nodes, interpolating to the pattern's
+  typedef std::tuple<const void *, int, int, int, int> CellKey;
+  std::map<CellKey, std::pair<size_t, int>> cell_tab;  // offset, a pattern with this table
+  auto cell_key = [&](int i) {
+    return CellKey(qsets[i], sum_grid[i].x.n, sum_grid[i].y.n, nodes[i].x.n, nodes[i].y.n);
+  };
+  auto cell_sizes = [&](int i, size_t n[3]) {
+    n[0] = ((size_t)3 * points[i] + 1) / 2 * 2;
+    n[1] = (size_t)nodes[i].x.n * coarse_ld(sum_grid[i].x.n);
+    n[2] = (size_t)nodes[i].y.n * coarse_ld(sum_grid[i].y.n);
   };
   size_t pix_total = 0;
   std::vector<size_t> pix_off(npat);
@@ -951,6 +1164,12 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
         size_t n[3];
         tab_sizes(i, n);
         tab_off[key] = tab_total;
+        tab_total += n[0] + n[1] + n[2];
+      }
+      if (cells[i].list && !cell_tab.count(cell_key(i))) {
+        size_t n[3];
+        cell_sizes(i, n);
+        cell_tab[cell_key(i)] = {tab_total, i};
         tab_total += n[0] + n[1] + n[2];
       }
       pix_off[i] = pix_total;
@@ -966,9 +1185,20 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     // (they are read back from L2), or one
     const long long strip = (long long)pl.max_nyn * pl.max_nx;
     pl.strip_size = strip * std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / strip));
+    if (pl.n_cells) {
+      pl.cell_nx = pl.cell_ny = pl.cell_nyn = 0;
+      for (int i = 0; i < npat; ++i) {
+        if (!cells[i].list) continue;
+        pl.cell_nx = std::max(pl.cell_nx, nodes[i].x.n);
+        pl.cell_ny = std::max(pl.cell_ny, nodes[i].y.n);
+        pl.cell_nyn = std::max(pl.cell_nyn, sum_grid[i].y.n);
+      }
+      const long long cs = (long long)pl.cell_nyn * pl.cell_nx;
+      pl.strip_size = std::max(pl.strip_size, cs * std::min<long long>(pl.n_cells, std::max<long long>(1, (4LL << 20) / cs)));
+    }
     auto round = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t at_cpats = round(tab_total * sizeof(double));
-    const size_t at_strip = at_cpats + round(npat * sizeof(CoarsePattern));
+    const size_t at_strip = at_cpats + round(((size_t)npat + pl.n_cells) * sizeof(CoarsePattern));
     const size_t at_acc = at_strip + round(pl.strip_size * sizeof(double2));
     CUDA_TRY(pl.grids.ensure(at_acc + (spec ? pix_total * sizeof(double2) : 0)));
     char *base = (char *)pl.grids.p;
@@ -1057,7 +1287,15 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     pt.ff = (double *)pl.ff.p + ffo[i];
     pt.npix = points[i];
     pt.hkl = pl.coarse ? nullptr : q->d_hkl;
-    pt.q64 = pl.coarse ? pl.tables + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)] : q->d_q64;
+    pt.q64 = cells[i].list ? pl.tables + cell_tab[cell_key(i)].first
+             : pl.coarse   ? pl.tables + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)]
+                           : q->d_q64;
+    if (const MoleculeCells *c = cells[i].list) {
+      pt.atomsd = c->d_atoms;
+      pt.tiles = c->d_tiles;
+      pt.n_tiles = (int)c->tiles.size();
+      pt.cell_tiles = (int)((points[i] + tile_pix - 1) / tile_pix);
+    }
     double qmax = q->qmax;
     if (rot) {
       const double *R = rot + 9 * (size_t)i;
@@ -1118,14 +1356,17 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     if (mols[i]->n_kept > 0 && qsets[i]->npix > 0 && qmax * mols[i]->rbound >= std::ldexp(1.0, 17)) pl.fixw = false;
   }
   if (pl.coarse) {
-    std::vector<CoarsePattern> cp(npat);
+    std::vector<CoarsePattern> cp((size_t)npat + pl.n_cells);
+    memset(cp.data(), 0, cp.size() * sizeof(CoarsePattern));
+    size_t next_cell = npat;
     for (int i = 0; i < npat; ++i) {
       const spsim_b200_qset *q = qsets[i];
       size_t n[3];
       tab_sizes(i, n);
-      const double *tab = pats[i].q64;
+      const double *tab = pl.tables + tab_off[TabKey(q, nodes[i].x.n, nodes[i].y.n)];
       CoarsePattern &c = cp[i];
-      c.nodes = pats[i].acc;
+      c.parent = i;  // of the pixel patterns
+      c.nodes = pl.sums() + node_off[i];
       c.mx = tab + n[0];
       c.my = tab + n[0] + n[1];
       c.nx = q->geom.nx;
@@ -1136,6 +1377,38 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       c.ldy = coarse_ld(c.nyn);
       c.B = B;
       c.out = spec ? pl.pix_acc + pix_off[i] : nullptr;
+      if (!cells[i].list) continue;
+      cell_sizes(i, n);
+      const double *ctab = pats[i].q64;
+      for (int k = 0; k < cells[i].list->n; ++k) {
+        CoarsePattern &d = cp[next_cell++];
+        d.parent = 2 * npat + i;
+        d.nodes = pats[i].acc + k * points[i];
+        d.mx = ctab + n[0];
+        d.my = ctab + n[0] + n[1];
+        d.nx = nodes[i].x.n;
+        d.ny = nodes[i].y.n;
+        d.nxn = sum_grid[i].x.n;
+        d.nyn = sum_grid[i].y.n;
+        d.ldx = coarse_ld(d.nxn);
+        d.ldy = coarse_ld(d.nyn);
+        d.sum = pl.sums() + node_off[i];
+        for (int e = 0; e < 3; ++e) d.shift[e] = cells[i].list->shift[3 * (size_t)k + e];
+      }
+    }
+    for (const auto &t : cell_tab) {
+      const int i = t.second.second;
+      size_t n[3];
+      cell_sizes(i, n);
+      CoarseGrid g = sum_grid[i];
+      g.x.to_n = nodes[i].x.n;
+      g.x.to_alpha = nodes[i].x.alpha;
+      g.x.to_asin = nodes[i].x.asin_alpha;
+      g.y.to_n = nodes[i].y.n;
+      g.y.to_alpha = nodes[i].y.alpha;
+      g.y.to_asin = nodes[i].y.asin_alpha;
+      double *tab = pl.tables + t.second.first;
+      CUDA_TRY(launch_coarse_tables(qsets[i]->geom, g.x, g.y, tab, tab + n[0], tab + n[0] + n[1], stream));
     }
     for (const auto &t : tab_off) {
       size_t n[3];
@@ -1146,9 +1419,9 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       CUDA_TRY(launch_coarse_tables(qsets[i]->geom, nodes[i].x, nodes[i].y, tab, tab + n[0], tab + n[0] + n[1],
                                     stream));
     }
-    CUDA_TRY(cudaMemcpyAsync(pl.cpats, cp.data(), npat * sizeof(CoarsePattern), cudaMemcpyHostToDevice, stream));
-    // the pixel patterns behind the node patterns
-    pats.resize(2 * (size_t)npat);
+    CUDA_TRY(cudaMemcpyAsync(pl.cpats, cp.data(), cp.size() * sizeof(CoarsePattern), cudaMemcpyHostToDevice, stream));
+    // the pixel patterns behind the patterns summed, and with cells the patterns on their own nodes
+    pats.resize((pl.n_cells ? 3 : 2) * (size_t)npat);
     for (int i = 0; i < npat; ++i) {
       SfPattern &pt = pats[npat + i];
       pt = pats[i];
@@ -1156,6 +1429,15 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       pt.q64 = qsets[i]->d_q64;
       pt.ff = nullptr;
       pt.acc = cp[i].out;
+      if (!pl.n_cells) continue;
+      SfPattern &nd = pats[2 * (size_t)npat + i];
+      nd = pats[i];
+      nd.npix = (long long)nodes[i].x.n * nodes[i].y.n;
+      nd.q64 = pl.tables + tab_off[TabKey(qsets[i], nodes[i].x.n, nodes[i].y.n)];
+      nd.ff = nullptr;
+      nd.acc = pl.sums() + node_off[i];
+      nd.F = nullptr;
+      nd.I = nullptr;
     }
   }
   CUDA_TRY(cudaMemcpyAsync(pl.pats.p, pats.data(), pats.size() * sizeof(SfPattern), cudaMemcpyHostToDevice, stream));
@@ -1174,34 +1456,50 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
                                           : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
     const long long slots = (long long)num_sms() * occ;
     long long total_ptiles = 0;
-    for (int i = 0; i < npat; ++i) total_ptiles += (points[i] + tile_pix - 1) / tile_pix;
+    double tile_products = 0;  // point tiles x atom tiles
+    for (int i = 0; i < npat; ++i) {
+      const long long nptile = (points[i] + tile_pix - 1) / tile_pix;
+      total_ptiles += nptile;
+      tile_products += (double)nptile * (cells[i].list ? cells[i].list->tiles.size() : mols[i]->tiles.size());
+    }
     // a row chunk of a pipelined shot splits its atoms as the whole shot
     // would: the next chunk, on the other stream, fills this one's tail
     if (g_split_pixels_hint > 0) total_ptiles = std::max(total_ptiles, (g_split_pixels_hint + tile_pix - 1) / tile_pix);
     // split atoms when pixel tiles alone cannot fill the GPU several times over
-    const long long want = 6 * slots;
+    // (cells' runs of an element are short, and a split in one costs another
+    // flush: 6 items per slot 265 us on 50,000 atoms in 65 cells, 4 256 us)
+    const long long want = (pl.n_cells ? 4 : 6) * slots;
     std::vector<WorkItem> items;
     std::vector<double> cost;
     for (int i = 0; i < npat; ++i) {
       const long long nptile = (points[i] + tile_pix - 1) / tile_pix;
-      const int ntile = (int)mols[i]->tiles.size();
-      if (ntile == 0 || points[i] == 0) continue;
-      int split = 1;
-      if (total_ptiles < want) split = (int)std::min<long long>((want + total_ptiles - 1) / total_ptiles, ntile);
-      split = std::max(1, std::min(split, std::max(1, pl.coarse ? ntile : ntile / 2)));
-      for (long long t = 0; t < nptile; ++t) {
-        const long long pix_here = std::min(tile_pix, points[i] - t * tile_pix);
-        for (int s = 0; s < split; ++s) {
-          WorkItem w;
-          w.pattern = i;
-          w.pixel_tile = (int)t;
-          w.k0 = (int)((long long)ntile * s / split);
-          w.k1 = (int)((long long)ntile * (s + 1) / split);
-          if (w.k1 <= w.k0) continue;
-          items.push_back(w);
-          int atoms_here = 0;
-          for (int k = w.k0; k < w.k1; ++k) atoms_here += mols[i]->tiles[k].count;
-          cost.push_back((double)pix_here * atoms_here);
+      const MoleculeCells *list = cells[i].list;
+      const std::vector<TileDesc> &tiles = list ? list->tiles : mols[i]->tiles;
+      if (tiles.empty() || points[i] == 0) continue;
+      for (int c = 0; c < (list ? list->n : 1); ++c) {
+        const int first = list ? list->tile_begin[c] : 0;
+        const int ntile = (list ? list->tile_begin[c + 1] : (int)tiles.size()) - first;
+        int split = 1;
+        if (pl.coarse) {  // by cost: molecules and cells are uneven, and the longest item is the launch's tail
+          split = (int)std::min<double>(std::ceil(want * (double)ntile / tile_products), ntile);
+        } else if (total_ptiles < want) {
+          split = (int)std::min<long long>((want + total_ptiles - 1) / total_ptiles, ntile);
+          split = std::max(1, std::min(split, std::max(1, ntile / 2)));
+        }
+        for (long long t = 0; t < nptile; ++t) {
+          const long long pix_here = std::min(tile_pix, points[i] - t * tile_pix);
+          for (int s = 0; s < split; ++s) {
+            WorkItem w;
+            w.pattern = i;
+            w.pixel_tile = (int)(c * nptile + t);
+            w.k0 = first + (int)((long long)ntile * s / split);
+            w.k1 = first + (int)((long long)ntile * (s + 1) / split);
+            if (w.k1 <= w.k0) continue;
+            items.push_back(w);
+            int atoms_here = 0;
+            for (int k = w.k0; k < w.k1; ++k) atoms_here += tiles[k].count;
+            cost.push_back((double)pix_here * atoms_here);
+          }
         }
       }
     }
@@ -1246,8 +1544,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 // gate: a stand-by plan, run only where the device sets *gate (nullptr: always).
 static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, cudaEvent_t ev1, int *gate = nullptr) {
   cudaError_t e;
-  long long acc_total = 0;
-  for (long long n : pl.npix_of) acc_total += n;
+  const long long acc_total = pl.acc_total;
   if (gate) {
     if ((e = launch_gate((const SfPattern *)pl.pats.p, pl.npat, pl.n_items, gate, pl.head() + 8, pl.sums(), acc_total,
                          stream)))
@@ -1275,6 +1572,11 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   if (pl.coarse) {
     CoarseBatch b;
     memset(&b, 0, sizeof(b));
+    b.pats = pats;
+    b.coarse = pl.cpats + pl.npat;
+    if (pl.n_cells && (e = launch_coarse_interp(b, pl.n_cells, pl.cell_nx, pl.cell_ny, pl.cell_nyn, pl.strip,
+                                                pl.strip_size, stream)))
+      return e;
     b.pats = pats + pixels;
     b.coarse = pl.cpats;
     if ((e = launch_coarse_interp(b, pl.npat, pl.max_nx, pl.max_ny, pl.max_nyn, pl.strip, pl.strip_size, stream)))
@@ -1340,7 +1642,7 @@ static cudaError_t refresh_descriptors(Plan &pl, const double *rot, float *const
       memcpy(pt.rot, rot + 9 * k, 9 * sizeof(double));
       changed = true;
     }
-    if (i < outputs || pl.spectrum) continue;  // (a spectrum's are the launch's arguments)
+    if (i < outputs || (outputs && i >= 2 * outputs) || pl.spectrum) continue;  // (a spectrum's are the launch's arguments)
     float2 *F = F_dev ? (float2 *)F_dev[k] : nullptr;
     float *I = I_dev ? I_dev[k] : nullptr;
     moved = moved || pt.F != F || pt.I != I;

@@ -27,6 +27,8 @@ CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, b
   a.half = 1.0;
   a.n = 0;
   a.alpha = a.asin_alpha = 0.0;
+  a.to_n = 0;
+  a.to_alpha = a.to_asin = 0.0;
   if (a.angular) {
     const double edge = 0.5 * (n_pix - 1) / n_pix * size;
     const double t0 = std::atan((-edge - centre) / distance), t1 = std::atan((edge - centre) / distance);
@@ -59,7 +61,10 @@ __device__ __forceinline__ double coarse_node_pos(const CoarseAxis &a, int k) {
   return (0.5 * (a.n_pix - 1) * X / a.n_pix) * a.size - a.centre;
 }
 
-// One row (pixel p) of an interpolation matrix by one warp:
+// points interpolated to
+__host__ __device__ __forceinline__ int coarse_rows(const CoarseAxis &a) { return a.to_n > 0 ? a.to_n : a.n_pix; }
+
+// One row (point p) of an interpolation matrix by one warp:
 // M[k] = (w_k / (xi - xi_k)) / sum_j w_j / (xi - xi_j), the barycentric weights
 // of the Chebyshev extreme points w_k = (-1)^k, halved at both ends.
 // mt: the transpose, [node][lt], or nullptr.
@@ -67,7 +72,9 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
                                            double *__restrict__ mt) {
   const int lane = threadIdx.x & 31, n = a.n;
   double X = 2.0 * p / (a.n_pix - 1) - 1.0;
-  if (a.angular) {
+  if (a.to_n > 0) {
+    X = asin(a.to_alpha * cospi((double)p / (a.to_n - 1))) / a.to_asin;
+  } else if (a.angular) {
     const double pos = ((p - (a.n_pix - 1.0) / 2.0) / a.n_pix) * a.size - a.centre;
     X = (atan(pos / a.distance) - a.mid) / a.half;
   }
@@ -94,7 +101,7 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
     m[(long long)p * ld + k] = v;
     if (mt && k < n) {
       mt[(long long)k * lt + p] = v;
-      if (p == a.n_pix - 1)
+      if (p == coarse_rows(a) - 1)
         for (int z = p + 1; z < lt; ++z) mt[(long long)k * lt + z] = 0.0;
     }
   }
@@ -102,7 +109,7 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
 
 __global__ void __launch_bounds__(256) coarse_tables_kernel(CoarseTables t) {
   const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  const int nx = t.x.n_pix, ny = t.y.n_pix;
+  const int nx = coarse_rows(t.x), ny = coarse_rows(t.y);
   if (warp < nx) {
     coarse_row(warp, t.x, t.ldx, t.mx, t.ltx, t.tx);
   } else if (warp < nx + ny) {
@@ -142,7 +149,7 @@ cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const Co
   t.lty = coarse_ld(y.n_pix);
   t.tx = tx;
   t.ty = ty;
-  const long long warps = (long long)x.n_pix + y.n_pix + ((long long)x.n * y.n + 31) / 32;
+  const long long warps = (long long)coarse_rows(x) + coarse_rows(y) + ((long long)x.n * y.n + 31) / 32;
   coarse_tables_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(t);
   return cudaGetLastError();
 }
@@ -274,11 +281,11 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
   float2 *F = batch.F ? batch.F + pattern * npix : nullptr;
   float *I = batch.I ? batch.I + pattern * npix : nullptr;
   if (batch.pats) {
-    const SfPattern &pt = batch.pats[pattern];
+    const SfPattern &pt = batch.pats[cp.parent];
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
     q64 = pt.q64;
     rot = pt.has_rot ? pt.rot : nullptr;
-    center = pt.center;
+    center = cp.sum ? cp.shift : pt.center;
     qscale = pt.qscale;
     F = pt.F;
     I = pt.I;
@@ -295,7 +302,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
       tile[(8 * i + fr) * TLD + 8 * (j >> 1) + 2 * fc + (j & 1)] =
           make_double2(re_[i][j >> 1][j & 1], im_[i][j >> 1][j & 1]);
   __syncwarp();
-  const bool need_q = F || cp.B != 0.0 || cp.out;
+  const bool need_q = F || cp.B != 0.0 || cp.out || cp.sum;
 #pragma unroll 1
   for (int e = lane; e < 8 * RM * TN; e += 32) {
     const int y = m0 + e / TN, x = n0 + e % TN;
@@ -314,7 +321,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
         cp.out[p] = make_double2(re, im);
         continue;
       }
-      if (F) {
+      if (F || cp.sum) {
         double ux = a, uy = b, uz = c;
         if (rot) {
           ux = rot[0] * a + rot[1] * b + rot[2] * c;
@@ -325,6 +332,11 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
         t -= rint(t);
         double sn, cs;
         sincospi(2.0 * t, &sn, &cs);
+        if (cp.sum) {
+          atomicAdd(&cp.sum[p].x, re * cs + im * sn);
+          atomicAdd(&cp.sum[p].y, im * cs - re * sn);
+          continue;
+        }
         F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
       }
     }
@@ -436,6 +448,84 @@ cudaError_t launch_coarse_adjoint(const CoarseAdjoint &a, int npat, double2 *H, 
     product(a.tx, coarse_ld(a.nx), a.nxn, H, a.ny, a.nx, strip, n, st);
     product(a.ty, coarse_ld(a.ny), a.nyn, strip, a.nxn, a.ny, nodes + (long long)p0 * a.nyn * a.nxn, n, st);
   }
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// atoms by cells
+
+__device__ __forceinline__ double cell_centre(const CellLattice &l, int i, int sub) {
+  return l.a * (i - l.reach + 0.5 * sub);
+}
+
+__global__ void __launch_bounds__(TILE_ATOMS)
+    cells_count_kernel(CellLattice l, const AtomD *__restrict__ atoms, const int *__restrict__ perm,
+                       const TileDesc *__restrict__ tiles, int n_elem, int *__restrict__ key, int *__restrict__ count) {
+  const TileDesc t = tiles[blockIdx.x];
+  if ((int)threadIdx.x >= t.count) return;
+  const int i = t.atom_begin + threadIdx.x;
+  if (perm[i] < 0) return;
+  const double r[3] = {atoms[i].x, atoms[i].y, atoms[i].z};
+  int at[2][3];
+  double d[2] = {0.0, 0.0};
+#pragma unroll
+  for (int sub = 0; sub < 2; ++sub)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      at[sub][k] = min(max((int)rint(r[k] / l.a - 0.5 * sub) + l.reach, 0), l.dim - 1);
+      const double e = r[k] - cell_centre(l, at[sub][k], sub);
+      d[sub] += e * e;
+    }
+  const int sub = d[1] < d[0];
+  const int cell = ((sub * l.dim + at[sub][2]) * l.dim + at[sub][1]) * l.dim + at[sub][0];
+  key[i] = cell * n_elem + t.elem;
+  atomicAdd(&count[cell * n_elem + t.elem], 1);
+}
+
+__global__ void __launch_bounds__(256)
+    cells_order_kernel(const int *__restrict__ perm, int n_padded, const int *__restrict__ key,
+                       const int *__restrict__ run_begin, int *__restrict__ cursor, int *__restrict__ order) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_padded || perm[i] < 0) return;
+  order[run_begin[key[i]] + atomicAdd(&cursor[key[i]], 1)] = i;
+}
+
+// each atom's place in its run by counting those before it, so that the sums'
+// order does not depend on the atomics'
+__global__ void __launch_bounds__(256)
+    cells_place_kernel(CellLattice l, const AtomD *__restrict__ atoms, const int *__restrict__ perm, int n_padded,
+                       int n_elem, const int *__restrict__ key, const int *__restrict__ count,
+                       const int *__restrict__ run_begin, const int *__restrict__ order, AtomD *__restrict__ out) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n_padded || perm[i] < 0) return;
+  const int k = key[i], begin = run_begin[k], n = count[k];
+  int rank = 0;
+#pragma unroll 8
+  for (int s = 0; s < n; ++s) rank += order[begin + s] < i;
+  const int cell = k / n_elem;
+  const int x = cell % l.dim, y = cell / l.dim % l.dim, z = cell / (l.dim * l.dim) % l.dim;
+  const int sub = cell / (l.dim * l.dim * l.dim);
+  AtomD a = atoms[i];
+  a.x -= cell_centre(l, x, sub);
+  a.y -= cell_centre(l, y, sub);
+  a.z -= cell_centre(l, z, sub);
+  out[begin + rank] = a;
+}
+
+cudaError_t launch_cells_count(const CellLattice &l, const AtomD *atoms, const int *perm, const TileDesc *tiles,
+                               int n_tiles, int n_elem, int *key, int *count, cudaStream_t st) {
+  if (n_tiles > 0) cells_count_kernel<<<n_tiles, TILE_ATOMS, 0, st>>>(l, atoms, perm, tiles, n_elem, key, count);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_cells_build(const CellLattice &l, const AtomD *atoms, const int *perm, int n_padded, int n_elem,
+                               const int *key, const int *count, const int *run_begin, int *cursor, int *order,
+                               AtomD *out, int n_slots, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(out, 0, n_slots * sizeof(AtomD), st);  // padding: weight 0
+  if (e != cudaSuccess || n_padded <= 0) return e;
+  const unsigned grid = (unsigned)((n_padded + 255) / 256);
+  cells_order_kernel<<<grid, 256, 0, st>>>(perm, n_padded, key, run_begin, cursor, order);
+  cells_place_kernel<<<grid, 256, 0, st>>>(l, atoms, perm, n_padded, n_elem, key, count, run_begin, order, out);
   return cudaGetLastError();
 }
 

@@ -34,6 +34,9 @@ struct CoarseAxis {
   double size, centre, distance, mid, half;
   int n;  // nodes
   double alpha, asin_alpha;
+  // the points to interpolate to: the pixels, or (to_n > 0) another grid's nodes
+  int to_n;
+  double to_alpha, to_asin;
 };
 
 constexpr int COARSE_MAX_NODES = 1024;  // per axis
@@ -56,6 +59,11 @@ struct CoarsePattern {
   int nx, ny, nxn, nyn, ldx, ldy;
   double B;              // global B factor, applied per pixel
   double2 *out;          // centred pixel amplitudes (FP64) instead of F and I, or nullptr
+  int parent;            // SfPattern of the points interpolated to
+  // one cell of a molecule (launch_cells_build): its amplitudes, times the phase
+  // of its centre `shift`, are added to sum on the pattern's own nodes
+  double2 *sum;
+  double shift[3];
 };
 
 __host__ __device__ inline int coarse_ld(int n) { return (n + 7) / 8 * 8; }
@@ -80,6 +88,25 @@ struct CoarseBatch {
 // (strip_size complex values, at least max_nyn * max_nx).
 cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
                                  long long strip_size, cudaStream_t st);
+
+// A molecule's atoms by cells, the Voronoi cells of a body-centred cubic
+// lattice of constant a about the molecule's centre (the lattice whose cells'
+// circumscribed sphere, of radius sqrt(5) / 4 a, is the smallest for their
+// volume): cell ((sub * dim + z) * dim + y) * dim + x has its centre at
+// a (x - reach + sub / 2, ...), dim = 2 reach + 1.
+struct CellLattice {
+  double a;
+  int reach, dim;
+};
+// The count of atoms per (cell, element), and each atom's such index in key.
+cudaError_t launch_cells_count(const CellLattice &l, const AtomD *atoms, const int *perm, const TileDesc *tiles,
+                               int n_tiles, int n_elem, int *key, int *count, cudaStream_t st);
+// The records of the cells: run_begin[key] is where (cell, element)'s begin, in
+// the atoms' own order, their positions about the cell's centre.  cursor: as
+// large as count, zero; order: n_slots, scratch.
+cudaError_t launch_cells_build(const CellLattice &l, const AtomD *atoms, const int *perm, int n_padded, int n_elem,
+                               const int *key, const int *count, const int *run_begin, int *cursor, int *order,
+                               AtomD *out, int n_slots, cudaStream_t st);
 
 // The adjoint of the interpolation: per pattern, from the forward's F and
 // G = dL/d|F|^2 on the pixels to the amplitudes H on the nodes.

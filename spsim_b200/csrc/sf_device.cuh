@@ -71,6 +71,8 @@ struct SfPattern {
   long long tile0;         // first pixel-tile index of this pattern in a grid-mapped launch
   const int *mol_err;      // the molecule's range word (atoms moved past its bounds), or nullptr
   int *plan_err;           // where the finalizing kernel reports it
+  int cell_tiles;          // point tiles per cell (acc: [cells][npix], a work item's pixel_tile
+                           // cell * cell_tiles + tile), or 0: the sum of the whole molecule
 };
 
 struct WorkItem {      // one CTA's unit of work

@@ -64,9 +64,11 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
     const long long npix = pt.npix;
     const AtomD *__restrict__ atomsd = pt.atomsd;
     const TileDesc *__restrict__ tiles = pt.tiles;
+    const int cell = pt.cell_tiles ? wi.pixel_tile / pt.cell_tiles : 0;
+    double2 *__restrict__ acc = pt.acc + cell * npix;
 
     // node i of this lane: pix0 + 128 (i / 4) + i % 4
-    const long long pix0 = (long long)wi.pixel_tile * NODE_TILE + 4 * lane;
+    const long long pix0 = (long long)(wi.pixel_tile - cell * pt.cell_tiles) * NODE_TILE + 4 * lane;
     double qx[P], qy[P], qz[P];
     float s2n[P];
 #pragma unroll
@@ -213,10 +215,10 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
       }
       if (p < npix) {
         if (whole) {
-          pt.acc[p] = v;
+          acc[p] = v;
         } else {
-          atomicAdd(&pt.acc[p].x, v.x);
-          atomicAdd(&pt.acc[p].y, v.y);
+          atomicAdd(&acc[p].x, v.x);
+          atomicAdd(&acc[p].y, v.y);
         }
       }
     }
@@ -266,8 +268,10 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPat
     const long long npix = pt.npix;
     const AtomD *__restrict__ atomsd = pt.atomsd;
     const TileDesc *__restrict__ tiles = pt.tiles;
+    const int cell = pt.cell_tiles ? wi.pixel_tile / pt.cell_tiles : 0;
+    double2 *__restrict__ acc = pt.acc + cell * npix;
 
-    const long long pix0 = (long long)wi.pixel_tile * (32 * P) + lane;  // node i of this lane: pix0 + 32 i
+    const long long pix0 = (long long)(wi.pixel_tile - cell * pt.cell_tiles) * (32 * P) + lane;  // node i of this lane: pix0 + 32 i
     double qx[P], qy[P], qz[P];
     double s2n[P];
 #pragma unroll
@@ -377,10 +381,10 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPat
       const long long p = pix0 + 32 * i;
       if (p < npix) {
         if (whole) {
-          pt.acc[p] = v;
+          acc[p] = v;
         } else {
-          atomicAdd(&pt.acc[p].x, v.x);
-          atomicAdd(&pt.acc[p].y, v.y);
+          atomicAdd(&acc[p].x, v.x);
+          atomicAdd(&acc[p].y, v.y);
         }
       }
     }

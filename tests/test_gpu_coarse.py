@@ -180,6 +180,75 @@ def test_calls_that_stay_on_every_pixel(cuda):
     assert not I.any()
 
 
+def _cells_case(shape, n, seed):
+    """Atoms of a ball, a rod, a sheet and two far balls, which leave cells empty, single and uneven."""
+    Z, pos = synth.random_molecule(n, 8.2e-9, seed)
+    if shape == "rod":
+        pos = pos * np.float32([0.2, 0.15, 1.0])
+    elif shape == "sheet":
+        pos = pos * np.float32([1.0, 0.04, 0.9])
+    elif shape == "pair":
+        pos = pos * np.float32(0.4) + np.float32([5e-9, 0, 0]) * np.sign(pos[:, :1])
+    return Z, (pos + np.float32([4e-9, -1e-9, 2e-9])).astype(np.float32)
+
+
+@pytest.mark.parametrize("shape", ["ball", "rod", "sheet", "pair"])
+@pytest.mark.parametrize("precision", ["f32", "fp64"])
+@pytest.mark.parametrize("det", [dict(center_x=0.007), dict(spherical=True)], ids=["off_axis", "spherical"])
+def test_cells(cuda, shape, precision, det):
+    # sums cell by cell: far fewer terms than on the patterns' own nodes, which a
+    # molecule whose positions were rewritten on the device still takes
+    Z, pos = _cells_case(shape, 12001, 221)
+    rng = np.random.Generator(np.random.PCG64(222))
+    occ = rng.uniform(-0.5, 1.0, len(Z)).astype(np.float32)
+    b = rng.uniform(0.0, 40.0, len(Z)).astype(np.float32)
+    d = _det(141, 118, pixel=280e-6, wavelength=0.13e-9, **det)
+    q, qs, R = _q(d), core.QSet.from_detector(**d), synth.haar_rotations(96, 223)
+    mol = core.Molecule(Z, pos, occ=occ, bfac=b)
+    F = torch.empty(len(R), d["ny"] * d["nx"], dtype=torch.complex64, device="cuda")
+    I = torch.empty(len(R), d["ny"] * d["nx"], device="cuda")
+    core.forward_batch([mol] * len(R), [qs] * len(R), rots=R, precision=precision, F=list(F), I=list(I), B=5.0)
+    terms = core.last_terms_evaluated()
+    for k in (0, 57, 95):
+        F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q @ R[k].T, occ=occ, bfac=b, B=5.0)
+        e_max, e_l2 = intensity_errors(I[k].cpu().numpy(), I64)
+        tol = TOL if precision == "f32" else (2e-7, 1e-7)
+        assert e_max < tol[0] and e_l2 < tol[1], (k, e_max, e_l2)
+        assert np.linalg.norm(F[k].cpu().numpy().reshape(F64.shape) - F64) < tol[1] * np.linalg.norm(F64)
+    # rotations of the next call go into the same plan
+    core.forward_batch([mol] * len(R), [qs] * len(R), rots=R[::-1].copy(), precision=precision, F=list(F), I=list(I), B=5.0)
+    assert core.last_terms_evaluated() == terms
+    F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q @ R[95].T, occ=occ, bfac=b, B=5.0)
+    assert intensity_errors(I[0].cpu().numpy(), I64)[1] < 1e-6
+    if precision == "f32":
+        moved = core.Molecule(Z, pos, occ=occ, bfac=b)
+        moved.update_device(torch.from_numpy(pos).cuda())
+        core.forward_batch([moved] * len(R), [qs] * len(R), rots=R, F=None, I=list(I), want_F=False, B=5.0)
+        assert core.last_terms_evaluated() > 1.3 * terms
+
+
+def test_cells_of_a_spectrum_and_of_uneven_molecules(cuda):
+    Z, pos = synth.random_molecule(30000, 9.0e-9, 224)
+    d = _det(256, 250, pixel=75e-6)
+    q, mol, qs = _q(d), core.Molecule(Z, pos), core.QSet.from_detector(**d)
+    F, I = core.forward(mol, qs)
+    whole = core.last_terms_evaluated()
+    _check(F, I, Z, pos, q)
+    F, I = core.forward_spectrum(mol, qs, d["wavelength"], 0.05, 4)
+    assert core.last_terms_evaluated() < 6 * whole
+    pick = np.arange(0, len(q), 97)  # the oracle on every 97th pixel
+    _, I64 = O.structure_factor_spectrum(Z, pos.astype(np.float64), q[pick], d["wavelength"], 0.05, 4)
+    e_max, e_l2 = intensity_errors(I.cpu().numpy().reshape(-1)[pick], I64)
+    assert e_max < TOL[0] and e_l2 < TOL[1], (e_max, e_l2)
+    # molecules with and without cells in one call
+    Zs, ps = synth.random_molecule(700, 1.5e-9, 225)
+    small = core.Molecule(Zs, ps)
+    Fs, Is = core.forward_batch([small, mol, small], [qs] * 3)
+    _check(Fs[1], Is[1], Z, pos, q)
+    for k in (0, 2):
+        _check(Fs[k], Is[k], Zs, ps, q)
+
+
 def _rel(a, b):
     return float(np.linalg.norm(a - b) / np.linalg.norm(b))
 
