@@ -590,6 +590,25 @@ static int check_detector(int nx, int ny, float width, float height, float dista
   return SPSIM_OK;
 }
 
+static DetGeom det_geom(int nx, int ny, float width, float height, float distance, float center_x, float center_y,
+                        float wavelength, int spherical) {
+  DetGeom g;
+  g.nx = nx;
+  g.ny = ny;
+  g.spherical = spherical ? 1 : 0;
+  g.width = width;
+  g.height = height;
+  g.distance = distance;
+  g.cx = center_x;
+  g.cy = center_y;
+  g.ewald = 1.0 / (double)wavelength;
+  g.px_size = (double)(width / nx);
+  g.py_size = (double)(height / ny);
+  g.fpx = 2 * std::sin(std::atan(g.px_size / distance) / 2) / wavelength;
+  g.fpy = 2 * std::sin(std::atan(g.py_size / distance) / 2) / wavelength;
+  return g;
+}
+
 extern "C" int spsim_b200_qset_from_detector(int nx, int ny, float width, float height, float distance,
                                              float center_x, float center_y, float wavelength, int spherical,
                                              spsim_b200_qset **out) {
@@ -605,23 +624,8 @@ extern "C" int spsim_b200_qset_from_detector(int nx, int ny, float width, float 
   q->device = dev;
   q->npix = (long long)nx * ny;
   q->row = nx;
-  {
-    DetGeom &g = q->geom;
-    g.nx = nx;
-    g.ny = ny;
-    g.spherical = spherical ? 1 : 0;
-    g.width = width;
-    g.height = height;
-    g.distance = distance;
-    g.cx = center_x;
-    g.cy = center_y;
-    g.ewald = 1.0 / (double)wavelength;
-    g.px_size = (double)(width / nx);
-    g.py_size = (double)(height / ny);
-    g.fpx = 2 * std::sin(std::atan(g.px_size / distance) / 2) / wavelength;
-    g.fpy = 2 * std::sin(std::atan(g.py_size / distance) / 2) / wavelength;
-    q->has_geom = true;
-  }
+  q->geom = det_geom(nx, ny, width, height, distance, center_x, center_y, wavelength, spherical);
+  q->has_geom = true;
   CUDA_TRY(cudaMalloc(&q->d_q64, 3 * q->npix * sizeof(double)));
   CUDA_TRY(launch_ewald(nx, ny, width, height, distance, center_x, center_y, wavelength, spherical, nullptr,
                         q->d_q64, 0));
@@ -717,6 +721,7 @@ struct Plan {
   // the interpolation of the cells' sums writes
   int n_cells = 0, cell_nx = 0, cell_ny = 0, cell_nyn = 0;
   long long acc_total = 0;  // FP64 sums
+  int n_interp = 0;         // patterns interpolated to pixels: npat, and a list's two derivatives
   // the same patterns on every pixel, run where a B factor rewritten on the
   // device is beyond what the coarse grids are sized for
   std::unique_ptr<Plan> direct;
@@ -1063,15 +1068,29 @@ static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const sp
   return SPSIM_OK;
 }
 
+// The amplitudes that launch_list_combine takes: two patterns, of a detector and
+// of the same lifted, and the first one's derivatives.
+struct ListSums {
+  double2 *out = nullptr;  // [4][npix]: A, A lifted, dA/dX, dA/dY
+  CoarseGrid grid;
+};
+
 static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
-                      cudaStream_t stream, const Spectrum *spec, bool allow_coarse = true) {
+                      cudaStream_t stream, const Spectrum *spec, bool allow_coarse = true,
+                      const ListSums *list = nullptr) {
   pl.npat = npat;
   pl.precision = precision;
   std::vector<CoarseGrid> nodes;
   for (int i = 0; i < npat; ++i)
     if (!mols[i] || !qsets[i]) return fail(SPSIM_ERR_INVALID_ARG, "pattern %d: NULL molecule or q set", i);
-  pl.coarse = allow_coarse && coarse_plan(npat, mols, qsets, rot, precision, spec, nodes);
+  if (list) {  // (admitted before the call)
+    nodes.assign(npat, list->grid);
+    pl.coarse = true;
+  } else {
+    pl.coarse = allow_coarse && coarse_plan(npat, mols, qsets, rot, precision, spec, nodes);
+  }
+  pl.n_interp = pl.coarse ? npat + (list ? 2 : 0) : 0;
   pl.mode = precision == SPSIM_PREC_F32_FAST && !pl.coarse ? PREC_MODE_MUFU : PREC_MODE_POLY;
   // cells, and the grid of each pattern's sums: its cells' or its own
   std::vector<PatternCells> cells(npat);
@@ -1175,6 +1194,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       pix_off[i] = pix_total;
       pix_total += qsets[i]->npix;
     }
+    if (list) tab_total += (size_t)(qsets[0]->geom.nx * coarse_ld(nodes[0].x.n) + qsets[0]->geom.ny * coarse_ld(nodes[0].y.n));
     pl.max_nx = pl.max_ny = pl.max_nyn = 0;
     for (int i = 0; i < npat; ++i) {
       pl.max_nx = std::max(pl.max_nx, qsets[i]->geom.nx);
@@ -1184,7 +1204,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     // the interpolation's strips: a group of patterns at a time, 64 MB of them
     // (they are read back from L2), or one
     const long long strip = (long long)pl.max_nyn * pl.max_nx;
-    pl.strip_size = strip * std::min<long long>(npat, std::max<long long>(1, (4LL << 20) / strip));
+    pl.strip_size = strip * std::min<long long>(pl.n_interp, std::max<long long>(1, (4LL << 20) / strip));
     if (pl.n_cells) {
       pl.cell_nx = pl.cell_ny = pl.cell_nyn = 0;
       for (int i = 0; i < npat; ++i) {
@@ -1198,7 +1218,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     }
     auto round = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t at_cpats = round(tab_total * sizeof(double));
-    const size_t at_strip = at_cpats + round(((size_t)npat + pl.n_cells) * sizeof(CoarsePattern));
+    const size_t at_strip = at_cpats + round(((size_t)pl.n_interp + pl.n_cells) * sizeof(CoarsePattern));
     const size_t at_acc = at_strip + round(pl.strip_size * sizeof(double2));
     CUDA_TRY(pl.grids.ensure(at_acc + (spec ? pix_total * sizeof(double2) : 0)));
     char *base = (char *)pl.grids.p;
@@ -1356,9 +1376,9 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     if (mols[i]->n_kept > 0 && qsets[i]->npix > 0 && qmax * mols[i]->rbound >= std::ldexp(1.0, 17)) pl.fixw = false;
   }
   if (pl.coarse) {
-    std::vector<CoarsePattern> cp((size_t)npat + pl.n_cells);
+    std::vector<CoarsePattern> cp((size_t)pl.n_interp + pl.n_cells);
     memset(cp.data(), 0, cp.size() * sizeof(CoarsePattern));
-    size_t next_cell = npat;
+    size_t next_cell = pl.n_interp;
     for (int i = 0; i < npat; ++i) {
       const spsim_b200_qset *q = qsets[i];
       size_t n[3];
@@ -1376,7 +1396,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       c.ldx = coarse_ld(c.nxn);
       c.ldy = coarse_ld(c.nyn);
       c.B = B;
-      c.out = spec ? pl.pix_acc + pix_off[i] : nullptr;
+      c.out = list ? list->out + i * q->npix : spec ? pl.pix_acc + pix_off[i] : nullptr;
       if (!cells[i].list) continue;
       cell_sizes(i, n);
       const double *ctab = pats[i].q64;
@@ -1395,6 +1415,20 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
         d.sum = pl.sums() + node_off[i];
         for (int e = 0; e < 3; ++e) d.shift[e] = cells[i].list->shift[3 * (size_t)k + e];
       }
+    }
+    if (list) {
+      const DetGeom &g = qsets[0]->geom;
+      double *dx = pl.tables + tab_total - ((size_t)g.nx * cp[0].ldx + (size_t)g.ny * cp[0].ldy);
+      double *dy = dx + (size_t)g.nx * cp[0].ldx;
+      cp[2] = cp[3] = cp[0];
+      cp[2].mx = dx;
+      cp[2].out = list->out + 2 * qsets[0]->npix;
+      cp[3].my = dy;
+      cp[3].out = list->out + 3 * qsets[0]->npix;
+      CoarseGrid d = nodes[0];
+      d.x.derivative = d.y.derivative = 1;
+      // (its node q vectors are the pattern's own, written again)
+      CUDA_TRY(launch_coarse_tables(g, d.x, d.y, pl.tables + tab_off[TabKey(qsets[0], d.x.n, d.y.n)], dx, dy, stream));
     }
     for (const auto &t : cell_tab) {
       const int i = t.second.second;
@@ -1573,13 +1607,13 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
     CoarseBatch b;
     memset(&b, 0, sizeof(b));
     b.pats = pats;
-    b.coarse = pl.cpats + pl.npat;
+    b.coarse = pl.cpats + pl.n_interp;
     if (pl.n_cells && (e = launch_coarse_interp(b, pl.n_cells, pl.cell_nx, pl.cell_ny, pl.cell_nyn, pl.strip,
                                                 pl.strip_size, stream)))
       return e;
     b.pats = pats + pixels;
     b.coarse = pl.cpats;
-    if ((e = launch_coarse_interp(b, pl.npat, pl.max_nx, pl.max_ny, pl.max_nyn, pl.strip, pl.strip_size, stream)))
+    if ((e = launch_coarse_interp(b, pl.n_interp, pl.max_nx, pl.max_ny, pl.max_nyn, pl.strip, pl.strip_size, stream)))
       return e;
   }
   if (pl.spectrum > 0)
@@ -1686,7 +1720,7 @@ static int check_flags(Plan &pl) {
 static int run_forward(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                        const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
                        cudaStream_t stream, bool cache, const Spectrum *spec = nullptr, bool sync = true,
-                       Plan *scratch = nullptr) {
+                       Plan *scratch = nullptr, const ListSums *list = nullptr) {
   if (npat < 0) return fail(SPSIM_ERR_INVALID_ARG, "npatterns < 0");
   if (npat == 0) return SPSIM_OK;
   if (!mols || !qsets) return fail(SPSIM_ERR_INVALID_ARG, "NULL molecule or q-set array");
@@ -1753,7 +1787,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     }
     pl->key_ptrs = kp;
     pl->key_vals = kv;
-    st = build_plan(*pl, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec);
+    st = build_plan(*pl, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec, true, list);
     if (st) return st;
   }
   g_last_terms = pl->terms;
@@ -1898,6 +1932,13 @@ struct HostSession {
   std::vector<Plan *> part_plans;
   int parts = 0;
   spsim_b200_qset *shot_q = nullptr;  // the shot's whole HKL list, borrowed (no copy)
+  // the shot on the nodes of its detector: the detector and the same lifted, the
+  // sums' plan and the pixels' amplitudes
+  spsim_b200_qset *nodes_q[2] = {nullptr, nullptr};
+  Plan *nodes_plan = nullptr;
+  DevBuf *nodes_out = nullptr;
+  ListCombine combine;
+  bool nodes_open = false;  // a shot prepared by spsim_internal_shot_nodes_begin
 };
 static thread_local HostSession g_host;
 static thread_local spsim_b200_molecule *g_shot_mol = nullptr;  // set by spsim_internal_shot_molecule
@@ -2002,6 +2043,9 @@ extern "C" void spsim_internal_release_host_session(void) {
       delete g_host.shot_q;
     }
     for (Plan *p : g_host.part_plans) delete p;
+    for (spsim_b200_qset *q : g_host.nodes_q) delete q;
+    delete g_host.nodes_plan;
+    delete g_host.nodes_out;
   }
   g_host = HostSession();
   g_shot_mol = nullptr;
@@ -2102,6 +2146,7 @@ extern "C" int spsim_internal_shot_molecule(int natoms, const int32_t *Z, const 
   }
   g_shot_mol = nullptr;
   g_host.parts = 0;
+  g_host.nodes_open = false;
   spsim_b200_molecule *m = nullptr;
   st = host_session_molecule(natoms, Z, pos, nullptr, nullptr, delta_atoms, beam, &m);
   if (st) return st;
@@ -2202,6 +2247,91 @@ extern "C" int spsim_internal_shot_part(int64_t p0, int64_t p1, float B, int pre
   return st;
 }
 
+// A shot on the nodes of its detector, from the direct sum's time up at which
+// two node sums, four interpolations and the plan's host work are cheaper
+// (512 x 480 pixels: from some 1,500 atoms); *used = 0 where it is not, or not
+// admitted.  Enqueues all but the pixels' combination on the legacy stream.
+extern "C" int spsim_internal_shot_nodes_begin(int64_t npix, const float *hkl_dev, int nx, int ny, float width,
+                                               float height, float distance, float center_x, float center_y,
+                                               float wavelength, int spherical, const float *rot, float B,
+                                               int precision, int *used) {
+  *used = 0;
+  g_host.nodes_open = false;
+  spsim_b200_molecule *m = g_shot_mol;
+  int dev;
+  int st = current_device(&dev);
+  if (st) return st;
+  if (precision == SPSIM_PREC_FP64 || !m || m != g_host.mol || g_host.device != dev || npix != (int64_t)nx * ny ||
+      m->n_kept == 0)
+    return SPSIM_OK;
+  // |direct| below this is not worth the look
+  const double direct = m->n_kept * (double)npix / 1.75e12;
+  if (!(direct > 1.5e-4)) return SPSIM_OK;
+  double R[9];
+  for (int k = 0; k < 9; ++k) R[k] = rot[k];
+  if (!is_orthonormal(R)) return SPSIM_OK;
+  for (spsim_b200_qset *&q : g_host.nodes_q) {
+    if (!q) q = new spsim_b200_qset();
+    q->device = dev;
+    q->id = __atomic_fetch_add(&g_next_id, 1, __ATOMIC_RELAXED);
+    q->npix = npix;
+    q->has_geom = true;
+    q->geom = det_geom(nx, ny, width, height, distance, center_x, center_y, wavelength, spherical);
+    q->qmax = detector_qmax(nx, ny, width, height, distance, center_x, center_y, wavelength, spherical);
+  }
+  spsim_b200_qset *q = g_host.nodes_q[0];
+  if (!(q->qmax * m->rbound < 100.0)) return SPSIM_OK;  // second order of the list's rounding: 1e-8
+  // a phase of 3e-4 along the beam: the difference's curvature and the sums'
+  // rounding leave 2e-4 of a correction of 1e-5
+  const double lift = 3e-4 / (2.0 * M_PI * m->rbound);
+  g_host.nodes_q[1]->geom.lift = lift;
+  const spsim_b200_molecule *mols[2] = {m, m};
+  const spsim_b200_qset *qs[2] = {q, g_host.nodes_q[1]};
+  const double rots[18] = {R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8],
+                           R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8]};
+  std::vector<CoarseGrid> nodes;
+  if (!coarse_plan(2, mols, qs, rots, precision, nullptr, nodes)) return SPSIM_OK;
+  const double nxn = nodes[0].x.n, nyn = nodes[0].y.n;
+  const double grid = 2.0 * m->n_kept * nxn * nyn / 1.3e12 + 4 * 2.0 * (npix + nx * nxn) * nyn / 1e13 + npix / 3e10;
+  if (!(grid + 1.2e-4 < 0.8 * direct)) return SPSIM_OK;
+  if (!g_host.nodes_out) g_host.nodes_out = new DevBuf();
+  if (!g_host.nodes_plan) g_host.nodes_plan = new Plan();
+  CUDA_TRY(g_host.nodes_out->ensure(4 * (size_t)npix * sizeof(double2)));
+  ListSums sums;
+  sums.out = (double2 *)g_host.nodes_out->p;
+  sums.grid = nodes[0];
+  st = run_forward(2, mols, qs, rots, 0.0f, precision, nullptr, nullptr, nullptr, false, nullptr, false,
+                   g_host.nodes_plan, &sums);
+  if (st) return st;
+  g_last_terms = m->n_kept * (double)npix;
+  ListCombine &c = g_host.combine;
+  c.g = q->geom;
+  c.x = nodes[0].x;
+  c.y = nodes[0].y;
+  memcpy(c.rot, R, sizeof(R));
+  c.hkl = hkl_dev;
+  c.a = sums.out;
+  c.lifted = sums.out + npix;
+  c.ax = sums.out + 2 * npix;
+  c.ay = sums.out + 3 * npix;
+  c.lift = lift;
+  c.B = B;
+  memcpy(c.center, m->center, sizeof(c.center));
+  g_host.nodes_open = true;
+  *used = 1;
+  return SPSIM_OK;
+}
+
+extern "C" int spsim_internal_shot_nodes_part(int64_t p0, int64_t p1, float *F_dev, float *I_dev, void *stream) {
+  if (!g_host.nodes_open) return fail(SPSIM_ERR_INVALID_ARG, "shot part without a prepared shot");
+  if (p0 < 0 || p1 > g_host.nodes_q[0]->npix) return fail(SPSIM_ERR_INVALID_ARG, "bad shot part");
+  ListCombine c = g_host.combine;
+  c.F = (float2 *)F_dev;
+  c.I = I_dev;
+  CUDA_TRY(launch_list_combine(c, p0, p1, (cudaStream_t)stream));
+  return SPSIM_OK;
+}
+
 static int nufft_check_flags(int dev);
 
 extern "C" int spsim_internal_shot_check(void) {
@@ -2211,6 +2341,10 @@ extern "C" int spsim_internal_shot_check(void) {
     std::lock_guard<std::mutex> lk(g_mu);
     int st = nufft_check_flags(dev);
     if (st) return st;
+  }
+  if (g_host.nodes_open) {
+    g_host.nodes_open = false;
+    return check_flags(*g_host.nodes_plan);
   }
   if (g_host.parts > 0) {
     const int n = g_host.parts;

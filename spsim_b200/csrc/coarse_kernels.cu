@@ -29,6 +29,7 @@ CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, b
   a.alpha = a.asin_alpha = 0.0;
   a.to_n = 0;
   a.to_alpha = a.to_asin = 0.0;
+  a.derivative = 0;
   if (a.angular) {
     const double edge = 0.5 * (n_pix - 1) / n_pix * size;
     const double t0 = std::atan((-edge - centre) / distance), t1 = std::atan((edge - centre) / distance);
@@ -77,6 +78,34 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
   } else if (a.angular) {
     const double pos = ((p - (a.n_pix - 1.0) / 2.0) / a.n_pix) * a.size - a.centre;
     X = (atan(pos / a.distance) - a.mid) / a.half;
+  }
+  if (a.derivative) {
+    // by a central difference: its own error is 1e-6 of the derivative at most
+    // (step 1e-5 of the half axis, 1,024 nodes)
+    const double step = 1e-5;
+    const double x1 = sin(a.asin_alpha * (X + step)) / a.alpha, x0 = sin(a.asin_alpha * (X - step)) / a.alpha;
+    double s1 = 0.0, s0 = 0.0;
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int k = lane; k < (pass ? ld : n); k += 32) {
+        const double node = cospi((double)k / (n - 1));
+        const double w = ((k & 1) ? -1.0 : 1.0) * ((k == 0 || k == n - 1) ? 0.5 : 1.0);
+        // a node within 1e-14 of a stepped point counts as 1e-14 away
+        const double d1 = copysign(fmax(fabs(x1 - node), 1e-14), x1 - node);
+        const double d0 = copysign(fmax(fabs(x0 - node), 1e-14), x0 - node);
+        if (!pass) {
+          s1 += w / d1;
+          s0 += w / d0;
+        } else {
+          m[(long long)p * ld + k] = k < n ? (w / d1 / s1 - w / d0 / s0) / (2.0 * step) : 0.0;
+        }
+      }
+      if (!pass)
+        for (int o = 16; o > 0; o >>= 1) {
+          s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+          s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        }
+    }
+    return;
   }
   const double xi = sin(a.asin_alpha * X) / a.alpha;
   double sum = 0.0;
@@ -128,6 +157,7 @@ __global__ void __launch_bounds__(256) coarse_tables_kernel(CoarseTables t) {
       q1 = py / r * t.g.ewald;
       q2 = (t.g.distance / r - 1.0) * t.g.ewald;
     }
+    q2 += t.g.lift;
     t.q64[3 * i] = q0;
     t.q64[3 * i + 1] = q1;
     t.q64[3 * i + 2] = q2;
@@ -302,7 +332,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
       tile[(8 * i + fr) * TLD + 8 * (j >> 1) + 2 * fc + (j & 1)] =
           make_double2(re_[i][j >> 1][j & 1], im_[i][j >> 1][j & 1]);
   __syncwarp();
-  const bool need_q = F || cp.B != 0.0 || cp.out || cp.sum;
+  const bool need_q = F || cp.B != 0.0 || cp.sum;
 #pragma unroll 1
   for (int e = lane; e < 8 * RM * TN; e += 32) {
     const int y = m0 + e / TN, x = n0 + e % TN;
@@ -316,10 +346,6 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
         const double w = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
         re *= w;
         im *= w;
-      }
-      if (cp.out) {
-        cp.out[p] = make_double2(re, im);
-        continue;
       }
       if (F || cp.sum) {
         double ux = a, uy = b, uz = c;
@@ -340,7 +366,10 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
         F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
       }
     }
-    if (I) I[p] = (float)(re * re + im * im);
+    if (cp.out)
+      cp.out[p] = make_double2(re, im);
+    else if (I)
+      I[p] = (float)(re * re + im * im);
   }
 }
 
@@ -448,6 +477,69 @@ cudaError_t launch_coarse_adjoint(const CoarseAdjoint &a, int npat, double2 *H, 
     product(a.tx, coarse_ld(a.nx), a.nxn, H, a.ny, a.nx, strip, n, st);
     product(a.ty, coarse_ld(a.ny), a.nyn, strip, a.nxn, a.ny, nodes + (long long)p0 * a.nyn * a.nxn, n, st);
   }
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// patterns on a detector's rounded HKL list
+
+// Bound by its FP64 arithmetic and 64 bytes of amplitudes per pixel.
+__global__ void __launch_bounds__(256) list_combine_kernel(const __grid_constant__ ListCombine c, long long p0,
+                                                           long long p1) {
+  const long long p = p0 + (long long)blockIdx.x * 256 + threadIdx.x;
+  if (p >= p1) return;
+  const DetGeom &g = c.g;
+  const int x = (int)(p % g.nx), y = (int)(p / g.nx);
+  const double px = ((x - (g.nx - 1.0) / 2.0) / g.nx) * g.width - g.cx;
+  const double py = ((y - (g.ny - 1.0) / 2.0) / g.ny) * g.height - g.cy;
+  // q of the detector and its derivatives by X and Y
+  double q[3], gx[3], gy[3];
+  if (g.spherical) {
+    const double hx = 0.5 * (g.nx - 1) / g.nx * g.width, hy = 0.5 * (g.ny - 1) / g.ny * g.height;
+    q[0] = g.fpx * px / g.px_size;
+    q[1] = g.fpy * py / g.py_size;
+    q[2] = 0.0;
+    gx[0] = g.fpx * hx / g.px_size;
+    gy[1] = g.fpy * hy / g.py_size;
+    gx[1] = gx[2] = gy[0] = gy[2] = 0.0;
+  } else {
+    const double d = g.distance, ir = rsqrt(px * px + py * py + d * d), ir2 = ir * ir;
+    const double v[3] = {px, py, d};
+    const double dx = c.x.half * (d + px * px / d) * ir * g.ewald, dy = c.y.half * (d + py * py / d) * ir * g.ewald;
+    for (int k = 0; k < 3; ++k) {
+      q[k] = v[k] * ir * g.ewald - (k == 2 ? g.ewald : 0.0);
+      gx[k] = ((k == 0 ? 1.0 : 0.0) - v[k] * px * ir2) * dx;
+      gy[k] = ((k == 1 ? 1.0 : 0.0) - v[k] * py * ir2) * dy;
+    }
+  }
+  const double l[3] = {c.hkl[3 * p], c.hkl[3 * p + 1], c.hkl[3 * p + 2]};
+  double e[3], d[3];  // the list's difference, in its frame and in the detector's
+  for (int k = 0; k < 3; ++k) e[k] = l[k] - (c.rot[3 * k] * q[0] + c.rot[3 * k + 1] * q[1] + c.rot[3 * k + 2] * q[2]);
+  for (int k = 0; k < 3; ++k) d[k] = c.rot[k] * e[0] + c.rot[3 + k] * e[1] + c.rot[6 + k] * e[2];
+  const double det = 1.0 / (gx[0] * gy[1] - gx[1] * gy[0]);
+  const double u = (d[0] * gy[1] - d[1] * gy[0]) * det, v = (gx[0] * d[1] - gx[1] * d[0]) * det;
+  const double w = (d[2] - u * gx[2] - v * gy[2]) / c.lift;
+  const double2 a = c.a[p], ax = c.ax[p], ay = c.ay[p], b = c.lifted[p];
+  double re = a.x + u * ax.x + v * ay.x + w * (b.x - a.x);
+  double im = a.y + u * ax.y + v * ay.y + w * (b.y - a.y);
+  if (c.B != 0.0) {
+    const double f = exp(-c.B * 0.25e-20 * (l[0] * l[0] + l[1] * l[1] + l[2] * l[2]));
+    re *= f;
+    im *= f;
+  }
+  if (c.I) c.I[p] = (float)(re * re + im * im);
+  if (c.F) {
+    double t = l[0] * c.center[0] + l[1] * c.center[1] + l[2] * c.center[2];
+    t -= rint(t);
+    double sn, cs;
+    sincospi(2.0 * t, &sn, &cs);
+    c.F[p] = make_float2((float)(re * cs + im * sn), (float)(im * cs - re * sn));
+  }
+}
+
+cudaError_t launch_list_combine(const ListCombine &c, long long p0, long long p1, cudaStream_t st) {
+  if (p1 <= p0) return cudaSuccess;
+  list_combine_kernel<<<(unsigned)((p1 - p0 + 255) / 256), 256, 0, st>>>(c, p0, p1);
   return cudaGetLastError();
 }
 

@@ -24,6 +24,7 @@ struct DetGeom {
   int nx, ny;
   int spherical;
   double width, height, distance, cx, cy, ewald, fpx, fpy, px_size, py_size;
+  double lift = 0.0;  // added to the nodes' q along the beam (launch_list_combine)
 };
 
 // One axis of a detector in the interpolation's coordinate X in [-1, 1]:
@@ -37,6 +38,7 @@ struct CoarseAxis {
   // the points to interpolate to: the pixels, or (to_n > 0) another grid's nodes
   int to_n;
   double to_alpha, to_asin;
+  int derivative;  // matrices of the interpolant's derivative by X instead
 };
 
 constexpr int COARSE_MAX_NODES = 1024;  // per axis
@@ -88,6 +90,25 @@ struct CoarseBatch {
 // (strip_size complex values, at least max_nyn * max_nx).
 cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
                                  long long strip_size, cudaStream_t st);
+
+// Patterns on a float HKL list that is a detector's own, rotated and rounded:
+// q = R q_detector + delta with delta of a few float roundings.  The amplitudes
+// on the detector's exact q, its derivatives along X and Y by the derivative
+// matrices, and those at `lift` along the beam (a second node sum) give
+// A + delta . grad A; the second order is below 1e-8 for the patterns admitted
+// (phases of at most 100 cycles), as are the derivatives' own errors.
+struct ListCombine {
+  DetGeom g;
+  CoarseAxis x, y;
+  double rot[9];              // q_list ~ rot q_detector
+  const float *hkl;           // [npix][3]
+  const double2 *a, *ax, *ay, *lifted;  // centred amplitudes of the pixels, A, dA/dX, dA/dY and A(q + lift)
+  double lift, B;
+  double center[3];
+  float2 *F;  // [npix] or nullptr
+  float *I;
+};
+cudaError_t launch_list_combine(const ListCombine &c, long long p0, long long p1, cudaStream_t st);
 
 // A molecule's atoms by cells, the Voronoi cells of a body-centred cubic
 // lattice of constant a about the molecule's centre (the lattice whose cells'

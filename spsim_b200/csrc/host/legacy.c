@@ -120,6 +120,10 @@ int spsim_internal_shot_part(int64_t p0, int64_t p1, float B, int precision, flo
                              void *stream);
 int spsim_internal_chain_rows(const spsim_b200_chain_params *p, const float *I_dev,
                               const spsim_b200_chain_outputs *out, int64_t row0, int64_t row1, void *stream);
+int spsim_internal_shot_nodes_begin(int64_t npix, const float *hkl_dev, int nx, int ny, float width, float height,
+                                    float distance, float center_x, float center_y, float wavelength, int spherical,
+                                    const float *rot, float B, int precision, int *used);
+int spsim_internal_shot_nodes_part(int64_t p0, int64_t p1, float *F_dev, float *I_dev, void *stream);
 int spsim_internal_rotate_hkl(int64_t npix, const float R[9], float *hkl_dev);
 
 /* Pinned staging buffer of simulate_shot's device-to-host copies (grow-only,
@@ -614,9 +618,9 @@ void calculate_noiseless_detector_output(CCD *det, Experiment *experiment) {
 /* ------------------------------------------------------------ orchestration */
 
 /* simulate_shot's HKL list to the pinned staging buffer on the copy stream,
- * after the work queued so far on the legacy stream; ev is recorded after it */
+ * after ev, recorded behind the list's kernels (not behind the structure
+ * factor's); ev is recorded again after the copy */
 static void queue_hkl_copy(cudaEvent_t ev, char *s_hkl, const float *d_hkl, size_t bytes) {
-  cudaEventRecord(ev, 0);
   cudaStreamWaitEvent(g_copy_stream, ev, 0);
   if (bytes) {
     cudaError_t e = cudaMemcpyAsync(s_hkl, d_hkl, bytes, cudaMemcpyDeviceToHost, g_copy_stream);
@@ -718,6 +722,7 @@ Diffraction_Pattern *simulate_shot(Molecule *mol, Options *opts) {
   cudaError_t e = cudaEventCreateWithFlags(&ev_hkl, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming);
   if (e != cudaSuccess) cuda_die("cudaEventCreate", e);
+  cudaEventRecord(ev_hkl, 0);
   /* the HKL list goes down on a side stream, beside the structure factor;
    * it is queued once the structure factor's q-set statistics have come
    * back, which would otherwise wait behind it on the copy engine */
@@ -753,9 +758,20 @@ Diffraction_Pattern *simulate_shot(Molecule *mol, Options *opts) {
   const int K = shot_row_chunks(det, n, opts->use_nfft_for_sf, poly, vol, rb);
   const long long bnx = det->nx / det->binning_x;
   cudaEvent_t ev_fi = NULL, ev_copied[MAX_SHOT_CHUNKS];
+  /* a flat detector's monochromatic direct sum: on the detector's nodes where
+   * that is cheaper (the chunks then only combine their pixels' amplitudes) */
+  int nodes = 0;
+  if (!opts->use_nfft_for_sf && !poly && !vol) {
+    st = spsim_internal_shot_nodes_begin(n, d_hkl, det->nx, det->ny, det->width, det->height, det->distance,
+                                         det->center_x, det->center_y, exp->wavelength, det->spherical, rot->data,
+                                         opts->b_factor, g_precision, &nodes);
+    if (st) die("simulate_shot structure factor", st);
+  }
 
   if (K == 1) {
-    if (opts->use_nfft_for_sf)
+    if (nodes)
+      st = spsim_internal_shot_nodes_part(0, n, dF, dI, NULL);
+    else if (opts->use_nfft_for_sf)
       st = spsim_internal_shot_structure_factor_nufft(mol->natoms, mol->atomic_number, mol->pos, opts->b_factor,
                                                       opts->delta_atoms, n, d_hkl, det->nx, g_nufft_eps, dF, dI);
     else
@@ -798,7 +814,7 @@ Diffraction_Pattern *simulate_shot(Molecule *mol, Options *opts) {
     if (nfft)
       st = spsim_internal_shot_nufft_begin(mol->natoms, mol->atomic_number, mol->pos, opts->b_factor,
                                            opts->delta_atoms, n, d_hkl, det->nx, g_nufft_eps);
-    else
+    else if (!nodes)
       st = spsim_internal_shot_parts_begin(n, d_hkl);
     if (st) die("simulate_shot structure factor", st);
     queue_hkl_copy(ev_hkl, s_hkl, d_hkl, b_hkl);
@@ -822,6 +838,8 @@ Diffraction_Pattern *simulate_shot(Molecule *mol, Options *opts) {
       cudaStream_t s = nfft ? (cudaStream_t)0 : g_comp_stream[c & 1];
       if (s) cudaStreamWaitEvent(s, ev_ready, 0);
       st = nfft ? spsim_internal_shot_nufft_part(p0, p1, dF, dI)
+           : nodes
+                ? spsim_internal_shot_nodes_part(p0, p1, dF, dI, s)
                 : spsim_internal_shot_part(p0, p1, opts->b_factor, g_precision, dF, dI, s);
       if (st) die("simulate_shot structure factor", st);
       st = spsim_internal_chain_rows(&p, dI, &o, r0, r1, s);

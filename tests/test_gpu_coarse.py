@@ -9,7 +9,7 @@ import torch
 
 from conftest import intensity_errors
 from oracle import oracle as O
-from spsim_b200 import core, synth
+from spsim_b200 import core, spsim as S, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -325,3 +325,49 @@ def test_nufft_at_the_nodes(cuda, eps, elements):
         assert np.linalg.norm(dF) < max(3 * eps, 2e-7) * np.linalg.norm(F64)
         assert dF.max() < max(30 * eps, 2e-6) * np.abs(F64).max()
         assert np.abs(I.cpu().numpy() - I64).max() < max(60 * eps, 4e-6) * I64.max()
+
+
+@pytest.mark.parametrize("nx,ny,chunks,kw", [
+    (400, 371, 1, dict()), (399, 357, 3, dict(b_factor=9.0)), (512, 300, 1, dict(spherical=1)),
+    (420, 401, 4, dict(center_x=0.011, center_y=-0.004)), (400, 380, 1, dict(distance=0.05)),
+    (450, 444, 2, dict(spherical=1, b_factor=4.0))],
+    ids=["one_pass", "chunks_b", "spherical", "off_axis", "wide", "spherical_chunks"])
+@pytest.mark.parametrize("fast", [False, True], ids=["f32", "f32_fast"])
+def test_simulate_shot_on_the_nodes(cuda, tmp_path, monkeypatch, nx, ny, chunks, kw, fast):
+    # the pattern is that of the shot's own float HKL list (its rounding is some
+    # 1e-5 of the amplitudes, two orders beyond the bounds here): the oracle on it
+    monkeypatch.chdir(tmp_path)
+    Z, pos = synth.random_molecule(9000, 6.0e-9, 231)
+    pos += np.float32(3e-9)
+    opts = S.set_defaults()
+    o = opts.contents
+    det, exp = o.detector.contents, o.experiment.contents
+    det.nx, det.ny, det.nz = nx, ny, 1
+    det.pixel_width = det.pixel_height = 75e-6
+    det.width, det.height = nx * det.pixel_width, ny * det.pixel_height
+    det.distance = kw.get("distance", 0.15)
+    det.center_x, det.center_y, det.spherical = kw.get("center_x", 0.0), kw.get("center_y", 0.0), kw.get("spherical", 0)
+    exp.wavelength = 1.5e-10
+    o.b_factor = kw.get("b_factor", 0.0)
+    o.verbosity_level = 0
+    o.random_orientation = 0
+    o.euler_orientation[0], o.euler_orientation[1], o.euler_orientation[2] = 0.4, -0.9, 1.7
+    mol = S.get_molecule_from_atoms(Z, pos)
+    S.set_precision("f32_fast" if fast else "f32")
+    S.set_shot_chunks(chunks)
+    try:
+        shot = S.simulate_shot(mol, opts)
+    finally:
+        S.set_shot_chunks(0)
+        S.set_precision("f32")
+    _on_grid()
+    n = nx * ny
+    q = S.as_array(shot.contents.HKL_list, 3 * n).reshape(-1, 3).astype(np.float64)
+    pick = np.arange(0, n, 7)
+    F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q[pick], B=kw.get("b_factor", 0.0))
+    e_max, e_l2 = intensity_errors(S.as_array(shot.contents.ints, n)[pick], I64)
+    assert e_max < TOL[0] and e_l2 < TOL[1], (e_max, e_l2)
+    F = S.as_array(shot.contents.F, n)[pick]
+    assert np.linalg.norm(F - F64) < 1e-6 * np.linalg.norm(F64)
+    S.free_stuff(shot, opts)
+    S.free_mol(mol)
