@@ -29,20 +29,23 @@ cudaError_t set_nodes_copy_stall(int on) {
 constexpr int NODE_THREADS = 128;
 constexpr int NODE_TILE = SF_NODES_TILE;  // nodes per work item: 8 per lane
 static_assert(NODE_TILE == 256, "eight nodes per lane");
+// Tiles in flight: those of most work items of a cell at once, so that its warps
+// meet only at the item's end (as many as static shared memory holds).
+constexpr int NODE_STAGES = 7;
 
 template <bool PERB, bool FIXW>
 __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
     const SfPattern *__restrict__ pats, const WorkItem *__restrict__ items, int n_items, int *__restrict__ queue,
     int *__restrict__ err, uint32_t m31) {
   constexpr int P = 8, NP = P / 2, WARPS = NODE_THREADS / 32;
-  __shared__ __align__(128) float4 ring[RING_STAGES][2 * TILE_ATOMS];
+  __shared__ __align__(128) float4 ring[NODE_STAGES][2 * TILE_ATOMS];
   __shared__ __align__(16) double2 sacc[P * NODE_THREADS];  // per-thread FP64 sums of the current work item
-  __shared__ __align__(8) uint64_t full_bar[RING_STAGES];
+  __shared__ __align__(8) uint64_t full_bar[NODE_STAGES];
   __shared__ int s_item;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int s = 0; s < RING_STAGES; ++s) mbar_init(&full_bar[s], 1);
+    for (int s = 0; s < NODE_STAGES; ++s) mbar_init(&full_bar[s], 1);
     fence_barrier_init();
   }
   __syncthreads();
@@ -89,9 +92,9 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
 
     const int k0 = wi.k0, k1 = wi.k1;
     if (tid == 0) {
-      for (int k = k0; k < k1 && k < k0 + RING_STAGES; ++k) {
+      for (int k = k0; k < k1 && k < k0 + NODE_STAGES; ++k) {
         const TileDesc td = tiles[k];
-        const uint32_t st = g_issue % RING_STAGES;
+        const uint32_t st = g_issue % NODE_STAGES;
         const uint32_t bytes = (uint32_t)td.count * (uint32_t)sizeof(AtomD);
         mbar_arrive_expect_tx(&full_bar[st], bytes);
         if (!(stall && g_issue == 0))  // the stall hook skips the CTA's first copy
@@ -100,23 +103,19 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
       }
     }
 
+    bool failed = false;
+    int groups = 0;  // of the tiles before, so that the warps' shares of a run's last groups even out
     for (int k = k0; k < k1; ++k) {
-      const uint32_t st = g_cons % RING_STAGES;
-      const uint32_t par = (g_cons / RING_STAGES) & 1u;
-      const bool ok = mbar_wait_bounded(&full_bar[st], par, kWaitCycles);
-      if (__syncthreads_or(!ok)) {
-        if (tid == 0) {
-          atomicOr(err, 1);
-          for (uint32_t g = g_cons; g < g_issue; ++g)
-            mbar_wait_bounded(&full_bar[g % RING_STAGES], (g / RING_STAGES) & 1u, kWaitCycles);
-        }
-        return;
-      }
+      const uint32_t st = g_cons % NODE_STAGES;
+      const uint32_t par = (g_cons / NODE_STAGES) & 1u;
+      // a copy that did not come: this item's rest is passed over, and the CTA returns at its end
+      if (!failed) failed = !mbar_wait_bounded(&full_bar[st], par, kWaitCycles);
       const TileDesc td = tiles[k];
       const float4 *__restrict__ ta = ring[st];
       // this warp's groups of eight atoms, in FP32 sums of four: of bright nodes'
       // sums, all of one sign, the rounding errors grow with the sum
-      for (int a = ATOM_GROUP * warp; a < td.count; a += ATOM_GROUP * WARPS)
+      const int end = failed ? 0 : td.count;
+      for (int a = ATOM_GROUP * ((warp - groups) & (WARPS - 1)); a < end; a += ATOM_GROUP * WARPS)
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         float2 bc[NP], bs[NP];
@@ -189,15 +188,25 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
           shc[j] = slc[j] = shs[j] = sls[j] = make_float2(0.f, 0.f);
         }
       }
+      groups += td.count / ATOM_GROUP;
+      ++g_cons;
+      if (k + NODE_STAGES >= k1) continue;
       __syncthreads();
-      if (tid == 0 && k + RING_STAGES < k1) {
-        const TileDesc tn = tiles[k + RING_STAGES];
+      if (tid == 0 && !failed) {
+        const TileDesc tn = tiles[k + NODE_STAGES];
         const uint32_t bytes = (uint32_t)tn.count * (uint32_t)sizeof(AtomD);
         mbar_arrive_expect_tx(&full_bar[st], bytes);
         bulk_copy_g2s(&ring[st][0], atomsd + tn.atom_begin, bytes, &full_bar[st]);
         ++g_issue;
       }
-      ++g_cons;
+    }
+    if (__syncthreads_or(failed)) {
+      if (tid == 0) {
+        atomicOr(err, 1);
+        for (uint32_t g = g_issue > NODE_STAGES ? g_issue - NODE_STAGES : 0; g < g_issue; ++g)
+          mbar_wait_bounded(&full_bar[g % NODE_STAGES], (g / NODE_STAGES) & 1u, kWaitCycles);
+      }
+      return;
     }
     // item done: the warps' sums of each node added, one write per node (a plain
     // store when the item covers every atom tile of the molecule)
