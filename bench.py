@@ -257,6 +257,9 @@ MIX = {
     "sf_dphase_kernel": {"fp32": 12, "dfma": 6, "imad": 1, "xu": 1},
     "sf_dphase_kernel+word/f32": {"fp32": 13, "dfma": 3, "imad": 1, "alu": 1, "i2f": 1},
     "sf_dphase_kernel+word/f32_fast": {"fp32": 4, "dfma": 3, "xu": 2, "i2f": 1},
+    # on the nodes of coarse grids: every term FP64-anchored, NODE polynomials,
+    # FP32 sums of 4 atoms (the sign's IMAD among the FP32 operations)
+    "sf_dquad_nodes_kernel+word": {"fp32": 14.6, "dfma": 3, "alu": 1, "i2f": 1},
     "sf_f32x2_kernel/f32": {"fp32": 27, "alu": 2},                   # compensated phase, HALF poly
     "sf_f32x2_kernel/f32_fast": {"fp32": 16, "xu": 2},               # compensated phase, MUFU sin/cos
 }
@@ -265,6 +268,9 @@ MIX = {
 def _kernel_key():
     """MIX key of the structure-factor kernel the last forward ran."""
     from spsim_b200 import core
+    terms, evaluated = core.last_forward_stats()[0], core.last_terms_evaluated()
+    if evaluated < terms:  # on coarse grids of nodes; the smallest sums in FP64
+        return "sf_dquad_nodes_kernel+word" if evaluated > 4e6 else "sf_nodes64_kernel"
     return (core.kernel_name() + ("+word" if core.last_phase_word() else "")
             + ("+narrow" if core.last_pair_narrow() else ""))
 
@@ -317,7 +323,7 @@ def _peaks(props):
     return min(p_fma / OPS_PER_TERM_FMA, p_mufu / OPS_PER_TERM_MUFU), p_mufu, p_fma, sm_max, src
 
 
-TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "sf_dquad_precision50k_traffic.md")
+TRAFFIC_PROFILE = os.path.join(ROOT, "profiles", "sf_nodes_precision50k_ncu.md")
 
 
 def _traffic_per_launch():
@@ -412,12 +418,13 @@ def run_b200(args):
     elapsed_ms, sf_avg, clocks = timed(prec, args.steps, args.warmup)
     value = world * args.steps * terms / (elapsed_ms * 1e-3)
     kname = _kernel_key()
+    evaluated = core.last_terms_evaluated()  # of the pattern's terms: on nodes far fewer
 
     line = None
     if rank == 0:
         props = torch.cuda.get_device_properties(local)
         R, p_mufu, p_fma, sm_max, src = _peaks(props)
-        achieved = terms / (sf_avg * 1e-3) if sf_avg else None
+        achieved = evaluated / (sf_avg * 1e-3) if sf_avg else None
         balanced = balanced_bound(kname, prec, measured_pipe_peaks())
         if balanced and achieved:
             balanced["frac"] = achieved / balanced["terms_per_s"]
@@ -428,19 +435,24 @@ def run_b200(args):
             "data": "synthetic (seeded molecule; no dataset)",
             "config": {"workload": workload_desc(), "precision": prec,
                        "parallelism": "one orientation per rank" if world > 1 else "single GPU",
+                       "sum": "atom.pixel terms of the pattern; evaluated on coarse grids of nodes and interpolated "
+                              "in FP64 (roofline.terms_per_launch), to the accuracy stated",
                        "l2": "flushed between timed steps (256 MiB write outside the timed events)"},
             "roofline": {
                 "bound": "sfu", "achieved": achieved, "peak": R, "unit": UNIT,
                 "frac": achieved / R if achieved else None, "traffic": _traffic_per_launch(),
                 "kernel": kname,
                 "kernel_ms": sf_avg,
+                "terms_per_launch": evaluated, "pattern_terms": terms,
                 "balanced": balanced,
                 "peak_source": "R = min(P_FMA/5, P_MUFU/2) terms/s; P_FMA = %.4g FMA lane-ops/s, P_MUFU = %.4g "
                                "ops/s, %s (MEASURED_PEAKS.json has no FP32-FMA or MUFU figure)" % (p_fma, p_mufu, src),
                 "peak_nominal": props.multi_processor_count * MUFU_PER_SM_CLK * 1965e6 / OPS_PER_TERM_MUFU,
             },
             "clocks": clocks.summary(),
-            "gpu_launches": 3 * args.steps,
+            # node sums, two interpolations of the cells, two of the pattern, chain;
+            # on every pixel: sums, finalize, chain
+            "gpu_launches": (6 if evaluated < terms else 3) * args.steps,
         }
     # the other precisions on the same workload, and accuracy against the FP64
     # GPU kernel: single-GPU extras (their timing takes no collective steps the
@@ -460,9 +472,9 @@ def run_b200(args):
     if rank == 0:
         if line.get("fp64_plain"):
             f = line["fp64_plain"]
-            f["f32_speedup"] = line["roofline"]["achieved"] / f["kernel_terms_per_s"] if line["roofline"]["achieved"] else None
-            if line.get("f32_fast", {}).get("kernel_terms_per_s"):
-                f["f32_fast_speedup"] = line["f32_fast"]["kernel_terms_per_s"] / f["kernel_terms_per_s"]
+            f["f32_speedup"] = line["value"] / f["kernel_terms_per_s"]
+            if line.get("f32_fast"):
+                f["f32_fast_speedup"] = line["f32_fast"]["value"] / f["kernel_terms_per_s"]
         # the batched workloads at their stated sizes (single-GPU extras: the
         # other ranks of a multi-GPU run would wait on them at the final barrier)
         batched = {}
@@ -502,13 +514,14 @@ def _modes(args, core, mol, qs, rot, terms, timed, prec):
     if prec != "f32_fast":
         ms, sf_ms, _ = timed("f32_fast", max(2, args.steps // 2), 1)
         kname = _kernel_key()
+        evaluated = core.last_terms_evaluated()
         bal = balanced_bound(kname, "f32_fast", measured_pipe_peaks())
         if bal and sf_ms:
-            bal["frac"] = terms / (sf_ms * 1e-3) / bal["terms_per_s"]
+            bal["frac"] = evaluated / (sf_ms * 1e-3) / bal["terms_per_s"]
         out["f32_fast"] = {"value": terms * max(2, args.steps // 2) / (ms * 1e-3), "unit": UNIT,
                            "kernel": kname,
-                           "kernel_terms_per_s": terms / (sf_ms * 1e-3) if sf_ms else None,
-                           "frac_of_R": terms / (sf_ms * 1e-3) / R if sf_ms else None,
+                           "kernel_terms_per_s": evaluated / (sf_ms * 1e-3) if sf_ms else None,
+                           "frac_of_R": evaluated / (sf_ms * 1e-3) / R if sf_ms else None,
                            "balanced": bal}
     q = qs.q()
     sub_rows = core.QSet.from_list(q.reshape(1024, 1024, 3)[::64].reshape(-1, 3))
@@ -769,7 +782,7 @@ def batched_orientations(prec, R0, n_orient=None, reps=2, nufft=True):
     with torch.cuda.stream(stream):
         t_batch = ev_time(lambda: core.forward_batch(mol, qs, rots=R, precision=prec, I=I, want_F=False,
                                                      stream=stream), reps=reps)
-        kname = _kernel_key()
+        kname, evaluated = _kernel_key(), core.last_terms_evaluated()
         nloop = min(n_orient, 64)
         Iloop = torch.empty(qs.npix, device="cuda")
         t_loop = ev_time(lambda: [core.forward(mol, qs, rot=R[i], precision=prec, I=Iloop, want_F=False,
@@ -789,20 +802,19 @@ def batched_orientations(prec, R0, n_orient=None, reps=2, nufft=True):
     out = {"workload": "orientations_20k: 20,000 atoms, 256^2 pixels of 150 um at 0.2 m, 0.2 nm, %d Haar rotations "
                        "in one batched forward (graph-replayed)" % n_orient,
            "precision": prec, "orientations": n_orient, "kernel": kname, "batch_ms": t_batch,
-           "terms_per_s": terms / t_batch * 1e3, "frac_of_R": terms / t_batch * 1e3 / R0,
+           "terms_per_s": terms / t_batch * 1e3, "terms_evaluated": evaluated,
+           "frac_of_R": evaluated / t_batch * 1e3 / R0,
            "loop_of_single_calls_ms": t_loop, "batch_speedup": t_loop / t_batch,
            "floored_max_rel_vs_fp64_first4": first4_error(Iall)}
     if prec == "f32":
-        # the same batch in the fast mode (pixels 4m+2, 4m+3 of each neighbour
-        # quad on MUFU sin/cos), with its error on the same patterns
+        # the same batch in the fast mode, with its error on the same patterns
         with torch.cuda.stream(stream):
             t_fast = ev_time(lambda: core.forward_batch(mol, qs, rots=R, precision="f32_fast", I=I, want_F=False,
                                                         stream=stream), reps=reps)
         out["f32_fast"] = {"batch_ms": t_fast, "terms_per_s": terms / t_fast * 1e3,
-                           "frac_of_R": terms / t_fast * 1e3 / R0,
+                           "frac_of_R": evaluated / t_fast * 1e3 / R0,
                            "floored_max_rel_vs_fp64_first4": first4_error(Iall),
-                           "note": "measured here; the fast mode's MUFU bias can reach ~1.7e-5 on random "
-                                   "high-|q| neighbour quads, so SPSIM_PREC_F32 is the mode held to 1e-5 everywhere"}
+                           "note": "on coarse grids of nodes both FP32 modes run the same kernel"}
     del Iall, I
     if nufft:
         with torch.cuda.stream(stream):
@@ -850,6 +862,7 @@ def batched_uneven(prec, R0, reps=3):
         F, I = core.forward_batch(mols, qsets, precision=prec, want_F=False, stream=stream)
         t_d = ev_time(lambda: core.forward_batch(mols, qsets, precision=prec, I=I, want_F=False, stream=stream),
                       reps=reps)
+        evaluated = core.last_terms_evaluated()
         try:
             tuned = core.autotune_batch(mols, qsets, precision=prec, stream=stream)
             t_u = ev_time(lambda: core.forward_batch(mols, qsets, precision=prec, I=I, want_F=False, stream=stream),
@@ -859,7 +872,7 @@ def batched_uneven(prec, R0, reps=3):
     return {"workload": "uneven_64: 64 molecules, 500..100,000 atoms (log-uniform), 128^2..1024^2 detectors, "
                         "lambda 0.1..0.3 nm, one batched forward after autotuning",
             "precision": prec, "terms": cost, "batch_ms": t_u, "terms_per_s": cost / t_u * 1e3,
-            "frac_of_R": cost / t_u * 1e3 / R0,
+            "terms_evaluated": evaluated, "frac_of_R": evaluated / t_u * 1e3 / R0,
             "autotuned_variant": {"threads": tuned[0], "pixels_per_thread": tuned[1], "form": tuned[2]},
             "untuned_default_ms": t_d}
 

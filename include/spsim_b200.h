@@ -114,8 +114,11 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
  * spectrum) therefore evaluate the sum on a tensor grid of nodes, a
  * little more than two per cycle along each axis, and interpolate it to the
  * pixels in FP64, to 1e-8 of an outermost atom's amplitude (1e-12 with
- * SPSIM_PREC_FP64) and far less for the others; form factors and per-atom B factors belong to the interpolated
- * sum, the global B factor and the centre phase are applied per pixel.  This
+ * SPSIM_PREC_FP64) and far less for the others; form factors and per-atom B
+ * factors belong to the interpolated sum, the global B factor and the centre
+ * phase are applied per pixel.  Large patterns are summed in two levels, by
+ * cells of the molecule's volume on still coarser grids of their own (lists of
+ * the cells' atoms stay with the molecule, 50 bytes per atom and list).  This
  * is done where it is faster (patterns of more than about 1e7 terms), for
  * whole batches or not at all, and in FP64 for molecules rewritten on the
  * device (refinements: a node's rounding error would enter the pixels around it
@@ -176,8 +179,9 @@ int spsim_b200_structure_factor_host_spectrum(int natoms, const int32_t *Z, cons
  * The same F(q) = sum_e f_e(|q|) sum_{j in e} w_j exp(-2 pi i q.r_j) as
  * spsim_b200_forward, computed per element as a type-3 non-uniform FFT
  * (atoms spread onto a real-space grid, one batched 3-D FFT, interpolation at
- * every pixel's q; FP64 spreading and FFT, an FP32 copy of the FFT grid for
- * the interpolation) in O(atoms w^3 + grid log grid + pixels w^3)
+ * every pixel's q, or of a detector's pixels from 2^16 on at the nodes of the
+ * forwards' coarse grid and from there to the pixels; FP64 spreading and FFT,
+ * an FP32 copy of the FFT grid for the interpolation at pixels) in O(atoms w^3 + grid log grid + pixels w^3)
  * instead of O(atoms x pixels).  Replaces the reference's NNFFT path
  * (compute_pattern_on_list_by_nfft, src/diffraction.c:528-675, dispatched by
  * compute_sf when use_nfft_for_sf is set, src/spsim.c:119-123), which runs
@@ -185,8 +189,8 @@ int spsim_b200_structure_factor_host_spectrum(int natoms, const int32_t *Z, cons
  * eps: target relative L2 error of F against the exact sum, in
  * [1e-14, 1e-2] (measured errors come out within a few eps, and not below the
  * complex64 output's ~3e-8); it sets the interpolation kernel width
- * w = ceil(-log10 eps) + 1 grid points (up to 15) and the spreading width
- * w + 3 (up to 16).  The grids follow the bounding box of R q and the
+ * w = ceil(-log10 eps) + 1 grid points (up to 15; one more at nodes) and the
+ * spreading width w + 3 (up to 16).  The grids follow the bounding box of R q and the
  * molecule's radius r_b: about 6 S_d r_b + w + 5 spreading points per axis
  * (S_d: half-width of the q box along d) and twice that, rounded up to a size
  * with factors 2, 3, 5, 7, for the FFT.
@@ -211,9 +215,11 @@ int spsim_b200_forward_nufft_batch(const spsim_b200_molecule *m, const spsim_b20
  * NUFFT forward on this thread. */
 int spsim_b200_last_nufft_grid(int *w_spread, int *w_interp, int *n2);
 /* Interpolation path of the NUFFT forwards (process-wide): 0 (default) lets
- * q sets made from a detector walk each 16 x 8 pixel tile's grid region in
- * shared memory together; 1 reads every pixel's stencil on its own.  Both
- * give the same bits.  Other values: SPSIM_ERR_INVALID_ARG. */
+ * q sets made from a detector interpolate at the nodes of a coarse grid and
+ * from there to the pixels (from 2^16 pixels of all patterns on), or below
+ * that walk each 16 x 8 pixel tile's grid region in shared memory together; 1
+ * reads every pixel's stencil on its own, with the same bits as the tiles'
+ * (the nodes' agree to eps).  Other values: SPSIM_ERR_INVALID_ARG. */
 int spsim_b200_set_nufft_interp(int mode);
 /* The NUFFT structure factor of host arrays with unit atom weights (the
  * reference NNFFT's semantics: no illumination weights), host F (complex64)
@@ -254,8 +260,8 @@ int spsim_b200_structure_factor_host_noalloc(int natoms, const int32_t *Z, const
  * precision) are built on the first call and reused by the next ones, which
  * allocate nothing.  Where the forward's coarse grids serve (see the structure
  * factor above), dL/dI F is taken to the nodes by the transposed interpolation
- * and the sum runs there in FP64; calls that share such a plan run in call order, whatever
- * their streams. */
+ * and the sum runs there in FP64; calls that share such a plan run in call
+ * order, whatever their streams. */
 int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200_qset *qs, int npat,
                        const double *rot, float B, int precision, const float *F_dev, const float *G_dev,
                        double *dpos_dev, double *docc_dev, double *dB_dev, void *stream);

@@ -205,8 +205,9 @@ def forward_nufft_batch(mol, qs, rots, B=0.0, eps=1e-8, F=None, I=None, want_F=T
 
 
 def set_nufft_interp(mode):
-    """NUFFT interpolation path: 0 (default) the shared-memory tile path for
-    detector q sets, 1 per-pixel stencil reads everywhere (same bits)."""
+    """NUFFT interpolation path: 0 (default) for detector q sets at the nodes of
+    a coarse grid (from 2^16 pixels on) or by shared-memory tiles, 1 per-pixel
+    stencil reads everywhere (the tiles' bits)."""
     check(lib().spsim_b200_set_nufft_interp(int(mode)))
 
 

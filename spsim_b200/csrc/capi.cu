@@ -1609,7 +1609,7 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
     b.pats = pats;
     b.coarse = pl.cpats + pl.n_interp;
     if (pl.n_cells && (e = launch_coarse_interp(b, pl.n_cells, pl.cell_nx, pl.cell_ny, pl.cell_nyn, pl.strip,
-                                                pl.strip_size, stream)))
+                                                pl.strip_size, stream, true)))
       return e;
     b.pats = pats + pixels;
     b.coarse = pl.cpats;
@@ -2476,7 +2476,7 @@ static int nufft_width(double eps) {
 // (each its own, the tile path shares nothing between nodes pixels apart), then
 // the interpolation to the pixels.  From 2^16 pixels on, where the stencils at
 // every pixel (1 ns each) take longer than the grid's three launches; 50,000
-// atoms x 1024^2 at 26,244 nodes: 1.07 ms -> 0.11 ms.
+// atoms x 1024^2: 1.07 ms -> 0.18 ms (26,244 nodes 0.12, to the pixels 0.06).
 static cudaError_t nufft_interp_coarse(NufftCtx &c, const NufftInterp &pixels, const spsim_b200_qset *qs,
                                        const CoarseGrid &grid, cudaStream_t st) {
   const DetGeom &g = qs->geom;

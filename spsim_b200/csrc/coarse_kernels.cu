@@ -188,14 +188,12 @@ cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const Co
 // Interpolation as two FP64 matrix products on the tensor pipe (m8n8k4):
 //   columns  strip[k][x] = sum_i M_x[x][i] nodes[k][i]
 //   rows     pixel[y][x] = sum_k M_y[y][k] strip[k][x]
-// with the complex values' parts as neighbouring columns of the right-hand
-// matrix, so that each lane's pair of results is one amplitude.  The rows'
-// kernel then applies the global B factor and the centre phase and writes F
+// The rows' kernel then applies the global B factor and the centre phase and writes F
 // and |F|^2 as sf_finalize_kernel does.  Fragments come straight from L1 / L2:
-// a warp's RM x RN tiles of 8 x 8 reuse each of its 2 (RM + RN) loads per four
-// k steps.  FP64 MMA runs at the FMA units' own rate but issues a quarter of
-// the loads of the same product written with FMAs from shared memory (50,000
-// atoms x 1024^2, 182 nodes a side: that form took 335 us).
+// a warp's RM x RN tiles of 8 x 8 complex values take RM + 2 RN 16-byte loads
+// per eight k.  FP64 MMA runs at the FMA units' own rate but issues a quarter of
+// the loads of the same product written with FMAs from shared memory (1024^2
+// pixels from 182 nodes a side: that form took 335 us, both products now 58).
 constexpr int INTERP_WARPS_M = 2, INTERP_WARPS_N = 2;
 constexpr int INTERP_THREADS = 32 * INTERP_WARPS_M * INTERP_WARPS_N;
 
@@ -263,8 +261,8 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, 
   }
 }
 
-// ROWS: the second product, else the first.
-template <int RM, int RN, int AHEAD, bool ROWS>
+// ROWS: the second product, else the first.  SUM: of a cell (CoarsePattern::sum).
+template <int RM, int RN, int AHEAD, bool ROWS, bool SUM>
 __global__ void __launch_bounds__(INTERP_THREADS, 7)
     coarse_interp_kernel(const __grid_constant__ CoarseBatch batch, int pattern0, double2 *__restrict__ strips,
                          long long strip_stride) {
@@ -315,7 +313,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && pt.mol_err && *pt.mol_err) atomicOr(pt.plan_err, 1);
     q64 = pt.q64;
     rot = pt.has_rot ? pt.rot : nullptr;
-    center = cp.sum ? cp.shift : pt.center;
+    center = SUM ? cp.shift : pt.center;
     qscale = pt.qscale;
     F = pt.F;
     I = pt.I;
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
       tile[(8 * i + fr) * TLD + 8 * (j >> 1) + 2 * fc + (j & 1)] =
           make_double2(re_[i][j >> 1][j & 1], im_[i][j >> 1][j & 1]);
   __syncwarp();
-  const bool need_q = F || cp.B != 0.0 || cp.sum;
+  const bool need_q = SUM || F || cp.B != 0.0;
 #pragma unroll 1
   for (int e = lane; e < 8 * RM * TN; e += 32) {
     const int y = m0 + e / TN, x = n0 + e % TN;
@@ -342,12 +340,12 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
     double re = v.x, im = v.y;
     if (need_q) {
       const double a = q64[3 * p], b = q64[3 * p + 1], c = q64[3 * p + 2];
-      if (cp.B != 0.0) {
+      if (!SUM && cp.B != 0.0) {
         const double w = exp(-cp.B * 0.25e-20 * (a * a + b * b + c * c));
         re *= w;
         im *= w;
       }
-      if (F || cp.sum) {
+      if (SUM || F) {
         double ux = a, uy = b, uz = c;
         if (rot) {
           ux = rot[0] * a + rot[1] * b + rot[2] * c;
@@ -358,7 +356,7 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
         t -= rint(t);
         double sn, cs;
         sincospi(2.0 * t, &sn, &cs);
-        if (cp.sum) {
+        if (SUM) {
           atomicAdd(&cp.sum[p].x, re * cs + im * sn);
           atomicAdd(&cp.sum[p].y, im * cs - re * sn);
           continue;
@@ -373,16 +371,91 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
   }
 }
 
-template <int RM, int RN, int AHEAD, bool ROWS>
+// The second product of many cells: as above onto the pattern's own nodes,
+// per_block cells in turn by one block, which adds them up in shared memory with
+// the phases of their centres and goes to the pattern's sums once per pattern.
+// 128 x 65 cells to 38^2 nodes: one cell per block, each adding to the sums,
+// 191 us, which the atomics bound; 133 us with nine, 153 with sixteen.  Where a
+// block takes one cell, the other kernel (65 cells to 167^2 nodes: 47 us, 62 here).
+__global__ void __launch_bounds__(INTERP_THREADS, 6)
+    cell_rows_kernel(const __grid_constant__ CoarseBatch batch, int cell0, int n, int per_block,
+                     const double2 *__restrict__ strips, long long strip_stride) {
+  constexpr int RM = 2, RN = 1, TN = 8 * RN, TLD = TN + 1, POINTS = 8 * RM * TN;
+  __shared__ double2 tiles[INTERP_WARPS_M * INTERP_WARPS_N][8 * RM * TLD];
+  __shared__ double2 sums[INTERP_WARPS_M * INTERP_WARPS_N][POINTS];
+  __shared__ double us[INTERP_WARPS_M * INTERP_WARPS_N][3][POINTS];  // R q of the warp's nodes
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
+  const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
+  const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);
+  double2 *tile = tiles[warp], *sum = sums[warp];
+  double(*u)[POINTS] = us[warp];
+  double2 *to = nullptr;
+  int to_nx = 0, to_ny = 0;
+  auto flush = [&]() {
+    for (int e = lane; e < POINTS && to; e += 32) {
+      const int y = m0 + e / TN, x = n0 + e % TN;
+      if (y >= to_ny || x >= to_nx) continue;
+      atomicAdd(&to[(long long)y * to_nx + x].x, sum[e].x);
+      atomicAdd(&to[(long long)y * to_nx + x].y, sum[e].y);
+    }
+  };
+  double qscale = 1.0;
+  const int first = blockIdx.z * per_block, end = min(first + per_block, n);
+  for (int c = first; c < end; ++c) {
+    const CoarsePattern &cp = batch.coarse[cell0 + c];
+    if (cp.sum != to) {
+      flush();
+      to = cp.sum;
+      to_nx = cp.nx;
+      to_ny = cp.ny;
+      const SfPattern &pt = batch.pats[cp.parent];
+      qscale = pt.qscale;
+      for (int e = lane; e < POINTS; e += 32) {
+        const int y = m0 + e / TN, x = n0 + e % TN;
+        sum[e] = make_double2(0.0, 0.0);
+        if (y >= to_ny || x >= to_nx) continue;
+        const double *q = pt.q64 + 3 * ((long long)y * to_nx + x), *R = pt.rot;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          u[k][e] = pt.has_rot ? R[3 * k] * q[0] + R[3 * k + 1] * q[1] + R[3 * k + 2] * q[2] : q[k];
+      }
+    }
+    if (m0 >= to_ny || n0 >= to_nx) continue;
+    const double2 *bcol[RN] = {strips + c * strip_stride + min(n0 + fr, to_nx - 1)};
+    double re[RM][RN][2], im[RM][RN][2];
+    dmma_tile<RM, RN, 1>(cp.my, cp.ldy, m0, to_ny, bcol, to_nx, cp.nyn, 0, cp.nyn, re, im);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) tile[(8 * i + fr) * TLD + 2 * fc + h] = make_double2(re[i][0][h], im[i][0][h]);
+    __syncwarp();
+#pragma unroll 2
+    for (int e = lane; e < POINTS; e += 32) {
+      const int y = m0 + e / TN, x = n0 + e % TN;
+      if (y >= to_ny || x >= to_nx) continue;
+      double t = (u[0][e] * cp.shift[0] + u[1][e] * cp.shift[1] + u[2][e] * cp.shift[2]) * qscale;
+      t -= rint(t);
+      double sn, cs;
+      sincospi(2.0 * t, &sn, &cs);
+      const double2 v = tile[e / TN * TLD + e % TN];
+      sum[e].x += v.x * cs + v.y * sn;
+      sum[e].y += v.y * cs - v.x * sn;
+    }
+  }
+  flush();
+}
+
+template <int RM, int RN, int AHEAD, bool ROWS, bool SUM = false>
 static void interp_t(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip, long long stride,
                      cudaStream_t st) {
   const int bm = 8 * RM * INTERP_WARPS_M, bn = 8 * RN * INTERP_WARPS_N;
   dim3 grid((unsigned)((n_max + bn - 1) / bn), (unsigned)((m_max + bm - 1) / bm), (unsigned)n);
-  coarse_interp_kernel<RM, RN, AHEAD, ROWS><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
+  coarse_interp_kernel<RM, RN, AHEAD, ROWS, SUM><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
 }
 
 cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
-                                 long long strip_size, cudaStream_t st) {
+                                 long long strip_size, cudaStream_t st, bool cells) {
   if (npat <= 0 || max_nx <= 0 || max_ny <= 0) return cudaSuccess;
   const long long stride = (long long)max_nyn * max_nx;
   const int group = (int)std::min<long long>(std::max<long long>(strip_size / stride, 1), 65535);
@@ -393,10 +466,19 @@ cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int
     // 32 x 16 46.5), but 8 x 8 where those leave most SMs without two blocks
     // (one 512^2 pattern: 6.4 us instead of 8.8; eight: 43 instead of 34).
     interp_t<1, 1, 2, false>(b, p0, n, max_nx, max_nyn, strip, stride, st);
-    if ((long long)n * ((max_ny + 31) / 32) * ((max_nx + 15) / 16) < 2 * 148)
+    const long long tiles = (long long)((max_ny + 31) / 32) * ((max_nx + 15) / 16);
+    // cells: as many per block as leave each SM's six blocks six turns
+    const int per_block = (int)std::min<long long>(n * tiles / (36 * 148), 16);
+    if (cells && per_block <= 1) {
+      interp_t<2, 1, 1, true, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
+    } else if (cells) {
+      dim3 grid((unsigned)((max_nx + 15) / 16), (unsigned)((max_ny + 31) / 32), (unsigned)((n + per_block - 1) / per_block));
+      cell_rows_kernel<<<grid, INTERP_THREADS, 0, st>>>(b, p0, n, per_block, strip, stride);
+    } else if (n * tiles < 2 * 148) {
       interp_t<1, 1, 2, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
-    else
+    } else {
       interp_t<2, 1, 1, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
+    }
   }
   return cudaGetLastError();
 }

@@ -118,13 +118,9 @@ unsigned long long nufft_double_to_key(double d);
 // leaves the grid is skipped and sets err[0].
 cudaError_t nufft_spread(const AtomD *atoms, const int *seg, int n_elem, int n_atoms, const NufftGeom &g,
                          double *grid, int copies, int *err, cudaStream_t st);
-// Step 2: zero `fine` and scatter the deconvolved spreading grid (the sum of
-// its copies) into it.  dec: 1 / phi2hat per spreading-grid index, x then y
-// then z.
-cudaError_t nufft_pad(const double2 *small, double2 *fine, const NufftGeom &g, int n_elem, int copies,
-                      const double *dec, cudaStream_t st);
 // Steps 2-3 by the hand-written passes: x (with the sum of the spreading-grid
-// copies and the deconvolution), y, z (with the FP32 element-interleaved
+// copies and the deconvolution; dec: 1 / phi2hat per spreading-grid index, x
+// then y then z), y, z (with the FP32 element-interleaved
 // output of nufft_pack_groups(n_elem) x box cells x nufft_pack_halves(n_elem)
 // float4; f64: the same cells in FP64, for nufft_nodes).  fa: E n1z n1y m_x, fb:
 // E n1z m_y m_x double2.

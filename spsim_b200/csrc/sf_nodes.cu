@@ -25,7 +25,11 @@ cudaError_t set_nodes_copy_stall(int on) {
 // nodes: 1.29e12 (1.27e12 with the sign on the ALU pipe, 1.24e12 with a full /
 // empty barrier pair per stage instead of the CTA barrier, 1.28e12 with three
 // CTAs per SM; FP32 sums of 16 atoms take the same time and have half as much
-// error again).
+// error again).  On cells (kCellSizes in capi.cu) the runs of an element are
+// short: 1.0e12 on 65 cells of 770 atoms x 71^2 nodes and on 65 of 308 x 22^2,
+// from the padding to groups, the flushes and the items' starts (not from their
+// latency: the next item's number and the form factors read ahead change
+// nothing).
 constexpr int NODE_THREADS = 128;
 constexpr int NODE_TILE = SF_NODES_TILE;  // nodes per work item: 8 per lane
 static_assert(NODE_TILE == 256, "eight nodes per lane");
@@ -235,14 +239,16 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
   }
 }
 
-// The same sum in FP64 throughout, phases by rounding.  B200's FP64 pipe runs at half the FP32 rate, and without the split
-// phase and the compensated sums a term is 21 operations, so this takes 1.8
-// times as long as the FP32 kernel (7.2e11 terms/s on 50,000 atoms x 26,244
-// nodes, P = 4; 80 % of the pipe).  It runs
-//   - for molecules rewritten on the device, that is in refinements: a node's
-//     rounding error goes into all the pixels around it alike, and the gradient
-//     of a loss adds it up where the pixels' own errors would average out (up
-//     to 6 times the gradient's error on a heavily oversampled detector);
+// The same sum in FP64 throughout, phases by rounding.  B200's FP64 pipe runs at
+// half the FP32 rate, and without the split phase and the compensated sums a
+// term is 21 operations, so this takes 1.8 times as long as the FP32 kernel
+// (7.2e11 terms/s on 50,000 atoms x 26,244 nodes, P = 4; 80 % of the pipe).  It
+// runs
+//   - in FP64, and for molecules rewritten on the device, that is in
+//     refinements: a node's rounding error goes into all the pixels around it
+//     alike, and the gradient of a loss adds it up where the pixels' own errors
+//     would average out (up to 6 times the gradient's error on a heavily
+//     oversampled detector);
 //   - for small grids, which latency bounds: with P = 2 a work item is 64 nodes
 //     (1,000 atoms x 340 nodes: 12 us against 17 us in FP32; 5,000 x 840 even).
 template <int P, bool PERB>
