@@ -716,7 +716,7 @@ struct Plan {
   CoarsePattern *cpats = nullptr;
   double2 *pix_acc = nullptr, *strip = nullptr;
   long long strip_size = 0;
-  int max_nx = 0, max_ny = 0, max_nyn = 0;
+  int max_nx = 0, max_ny = 0, max_nxn = 0, max_nyn = 0;
   // cells: the last npat descriptors hold the patterns on their own nodes, which
   // the interpolation of the cells' sums writes
   int n_cells = 0, cell_nx = 0, cell_ny = 0, cell_nyn = 0;
@@ -1024,7 +1024,10 @@ static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stre
 }
 
 // Cells for the patterns of a plan on coarse grids: where they save more than
-// their two launches, in all less than kMaxCellSums of sums.
+// their two launches, in all less than kMaxCellSums of sums.  Making a list takes
+// 0.15 ms once per molecule, which a few passes of a large pattern or some ten of
+// a batch of uneven molecules repay (16 of them, 500 to 60,000 atoms: 277 us a
+// pass; 343 with lists only for those that save 12 us, 400 for those of 50 us).
 struct PatternCells {
   const MoleculeCells *list = nullptr;
   CoarseGrid grid;  // of each cell
@@ -1195,10 +1198,11 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       pix_total += qsets[i]->npix;
     }
     if (list) tab_total += (size_t)(qsets[0]->geom.nx * coarse_ld(nodes[0].x.n) + qsets[0]->geom.ny * coarse_ld(nodes[0].y.n));
-    pl.max_nx = pl.max_ny = pl.max_nyn = 0;
+    pl.max_nx = pl.max_ny = pl.max_nxn = pl.max_nyn = 0;
     for (int i = 0; i < npat; ++i) {
       pl.max_nx = std::max(pl.max_nx, qsets[i]->geom.nx);
       pl.max_ny = std::max(pl.max_ny, qsets[i]->geom.ny);
+      pl.max_nxn = std::max(pl.max_nxn, nodes[i].x.n);
       pl.max_nyn = std::max(pl.max_nyn, nodes[i].y.n);
     }
     // the interpolation's strips: a group of patterns at a time, 64 MB of them
@@ -1608,12 +1612,13 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
     memset(&b, 0, sizeof(b));
     b.pats = pats;
     b.coarse = pl.cpats + pl.n_interp;
-    if (pl.n_cells && (e = launch_coarse_interp(b, pl.n_cells, pl.cell_nx, pl.cell_ny, pl.cell_nyn, pl.strip,
-                                                pl.strip_size, stream, true)))
+    if (pl.n_cells && (e = launch_coarse_interp(b, pl.n_cells, pl.cell_nx, pl.cell_ny, 0, pl.cell_nyn,
+                                                pl.strip, pl.strip_size, stream, true)))
       return e;
     b.pats = pats + pixels;
     b.coarse = pl.cpats;
-    if ((e = launch_coarse_interp(b, pl.n_interp, pl.max_nx, pl.max_ny, pl.max_nyn, pl.strip, pl.strip_size, stream)))
+    if ((e = launch_coarse_interp(b, pl.n_interp, pl.max_nx, pl.max_ny, pl.max_nxn, pl.max_nyn, pl.strip, pl.strip_size,
+                                  stream)))
       return e;
   }
   if (pl.spectrum > 0)
@@ -2524,7 +2529,7 @@ static cudaError_t nufft_interp_coarse(NufftCtx &c, const NufftInterp &pixels, c
   memcpy(b.center, pixels.g.center, sizeof(b.center));
   b.F = pixels.F;
   b.I = pixels.I;
-  return launch_coarse_interp(b, pixels.npat, g.nx, g.ny, nyn, (double2 *)c.strip.p, strips, st);
+  return launch_coarse_interp(b, pixels.npat, g.nx, g.ny, nxn, nyn, (double2 *)c.strip.p, strips, st);
 }
 
 // npat patterns of one molecule and q set, pattern i rotated by rot[9 i] (or

@@ -262,7 +262,10 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, 
 }
 
 // ROWS: the second product, else the first.  SUM: of a cell (CoarsePattern::sum).
-template <int RM, int RN, int AHEAD, bool ROWS, bool SUM>
+// BOTH: the second product after the first one's for the block's own 16 columns,
+// in shared memory, on grids of up to 64 x 64 nodes.
+constexpr int BOTH_NODES = 64;
+template <int RM, int RN, int AHEAD, bool ROWS, bool SUM, bool BOTH>
 __global__ void __launch_bounds__(INTERP_THREADS, 7)
     coarse_interp_kernel(const __grid_constant__ CoarseBatch batch, int pattern0, double2 *__restrict__ strips,
                          long long strip_stride) {
@@ -278,17 +281,35 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
   const double *__restrict__ M = ROWS ? cp.my : cp.mx;
   const int m0 = (blockIdx.y * INTERP_WARPS_M + warp % INTERP_WARPS_M) * (8 * RM);
   const int n0 = (blockIdx.x * INTERP_WARPS_N + warp / INTERP_WARPS_M) * (8 * RN);
-  if (m0 >= m_all || n0 >= n_all) return;
   const int fr = lane >> 2, fc = lane & 3;
+  constexpr int CLD = 17;
+  __shared__ double2 columns[BOTH ? BOTH_NODES * CLD : 1];
+  if (BOTH) {
+    static_assert(!BOTH || (RN == 1 && INTERP_WARPS_N == 2), "16 columns per block");
+    const int x0 = blockIdx.x * 16 + 8 * (warp & 1);
+    for (int kb = 16 * (warp >> 1); kb < cp.nyn; kb += 32) {
+      const double2 *col[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) col[j] = cp.nodes + (long long)min(kb + 8 * j + fr, cp.nyn - 1) * cp.nxn;
+      double cr[1][2][2], ci[1][2][2];
+      dmma_tile<1, 2, 2>(cp.mx, cp.ldx, x0, cp.nx, col, 1, cp.nxn, 0, cp.nxn, cr, ci);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        columns[(kb + 8 * (j >> 1) + 2 * fc + (j & 1)) * CLD + 8 * (warp & 1) + fr] =
+            make_double2(cr[0][j >> 1][j & 1], ci[0][j >> 1][j & 1]);
+    }
+    __syncthreads();
+  }
+  if (m0 >= m_all || n0 >= n_all) return;
 
   const double2 *bcol[RN];
 #pragma unroll
   for (int j = 0; j < RN; ++j) {
     const int n = min(n0 + 8 * j + fr, n_all - 1);
-    bcol[j] = ROWS ? strip + n : cp.nodes + (long long)n * cp.nxn;
+    bcol[j] = BOTH ? columns + (n0 - (int)blockIdx.x * 16 + 8 * j + fr) : ROWS ? strip + n : cp.nodes + (long long)n * cp.nxn;
   }
   double re_[RM][RN][2], im_[RM][RN][2];
-  dmma_tile<RM, RN, AHEAD>(M, ld, m0, m_all, bcol, ROWS ? cp.nx : 1, k_all, 0, k_all, re_, im_);
+  dmma_tile<RM, RN, AHEAD>(M, ld, m0, m_all, bcol, BOTH ? CLD : ROWS ? cp.nx : 1, k_all, 0, k_all, re_, im_);
 
   if (!ROWS) {
 #pragma unroll
@@ -446,15 +467,15 @@ __global__ void __launch_bounds__(INTERP_THREADS, 6)
   flush();
 }
 
-template <int RM, int RN, int AHEAD, bool ROWS, bool SUM = false>
+template <int RM, int RN, int AHEAD, bool ROWS, bool SUM = false, bool BOTH = false>
 static void interp_t(const CoarseBatch &b, int pattern0, int n, int m_max, int n_max, double2 *strip, long long stride,
                      cudaStream_t st) {
   const int bm = 8 * RM * INTERP_WARPS_M, bn = 8 * RN * INTERP_WARPS_N;
   dim3 grid((unsigned)((n_max + bn - 1) / bn), (unsigned)((m_max + bm - 1) / bm), (unsigned)n);
-  coarse_interp_kernel<RM, RN, AHEAD, ROWS, SUM><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
+  coarse_interp_kernel<RM, RN, AHEAD, ROWS, SUM, BOTH><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
 }
 
-cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
+cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nxn, int max_nyn, double2 *strip,
                                  long long strip_size, cudaStream_t st, bool cells) {
   if (npat <= 0 || max_nx <= 0 || max_ny <= 0) return cudaSuccess;
   const long long stride = (long long)max_nyn * max_nx;
@@ -465,8 +486,16 @@ cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int
     // 10.3 us, with 16 x 8 11.8, 16 x 16 14).  Rows: 16 x 8 (46 us; 8 x 8 64,
     // 32 x 16 46.5), but 8 x 8 where those leave most SMs without two blocks
     // (one 512^2 pattern: 6.4 us instead of 8.8; eight: 43 instead of 34).
-    interp_t<1, 1, 2, false>(b, p0, n, max_nx, max_nyn, strip, stride, st);
     const long long tiles = (long long)((max_ny + 31) / 32) * ((max_nx + 15) / 16);
+    // Both products in one launch where the second leaves SMs without two blocks
+    // and the first is short: one 256^2 pattern 7.3 us instead of 3.3 + 6.0 and a
+    // launch (the call 16.4 us instead of 20.5).  Not beyond: 517 x 389 pixels from
+    // 54 x 45 nodes 21 us against 5 + 11, eight 512^2 patterns 53 against 4 + 33.
+    if (!cells && max_nxn <= BOTH_NODES && max_nyn <= BOTH_NODES && n * tiles < 2 * 148) {
+      interp_t<1, 1, 2, true, false, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
+      continue;
+    }
+    interp_t<1, 1, 2, false>(b, p0, n, max_nx, max_nyn, strip, stride, st);
     // cells: as many per block as leave each SM's six blocks six turns
     const int per_block = (int)std::min<long long>(n * tiles / (36 * 148), 16);
     if (cells && per_block <= 1) {

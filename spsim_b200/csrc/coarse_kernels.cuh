@@ -89,8 +89,8 @@ struct CoarseBatch {
 // Interpolates npat patterns in groups of as many as the strip buffer holds
 // (strip_size complex values, at least max_nyn * max_nx).
 // cells: the patterns are cells, added to the sums of the patterns they belong to.
-cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nyn, double2 *strip,
-                                 long long strip_size, cudaStream_t st, bool cells = false);
+cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nxn, int max_nyn,
+                                 double2 *strip, long long strip_size, cudaStream_t st, bool cells = false);
 
 // Patterns on a float HKL list that is a detector's own, rotated and rounded:
 // q = R q_detector + delta with delta of a few float roundings.  The amplitudes
