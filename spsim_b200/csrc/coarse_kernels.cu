@@ -65,6 +65,10 @@ __device__ __forceinline__ double coarse_node_pos(const CoarseAxis &a, int k) {
 // points interpolated to
 __host__ __device__ __forceinline__ int coarse_rows(const CoarseAxis &a) { return a.to_n > 0 ? a.to_n : a.n_pix; }
 
+// Where column k of a matrix row is stored: of each eight, k and k + 4 are
+// neighbours, a lane's pair in dmma_tile.
+__device__ __forceinline__ int coarse_slot(int k) { return (k & ~7) | (2 * (k & 3) + ((k >> 2) & 1)); }
+
 // One row (point p) of an interpolation matrix by one warp:
 // M[k] = (w_k / (xi - xi_k)) / sum_j w_j / (xi - xi_j), the barycentric weights
 // of the Chebyshev extreme points w_k = (-1)^k, halved at both ends.
@@ -96,7 +100,7 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
           s1 += w / d1;
           s0 += w / d0;
         } else {
-          m[(long long)p * ld + k] = k < n ? (w / d1 / s1 - w / d0 / s0) / (2.0 * step) : 0.0;
+          m[(long long)p * ld + coarse_slot(k)] = k < n ? (w / d1 / s1 - w / d0 / s0) / (2.0 * step) : 0.0;
         }
       }
       if (!pass)
@@ -127,11 +131,11 @@ __device__ __forceinline__ void coarse_row(int p, const CoarseAxis &a, int ld, d
       const double w = ((k & 1) ? -1.0 : 1.0) * ((k == 0 || k == n - 1) ? 0.5 : 1.0);
       v = hit >= 0 ? (k == hit ? 1.0 : 0.0) : w / d / sum;
     }
-    m[(long long)p * ld + k] = v;
+    m[(long long)p * ld + coarse_slot(k)] = v;
     if (mt && k < n) {
-      mt[(long long)k * lt + p] = v;
+      mt[(long long)k * lt + coarse_slot(p)] = v;
       if (p == coarse_rows(a) - 1)
-        for (int z = p + 1; z < lt; ++z) mt[(long long)k * lt + z] = 0.0;
+        for (int z = p + 1; z < lt; ++z) mt[(long long)k * lt + coarse_slot(z)] = 0.0;
     }
   }
 }
@@ -207,8 +211,9 @@ __device__ __forceinline__ void dmma(double c[2], double a, double b) {
 // (in range, clamped), B's column n0 + 8 j + fr from bcol[j], bstep values from
 // one k to the next.  A tile's real and imaginary parts are two MMA tiles, so
 // that a lane reads a complex value at a time.  Of each group of eight k the
-// lane's entries are k = 2 fc + s in step s, so that M is read in pairs; M
-// holds zeros from k_all to its padded end, where B is read at its last row.
+// lane's entries are k = fc + 4 s in step s: neighbours in M (coarse_slot), and
+// of B's rows four lanes read 64 bytes (with k = 2 fc + s every other 16: the
+// columns of 65 cells 20 us instead of 15).  M holds zeros from k_all to its padded end, where B is read at its last row.
 // AHEAD: the groups whose fragments are read ahead of the one multiplied (L2's
 // latency bounds the small tiles, registers the large ones).
 template <int RM, int RN, int AHEAD>
@@ -225,7 +230,7 @@ __device__ __forceinline__ void dmma_tile(const double *__restrict__ M, int ld, 
     for (int j = 0; j < RN; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
   double2 a[AHEAD + 1][RM], b0[AHEAD + 1][RN], b1[AHEAD + 1][RN];
   auto load = [&](int k, int slot) {
-    const long long kb0 = min(k + 2 * fc, k_all - 1) * bstep, kb1 = min(k + 2 * fc + 1, k_all - 1) * bstep;
+    const long long kb0 = min(k + fc, k_all - 1) * bstep, kb1 = min(k + fc + 4, k_all - 1) * bstep;
 #pragma unroll
     for (int i = 0; i < RM; ++i) a[slot][i] = arow[i][k / 2];
 #pragma unroll
@@ -483,7 +488,7 @@ cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int
   for (int p0 = 0; p0 < npat; p0 += group) {
     const int n = std::min(group, npat - p0);
     // Columns: 8 x 8 values per warp (50,000 atoms x 1024^2, 161 nodes a side:
-    // 10.3 us, with 16 x 8 11.8, 16 x 16 14).  Rows: 16 x 8 (46 us; 8 x 8 64,
+    // 10.4 us, with 16 x 8 11.8, 16 x 16 14).  Rows: 16 x 8 (44 us; 8 x 8 64,
     // 32 x 16 46.5), but 8 x 8 where those leave most SMs without two blocks
     // (one 512^2 pattern: 6.4 us instead of 8.8; eight: 43 instead of 34).
     const long long tiles = (long long)((max_ny + 31) / 32) * ((max_nx + 15) / 16);

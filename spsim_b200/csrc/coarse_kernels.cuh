@@ -56,7 +56,7 @@ void coarse_set_nodes(CoarseAxis &a, int n);
 // SfPattern of pixels.
 struct CoarsePattern {
   const double2 *nodes;  // [nyn][nxn] centred amplitudes
-  const double *mx;      // [nx][ldx]: weight of node column i for pixel column x at mx[x * ldx + i]
+  const double *mx;      // [nx][ldx]: weight of node column i for pixel column x at mx[x * ldx + coarse_slot(i)]
   const double *my;      // [ny][ldy]
   int nx, ny, nxn, nyn, ldx, ldy;
   double B;              // global B factor, applied per pixel
@@ -71,7 +71,7 @@ struct CoarsePattern {
 __host__ __device__ inline int coarse_ld(int n) { return (n + 7) / 8 * 8; }
 
 // Node q vectors [y.n * x.n][3] and both interpolation matrices of one
-// detector; tx, ty: also their transposes, [nodes][coarse_ld(pixels)].
+// detector, columns at coarse_slot; tx, ty: also their transposes, [nodes][coarse_ld(pixels)].
 cudaError_t launch_coarse_tables(const DetGeom &g, const CoarseAxis &x, const CoarseAxis &y, double *q64, double *mx,
                                  double *my, cudaStream_t st, double *tx = nullptr, double *ty = nullptr);
 // The patterns of one interpolation: either described one by one (pats, coarse)
