@@ -457,7 +457,7 @@ def run_b200(args):
     # the other precisions on the same workload, and accuracy against the FP64
     # GPU kernel: single-GPU extras (their timing takes no collective steps the
     # other ranks would have to match)
-    extra = _modes(args, core, mol, qs, rot, terms, timed, prec) if world == 1 and not args.no_modes else None
+    extra = _modes(args, core, mol, qs, rot, terms, timed, prec, w, Z, pos) if world == 1 and not args.no_modes else None
     if rank == 0 and extra:
         line.update(extra)
     # end to end through the reference-facing simulate_shot (host buffers), on every rank
@@ -501,10 +501,10 @@ def run_b200(args):
     return 0
 
 
-def _modes(args, core, mol, qs, rot, terms, timed, prec):
+def _modes(args, core, mol, qs, rot, terms, timed, prec, w, Z, pos):
     """f32_fast throughput, the plain FP64 kernel on every 8th pixel, and the
-    relative |F|^2 errors of both FP32 modes against that FP64 kernel (itself
-    within 2e-7 of the FP64 oracle: tests/test_gpu_sf.py) on every 64th row."""
+    relative |F|^2 errors of both FP32 modes against the FP64 oracle on every
+    64th row."""
     import torch
 
     out = {}
@@ -524,7 +524,6 @@ def _modes(args, core, mol, qs, rot, terms, timed, prec):
                            "frac_of_R": evaluated / (sf_ms * 1e-3) / R if sf_ms else None,
                            "balanced": bal}
     q = qs.q()
-    sub_rows = core.QSet.from_list(q.reshape(1024, 1024, 3)[::64].reshape(-1, 3))
     sub8 = core.QSet.from_list(q[::8])
     with core.timing() as t:
         for _ in range(3):
@@ -532,26 +531,32 @@ def _modes(args, core, mol, qs, rot, terms, timed, prec):
         torch.cuda.synchronize()
     fp64_ms = statistics.median(t.ms[1:])
     fp64_rate = terms / 8 / (fp64_ms * 1e-3)
-    _, I64 = core.forward(mol, sub_rows, rot=rot, precision="fp64")
-    I64 = I64.double().cpu().numpy()
+    # the outputs of the timed calls against the FP64 oracle on every 64th row
+    from oracle import oracle as O
+    d = w["det"]
+    q64 = O.hkl_detector(d["nx"], d["ny"], d["width"], d["height"], d["distance"], d["wavelength"])
+    q64 = q64.reshape(d["ny"], d["nx"], 3)[::64].reshape(-1, 3)
+    if rot is not None:
+        q64 = q64 @ np.asarray(rot, np.float64).reshape(3, 3).T
+    _, I64 = O.structure_factor(Z, pos.astype(np.float64), q64)
+    rows = lambda I: I.reshape(d["ny"], d["nx"])[::64].reshape(-1).double().cpu().numpy()
     acc = {}
     for p in ("f32", "f32_fast"):
-        _, Ip = core.forward(mol, sub_rows, rot=rot, precision=p)
-        Ip = Ip.double().cpu().numpy()
+        Ip = rows(core.forward(mol, qs, rot=rot, precision=p)[1])
         den = np.maximum(I64, 1e-3 * I64.mean())
         acc[p] = {"floored_max_rel": float(np.max(np.abs(Ip - I64) / den)),
                   "l2_rel": float(np.linalg.norm(Ip - I64) / np.linalg.norm(I64)),
                   "p99_rel": float(np.percentile(np.abs(Ip - I64) / np.maximum(I64, 1e-30), 99))}
     torch.cuda.synchronize()
-    out["accuracy"] = {"reference": "plain FP64 GPU kernel", "pixels": "every 64th detector row (16,384)",
+    out["accuracy"] = {"reference": "FP64 oracle", "pixels": "every 64th detector row (16,384)",
                        "floor": "1e-3 x mean intensity", **acc}
-    out["nufft"] = _nufft_mode(core, mol, qs, rot, terms, sub_rows, I64)
+    out["nufft"] = _nufft_mode(core, mol, qs, rot, terms, rows, I64)
     out["fp64_plain"] = {"kernel_terms_per_s": fp64_rate, "sample": "every 8th pixel",
                          "f32_speedup": None, "f32_fast_speedup": None}
     return out
 
 
-def _nufft_mode(core, mol, qs, rot, terms, sub_rows, I64, eps=1e-8, steps=5):
+def _nufft_mode(core, mol, qs, rot, terms, rows, I64, eps=1e-8, steps=5):
     """The same structure factor by the type-3 NUFFT (spsim_b200_forward_nufft,
     the reference's use_nfft_for_sf path): device-resident time per pattern
     (CUDA events around the call, L2 flushed between calls), the equivalent
@@ -575,8 +580,7 @@ def _nufft_mode(core, mol, qs, rot, terms, sub_rows, I64, eps=1e-8, steps=5):
     core.synchronize()
     ms = statistics.median(a.elapsed_time(b) for a, b in evs)
     w1, w2, n2 = core.last_nufft_grid()
-    _, In = core.forward_nufft(mol, sub_rows, rot=rot, eps=eps)
-    In = In.double().cpu().numpy()
+    In = rows(I)
     den = np.maximum(I64, 1e-3 * I64.mean())
     return {"ms_per_pattern": ms, "equivalent_terms_per_s": terms / (ms * 1e-3), "eps": eps,
             "kernel_widths": [w1, w2], "fft_grid": list(n2),
@@ -584,7 +588,7 @@ def _nufft_mode(core, mol, qs, rot, terms, sub_rows, I64, eps=1e-8, steps=5):
                          "l2_rel": float(np.linalg.norm(In - I64) / np.linalg.norm(I64))},
             "note": "type-3 NUFFT per element (spread; pruned x, y, z FFT passes with the deconvolution and the "
                     "FP32 packing fused; interpolate; FP64 spreading and FFT, "
-                    "FP32 interpolation grid), a different algorithm from the direct sum the headline value times"}
+                    "interpolation at the nodes of the detector's coarse grid), a different algorithm from the direct sum the headline value times"}
 
 
 def _e2e(args, w, Z, pos, terms, world, dist=None):
