@@ -120,7 +120,11 @@ void spsim_b200_set_noise_seed(unsigned long long seed);
  * 2^19 pixels on, none below; 1: none; at most 8.  Every output is that of
  * one whole-detector pass (each pixel keeps its noise stream; chunk rows are
  * a multiple of the y binning), up to the FP32 summation order of the
- * structure factor. */
+ * structure factor.  Where the direct sum of a shot is long (from some 2.5e8
+ * atom.pixel terms on) it runs on a coarse grid of the detector
+ * (spsim_b200_forward), the float HKL list's rounding added to first order,
+ * and the chunks only combine their pixels: within 1e-7 (relative L2 of
+ * |F|^2) of the sum on every pixel. */
 void spsim_b200_set_shot_chunks(int chunks);
 int spsim_b200_get_shot_chunks(void);
 

@@ -912,8 +912,8 @@ static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const 
 // each cell's sum runs on a coarser grid of its own, which is interpolated to
 // the pattern's nodes and multiplied there by the phase of the cell's centre.
 // 50,000 atoms on 167^2 nodes, 1,065 us of node kernel: 65 cells of 71^2 nodes
-// take 256 us, and 75 us to interpolate; 128 orientations of 20,000 atoms on
-// 38^2 nodes 2,890 us: 65 cells of 22^2, 1,361 and 232 us.  The cells' size is
+// take 250 us, and 62 us to interpolate; 128 orientations of 20,000 atoms on
+// 38^2 nodes 2,890 us: 65 cells of 22^2, 1,276 and 176 us.  The cells' size is
 // the cheapest of these by the measured rates.
 struct CellSize {
   double a;   // lattice constant per bound of the molecule
@@ -1024,15 +1024,16 @@ static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stre
 }
 
 // Cells for the patterns of a plan on coarse grids: where they save more than
-// their two launches, in all less than kMaxCellSums of sums.  Making a list takes
-// 0.15 ms once per molecule, which a few passes of a large pattern or some ten of
-// a batch of uneven molecules repay (16 of them, 500 to 60,000 atoms: 277 us a
-// pass; 343 with lists only for those that save 12 us, 400 for those of 50 us).
+// their two launches, and their sums take no more memory than kMaxCellSums or
+// the pixels' own would.  Making a list takes 0.15 ms once per molecule, which a
+// few passes of a large pattern or some ten of a batch of uneven molecules repay
+// (16 of them, 500 to 60,000 atoms: 277 us a pass; 343 with lists only for those
+// that save 12 us, 400 for those of 50 us).
 struct PatternCells {
   const MoleculeCells *list = nullptr;
   CoarseGrid grid;  // of each cell
 };
-constexpr double kMaxCellSums = 4e9, kCellsMinSaved = 15e-6;
+constexpr double kMaxCellSums = 256e6, kCellsMinSaved = 15e-6;
 static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, int precision, const Spectrum *spec, const std::vector<CoarseGrid> &nodes,
                       cudaStream_t stream, std::vector<PatternCells> &cells) {
@@ -1067,7 +1068,9 @@ static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const sp
     cells[i].grid = grid[i];
     if (cells[i].list) bytes += (double)cells[i].list->n * grid[i].x.n * grid[i].y.n * sizeof(double2);
   }
-  if (bytes > kMaxCellSums) cells.assign(npat, PatternCells());
+  double pixels = 0.0;
+  for (int i = 0; i < npat; ++i) pixels += (double)qsets[i]->npix * sizeof(double2);
+  if (bytes > std::max(kMaxCellSums, pixels)) cells.assign(npat, PatternCells());
   return SPSIM_OK;
 }
 
