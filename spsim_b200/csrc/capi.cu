@@ -877,7 +877,8 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
 // All of them or none: a batch is one launch of one kernel.  The times weighed
 // are the measured rates on B200 (direct sum on neighbour quads 1.75e12 terms/s;
 // on nodes, each with its own FP64 phase, 1.3e12; in FP64 on pixels 2e11, on
-// nodes 7e11; the interpolation 1e13 FP64 multiply-adds/s) and the interpolation's launches and tail, ~4 us: patterns of
+// nodes 7e11; the interpolation 1e13 FP64 multiply-adds/s) and the
+// interpolation's launches and tail, ~4 us: patterns of
 // less than about 1e7 terms stay on the direct sum.
 static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                         const double *rot, int precision, const Spectrum *spec, std::vector<CoarseGrid> &nodes) {
@@ -1014,7 +1015,8 @@ static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stre
   c->tile_begin.push_back((int)c->tiles.size());
   CUDA_TRY(cudaMemcpyAsync(run, begin.data(), keys * sizeof(int), cudaMemcpyHostToDevice, stream));
   CUDA_TRY(cudaMemsetAsync(cursor, 0, keys * sizeof(int), stream));
-  CUDA_TRY(cudaMemcpyAsync(c->d_tiles, c->tiles.data(), c->tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice, stream));
+  CUDA_TRY(cudaMemcpyAsync(c->d_tiles, c->tiles.data(), c->tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice,
+                           stream));
   CUDA_TRY(launch_cells_build(c->lattice, m->d_atomsd, m->d_perm, m->n_padded, n_elem, key, count, run, cursor, order,
                               c->d_atoms, slots, stream));
   CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1200,7 +1202,10 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
       pix_off[i] = pix_total;
       pix_total += qsets[i]->npix;
     }
-    if (list) tab_total += (size_t)(qsets[0]->geom.nx * coarse_ld(nodes[0].x.n) + qsets[0]->geom.ny * coarse_ld(nodes[0].y.n));
+    if (list) {  // the derivative matrices
+      const DetGeom &g = qsets[0]->geom;
+      tab_total += (size_t)g.nx * coarse_ld(nodes[0].x.n) + (size_t)g.ny * coarse_ld(nodes[0].y.n);
+    }
     pl.max_nx = pl.max_ny = pl.max_nxn = pl.max_nyn = 0;
     for (int i = 0; i < npat; ++i) {
       pl.max_nx = std::max(pl.max_nx, qsets[i]->geom.nx);
@@ -1221,7 +1226,8 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
         pl.cell_nyn = std::max(pl.cell_nyn, sum_grid[i].y.n);
       }
       const long long cs = (long long)pl.cell_nyn * pl.cell_nx;
-      pl.strip_size = std::max(pl.strip_size, cs * std::min<long long>(pl.n_cells, std::max<long long>(1, (4LL << 20) / cs)));
+      const long long group = std::min<long long>(pl.n_cells, std::max<long long>(1, (4LL << 20) / cs));
+      pl.strip_size = std::max(pl.strip_size, cs * group);
     }
     auto round = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t at_cpats = round(tab_total * sizeof(double));

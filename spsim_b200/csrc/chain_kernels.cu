@@ -174,7 +174,8 @@ __device__ __forceinline__ float solid_angle_factor(const ChainDev &c, const Pix
 // pixel indices and a division per Poisson term; 41 us without those; 35 us
 // with a block drawn before the samplers' branches and one rsqrt for both
 // angles; 33 us at 40 registers (six blocks per SM instead of four).
-__global__ void __launch_bounds__(256, 6) chain_pixel_kernel(ChainDev c, const float *__restrict__ I, ChainOut o, bool small) {
+__global__ void __launch_bounds__(256, 6)
+    chain_pixel_kernel(ChainDev c, const float *__restrict__ I, ChainOut o, bool small) {
   const long long i = c.i0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= c.i1) return;
   int x, y;

@@ -213,7 +213,8 @@ __device__ __forceinline__ void dmma(double c[2], double a, double b) {
 // that a lane reads a complex value at a time.  Of each group of eight k the
 // lane's entries are k = fc + 4 s in step s: neighbours in M (coarse_slot), and
 // of B's rows four lanes read 64 bytes (with k = 2 fc + s every other 16: the
-// columns of 65 cells 20 us instead of 15).  M holds zeros from k_all to its padded end, where B is read at its last row.
+// columns of 65 cells 20 us instead of 15).  M holds zeros from k_all to its
+// padded end, where B is read at its last row.
 // AHEAD: the groups whose fragments are read ahead of the one multiplied (L2's
 // latency bounds the small tiles, registers the large ones).
 template <int RM, int RN, int AHEAD>
@@ -311,7 +312,9 @@ __global__ void __launch_bounds__(INTERP_THREADS, 7)
 #pragma unroll
   for (int j = 0; j < RN; ++j) {
     const int n = min(n0 + 8 * j + fr, n_all - 1);
-    bcol[j] = BOTH ? columns + (n0 - (int)blockIdx.x * 16 + 8 * j + fr) : ROWS ? strip + n : cp.nodes + (long long)n * cp.nxn;
+    bcol[j] = BOTH   ? columns + (n0 - (int)blockIdx.x * 16 + 8 * j + fr)
+              : ROWS ? strip + n
+                     : cp.nodes + (long long)n * cp.nxn;
   }
   double re_[RM][RN][2], im_[RM][RN][2];
   dmma_tile<RM, RN, AHEAD>(M, ld, m0, m_all, bcol, BOTH ? CLD : ROWS ? cp.nx : 1, k_all, 0, k_all, re_, im_);
@@ -480,8 +483,8 @@ static void interp_t(const CoarseBatch &b, int pattern0, int n, int m_max, int n
   coarse_interp_kernel<RM, RN, AHEAD, ROWS, SUM, BOTH><<<grid, INTERP_THREADS, 0, st>>>(b, pattern0, strip, stride);
 }
 
-cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nxn, int max_nyn, double2 *strip,
-                                 long long strip_size, cudaStream_t st, bool cells) {
+cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int max_ny, int max_nxn, int max_nyn,
+                                 double2 *strip, long long strip_size, cudaStream_t st, bool cells) {
   if (npat <= 0 || max_nx <= 0 || max_ny <= 0) return cudaSuccess;
   const long long stride = (long long)max_nyn * max_nx;
   const int group = (int)std::min<long long>(std::max<long long>(strip_size / stride, 1), 65535);
@@ -506,7 +509,8 @@ cudaError_t launch_coarse_interp(const CoarseBatch &b, int npat, int max_nx, int
     if (cells && per_block <= 1) {
       interp_t<2, 1, 1, true, true>(b, p0, n, max_ny, max_nx, strip, stride, st);
     } else if (cells) {
-      dim3 grid((unsigned)((max_nx + 15) / 16), (unsigned)((max_ny + 31) / 32), (unsigned)((n + per_block - 1) / per_block));
+      dim3 grid((unsigned)((max_nx + 15) / 16), (unsigned)((max_ny + 31) / 32),
+                (unsigned)((n + per_block - 1) / per_block));
       cell_rows_kernel<<<grid, INTERP_THREADS, 0, st>>>(b, p0, n, per_block, strip, stride);
     } else if (n * tiles < 2 * 148) {
       interp_t<1, 1, 2, true>(b, p0, n, max_ny, max_nx, strip, stride, st);

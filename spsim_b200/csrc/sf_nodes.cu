@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPat
     const int cell = pt.cell_tiles ? wi.pixel_tile / pt.cell_tiles : 0;
     double2 *__restrict__ acc = pt.acc + cell * npix;
 
-    const long long pix0 = (long long)(wi.pixel_tile - cell * pt.cell_tiles) * (32 * P) + lane;  // node i of this lane: pix0 + 32 i
+    // node i of this lane: pix0 + 32 i
+    const long long pix0 = (long long)(wi.pixel_tile - cell * pt.cell_tiles) * (32 * P) + lane;
     double qx[P], qy[P], qz[P];
     double s2n[P];
 #pragma unroll
