@@ -392,17 +392,29 @@ def run_b200(args):
         torch.cuda.synchronize()
         core.synchronize()
         evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(steps)]
-        if dist:
-            dist.barrier()
-        torch.cuda.synchronize()
-        with core.timing() as kt, ClockSampler(local) as clocks:
-            for i, (a, b) in enumerate(evs):
-                flush.zero_()  # L2 flush between timed steps, outside the events
-                a.record()
-                step(warmup + i, prec)
-                b.record()
+        def load(seconds):
+            # the same steps, untimed: the timed ones take milliseconds, a clock
+            # sample 0.2 s, so the samples are of the load around them
+            end = time.perf_counter() + seconds
+            while time.perf_counter() < end:
+                for i in range(20):
+                    step(i, prec)
+                torch.cuda.synchronize()
+
+        with ClockSampler(local) as clocks:
+            load(1.0)
+            if dist:
+                dist.barrier()
             torch.cuda.synchronize()
-            kt.read()
+            with core.timing() as kt:
+                for i, (a, b) in enumerate(evs):
+                    flush.zero_()  # L2 flush between timed steps, outside the events
+                    a.record()
+                    step(warmup + i, prec)
+                    b.record()
+                torch.cuda.synchronize()
+                kt.read()
+            load(0.5)
         if dist:
             dist.barrier()
         torch.cuda.synchronize()
