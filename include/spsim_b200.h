@@ -122,7 +122,10 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
  * is done where it is faster (patterns of more than about 1e7 terms), for
  * whole batches or not at all, and in FP64 for molecules rewritten on the
  * device (refinements: a node's rounding error would enter the pixels around it
- * alike and add up in a gradient); q lists, forced variants
+ * alike and add up in a gradient) and where form factors and per-atom B factors
+ * let the amplitudes fall below e^-4 at the edge of an axis (dim pixels would
+ * take over the bright nodes' rounding).  Amplitudes falling below e^-10 (e^-5
+ * with SPSIM_PREC_FP64), q lists, forced variants
  * (spsim_b200_set_variant), detectors further than 1.2 detector distances off
  * the beam axis and per-atom B factors beyond twice their largest at creation
  * + 100 A^2 (checked on the device when they are rewritten there) take the

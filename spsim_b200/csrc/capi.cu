@@ -226,6 +226,7 @@ struct spsim_b200_molecule {
   int n_padded = 0;
   int n_elem = 0;
   int elem_Z[MAX_ELEM];
+  int elem_count[MAX_ELEM] = {0};  // atoms kept
   std::vector<float> coeffs;  // n_elem x 9
   std::vector<int> perm;      // padded index -> caller index (-1 = padding)
   std::vector<TileDesc> tiles;
@@ -235,6 +236,7 @@ struct spsim_b200_molecule {
   float dr = 1, inv_dr = 1;
   int per_atom_b = 0, delta_atoms = 0;
   float b_limit = 0;        // largest |per-atom B| the coarse grids are sized for
+  float b_low = 0;          // a quarter of the atoms' |per-atom B| at creation are below it
   bool updated = false;     // atoms rewritten on the device
   bool b_updated = false;   // B factors rewritten on the device: b_limit is checked there (d_flags[1])
   // device views of the buffers below
@@ -331,10 +333,19 @@ static int molecule_create_impl(int natoms, const int32_t *Z, const PosT *pos, c
   // B factors may double (and rise by 100 A^2) in a refinement before its
   // patterns leave the coarse grids
   if (bfac) {
+    std::vector<float> mag;
     float bmax = 0.0f;
-    for (int j = 0; j < natoms; ++j)
-      if (Z[j]) bmax = std::max(bmax, std::isfinite(bfac[j]) ? std::fabs(bfac[j]) : 1e30f);
+    for (int j = 0; j < natoms; ++j) {
+      if (!Z[j]) continue;
+      const float b = std::isfinite(bfac[j]) ? std::fabs(bfac[j]) : 1e30f;
+      bmax = std::max(bmax, b);
+      if (!occ || occ[j] != 0.0f) mag.push_back(b);
+    }
     m->b_limit = 2.0f * bmax + 100.0f;
+    if (!mag.empty()) {
+      std::nth_element(mag.begin(), mag.begin() + mag.size() / 4, mag.end());
+      m->b_low = mag[mag.size() / 4];
+    }
   }
 
   // element segments (ascending Z), padded to ATOM_GROUP
@@ -344,6 +355,7 @@ static int molecule_create_impl(int natoms, const int32_t *Z, const PosT *pos, c
     if (!count[z]) continue;
     if (m->n_elem >= MAX_ELEM) return fail(SPSIM_ERR_INVALID_ARG, "too many elements");
     m->elem_Z[m->n_elem] = z;
+    m->elem_count[m->n_elem] = count[z];
     for (int k = 0; k < 9; ++k) m->coeffs.push_back(g_atomsf[z][k]);
     seg_begin.push_back(n_pad);
     n_pad += (count[z] + ATOM_GROUP - 1) / ATOM_GROUP * ATOM_GROUP;
@@ -834,12 +846,12 @@ static double frobenius(const double *R) {
 // or more nodes than 80 % of the pixels.
 struct CoarseGrid {
   CoarseAxis x, y;
+  int digits = 0;  // of the interpolation (coarse_node_count)
 };
 
-// fp64: nodes for FP64 sums (1e-12 instead of 1e-8).
 // rbound: of the atoms about the centre of their phases (0: the molecule's).
 static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale,
-                       CoarseGrid *grid, bool fp64 = false, double rbound = 0.0) {
+                       CoarseGrid *grid, int digits = COARSE_DIGITS_F32, double rbound = 0.0) {
   if (!(rbound > 0.0)) rbound = m->rbound;
   const DetGeom &g = q->geom;
   if (!q->has_geom || m->n_kept == 0 || g.nx < 16 || g.ny < 16) return false;
@@ -851,6 +863,7 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
       for (int k = 4; k < 8; ++k) c = std::max(c, (double)std::fabs(m->coeffs[9 * e + k]));
     bmax += c;
   }
+  grid->digits = digits;
   grid->x = coarse_axis(g.nx, g.width, g.cx, g.distance, g.spherical != 0);
   grid->y = coarse_axis(g.ny, g.height, g.cy, g.distance, g.spherical != 0);
   for (int d = 0; d < 2; ++d) {
@@ -866,12 +879,61 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
     const double c = 2.0 * M_PI * rbound * scale * arc * (t > 1.0 ? 1.02 : 1.0);
     const double a = bmax * 0.25e-20 * reach * reach;
     if (!(c <= 1.5 * COARSE_MAX_NODES) || !(t <= 1.2) || !(a <= 60.0)) return false;
-    const int n = coarse_node_count(c, t, a, fp64);
+    const int n = coarse_node_count(c, t, a, digits);
     if (n > COARSE_MAX_NODES) return false;
     coarse_set_nodes(ax, n);
   }
   return (double)grid->x.n * grid->y.n < 0.8 * (double)g.nx * g.ny;
 }
+
+// By how much the patterns' amplitudes fall from the beam to the edge of either
+// axis (e^-fall, rms over the atoms: the form factors', times the per-atom B
+// factor of the quarter of the atoms that it dims least, or of b_limit where the
+// device may have rewritten them).  bscale as coarse_fit's.
+static double coarse_fall(const spsim_b200_molecule *m, const spsim_b200_qset *q, double bscale) {
+  const DetGeom &g = q->geom;
+  double fall = 0.0;
+  for (int d = 0; d < 2; ++d) {
+    const CoarseAxis ax = d ? coarse_axis(g.ny, g.height, g.cy, g.distance, g.spherical != 0)
+                            : coarse_axis(g.nx, g.width, g.cx, g.distance, g.spherical != 0);
+    double edge = 2.0 * std::sin(0.5 * (std::fabs(ax.mid) + ax.half)) * g.ewald;
+    if (!ax.angular)
+      edge = d ? g.fpy * (0.5 * (g.ny - 1) / g.ny * g.height + std::fabs(g.cy)) / g.py_size
+               : g.fpx * (0.5 * (g.nx - 1) / g.nx * g.width + std::fabs(g.cx)) / g.px_size;
+    const double s2 = 0.25e-20 * edge * edge;
+    double now = 0.0, before = 0.0;
+    for (int e = 0; e < m->n_elem && !m->delta_atoms; ++e) {
+      const float *c = &m->coeffs[9 * e];
+      double f0 = c[8], f = c[8];
+      for (int k = 0; k < 4; ++k) {
+        f0 += c[k];
+        f += c[k] * std::exp(-c[4 + k] * s2);
+      }
+      before += m->elem_count[e] * f0 * f0;
+      now += m->elem_count[e] * f * f;
+    }
+    const double b = m->per_atom_b ? (m->b_updated ? m->b_limit : m->b_low) * bscale * bscale : 0.0;
+    fall = std::max(fall, b * s2 + (now > 0.0 && before > now ? 0.5 * std::log(before / now) : 0.0));
+  }
+  return fall;
+}
+
+// The interpolation's digits for amplitudes that fall by e^-fall, or 0 where no
+// grid is admitted.  Every pixel's amplitude is interpolated from all nodes, the
+// bright ones in the middle among them, and takes over a part of their errors: of
+// FP32 sums' some 1e-9 of the bright amplitude at the edge of an axis, which stays
+// below the dim pixel's own rounding up to a fall of e^-4 (3,000 atoms of B = 200
+// A^2 to 1.4 A, falling by e^-13: 7 % of the dim pixels' amplitude; on every pixel
+// 9e-7).  Beyond, the sums are in FP64 and to more digits, and from e^-10 on the
+// patterns stay on every pixel.  FP64 results: to the rounding of FP64 phases, up
+// to e^-5.
+static int coarse_digits(bool fp64, double fall) {
+  if (fp64) return fall <= 5.0 ? COARSE_DIGITS_FULL : 0;
+  return fall <= 4.0 ? COARSE_DIGITS_F32 : fall <= 10.0 ? COARSE_DIGITS_F64 : 0;
+}
+
+// Node kernel's rate (terms/s).
+static double node_rate(int digits) { return digits > COARSE_DIGITS_F32 ? 7e11 : 1.3e12; }
 
 // Whether the plan's patterns run on coarse grids, with their node counts.
 // All of them or none: a batch is one launch of one kernel.  The times weighed
@@ -888,6 +950,18 @@ static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const 
   if (spec)
     for (int i = 0; i < npat; ++i) qscale = std::max(qscale, std::fabs(spec->qscale[i]));
   nodes.resize(npat);
+  // one number of digits for the plan: it runs one kernel
+  int digits = COARSE_DIGITS_F32;
+  for (int i = 0; i < npat; ++i) {
+    if (!qsets[i]->has_geom) return false;
+    const bool general = rot && !is_orthonormal(rot + 9 * (size_t)i);
+    if (i > 0 && mols[i] == mols[i - 1] && qsets[i] == qsets[i - 1] && !general) continue;
+    const double stretch = general ? std::max(1.0, frobenius(rot + 9 * (size_t)i)) : 1.0;
+    const int d = coarse_digits(fp64, coarse_fall(mols[i], qsets[i], stretch));
+    if (d == 0) return false;
+    digits = std::max(digits, d);
+  }
+  const double rate = node_rate(digits);
   double direct = 0, grid = 4e-6;
   for (int i = 0; i < npat; ++i) {
     double stretch = 1.0;  // of |q| under this pattern's matrix
@@ -896,13 +970,13 @@ static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const 
     if (i > 0 && stretch == 1.0 && mols[i] == mols[i - 1] && qsets[i] == qsets[i - 1] &&
         !(rot && !is_orthonormal(rot + 9 * (size_t)(i - 1)))) {
       nodes[i] = nodes[i - 1];
-    } else if (!coarse_fit(mols[i], qsets[i], qscale * stretch, stretch, &nodes[i], fp64)) {
+    } else if (!coarse_fit(mols[i], qsets[i], qscale * stretch, stretch, &nodes[i], digits)) {
       return false;
     }
     const double npix = (double)qsets[i]->npix, kept = mols[i]->n_kept;
     const double nxn = nodes[i].x.n, nyn = nodes[i].y.n;
     direct += kept * npix / (fp64 ? 2e11 : 1.75e12);
-    grid += kept * nxn * nyn / (fp64 ? 7e11 : 1.3e12) + 2.0 * (npix + qsets[i]->geom.nx * nxn) * nyn / 1e13;
+    grid += kept * nxn * nyn / rate + 2.0 * (npix + qsets[i]->geom.nx * nxn) * nyn / 1e13;
   }
   return grid < 0.8 * direct;
 }
@@ -924,16 +998,16 @@ static const CellSize kCellSizes[] = {{1.07, 15}, {0.85, 27},  {0.74, 51},  {0.6
                                       {0.495, 113}, {0.46, 137}, {0.41, 169}, {0.39, 181}, {0.36, 259},
                                       {0.32, 331}, {0.275, 531}, {0.25, 609}, {0.225, 868}, {0.2, 1133}};
 
-// Node kernel's rate (terms/s) and, per (cell, element), the atoms that the
-// padding, the flush and the idle warps of a short run cost.
-static double node_rate(bool fp64) { return fp64 ? 7e11 : 1.3e12; }
+// Per (cell, element), the atoms that the padding, the flush and the idle warps
+// of a short run cost.
 constexpr double kRunAtoms = 50.0;
 
 // The cheapest cells of one pattern: index into kCellSizes or -1, their grid,
 // and the time saved against the sum of all atoms on `outer`.
-static int choose_cells(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale, bool fp64,
+static int choose_cells(const spsim_b200_molecule *m, const spsim_b200_qset *q, double scale, double bscale,
                         const CoarseGrid &outer, CoarseGrid *inner, double *saved) {
-  const double no = (double)outer.x.n * outer.y.n, whole = m->n_kept * no / node_rate(fp64);
+  const double rate = node_rate(outer.digits);
+  const double no = (double)outer.x.n * outer.y.n, whole = m->n_kept * no / rate;
   int best = -1;
   double best_time = 0.85 * whole;
   *saved = 0.0;
@@ -941,10 +1015,10 @@ static int choose_cells(const spsim_b200_molecule *m, const spsim_b200_qset *q, 
   for (int k = 0; k < (int)(sizeof(kCellSizes) / sizeof(kCellSizes[0])); ++k) {
     const double cells = kCellSizes[k].cells;
     CoarseGrid g;
-    if (!coarse_fit(m, q, scale, bscale, &g, fp64, 0.5591 * kCellSizes[k].a * m->rbound)) continue;
+    if (!coarse_fit(m, q, scale, bscale, &g, outer.digits, 0.5591 * kCellSizes[k].a * m->rbound)) continue;
     const double ni = (double)g.x.n * g.y.n;
-    const double tile = fp64 ? SF_NODES64_TILE : SF_NODES_TILE;
-    const double time = (m->n_kept + cells * m->n_elem * kRunAtoms) * std::ceil(ni / tile) * tile / node_rate(fp64) +
+    const double tile = outer.digits > COARSE_DIGITS_F32 ? SF_NODES64_TILE : SF_NODES_TILE;
+    const double time = (m->n_kept + cells * m->n_elem * kRunAtoms) * std::ceil(ni / tile) * tile / rate +
                         cells * (2.0 * outer.x.n * g.y.n * (g.x.n + outer.y.n) / 6e12 + no / 1.2e11);
     if (time < best_time) {
       best = k;
@@ -1037,10 +1111,9 @@ struct PatternCells {
 };
 constexpr double kMaxCellSums = 256e6, kCellsMinSaved = 15e-6;
 static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
-                      const double *rot, int precision, const Spectrum *spec, const std::vector<CoarseGrid> &nodes,
+                      const double *rot, const Spectrum *spec, const std::vector<CoarseGrid> &nodes,
                       cudaStream_t stream, std::vector<PatternCells> &cells) {
   cells.assign(npat, PatternCells());
-  const bool fp64 = precision == SPSIM_PREC_FP64;
   std::vector<int> size(npat, -1);
   std::vector<CoarseGrid> grid(npat);
   double saved = 0.0, bytes = 0.0;
@@ -1058,7 +1131,7 @@ static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const sp
       size[i] = size[i - 1];
       grid[i] = grid[i - 1];
     } else {
-      size[i] = choose_cells(mols[i], qsets[i], qscale * stretch, stretch, fp64, nodes[i], &grid[i], &last);
+      size[i] = choose_cells(mols[i], qsets[i], qscale * stretch, stretch, nodes[i], &grid[i], &last);
     }
     saved += last;
   }
@@ -1103,7 +1176,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   // cells, and the grid of each pattern's sums: its cells' or its own
   std::vector<PatternCells> cells(npat);
   if (pl.coarse) {
-    const int st = plan_cells(npat, mols, qsets, rot, precision, spec, nodes, stream, cells);
+    const int st = plan_cells(npat, mols, qsets, rot, spec, nodes, stream, cells);
     if (st) return st;
   }
   std::vector<CoarseGrid> sum_grid(nodes);
@@ -1293,13 +1366,12 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   pl.ppt = var.p;
   pl.packed = var.packed;
   if (pl.coarse) {
-    // the FP64 kernel (sf_nodes.cu) for FP64, for molecules rewritten on the device
-    // and for grids that latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
-    bool updated = false;
-    for (int i = 0; i < npat; ++i) updated = updated || mols[i]->updated;
-    pl.node_tile = pl.evaluated <= 4e6                            ? SF_NODES64_SMALL_TILE
-                   : updated || precision == SPSIM_PREC_FP64 ? SF_NODES64_TILE
-                                                             : SF_NODES_TILE;
+    // the FP64 kernel (sf_nodes.cu) for FP64, for amplitudes that fall far
+    // (coarse_digits), for molecules rewritten on the device and for grids that
+    // latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
+    bool wide = nodes[0].digits > COARSE_DIGITS_F32;
+    for (int i = 0; i < npat; ++i) wide = wide || mols[i]->updated;
+    pl.node_tile = pl.evaluated <= 4e6 ? SF_NODES64_SMALL_TILE : wide ? SF_NODES64_TILE : SF_NODES_TILE;
   }
   const long long tile_pix = pl.coarse ? pl.node_tile : (long long)nt * ppt;
 
@@ -3426,7 +3498,7 @@ static int adjoint_plan(const spsim_b200_molecule *m, const spsim_b200_qset *qs,
   for (size_t i = 0; i < g_adj_plans.size(); ++i) {
     AdjPlan &c = *g_adj_plans[i];
     if (c.mol_id == m->id && c.qs_id == qs->id && c.npat == npat && c.B == B && c.mode == mode && c.device == dev &&
-        c.coarse == (grid != nullptr) && c.stretch == stretch) {
+        c.coarse == (grid != nullptr) && c.stretch == stretch && (!grid || c.grid.digits == grid->digits)) {
       std::unique_ptr<AdjPlan> keep = std::move(g_adj_plans[i]);
       g_adj_plans.erase(g_adj_plans.begin() + i);
       g_adj_plans.push_back(std::move(keep));
@@ -3667,7 +3739,11 @@ extern "C" int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200
   // 4 TB/s, its launches ~15 us); both FP32 precisions take the FP64 kernel there
   const double stretch = qs->qmax > 0 ? qmax / qs->qmax : 1.0;
   CoarseGrid grid;
-  bool coarse = precision != SPSIM_PREC_FP64 && g_force_nt <= 0 && coarse_fit(m, qs, stretch, stretch, &grid);
+  bool coarse = precision != SPSIM_PREC_FP64 && g_force_nt <= 0 && qs->has_geom;
+  if (coarse) {  // (dim pixels enter with large dL/d|F|^2)
+    const int digits = coarse_digits(false, coarse_fall(m, qs, stretch));
+    coarse = digits > 0 && coarse_fit(m, qs, stretch, stretch, &grid, digits);
+  }
   if (coarse) {
     const double nxn = grid.x.n, nyn = grid.y.n, pix = (double)npix;
     const double on_nodes = npat * (m->n_kept * nxn * nyn / 5e11 + 2 * (pix * nxn + nxn * nyn * qs->geom.ny) / 8e12 +

@@ -7,12 +7,12 @@
 
 namespace spsim {
 
-int coarse_node_count(double c, double t, double a, bool fp64) {
+int coarse_node_count(double c, double t, double a, int digits) {
   const double cc = c > 1.0 ? c : 1.0;
   double n = 0.66 * cc + 8.9 * std::pow(cc, 0.253);
   if (t > 0.0) n += (3.5 + 11.5 * std::sqrt(cc / 320.0)) * std::pow(t, 1.2);
   if (a > 0.0) n += 6.6 * std::sqrt(a) / (1.0 + 0.5 * std::pow(cc / (8.0 * a), 0.6));
-  if (fp64) n += 10.0 + cc / 100.0;
+  if (digits > COARSE_DIGITS_F32) n += 10.0 + cc / 100.0;
   return (int)std::ceil(n);
 }
 

@@ -120,6 +120,32 @@ def test_b_factors_rewritten_beyond_the_grids_limit(cuda):
             _check(F[k], I[k], Z, pos, q @ R[k].T, bfac=bk)
 
 
+@pytest.mark.parametrize("B,nodes", [(20.0, True), (60.0, True), (100.0, True), (200.0, False)])
+def test_amplitudes_that_fall_far(cuda, B, nodes):
+    # amplitudes that fall by e^-2 to e^-17 along an axis, e^-4 to e^-33 to the
+    # corners: the dim pixels keep their own accuracy beside the bright ones.  A
+    # ring's rms error against its rms amplitude: the FP32 weight's exponent, up
+    # to 33 / ln 2 = 48, rounds to 48 * 2^-24 * ln 2 = 2e-6
+    Z, pos = synth.random_molecule(3000, 3.0e-9, 214)
+    b = np.full(len(Z), B, np.float32)
+    d = _det(400, 400, pixel=192e-6, distance=0.06, wavelength=0.1e-9)
+    q, qs, mol = _q(d), core.QSet.from_detector(**d), core.Molecule(Z, pos, bfac=b)
+    F, _ = core.forward(mol, qs)
+    _on_grid(nodes)
+    F64, I64 = O.structure_factor(Z, pos.astype(np.float64), q, bfac=b)
+    s2 = (q * q).sum(1)
+    ring = np.minimum(6 * s2 / s2.max(), 5).astype(int)
+    err = np.abs(F.cpu().numpy() - F64) ** 2
+    for k in range(6):
+        assert np.sqrt(err[ring == k].mean() / I64[ring == k].mean()) < 2e-6, k
+    # the gradient of a loss that weighs every pixel's logarithm alike
+    g = (np.random.Generator(np.random.PCG64(215)).normal(size=len(q)) / (I64 + 1e-12 * I64.max())).astype(np.float32)
+    grads = core.adjoint(mol, qs, torch.from_numpy(F64.astype(np.complex64)).cuda(), torch.from_numpy(g).cuda())
+    exact = O.structure_factor_vjp(Z, pos.astype(np.float64), q, g.astype(np.float64), bfac=b)
+    for ours, e in zip(grads, exact):
+        assert _rel(ours.cpu().numpy(), e) < 1e-5
+
+
 def test_fp64_at_its_own_tolerance(cuda):
     # 2e-7 floored maximum, 1e-7 L2: the float32 outputs' rounding; weights, B factors, a wide detector
     Z, pos = synth.random_molecule(1500, 2.5e-9, 212)
