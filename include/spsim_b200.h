@@ -113,8 +113,8 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
  * |dq/dx| |r - c|max cycles per pixel.  The forwards (one pattern, a batch, a
  * spectrum) therefore evaluate the sum on a tensor grid of nodes, a
  * little more than two per cycle along each axis, and interpolate it to the
- * pixels in FP64, to 1e-8 of an outermost atom's amplitude (1e-12 with
- * SPSIM_PREC_FP64) and far less for the others; form factors and per-atom B
+ * pixels in FP64, to 1e-8 of an outermost atom's amplitude (1e-15 with
+ * SPSIM_PREC_FP64, whose terms keep the rounding of FP64) and far less for the others; form factors and per-atom B
  * factors belong to the interpolated sum, the global B factor and the centre
  * phase are applied per pixel.  Large patterns are summed in two levels, by
  * cells of the molecule's volume on still coarser grids of their own (lists of

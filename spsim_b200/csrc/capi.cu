@@ -881,7 +881,7 @@ static bool coarse_fit(const spsim_b200_molecule *m, const spsim_b200_qset *q, d
     if (!(c <= 1.5 * COARSE_MAX_NODES) || !(t <= 1.2) || !(a <= 60.0)) return false;
     const int n = coarse_node_count(c, t, a, digits);
     if (n > COARSE_MAX_NODES) return false;
-    coarse_set_nodes(ax, n);
+    coarse_set_nodes(ax, n, digits);
   }
   return (double)grid->x.n * grid->y.n < 0.8 * (double)g.nx * g.ny;
 }
@@ -933,13 +933,15 @@ static int coarse_digits(bool fp64, double fall) {
 }
 
 // Node kernel's rate (terms/s).
-static double node_rate(int digits) { return digits > COARSE_DIGITS_F32 ? 7e11 : 1.3e12; }
+static double node_rate(int digits) {
+  return digits == COARSE_DIGITS_FULL ? 5.6e11 : digits == COARSE_DIGITS_F64 ? 7e11 : 1.3e12;
+}
 
 // Whether the plan's patterns run on coarse grids, with their node counts.
 // All of them or none: a batch is one launch of one kernel.  The times weighed
 // are the measured rates on B200 (direct sum on neighbour quads 1.75e12 terms/s;
 // on nodes, each with its own FP64 phase, 1.3e12; in FP64 on pixels 2e11, on
-// nodes 7e11; the interpolation 1e13 FP64 multiply-adds/s) and the
+// nodes 5.6e11; the interpolation 1e13 FP64 multiply-adds/s) and the
 // interpolation's launches and tail, ~4 us: patterns of
 // less than about 1e7 terms stay on the direct sum.
 static bool coarse_plan(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
@@ -1571,7 +1573,8 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 
   if (precision != SPSIM_PREC_FP64 || pl.coarse) {
     // work items: pixel tile x atom-tile range, cost-sorted (largest first)
-    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw)
+    const bool full = precision == SPSIM_PREC_FP64;
+    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw, full)
                                           : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
     const long long slots = (long long)num_sms() * occ;
     long long total_ptiles = 0;
@@ -1678,8 +1681,8 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   } else if (pl.n_items > 0) {
     int *queue = pl.head() + 8, *err = pl.head() + 4;
     if (pl.coarse)
-      e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
-                          pl.n_items, queue, err, pl.grid, stream);
+      e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, pl.precision == SPSIM_PREC_FP64,
+                          (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p, pl.n_items, queue, err, pl.grid, stream);
     else
       e = launch_sf_f32(pl.mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,
                         pl.n_items, queue, err, pl.grid, stream, pl.fixw, pl.narrow);

@@ -12,7 +12,8 @@ int coarse_node_count(double c, double t, double a, int digits) {
   double n = 0.66 * cc + 8.9 * std::pow(cc, 0.253);
   if (t > 0.0) n += (3.5 + 11.5 * std::sqrt(cc / 320.0)) * std::pow(t, 1.2);
   if (a > 0.0) n += 6.6 * std::sqrt(a) / (1.0 + 0.5 * std::pow(cc / (8.0 * a), 0.6));
-  if (digits > COARSE_DIGITS_F32) n += 10.0 + cc / 100.0;
+  if (digits == COARSE_DIGITS_F64) n += 10.0 + cc / 100.0;
+  if (digits == COARSE_DIGITS_FULL) n += 18.0 + cc / 25.0;
   return (int)std::ceil(n);
 }
 
@@ -39,9 +40,14 @@ CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, b
   return a;
 }
 
-void coarse_set_nodes(CoarseAxis &a, int n) {
+// The stretch leaves errors of e^-(n acosh(1 / alpha)) whatever the function:
+// e^-(9.3 n^(1/3)) is small enough for 1e-8 at eight nodes and for 1e-12 at the
+// twenty that these take; for 1e-15 e^-36 at least.
+void coarse_set_nodes(CoarseAxis &a, int n, int digits) {
   a.n = n;
-  a.alpha = 1.0 / std::cosh(9.3 * std::cbrt((double)n) / n);
+  double stretch = 9.3 * std::cbrt((double)n);
+  if (digits == COARSE_DIGITS_FULL) stretch = std::max(stretch, 36.0);
+  a.alpha = 1.0 / std::cosh(stretch / n);
   a.asin_alpha = std::asin(a.alpha);
 }
 

@@ -47,11 +47,13 @@ CoarseAxis coarse_axis(int n_pix, double size, double centre, double distance, b
 // Nodes along one axis for phases of at most c radians over half of it, pixels
 // up to t detector distances off the beam axis and form factors falling as
 // exp(-a X^2): a fit, from above, to the smallest node counts that interpolate
-// every such function to 1e-8 of its maximum or, by digits, to 1e-12
-// (tests/test_coarse_grid.py restates it and measures the errors).
-constexpr int COARSE_DIGITS_F32 = 8, COARSE_DIGITS_F64 = 12, COARSE_DIGITS_FULL = 12;
+// every such function to 1e-8 of its maximum or, by digits, to 1e-12 or 1e-15
+// (tests/test_coarse_grid.py restates it and measures the errors): FP32 results,
+// FP32 results from FP64 sums, and FP64 results, whose phases' own rounding is
+// larger (1e-16 of up to some thousand radians).
+constexpr int COARSE_DIGITS_F32 = 8, COARSE_DIGITS_F64 = 12, COARSE_DIGITS_FULL = 15;
 int coarse_node_count(double c, double t, double a, int digits);
-void coarse_set_nodes(CoarseAxis &a, int n);
+void coarse_set_nodes(CoarseAxis &a, int n, int digits);
 
 // What the interpolation of one pattern reads and writes beside its
 // SfPattern of pixels.

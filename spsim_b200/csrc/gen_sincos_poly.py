@@ -141,6 +141,54 @@ def emit64(name, Y, sdeg, cdeg, out):
         out.append("#define SPSIM_%s_C%d %.17e" % (name, k, c))
 
 
+def emit_full(name, Y, sdeg, cdeg, out):
+    """FP64 pair to the rounding: the Taylor polynomials in z = y^2 economised
+    (expanded in Chebyshev polynomials on [0, Y^2] and cut), in extended
+    precision, since Remez' linear systems lose the last digits in FP64."""
+    from numpy.polynomial import chebyshev as T, polynomial as P
+
+    x = np.longdouble
+    two_pi = x("6.28318530717958647692528676655900577")
+    terms = 16
+    t = [x(1)]
+    for k in range(1, 2 * terms):
+        t.append(t[-1] * two_pi / k)  # (2 pi)^k / k!
+    sign = np.where(np.arange(terms) & 1, x(-1), x(1))
+    # of (P - P_0) / z, so that the constants stay 2 pi and 1
+    full = {"S": sign * np.array(t[1::2]), "C": sign * np.array(t[0::2])}
+    coeffs = {}
+    for key, deg in (("S", sdeg), ("C", cdeg)):
+        half = x(Y) ** 2 / 2
+        u = np.zeros(1, x)  # the rest as a polynomial in u, z = half (1 + u)
+        for c in full[key][:0:-1]:
+            u = P.polymul(u, np.array([half, half], x))
+            u[0] += c
+        c = np.zeros(terms, x)  # u^k in Chebyshev polynomials, summed
+        power = np.array([x(1)])
+        for v in u:
+            c[:len(power)] += v * power
+            power = T.chebmulx(power)
+        rest, low = np.zeros(1, x), [np.array([x(1)]), np.array([x(0), x(1)])]
+        for k in range(deg):
+            if k > 1:
+                low.append(P.polysub(P.polymul(np.array([x(0), x(2)]), low[-1]), low[-2]))
+            rest = P.polyadd(rest, c[k] * low[k])
+        inner = np.zeros(1, x)  # back to z: u = z / half - 1
+        for v in rest[::-1]:
+            inner = P.polymul(inner, np.array([x(-1), 1 / half], x))
+            inner[0] += v
+        coeffs[key] = np.concatenate([full[key][:1], inner[:deg]])
+    y = np.linspace(0, Y, 20001).astype(x)
+    z = y * y
+    ps, pc = (coeffs[k].astype(np.float64).astype(x) for k in "SC")
+    es = np.max(np.abs(y * P.polyval(z, ps) - np.sin(two_pi * y)))
+    ec = np.max(np.abs(P.polyval(z, pc) - np.cos(two_pi * y)))
+    out.append("/* %s: |y| <= %.6f cycles, FP64 coefficients: sin max %.1e, cos max %.1e */" % (name, Y, es, ec))
+    for key in "SC":
+        for k, c in enumerate(coeffs[key]):
+            out.append("#define SPSIM_%s_%s%d %.17e" % (name, key, k, c))
+
+
 def main():
     out = [
         "/* Generated by gen_sincos_poly.py (Remez minimax, float32 coefficients).",
@@ -156,6 +204,7 @@ def main():
     emit("NARROW", 0.32, 4, 5, out)
     emit("WIDER", 0.41, 5, 5, out)
     emit64("NODE64", 0.25, 5, 6, out)
+    emit_full("FULL64", 0.25, 8, 8, out)
     out += ["#endif", ""]
     print("\n".join(out))
 

@@ -371,6 +371,31 @@ __device__ __forceinline__ double exp2_poly(double x) {
   return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
 }
 
+// The same to the rounding of FP64, for FP64 results.
+__device__ __forceinline__ double exp2_full(double x) {
+  const double M52 = 6755399441055744.0;  // 1.5 * 2^52
+  constexpr double L = 0.69314718055994530942;
+  constexpr double c2 = L * L / 2, c3 = c2 * L / 3, c4 = c3 * L / 4, c5 = c4 * L / 5, c6 = c5 * L / 6, c7 = c6 * L / 7,
+                   c8 = c7 * L / 8, c9 = c8 * L / 9, c10 = c9 * L / 10, c11 = c10 * L / 11, c12 = c11 * L / 12,
+                   c13 = c12 * L / 13;
+  const double t = x + M52;
+  const double f = x - (t - M52);
+  double p = fma(f, c13, c12);
+  p = fma(f, p, c11);
+  p = fma(f, p, c10);
+  p = fma(f, p, c9);
+  p = fma(f, p, c8);
+  p = fma(f, p, c7);
+  p = fma(f, p, c6);
+  p = fma(f, p, c5);
+  p = fma(f, p, c4);
+  p = fma(f, p, c3);
+  p = fma(f, p, c2);
+  p = fma(f, p, L);
+  p = fma(f, p, 1.0);
+  return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
+}
+
 // log2(x) by the XU pipe's approximation (PTX lg2.approx.ftz.f32; -inf at 0)
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;

@@ -20,11 +20,11 @@ cudaError_t set_copy_stall(int on);
 cudaError_t set_nodes_copy_stall(int on);  // its part in sf_nodes.cu
 int sf_f32_occupancy(int mode, int nt, int p, int packed, bool perb, bool fixw = false, bool narrow = false);
 // The sum on a coarse grid's nodes, in work items of `tile` nodes: SF_NODES_TILE
-// selects the FP32 quad form, the other two the FP64 kernel.
+// selects the FP32 quad form, the other two the FP64 kernel (full: for FP64 results).
 constexpr int SF_NODES_TILE = 256, SF_NODES64_TILE = 128, SF_NODES64_SMALL_TILE = 64;
-cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items,
-                            int *queue, int *err, int grid, cudaStream_t st);
-int sf_nodes_occupancy(int tile, bool perb, bool fixw);
+cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, bool full, const SfPattern *pats, const WorkItem *items,
+                            int n_items, int *queue, int *err, int grid, cudaStream_t st);
+int sf_nodes_occupancy(int tile, bool perb, bool fixw, bool full);
 bool sf_f32_variant_exists(int mode, int nt, int p, int packed);
 cudaError_t launch_sf_f64(const SfPattern *pats, int pattern, long long npix, cudaStream_t st);
 cudaError_t launch_spectrum_combine(const SfPattern *pats, int pattern0, int S, const double *weight, float *F,

@@ -239,19 +239,58 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
   }
 }
 
+// FP64 term of the nodes: cos and sin / y of 2 pi y, |y| <= 1/4, z = y^2, and the
+// weight's exponential.  FULL, for FP64 results: to the rounding (FULL64 and
+// exp2_full, seven more operations); else to 1.7e-11 for FP32 results.
+template <bool FULL>
+__device__ __forceinline__ void node64_sincos(double z, double &ps, double &pc) {
+  if (FULL) {
+    ps = fma(z, SPSIM_FULL64_S8, SPSIM_FULL64_S7);
+    pc = fma(z, SPSIM_FULL64_C8, SPSIM_FULL64_C7);
+    ps = fma(z, ps, SPSIM_FULL64_S6);
+    pc = fma(z, pc, SPSIM_FULL64_C6);
+    ps = fma(z, ps, SPSIM_FULL64_S5);
+    pc = fma(z, pc, SPSIM_FULL64_C5);
+    ps = fma(z, ps, SPSIM_FULL64_S4);
+    pc = fma(z, pc, SPSIM_FULL64_C4);
+    ps = fma(z, ps, SPSIM_FULL64_S3);
+    pc = fma(z, pc, SPSIM_FULL64_C3);
+    ps = fma(z, ps, SPSIM_FULL64_S2);
+    pc = fma(z, pc, SPSIM_FULL64_C2);
+    ps = fma(z, ps, SPSIM_FULL64_S1);
+    pc = fma(z, pc, SPSIM_FULL64_C1);
+    ps = fma(z, ps, SPSIM_FULL64_S0);
+    pc = fma(z, pc, SPSIM_FULL64_C0);
+  } else {
+    ps = fma(z, SPSIM_NODE64_S5, SPSIM_NODE64_S4);
+    pc = fma(z, SPSIM_NODE64_C6, SPSIM_NODE64_C5);
+    ps = fma(z, ps, SPSIM_NODE64_S3);
+    pc = fma(z, pc, SPSIM_NODE64_C4);
+    ps = fma(z, ps, SPSIM_NODE64_S2);
+    pc = fma(z, pc, SPSIM_NODE64_C3);
+    ps = fma(z, ps, SPSIM_NODE64_S1);
+    pc = fma(z, pc, SPSIM_NODE64_C2);
+    ps = fma(z, ps, SPSIM_NODE64_S0);
+    pc = fma(z, pc, SPSIM_NODE64_C1);
+    pc = fma(z, pc, SPSIM_NODE64_C0);
+  }
+}
+
 // The same sum in FP64 throughout, phases by rounding.  B200's FP64 pipe runs at
 // half the FP32 rate, and without the split phase and the compensated sums a
 // term is 21 operations, so this takes 1.8 times as long as the FP32 kernel
 // (7.2e11 terms/s on 50,000 atoms x 26,244 nodes, P = 4; 80 % of the pipe).  It
 // runs
-//   - in FP64, and for molecules rewritten on the device, that is in
-//     refinements: a node's rounding error goes into all the pixels around it
+//   - in FP64 (FULL: 28 operations, 5.6e11 terms/s on 50,000 atoms in cells of
+//     1024^2 pixels where the shorter polynomials take 6.5e11), where amplitudes
+//     fall far (coarse_digits in capi.cu), and for molecules rewritten on the
+//     device, that is in refinements: a node's rounding error goes into all the pixels around it
 //     alike, and the gradient of a loss adds it up where the pixels' own errors
 //     would average out (up to 6 times the gradient's error on a heavily
 //     oversampled detector);
 //   - for small grids, which latency bounds: with P = 2 a work item is 64 nodes
 //     (1,000 atoms x 340 nodes: 12 us against 17 us in FP32; 5,000 x 840 even).
-template <int P, bool PERB>
+template <int P, bool PERB, bool FULL>
 __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPattern *__restrict__ pats,
                                                                   const WorkItem *__restrict__ items, int n_items,
                                                                   int *__restrict__ queue, int *__restrict__ err) {
@@ -344,20 +383,11 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPat
           u = fma(qz[i], rz, u);
           const double t = fma(u, 2.0, M52);  // rint(2u) in the low bits
           const double y = fma(t - M52, -0.5, u);
-          double w = PERB ? W * exp2_poly(Bj * s2n[i]) : W;
+          double w = PERB ? W * (FULL ? exp2_full(Bj * s2n[i]) : exp2_poly(Bj * s2n[i])) : W;
           w = __hiloint2double(__double2hiint(w) ^ (__double2loint(t) << 31), __double2loint(w));
           const double z = y * y;
-          double ps = fma(z, SPSIM_NODE64_S5, SPSIM_NODE64_S4);
-          double pc = fma(z, SPSIM_NODE64_C6, SPSIM_NODE64_C5);
-          ps = fma(z, ps, SPSIM_NODE64_S3);
-          pc = fma(z, pc, SPSIM_NODE64_C4);
-          ps = fma(z, ps, SPSIM_NODE64_S2);
-          pc = fma(z, pc, SPSIM_NODE64_C3);
-          ps = fma(z, ps, SPSIM_NODE64_S1);
-          pc = fma(z, pc, SPSIM_NODE64_C2);
-          ps = fma(z, ps, SPSIM_NODE64_S0);
-          pc = fma(z, pc, SPSIM_NODE64_C1);
-          pc = fma(z, pc, SPSIM_NODE64_C0);
+          double ps, pc;
+          node64_sincos<FULL>(z, ps, pc);
           ec[i] = fma(w, pc, ec[i]);
           es[i] = fma(w * y, ps, es[i]);
         }
@@ -409,18 +439,22 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_nodes64_kernel(const SfPat
 }
 
 // f(the kernel of node form `tile`), called with its arguments or queried for its occupancy
-template <typename F>
-static void with_nodes64(int tile, bool perb, F f) {
-  if (tile == SF_NODES64_TILE)
-    perb ? f(sf_nodes64_kernel<4, true>) : f(sf_nodes64_kernel<4, false>);
+template <int P, typename F>
+static void with_nodes64_p(bool perb, bool full, F f) {
+  if (full)
+    perb ? f(sf_nodes64_kernel<P, true, true>) : f(sf_nodes64_kernel<P, false, true>);
   else
-    perb ? f(sf_nodes64_kernel<2, true>) : f(sf_nodes64_kernel<2, false>);
+    perb ? f(sf_nodes64_kernel<P, true, false>) : f(sf_nodes64_kernel<P, false, false>);
+}
+template <typename F>
+static void with_nodes64(int tile, bool perb, bool full, F f) {
+  tile == SF_NODES64_TILE ? with_nodes64_p<4>(perb, full, f) : with_nodes64_p<2>(perb, full, f);
 }
 
-cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, const SfPattern *pats, const WorkItem *items, int n_items,
-                            int *queue, int *err, int grid, cudaStream_t st) {
+cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, bool full, const SfPattern *pats, const WorkItem *items,
+                            int n_items, int *queue, int *err, int grid, cudaStream_t st) {
   if (tile != SF_NODES_TILE)
-    with_nodes64(tile, perb,
+    with_nodes64(tile, perb, full,
                  [&](auto kernel) { kernel<<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err); });
   else if (perb)
     fixw ? sf_dquad_nodes_kernel<true, true><<<grid, NODE_THREADS, 0, st>>>(pats, items, n_items, queue, err, 0x80000000u)
@@ -434,10 +468,10 @@ cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, const SfPattern *pat
   return cudaGetLastError();
 }
 
-int sf_nodes_occupancy(int tile, bool perb, bool fixw) {
+int sf_nodes_occupancy(int tile, bool perb, bool fixw, bool full) {
   int n = 0;
   if (tile != SF_NODES_TILE) {
-    with_nodes64(tile, perb,
+    with_nodes64(tile, perb, full,
                  [&](auto kernel) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NODE_THREADS, 0); });
     return n;
   }
