@@ -1032,18 +1032,12 @@ static int choose_cells(const spsim_b200_molecule *m, const spsim_b200_qset *q, 
   return best;
 }
 
-// The molecule's cells of size k; nullptr while the stream is being captured
-// and they are not there yet.  Complete before return.
+// The molecule's cells of size k.  Complete before return.
 static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stream, const MoleculeCells **out) {
   *out = nullptr;
   auto &slot = m->cells[k];
   if (slot) {
     *out = slot.get();
-    return SPSIM_OK;
-  }
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
     return SPSIM_OK;
   }
   std::unique_ptr<MoleculeCells> c(new MoleculeCells());
@@ -1752,11 +1746,10 @@ static void plan_key(int npat, const spsim_b200_molecule *const *mols, const sps
 }
 
 // Write this call's rotations and outputs into the plan's descriptors (device
-// copy ordered on `stream`).  New outputs cannot be written while the stream is
-// being captured: the copy's source would be read again at every replay.
+// copy ordered on `stream`).
 static cudaError_t refresh_descriptors(Plan &pl, const double *rot, float *const *F_dev, float *const *I_dev,
                                        cudaStream_t stream) {
-  bool changed = false, moved = false;
+  bool changed = false;
   const size_t outputs = pl.coarse ? pl.npat : 0;  // the first pattern with pixels to write
   for (size_t i = 0; i < pl.host_pats.size(); ++i) {
     SfPattern &pt = pl.host_pats[i];
@@ -1768,7 +1761,7 @@ static cudaError_t refresh_descriptors(Plan &pl, const double *rot, float *const
     if (i < outputs || (outputs && i >= 2 * outputs) || pl.spectrum) continue;  // (a spectrum's are the launch's arguments)
     float2 *F = F_dev ? (float2 *)F_dev[k] : nullptr;
     float *I = I_dev ? I_dev[k] : nullptr;
-    moved = moved || pt.F != F || pt.I != I;
+    changed = changed || pt.F != F || pt.I != I;
     pt.F = F;
     pt.I = I;
   }
@@ -1776,13 +1769,7 @@ static cudaError_t refresh_descriptors(Plan &pl, const double *rot, float *const
     const cudaError_t e = refresh_descriptors(*pl.direct, rot, F_dev, I_dev, stream);
     if (e != cudaSuccess) return e;
   }
-  if (!changed && !moved) return cudaSuccess;
-  if (moved && stream) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const cudaError_t e = cudaStreamIsCapturing(stream, &capture);
-    if (e != cudaSuccess) return e;
-    if (capture != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
-  }
+  if (!changed) return cudaSuccess;
   return cudaMemcpyAsync(pl.pats.p, pl.host_pats.data(), pl.host_pats.size() * sizeof(SfPattern),
                          cudaMemcpyHostToDevice, stream);
 }
@@ -1801,6 +1788,18 @@ static int check_flags(Plan &pl) {
     return fail(SPSIM_ERR_RANGE, "atoms moved outside the molecule's creation-time bounds");
   }
   return pl.direct ? check_flags(*pl.direct) : SPSIM_OK;
+}
+
+// Forwards, adjoints and the NUFFT refuse a stream that is being captured before
+// they touch anything: their plans' tables would be uploaded by the graph's
+// replays only, from host arrays that are gone by then, while the cache would
+// hold the plan as made; and a plan's buffers belong to one launch at a time.
+static int refuse_capture(cudaStream_t stream) {
+  if (!stream) return SPSIM_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(stream, &capture));
+  if (capture == cudaStreamCaptureStatusNone) return SPSIM_OK;
+  return fail(SPSIM_ERR_CUDA, "the stream is being captured: this call cannot be part of a graph");
 }
 
 // cache == false: a one-shot plan (host convenience path), synchronised before return
@@ -1823,6 +1822,8 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     if (mols[i]->device != dev || qsets[i]->device != dev)
       return fail(SPSIM_ERR_INVALID_ARG, "pattern %d: handle belongs to another device", i);
   }
+  st = refuse_capture(stream);
+  if (st) return st;
   std::lock_guard<std::mutex> lk(g_mu);
   std::vector<const void *> kp;
   std::vector<double> kv;
@@ -2652,6 +2653,8 @@ static int nufft_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs
         for (int k = 0; k < 9; ++k) fro += rot[9 * (size_t)i + k] * rot[9 * (size_t)i + k];
         qball = std::max(qball, qs->qmax * std::sqrt(fro));
       }
+  st0 = refuse_capture(st);
+  if (st0) return st0;
   std::unique_lock<std::mutex> lk(g_mu);
   g_nufft_cv.wait(lk, [dev] { return nufft_free_for_this_thread(dev); });
   NufftCtx &c = g_nufft[dev];
@@ -3723,6 +3726,10 @@ extern "C" int spsim_b200_adjoint(const spsim_b200_molecule *m, const spsim_b200
     const double lim = precision == SPSIM_PREC_F32 ? 1.0 / 16 : 0.25;
     if (qmax * m->rbound >= std::ldexp(1.0, 19) || cmax > lim)
       return fail(SPSIM_ERR_RANGE, "adjoint: phase range outside the FP32 kernel's domain; use SPSIM_PREC_FP64");
+  }
+  if (m->n_kept > 0 && total > 0) {
+    const int refused = refuse_capture(st);
+    if (refused) return refused;
   }
   CUDA_TRY(cudaMemsetAsync(dpos_dev, 0, 3 * (size_t)m->natoms_in * sizeof(double), st));
   if (docc_dev) CUDA_TRY(cudaMemsetAsync(docc_dev, 0, (size_t)m->natoms_in * sizeof(double), st));

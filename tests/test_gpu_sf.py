@@ -16,7 +16,7 @@ import torch
 
 from conftest import golden, intensity_errors
 from oracle import oracle as O
-from spsim_b200 import core, synth
+from spsim_b200 import _native, core, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -468,3 +468,45 @@ def test_atoms_moved_outside_bounds_are_reported(cuda):
         _, I64 = O.structure_factor(Z, pos.astype(np.float64), qs.q().astype(np.float64))
         e_max, _ = intensity_errors(I.cpu().numpy(), I64)
         assert e_max < 1e-5
+
+
+def test_a_stream_under_capture_is_refused(cuda):
+    # before anything is touched: the capture stays valid, and the plan that the
+    # call would have made over an older one's buffers is made afterwards
+    Z, pos = synth.random_molecule(400, 2.0e-9, 61)
+    qs = core.QSet.from_detector(64, 60, 64 * 150e-6, 60 * 150e-6, 0.2, 0.2e-9)
+    F = torch.empty(qs.npix, dtype=torch.complex64, device="cuda")
+    G, I = torch.rand(qs.npix, device="cuda"), torch.empty(qs.npix, device="cuda")
+    s = torch.cuda.Stream()
+    mols = [core.Molecule(Z, pos + np.float32(1e-11 * k)) for k in range(12)]
+    new = core.Molecule(Z, pos)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        for m in mols:  # more than the caches hold
+            core.forward(m, qs, F=F, I=I)
+            core.adjoint(m, qs, F, G)
+            core.forward_nufft(m, qs, F=F, I=I)
+    torch.cuda.synchronize()
+    x = torch.zeros(4, device="cuda")
+    calls = [lambda m: core.forward(m, qs, F=F, I=I), lambda m: core.adjoint(m, qs, F, G),
+             lambda m: core.forward_nufft(m, qs, F=F, I=I)]
+    for call in calls:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            x += 1
+            for m in (new, mols[-1]):
+                with pytest.raises(_native.SpsimError, match="captured"):
+                    call(m)
+        x.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert x.tolist() == [1.0] * 4
+    with torch.cuda.stream(s):
+        core.forward(new, qs, F=F, I=I)
+        grad = core.adjoint(new, qs, F, G)[0]
+    torch.cuda.synchronize()
+    F64, I64 = O.structure_factor(Z, pos.astype(np.float64), qs.q().astype(np.float64))
+    assert np.abs(I.cpu().numpy() - I64).max() < 1e-5 * I64.max()
+    other = core.adjoint(mols[0], qs, core.forward(mols[0], qs)[0], G)[0]  # (the same molecule)
+    torch.cuda.synchronize()
+    assert float((grad - other).norm() / other.norm()) < 1e-5
