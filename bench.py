@@ -268,11 +268,11 @@ MIX = {
 def _kernel_key():
     """MIX key of the structure-factor kernel the last forward ran."""
     from spsim_b200 import core
-    terms, evaluated = core.last_forward_stats()[0], core.last_terms_evaluated()
-    if evaluated < terms:  # on coarse grids of nodes; the smallest sums in FP64
-        return "sf_dquad_nodes_kernel+word" if evaluated > 4e6 else "sf_nodes64_kernel"
-    return (core.kernel_name() + ("+word" if core.last_phase_word() else "")
-            + ("+narrow" if core.last_pair_narrow() else ""))
+    tile = core.last_node_tile()
+    if tile and tile < 256:  # on coarse grids of nodes, in FP64
+        return "sf_nodes64_kernel"
+    return (("sf_dquad_nodes_kernel" if tile else core.kernel_name()) + ("+word" if core.last_phase_word() else "")
+            + ("+narrow" if not tile and core.last_pair_narrow() else ""))
 
 
 def balanced_bound(kernel, prec, probe):
@@ -484,9 +484,13 @@ def run_b200(args):
     if rank == 0:
         if line.get("fp64_plain"):
             f = line["fp64_plain"]
-            f["f32_speedup"] = line["value"] / f["kernel_terms_per_s"]
+            # the precisions on the same detector, and the pattern on its coarse
+            # grids against the FP64 sum on every pixel
+            f["f32_speedup"] = line["value"] / f["value"]
+            f["f32_vs_every_pixel"] = line["value"] / f["kernel_terms_per_s"]
             if line.get("f32_fast"):
-                f["f32_fast_speedup"] = line["f32_fast"]["value"] / f["kernel_terms_per_s"]
+                f["f32_fast_speedup"] = line["f32_fast"]["value"] / f["value"]
+                f["f32_fast_vs_every_pixel"] = line["f32_fast"]["value"] / f["kernel_terms_per_s"]
         # the batched workloads at their stated sizes (single-GPU extras: the
         # other ranks of a multi-GPU run would wait on them at the final barrier)
         batched = {}
@@ -495,7 +499,8 @@ def run_b200(args):
             batched["uneven_64"] = batched_uneven(prec, line["roofline"]["peak"])
             fp64 = line.get("fp64_plain", {}).get("kernel_terms_per_s")
             if fp64:
-                # the batched forwards against the plain per-pattern FP64 kernel
+                # the batched forwards (on coarse grids) against the plain FP64
+                # kernel's sum on every pixel
                 o = batched["orientations_20k"]
                 o["vs_fp64_plain"] = o["terms_per_s"] / fp64
                 if "f32_fast" in o:
@@ -514,8 +519,8 @@ def run_b200(args):
 
 
 def _modes(args, core, mol, qs, rot, terms, timed, prec, w, Z, pos):
-    """f32_fast throughput, the plain FP64 kernel on every 8th pixel, and the
-    relative |F|^2 errors of both FP32 modes against the FP64 oracle on every
+    """f32_fast and fp64 throughput, the plain FP64 kernel's sum on every 8th
+    pixel, and the relative |F|^2 errors of both FP32 modes against the FP64 oracle on every
     64th row."""
     import torch
 
@@ -535,6 +540,8 @@ def _modes(args, core, mol, qs, rot, terms, timed, prec, w, Z, pos):
                            "kernel_terms_per_s": evaluated / (sf_ms * 1e-3) if sf_ms else None,
                            "frac_of_R": evaluated / (sf_ms * 1e-3) / R if sf_ms else None,
                            "balanced": bal}
+    fp64_steps = max(2, args.steps // 2)
+    fp64_step_ms = timed("fp64", fp64_steps, 1)[0]
     q = qs.q()
     sub8 = core.QSet.from_list(q[::8])
     with core.timing() as t:
@@ -563,7 +570,8 @@ def _modes(args, core, mol, qs, rot, terms, timed, prec, w, Z, pos):
     out["accuracy"] = {"reference": "FP64 oracle", "pixels": "every 64th detector row (16,384)",
                        "floor": "1e-3 x mean intensity", **acc}
     out["nufft"] = _nufft_mode(core, mol, qs, rot, terms, rows, I64)
-    out["fp64_plain"] = {"kernel_terms_per_s": fp64_rate, "sample": "every 8th pixel",
+    out["fp64_plain"] = {"value": terms * fp64_steps / (fp64_step_ms * 1e-3), "unit": UNIT,
+                         "kernel_terms_per_s": fp64_rate, "sample": "every pixel's sum: every 8th pixel as a list",
                          "f32_speedup": None, "f32_fast_speedup": None}
     return out
 
@@ -599,8 +607,8 @@ def _nufft_mode(core, mol, qs, rot, terms, rows, I64, eps=1e-8, steps=5):
             "accuracy": {"floored_max_rel": float(np.max(np.abs(In - I64) / den)),
                          "l2_rel": float(np.linalg.norm(In - I64) / np.linalg.norm(I64))},
             "note": "type-3 NUFFT per element (spread; pruned x, y, z FFT passes with the deconvolution and the "
-                    "FP32 packing fused; interpolate; FP64 spreading and FFT, "
-                    "interpolation at the nodes of the detector's coarse grid), a different algorithm from the direct sum the headline value times"}
+                    "packing fused; interpolate at the nodes of the detector's coarse grid and from there to the "
+                    "pixels; FP64 throughout), a different algorithm from the sum the headline value times"}
 
 
 def _e2e(args, w, Z, pos, terms, world, dist=None):

@@ -432,8 +432,9 @@ void spsim_b200_set_formula_seed(unsigned long long seed);
  * FP64 FMAs) while |q|max |r - centre|max < 2^17 cycles, and reduce by FP64
  * rounding (six FP64 operations, up to 2^48 cycles) beyond.
  * On coarse grids form 4's kernel for nodes runs, whose points each take their
- * own FP64 phase; it has one shape, and the variant reported (the default's or
- * the tuned threads and pixels per thread) is that of its size class on pixels.
+ * own FP64 phase, or an FP64 kernel (spsim_b200_last_node_tile); they have one
+ * shape each, and the variant reported (the default's or the tuned threads and
+ * pixels per thread) is that of the size class on pixels.
  * threads < 0 restores automatic choice; autotune times every compiled
  * variant on the given workload and keeps the fastest for workloads of that
  * size class. */
@@ -441,6 +442,10 @@ int spsim_b200_set_variant(int threads, int pixels_per_thread, int form);
 /* The kernel variant the last forward on this thread ran: threads per CTA,
  * pixels per thread and form (-1 for the plain FP64 kernel). */
 int spsim_b200_last_variant(int *threads, int *pixels_per_thread, int *form);
+/* The node kernel the last forward on this thread ran: 256 nodes per work item,
+ * the FP32 quad form for nodes; 128 or 64, the FP64 kernel; 0, none (the sum ran
+ * on every pixel, by spsim_b200_last_variant's kernel). */
+int spsim_b200_last_node_tile(int *nodes);
 /* Whether the last forward on this thread (forms 2, 3 and 4) took the phase from
  * the fixed-point phase word (1) or reduced it by FP64 rounding (0); 0 for the
  * other forms and the plain FP64 kernel.  No reference counterpart. */

@@ -124,6 +124,7 @@ _SIGNATURES = {
     "spsim_b200_last_forward_stats": (c_int, [POINTER(c_double), POINTER(c_double)]),
     "spsim_b200_last_terms_evaluated": (c_int, [POINTER(c_double)]),
     "spsim_b200_set_variant": (c_int, [c_int, c_int, c_int]),
+    "spsim_b200_last_node_tile": (c_int, [POINTER(c_int)]),
     "spsim_b200_last_variant": (c_int, [POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
     "spsim_b200_last_phase_word": (c_int, [POINTER(c_int)]),
     "spsim_b200_last_pair_narrow": (c_int, [POINTER(c_int)]),

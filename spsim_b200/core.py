@@ -21,7 +21,7 @@ from ._native import PRECISIONS, ChainOutputs, ChainParams, check, lib
 __all__ = [
     "Molecule", "QSet", "forward", "forward_batch", "adjoint", "detector_chain", "chain_params",
     "hkl_for_detector", "synchronize", "forward_spectrum", "timing", "autotune", "set_variant", "last_forward_stats",
-    "last_terms_evaluated", "last_variant", "last_phase_word", "last_pair_narrow", "kernel_name", "autotune_batch", "clear_tuning",
+    "last_terms_evaluated", "last_node_tile", "last_variant", "last_phase_word", "last_pair_narrow", "kernel_name", "autotune_batch", "clear_tuning",
     "forward_nufft", "forward_nufft_batch", "last_nufft_grid",
 ]
 
@@ -405,8 +405,18 @@ KERNELS = {-1: "sf_f64_kernel", 0: "sf_f32_kernel", 1: "sf_f32x2_kernel", 2: "sf
            4: "sf_dquad_kernel"}
 
 
+def last_node_tile():
+    """Nodes per work item where the last forward on this thread ran on coarse
+    grids: 256 for sf_dquad_nodes_kernel, 128 or 64 for sf_nodes64_kernel; 0 where
+    it ran on every pixel."""
+    n = c_int(0)
+    check(lib().spsim_b200_last_node_tile(byref(n)))
+    return n.value
+
+
 def last_variant():
-    """(threads, pixels_per_thread, form) of the last forward on this thread; form -1 = plain FP64."""
+    """(threads, pixels_per_thread, form) of the last forward on this thread; form -1 = plain FP64.
+    On coarse grids (last_node_tile() > 0) those of its size class on every pixel."""
     t, p, f = c_int(0), c_int(0), c_int(0)
     check(lib().spsim_b200_last_variant(byref(t), byref(p), byref(f)))
     return t.value, p.value, f.value
@@ -431,7 +441,8 @@ def last_pair_narrow():
 
 
 def kernel_name():
-    """Name of the structure-factor kernel the last forward on this thread ran."""
+    """Name of last_variant()'s kernel: the one the last forward on this thread ran
+    on every pixel, or on coarse grids the one of its size class there."""
     return KERNELS[last_variant()[2]]
 
 

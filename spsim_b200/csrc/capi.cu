@@ -777,6 +777,7 @@ static bool g_timing = false;
 static std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_timing_events;
 static thread_local double g_last_terms = 0, g_last_evaluated = 0, g_last_ms = 0;
 static thread_local int g_last_variant[3] = {0, 0, -1};  // threads, pixels per thread, form (-1: FP64 kernel)
+static thread_local int g_last_node_tile = 0;             // coarse grids: nodes per work item, else 0
 static thread_local int g_last_phase_word = 0;            // forms 2/3: fixed-point phase word used
 static thread_local int g_last_pair_narrow = 0;           // form 3: NARROW second-pixel polynomial used
 static int g_num_sms = 0;
@@ -1882,6 +1883,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
   }
   g_last_terms = pl->terms;
   g_last_evaluated = pl->evaluated;
+  g_last_node_tile = pl->coarse ? pl->node_tile : 0;
   g_last_variant[0] = pl->precision == SPSIM_PREC_FP64 ? 256 : pl->nt;
   g_last_variant[1] = pl->precision == SPSIM_PREC_FP64 ? 1 : pl->ppt;
   g_last_variant[2] = pl->precision == SPSIM_PREC_FP64 ? -1 : pl->packed;
@@ -3107,6 +3109,12 @@ extern "C" int spsim_b200_last_forward_stats(double *terms, double *kernel_ms) {
 extern "C" int spsim_b200_last_terms_evaluated(double *terms) {
   if (!terms) return fail(SPSIM_ERR_INVALID_ARG, "NULL argument");
   *terms = g_last_evaluated;
+  return SPSIM_OK;
+}
+
+extern "C" int spsim_b200_last_node_tile(int *nodes) {
+  if (!nodes) return fail(SPSIM_ERR_INVALID_ARG, "NULL argument");
+  *nodes = g_last_node_tile;
   return SPSIM_OK;
 }
 

@@ -163,6 +163,21 @@ def test_fp64_at_its_own_tolerance(cuda):
             assert np.linalg.norm(F.cpu().numpy() - F64) < 1e-7 * np.linalg.norm(F64)
 
 
+@pytest.mark.parametrize("natoms,precision,update,tile", [(400, "f32", False, 64), (6000, "f32", False, 256),
+                                                          (6000, "f32_fast", False, 256), (6000, "f32", True, 128),
+                                                          (6000, "fp64", False, 128)])
+def test_the_node_kernel_that_ran(cuda, natoms, precision, update, tile):
+    Z, pos = synth.random_molecule(natoms, 3.6e-9, 216)
+    d = _det(256, 250)
+    mol, qs = core.Molecule(Z, pos), core.QSet.from_detector(**d)
+    if update:
+        mol.update_device(torch.from_numpy(pos).cuda())
+    core.forward(mol, qs, precision=precision)
+    assert core.last_node_tile() == tile
+    core.forward(mol, core.QSet.from_list(qs.q()[:5000]), precision=precision)
+    assert core.last_node_tile() == 0
+
+
 def test_general_matrices_and_spectrum(cuda):
     Z, pos = synth.random_molecule(2500, 2.6e-9, 209)
     d = _det(132, 136)
