@@ -93,3 +93,35 @@ def test_synchronous_host_calls_return_timeout(cuda):
         assert st == 0
         e_max, e_l2 = intensity_errors(I, I64)
         assert e_max < 1e-5 and e_l2 < 1e-6, (e_max, e_l2)
+
+
+@pytest.mark.parametrize("natoms,radius,n,precision,tile", [(1000, 2.5e-9, 128, "f32", 64), (6000, 3.6e-9, 320, "f32", 256),
+                                                            (50000, 12e-9, 512, "f32", 256),
+                                                            (6000, 3.6e-9, 256, "fp64", 128)],
+                         ids=["small", "f32", "cells", "fp64"])
+def test_stalled_copy_on_the_nodes(cuda, natoms, radius, n, precision, tile):
+    # the node kernels' own exits, on detectors that take the coarse grids
+    Z, pos = synth.random_molecule(natoms, radius, 35)
+    mol = core.Molecule(Z, pos)
+    d = dict(nx=n, ny=n, width=n * 150e-6, height=n * 150e-6, distance=0.2, wavelength=0.2e-9)
+    qs = core.QSet.from_detector(**d)
+    side = torch.cuda.Stream()
+    _stall(True)
+    try:
+        for stream in (None, side):
+            core.forward(mol, qs, precision=precision, stream=stream)
+            with pytest.raises(SpsimError) as e:
+                core.synchronize(stream)
+            assert e.value.status == SPSIM_ERR_TIMEOUT
+            assert core.last_node_tile() == tile
+    finally:
+        _stall(False)
+    if natoms == 50000:  # by cells: fewer terms than atoms times the pattern's nodes, 77 a side
+        assert core.last_terms_evaluated() < 0.6 * natoms * 77 ** 2
+    some = np.arange(0, n * n, 41)
+    _, I64 = O.structure_factor(Z, pos.astype(np.float64), O.hkl_detector(**d)[some])
+    for stream in (None, side):
+        _, I = core.forward(mol, qs, precision=precision, stream=stream)
+        core.synchronize(stream)
+        e_max, e_l2 = intensity_errors(I.cpu().numpy()[some], I64)
+        assert e_max < 1e-5 and e_l2 < 1e-6, (e_max, e_l2)
