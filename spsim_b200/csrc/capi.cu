@@ -252,6 +252,8 @@ struct spsim_b200_molecule {
   DevBuf b_atoms, b_atoms2, b_atomsd, b_tiles, b_perm, b_wbase, b_coeffs, b_flags, b_inputs;
   // by index of kCellSizes, made when a plan first wants them, under g_mu
   mutable std::map<int, std::unique_ptr<MoleculeCells>> cells;
+  mutable DevBuf b_cells;           // of a dropped molecule's list, for this one's first
+  mutable bool planned_once = false;  // a plan for one call has been made without lists, under g_mu
   void take_buffers(spsim_b200_molecule &o) {
     b_atoms.swap(o.b_atoms);
     b_atoms2.swap(o.b_atoms2);
@@ -262,6 +264,9 @@ struct spsim_b200_molecule {
     b_coeffs.swap(o.b_coeffs);
     b_flags.swap(o.b_flags);
     b_inputs.swap(o.b_inputs);
+    b_cells.swap(o.b_cells);
+    for (auto &c : o.cells)
+      if (c.second && c.second->buf.cap > b_cells.cap) b_cells.swap(c.second->buf);
   }
 };
 
@@ -1042,6 +1047,7 @@ static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stre
     return SPSIM_OK;
   }
   std::unique_ptr<MoleculeCells> c(new MoleculeCells());
+  c->buf.swap(m->b_cells);
   c->lattice.a = kCellSizes[k].a * m->rbound;
   c->lattice.reach = (int)std::ceil(1.0 / kCellSizes[k].a) + 1;
   c->lattice.dim = 2 * c->lattice.reach + 1;
@@ -1101,15 +1107,16 @@ static int molecule_cells(const spsim_b200_molecule *m, int k, cudaStream_t stre
 // the pixels' own would.  Making a list takes 0.15 ms once per molecule, which a
 // few passes of a large pattern or some ten of a batch of uneven molecules repay
 // (16 of them, 500 to 60,000 atoms: 277 us a pass; 343 with lists only for those
-// that save 12 us, 400 for those of 50 us).
+// that save 12 us, 400 for those of 50 us).  once: a plan for one call, which has
+// to repay them itself, unless the molecule comes to such a plan again.
 struct PatternCells {
   const MoleculeCells *list = nullptr;
   CoarseGrid grid;  // of each cell
 };
-constexpr double kMaxCellSums = 256e6, kCellsMinSaved = 15e-6;
+constexpr double kMaxCellSums = 256e6, kCellsMinSaved = 15e-6, kCellsBuild = 150e-6;
 static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, const Spectrum *spec, const std::vector<CoarseGrid> &nodes,
-                      cudaStream_t stream, std::vector<PatternCells> &cells) {
+                      cudaStream_t stream, bool once, std::vector<PatternCells> &cells) {
   cells.assign(npat, PatternCells());
   std::vector<int> size(npat, -1);
   std::vector<CoarseGrid> grid(npat);
@@ -1131,6 +1138,16 @@ static int plan_cells(int npat, const spsim_b200_molecule *const *mols, const sp
       size[i] = choose_cells(mols[i], qsets[i], qscale * stretch, stretch, nodes[i], &grid[i], &last);
     }
     saved += last;
+  }
+  if (once) {
+    double build = 0.0;
+    for (int i = 0; i < npat; ++i) {
+      if (size[i] < 0 || (i > 0 && mols[i] == mols[i - 1])) continue;
+      const auto made = mols[i]->cells.find(size[i]);
+      if (!mols[i]->planned_once && (made == mols[i]->cells.end() || !made->second)) build += kCellsBuild;
+      mols[i]->planned_once = true;
+    }
+    saved -= build;
   }
   if (saved < kCellsMinSaved) return SPSIM_OK;
   for (int i = 0; i < npat; ++i) {
@@ -1156,7 +1173,7 @@ struct ListSums {
 static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols, const spsim_b200_qset *const *qsets,
                       const double *rot, float B, int precision, float *const *F_dev, float *const *I_dev,
                       cudaStream_t stream, const Spectrum *spec, bool allow_coarse = true,
-                      const ListSums *list = nullptr) {
+                      const ListSums *list = nullptr, bool once = false) {
   pl.npat = npat;
   pl.precision = precision;
   std::vector<CoarseGrid> nodes;
@@ -1173,7 +1190,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
   // cells, and the grid of each pattern's sums: its cells' or its own
   std::vector<PatternCells> cells(npat);
   if (pl.coarse) {
-    const int st = plan_cells(npat, mols, qsets, rot, spec, nodes, stream, cells);
+    const int st = plan_cells(npat, mols, qsets, rot, spec, nodes, stream, once, cells);
     if (st) return st;
   }
   std::vector<CoarseGrid> sum_grid(nodes);
@@ -1878,7 +1895,7 @@ static int run_forward(int npat, const spsim_b200_molecule *const *mols, const s
     }
     pl->key_ptrs = kp;
     pl->key_vals = kv;
-    st = build_plan(*pl, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec, true, list);
+    st = build_plan(*pl, npat, mols, qsets, rot, B, precision, F_dev, I_dev, stream, spec, true, list, true);
     if (st) return st;
   }
   g_last_terms = pl->terms;
