@@ -2405,7 +2405,11 @@ extern "C" int spsim_internal_shot_nodes_begin(int64_t npix, const float *hkl_de
   if (!(grid + 1.2e-4 < 0.8 * direct)) return SPSIM_OK;
   if (!g_host.nodes_out) g_host.nodes_out = new DevBuf();
   if (!g_host.nodes_plan) g_host.nodes_plan = new Plan();
-  CUDA_TRY(g_host.nodes_out->ensure(4 * (size_t)npix * sizeof(double2)));
+  // 64 bytes a pixel more than the sum on every pixel takes: that one where they do not fit
+  if (g_host.nodes_out->ensure(4 * (size_t)npix * sizeof(double2)) != cudaSuccess) {
+    cudaGetLastError();
+    return SPSIM_OK;
+  }
   ListSums sums;
   sums.out = (double2 *)g_host.nodes_out->p;
   sums.grid = nodes[0];
