@@ -142,8 +142,10 @@ int spsim_b200_forward(const spsim_b200_molecule *m, const spsim_b200_qset *qs, 
  * rot[9*i] (NULL = identity for all) and writes F_dev[i] / I_dev[i] (device
  * pointers, entries may be NULL).  Work items (pixel tile x atom range) are
  * cost-sorted and drained by a persistent kernel; the whole launch sequence
- * is captured once per plan into a CUDA graph and replayed while the plan's
- * shapes and pointers stay the same. */
+ * is captured once per plan into a CUDA graph and replayed while molecules, q
+ * sets, B, precision and stream stay the same (rotations and outputs may
+ * change).  Forwards, adjoints and the NUFFT cannot be part of a caller's own
+ * stream capture: SPSIM_ERR_CUDA, before anything is touched. */
 int spsim_b200_forward_batch(int npatterns, const spsim_b200_molecule *const *mols,
                              const spsim_b200_qset *const *qsets, const double *rot, float B,
                              int precision, float *const *F_dev, float *const *I_dev, void *stream);
@@ -460,7 +462,8 @@ int spsim_b200_autotune(const spsim_b200_molecule *m, const spsim_b200_qset *qs,
 /* The same over a batch (the arguments of spsim_b200_forward_batch, without
  * B and outputs): every variant is timed on the whole batched launch, and the
  * fastest is kept for batches of that size class (total atom.pixel terms).
- * No reference counterpart. */
+ * The variants are those of the sum on every pixel, which q lists take; on
+ * coarse grids a tuned choice changes nothing.  No reference counterpart. */
 int spsim_b200_autotune_batch(int npatterns, const spsim_b200_molecule *const *mols,
                               const spsim_b200_qset *const *qsets, const double *rot, int precision, void *stream,
                               int *best_threads, int *best_pixels_per_thread, int *best_form);
