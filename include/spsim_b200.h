@@ -124,7 +124,7 @@ int spsim_b200_qset_destroy(spsim_b200_qset *qs);
  * device (refinements: a node's rounding error would enter the pixels around it
  * alike and add up in a gradient) and where form factors and per-atom B factors
  * let the amplitudes fall below e^-4 at the edge of an axis (dim pixels would
- * take over the bright nodes' rounding).  Amplitudes falling below e^-10 (e^-5
+ * take over the bright nodes' rounding).  Amplitudes falling below e^-16 (e^-5
  * with SPSIM_PREC_FP64), q lists, forced variants
  * (spsim_b200_set_variant), detectors further than 1.2 detector distances off
  * the beam axis and per-atom B factors beyond twice their largest at creation

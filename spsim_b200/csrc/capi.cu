@@ -717,6 +717,7 @@ struct Plan {
   int precision = 0, nt = 128, ppt = 4, packed = 1;
   int mode = PREC_MODE_POLY;
   int node_tile = 0;  // coarse grids: nodes per work item, which selects the kernel (launch_sf_nodes)
+  bool full = false;  // coarse grids: the FP64 kernel to the rounding
   bool perb = false;
   bool fixw = false;  // FP64-phase forms: fixed-point phase word (every pattern within 2^17 cycles)
   bool narrow = false;  // neighbour pairs: every step within 0.07 cycle (the NARROW second-pixel polynomial)
@@ -930,12 +931,13 @@ static double coarse_fall(const spsim_b200_molecule *m, const spsim_b200_qset *q
 // FP32 sums' some 1e-9 of the bright amplitude at the edge of an axis, which stays
 // below the dim pixel's own rounding up to a fall of e^-4 (3,000 atoms of B = 200
 // A^2 to 1.4 A, falling by e^-13: 7 % of the dim pixels' amplitude; on every pixel
-// 9e-7).  Beyond, the sums are in FP64 and to more digits, and from e^-10 on the
-// patterns stay on every pixel.  FP64 results: to the rounding of FP64 phases, up
-// to e^-5.
+// 9e-7).  Beyond, the sums are in FP64 and to more digits (from e^-10 on with the
+// FP64 results' own kernel, so that refinements to 1.7 A, whose B factors may reach
+// their limit, keep the grids), and from e^-16 on the patterns stay on every pixel.
+// FP64 results: to the rounding of FP64 phases, up to e^-5.
 static int coarse_digits(bool fp64, double fall) {
   if (fp64) return fall <= 5.0 ? COARSE_DIGITS_FULL : 0;
-  return fall <= 4.0 ? COARSE_DIGITS_F32 : fall <= 10.0 ? COARSE_DIGITS_F64 : 0;
+  return fall <= 4.0 ? COARSE_DIGITS_F32 : fall <= 10.0 ? COARSE_DIGITS_F64 : fall <= 16.0 ? COARSE_DIGITS_FULL : 0;
 }
 
 // Node kernel's rate (terms/s).
@@ -1383,6 +1385,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
     // the FP64 kernel (sf_nodes.cu) for FP64, for amplitudes that fall far
     // (coarse_digits), for molecules rewritten on the device and for grids that
     // latency bounds: its items of 64 nodes up to 4e6 terms, of 128 beyond
+    pl.full = nodes[0].digits == COARSE_DIGITS_FULL;
     bool wide = nodes[0].digits > COARSE_DIGITS_F32;
     for (int i = 0; i < npat; ++i) wide = wide || mols[i]->updated;
     pl.node_tile = pl.evaluated <= 4e6 ? SF_NODES64_SMALL_TILE : wide ? SF_NODES64_TILE : SF_NODES_TILE;
@@ -1585,8 +1588,7 @@ static int build_plan(Plan &pl, int npat, const spsim_b200_molecule *const *mols
 
   if (precision != SPSIM_PREC_FP64 || pl.coarse) {
     // work items: pixel tile x atom-tile range, cost-sorted (largest first)
-    const bool full = precision == SPSIM_PREC_FP64;
-    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw, full)
+    const int occ = std::max(1, pl.coarse ? sf_nodes_occupancy(pl.node_tile, perb, pl.fixw, pl.full)
                                           : sf_f32_occupancy(pl.mode, nt, ppt, pl.packed, perb, pl.fixw, pl.narrow));
     const long long slots = (long long)num_sms() * occ;
     long long total_ptiles = 0;
@@ -1693,7 +1695,7 @@ static cudaError_t enqueue_plan(Plan &pl, cudaStream_t stream, cudaEvent_t ev0, 
   } else if (pl.n_items > 0) {
     int *queue = pl.head() + 8, *err = pl.head() + 4;
     if (pl.coarse)
-      e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, pl.precision == SPSIM_PREC_FP64,
+      e = launch_sf_nodes(pl.node_tile, pl.perb, pl.fixw, pl.full,
                           (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p, pl.n_items, queue, err, pl.grid, stream);
     else
       e = launch_sf_f32(pl.mode, pl.nt, pl.ppt, pl.packed, pl.perb, (const SfPattern *)pl.pats.p, (const WorkItem *)pl.items.p,

@@ -20,7 +20,7 @@ cudaError_t set_copy_stall(int on);
 cudaError_t set_nodes_copy_stall(int on);  // its part in sf_nodes.cu
 int sf_f32_occupancy(int mode, int nt, int p, int packed, bool perb, bool fixw = false, bool narrow = false);
 // The sum on a coarse grid's nodes, in work items of `tile` nodes: SF_NODES_TILE
-// selects the FP32 quad form, the other two the FP64 kernel (full: for FP64 results).
+// selects the FP32 quad form, the other two the FP64 kernel (full: to the rounding of FP64, else to 1.7e-11).
 constexpr int SF_NODES_TILE = 256, SF_NODES64_TILE = 128, SF_NODES64_SMALL_TILE = 64;
 cudaError_t launch_sf_nodes(int tile, bool perb, bool fixw, bool full, const SfPattern *pats, const WorkItem *items,
                             int n_items, int *queue, int *err, int grid, cudaStream_t st);

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(NODE_THREADS, 1) sf_dquad_nodes_kernel(
 }
 
 // FP64 term of the nodes: cos and sin / y of 2 pi y, |y| <= 1/4, z = y^2, and the
-// weight's exponential.  FULL, for FP64 results: to the rounding (FULL64 and
+// weight's exponential.  FULL (coarse_digits in capi.cu): to the rounding (FULL64 and
 // exp2_full, seven more operations); else to 1.7e-11 for FP32 results.
 template <bool FULL>
 __device__ __forceinline__ void node64_sincos(double z, double &ps, double &pc) {

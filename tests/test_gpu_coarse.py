@@ -120,7 +120,7 @@ def test_b_factors_rewritten_beyond_the_grids_limit(cuda):
             _check(F[k], I[k], Z, pos, q @ R[k].T, bfac=bk)
 
 
-@pytest.mark.parametrize("B,nodes", [(20.0, True), (60.0, True), (100.0, True), (200.0, False)])
+@pytest.mark.parametrize("B,nodes", [(20.0, True), (60.0, True), (100.0, True), (180.0, True), (200.0, False)])
 def test_amplitudes_that_fall_far(cuda, B, nodes):
     # amplitudes that fall by e^-2 to e^-17 along an axis, e^-4 to e^-33 to the
     # corners: the dim pixels keep their own accuracy beside the bright ones.  A
